@@ -537,14 +537,13 @@ VVPT_API vvpt_status vvpt_render(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_sc
         stats.kernel_launches += 1;
         VV_CUDA(cudaGetLastError(), "launch init");
         const uint64_t max_iters =
-            (uint64_t)hp.batch_size * (hp.depth + 1) * ((hp.total_items + slots - 1) / slots + 1) + 64;
+            (uint64_t)hp.batch_size * (hp.depth + 2) * ((hp.total_items + slots - 1) / slots + 1) + 64;
 
         if (info->flags & VVPT_RENDER_PROFILE_KERNELS) {
             // one kernel at a time with events around each launch
-            static const char *names[K_NUM] = {"k_begin", "k_regen",  "k_extend", "k_partition",
-                                               "k_walk",  "k_shade", "k_shadow"};
-            static const double bpu[K_NUM] = {0.0,        kBytesRegen, kBytesExtend, kBytesPartition,
-                                              kBytesWalk, kBytesShade, kBytesShadow};
+            static const char *names[K_NUM] = {"k_begin", "k_regen", "k_trace", "k_partition", "k_walk", "k_shade"};
+            static const double bpu[K_NUM] = {0.0,        kBytesRegen, kBytesTrace, kBytesPartition,
+                                              kBytesWalk, kBytesShade};
             vvpt_kernel_profile prof{};
             prof.count = K_NUM;
             for (int k = 0; k < K_NUM; k++) {
@@ -565,10 +564,10 @@ VVPT_API vvpt_status vvpt_render(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_sc
                     VV_CUDA(cudaStreamSynchronize(vv_stream(ctx)), "profile sync");
                     const uint32_t *c = ctx->counters_pinned;
                     uint64_t units = k == K_REGEN    ? c[C_REGEN0 + pp]
-                                     : (k == K_EXTEND || k == K_PARTITION) ? c[C_EXT0 + pp]
-                                     : k == K_WALK   ? c[C_WALK]
+                                     : k == K_TRACE ? (uint64_t)c[C_EXT0 + pp] + c[C_CONN]
+                                     : k == K_PARTITION ? c[C_EXT0 + pp]
+                                     : k == K_WALK   ? (uint64_t)c[C_WALK] + c[C_NEE_RUN]
                                      : k == K_SHADE  ? (uint64_t)c[C_SHADE_L] + c[C_SHADE_P] + c[C_SHADE_M]
-                                     : k == K_SHADOW ? (uint64_t)c[C_CONN] + c[C_NEEQ]
                                                       : 1;
                     cudaEventRecord(ka, vv_stream(ctx));
                     launch_kernel((KernelId)k, jt, ps, q, pp, shape, vv_stream(ctx));
@@ -985,7 +984,7 @@ VVPT_API vvpt_status vvpt_render_noalloc(vvpt_ctx *ctx, vvpt_scene *scene, const
     launch_init_slots(q, ps, jt, slots, stream);
     VV_CUDA(cudaGetLastError(), "launch init");
     const uint64_t max_iters =
-        (uint64_t)hp.batch_size * (hp.depth + 1) * ((hp.total_items + slots - 1) / slots + 1) + 64;
+        (uint64_t)hp.batch_size * (hp.depth + 2) * ((hp.total_items + slots - 1) / slots + 1) + 64;
     // kernels are launched one by one (no graph objects); the pinned counter
     // buffer was allocated when the context was created
     vvpt_render_stats stats{};

@@ -1,14 +1,16 @@
-// Wavefront integrator kernels: regen (camera rays), extend (closest hit),
-// shade (surface / medium / miss events, light and BSDF sampling, Russian
-// roulette) and connect (shadow rays and BSDF-direction emitter rays).
+// Wavefront integrator kernels: regen (camera rays), trace (closest hits of
+// the extension rays and the shadow rays of the previous shading), partition,
+// walk (the rays that need the full any-hit candidate walk) and shade
+// (surface / medium / miss events, light and BSDF sampling, Russian roulette).
 //
-// One iteration of the five kernels advances every live path by one traced
+// One iteration of the kernels advances every live path by one traced
 // segment, i.e. one pass of the `for d < depth` loop of
 // src/lib/vengine/shaders/pt/raygen.rgen.glsl:100-124 with the closest-hit /
 // miss shader that follows it. The shadow and emitter rays the reference
 // traces inside its hit shaders (lightSampling.glsl:108-144,
-// next_event_estimation.glsl:1-33) are deferred to `connect`; they consume no
-// random numbers, so the RNG stream per path is the reference's.
+// next_event_estimation.glsl:1-33) are traced with the next iteration's
+// extension rays; they consume no random numbers, so the RNG stream per path
+// is the reference's.
 #include "shade.cuh"
 #include "traverse.cuh"
 #include "wavefront.cuh"
@@ -21,9 +23,10 @@ constexpr uint32_t F_INSIDE = 1u;       // rayPayloadPrimary.insideVolume
 constexpr uint32_t F_DONE = 2u;         // sample finished, finalize in regen
 constexpr uint32_t F_ITEM = 4u;         // slot holds a work item
 constexpr uint32_t F_SHADOW = 8u;       // pending shadow connection
-constexpr uint32_t F_NEE = 16u;         // pending emitter connection (path ends at this event)
+constexpr uint32_t F_NEE = 16u;         // pending emitter connection (traced on its own, result in nee_c)
 constexpr uint32_t F_NEE_FUSED = 32u;   // emitter ray rides on the next extension ray
-constexpr uint32_t F_NEE_FULL = 64u;    // ... but needs the full candidate walk (set by extend)
+constexpr uint32_t F_NEE_FULL = 64u;    // ... but needs the full candidate walk (set by k_partition)
+constexpr uint32_t F_SHADOW_WALK = 1u << 24; // shadow ray needs the candidate walk (set by k_trace)
 constexpr int kDepthShift = 8;          // recursionDepth d
 constexpr int kSurfShift = 16;          // surfaceDepth
 constexpr uint32_t kByteMask = 0xFFu;
@@ -32,27 +35,6 @@ constexpr float kExtTmin = 0.001f;      // raygen.rgen.glsl:110
 constexpr float kExtTmax = 10000.0f;
 constexpr float kConnTmin = 0.0001f;    // lightSampling.glsl:112, next_event_estimation.glsl:3
 constexpr int kCandidateCap = 1024;     // per-segment candidate bound for any-hit loops
-
-// Who traces a ray in the candidate walks below: one lane on its own
-// (trace_after), or a group of eight lanes that all run the walk with the
-// same data (trace_after_group, the traversal kernels' form).
-struct LaneTracer {
-    __device__ __forceinline__ Hit operator()(const SceneView &s, const float3 &o, const float3 &d, float tmin,
-                                              float tmax, const Hit &after, uint32_t &err) const
-    {
-        return trace_after(s, o, d, tmin, tmax, after, err);
-    }
-};
-#if VVPT_BLAS_WIDE && VVPT_GROUP_TRAVERSAL
-struct GroupTracer {
-    LaneGroup g;
-    __device__ __forceinline__ Hit operator()(const SceneView &s, const float3 &o, const float3 &d, float tmin,
-                                              float tmax, const Hit &after, uint32_t &err) const
-    {
-        return trace_after_group(s, o, d, tmin, tmax, after, err, g);
-    }
-};
-#endif
 
 // One atomic per warp for a per-lane count. All 32 lanes call it.
 __device__ __forceinline__ void warp_add(uint32_t *counter, uint32_t v)
@@ -471,12 +453,8 @@ __global__ void k_begin(Queues q, int pp)
         q.counters[C_SHADE_P] = 0u;
         q.counters[C_SHADE_M] = 0u;
         q.counters[C_WALK] = 0u;
-        q.counters[C_CONN] = 0u;
-        q.counters[C_NEEQ] = 0u;
-        q.counters[C_FETCH_EXT] = 0u;
-        q.counters[C_FETCH_SHADOW] = 0u;
+        q.counters[C_FETCH] = 0u;
         q.counters[C_EXT0 + (1 - pp)] = 0u;
-        q.counters[C_REGEN0 + (1 - pp)] = 0u;
     }
 }
 
@@ -641,15 +619,10 @@ __global__ void __launch_bounds__(256, VVPT_REGEN_MIN_BLOCKS) k_regen(JobTable j
     }
 }
 
-// Closest hit for every queued extension ray; hits are binned by material
-// model into the shade queues (material-sorted shading).
 // Minimum resident blocks of 256 threads per SM requested for the traversal
 // kernels, which caps their registers (4: 64 registers, 50% occupancy); the
 // traversal is latency bound and gains more from resident warps than it
 // loses to the few spilled registers.
-#ifndef VVPT_EXTEND_MIN_BLOCKS
-#define VVPT_EXTEND_MIN_BLOCKS 4
-#endif
 #ifndef VVPT_TRACE_MIN_BLOCKS
 #define VVPT_TRACE_MIN_BLOCKS 4
 #endif
@@ -660,24 +633,9 @@ __global__ void __launch_bounds__(256, VVPT_REGEN_MIN_BLOCKS) k_regen(JobTable j
 #ifndef VVPT_SHADE_LM_MIN_BLOCKS
 #define VVPT_SHADE_LM_MIN_BLOCKS 2
 #endif
-// Rays per traversal-kernel lane: one (the one-ray-per-lane loop) or, with
-// the wide BLAS, one per group of eight lanes (trace_after_group). first_ray
-// is the queue index of a block's first ray, ray_stride the grid stride.
-#if VVPT_BLAS_WIDE && VVPT_GROUP_TRAVERSAL
-constexpr uint32_t kLanesPerRay = 8;
-#else
-constexpr uint32_t kLanesPerRay = 1;
-#endif
-__device__ __forceinline__ uint32_t first_ray() { return blockIdx.x * (blockDim.x / kLanesPerRay); }
-__device__ __forceinline__ uint32_t my_ray() { return (blockIdx.x * blockDim.x + threadIdx.x) / kLanesPerRay; }
-__device__ __forceinline__ uint32_t ray_stride() { return gridDim.x * blockDim.x / kLanesPerRay; }
-// Before a group's lane 0 writes what every lane of the group has read.
-__device__ __forceinline__ void group_sync()
-{
-#if VVPT_BLAS_WIDE && VVPT_GROUP_TRAVERSAL
-    __syncwarp(0xFFu << (threadIdx.x & 24u));
-#endif
-}
+__device__ __forceinline__ uint32_t first_ray() { return blockIdx.x * blockDim.x; }
+__device__ __forceinline__ uint32_t my_ray() { return blockIdx.x * blockDim.x + threadIdx.x; }
+__device__ __forceinline__ uint32_t ray_stride() { return gridDim.x * blockDim.x; }
 
 // Shade bin of a closest hit (0 Lambert, 1 PBR, 2 miss; | 4: the fused
 // emitter ray takes the full candidate walk).
@@ -701,17 +659,14 @@ __device__ __forceinline__ uint32_t extend_key(const SceneView &s, const Hit &h,
 // then share a warp's steps instead of the warp running until its longest
 // ray ends, and the code between traversals runs for many lanes at once.
 // Per-lane values that only that code reads stay in shared memory (one entry
-// per thread), so the traversal state keeps the registers. Binary BLAS only.
+// per thread), so the traversal state keeps the registers.
 #ifndef VVPT_REFILL_BELOW
 #define VVPT_REFILL_BELOW 16
 #endif
 constexpr uint32_t kLaneFree = 0, kLaneTracing = 1, kLaneDone = 2;
-// Step turns (k_extend): triangle tests and the other kinds of step in
-// separate warp steps, triangle tests when at least VVPT_TRI_TURN_PCT % of
-// the tracing lanes have one pending.
-#ifndef VVPT_STEP_TURNS
-#define VVPT_STEP_TURNS 1
-#endif
+// Step turns: triangle tests and the other kinds of step in separate warp
+// steps, triangle tests when at least VVPT_TRI_TURN_PCT % of the tracing
+// lanes have one pending.
 #ifndef VVPT_TRI_TURN_PCT
 #define VVPT_TRI_TURN_PCT 33
 #endif
@@ -735,17 +690,60 @@ __device__ __forceinline__ uint32_t refill_take(bool free, uint32_t *counter, ui
     return idx;
 }
 
-__global__ void __launch_bounds__(256, VVPT_EXTEND_MIN_BLOCKS) k_extend(JobTable jt, PathState ps, Queues q, int pp)
+__device__ __forceinline__ float3 medium_transmittance(const SceneView &s, uint32_t vol, float vtstart, float vtend);
+
+// A shadow ray whose nearest candidate is known: opaque, the light is hidden;
+// none, the light is seen through the medium at the event (the miss shader of
+// raySecondary.rmiss.glsl:17-44); transparent, the candidates have to be
+// walked (k_walk), which returns true.
+__device__ __forceinline__ bool shadow_finish(const JobView &J, const PathState &ps, uint32_t slot, const Hit &h)
 {
-    const uint32_t n = q.counters[C_EXT0 + pp];
-    const uint32_t *queue = q.ext[pp];
+    const SceneView &s = J.scene;
+    if (h.inst != kNoHit) {
+        if (!(s.materials[s.instances[h.inst].material].mrao.w >= 0.99f))
+            return false;
+        ps.flags[slot] |= F_SHADOW_WALK;
+        return true;
+    }
+    float3 T = f3(1.0f);
+    if (ps.flags[slot] & F_INSIDE) {
+        const uint32_t vol = ps.vol[slot];
+        if (vol < s.num_materials) {
+            T *= medium_transmittance(s, vol, kConnTmin, fminf(J.params.zfar_trunc, h.t));
+            if (!(max3f(T) > kEps))
+                T = f3(0.0f);
+        }
+    }
+    if (!is_black(T))
+        ps.rad[slot] = f4(f3(ps.rad[slot]) + f3(ps.sh_c[slot]) * T, 0.0f);
+    return false;
+}
+
+// Closest hits: the extension rays of this iteration, then the shadow rays of
+// the events shaded in the previous one and the emitter rays of the paths that
+// ended there, from one hand-out sequence, so that all share the lane refill
+// and a launch has one tail of long rays instead of three. Issue-bound under
+// divergence, then bound by the latency of dependent node fetches. Measured
+// against a shadow launch of its own after k_shade (one ray per lane to its
+// end, walks and emitter rays inline): 1920 x 1080 x 32 medium scene, 143 ms
+// of extension + 135 ms of shadow launches -> 211 ms; 4096 shadow rays under
+// the open sky (512 instances) took 215 us a launch, nearly all of it the
+// tail, and now disappear behind the extension rays: 106 -> 92 ms.
+constexpr uint32_t kColdFused = 1u, kColdShadow = 2u, kColdEmitter = 4u; // cold[].z; shade-bin bits above them
+__global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_trace(JobTable jt, PathState ps, Queues q, int pp)
+{
+    const uint32_t ne = q.counters[C_EXT0 + pp], ns = q.counters[C_CONN];
+    const uint32_t n = ne + ns + q.counters[C_NEEQ];
     uint32_t err = 0;
-#if VVPT_EXTEND_REFILL
-    if (n > 0)
-        tlas_cache_fill(jt.jobs[ps.job[queue[min(first_ray(), n - 1u)]]].scene);
-    else
+    auto entry = [&](uint32_t i) {
+        return i < ne ? q.ext[pp][i] : (i < ne + ns ? q.conn[i - ne] : q.nee[i - ne - ns]);
+    };
+    if (n > 0) {
+        tlas_cache_fill(jt.jobs[ps.job[entry(min(first_ray(), n - 1u))]].scene);
+    } else {
         tlas_cache_none();
-    // per lane: queue index, slot, fused (bit 0) | shade-bin bits (<< 1)
+    }
+    // per lane: queue index, slot, kind of ray and shade-bin bits
     __shared__ uint4 cold[256];
     TraceState st;
     TraceStack stack;
@@ -754,63 +752,59 @@ __global__ void __launch_bounds__(256, VVPT_EXTEND_MIN_BLOCKS) k_extend(JobTable
     for (;;) {
         uint32_t tr = __ballot_sync(0xFFFFFFFFu, state == kLaneTracing);
         if (__popc(tr) <= VVPT_REFILL_BELOW) {
-            // finished rays go straight to the shade queues (material
-            // bins) and the emitter-walk queue: warp-uniform appends
-            uint32_t fin_slot = 0, fin_key = 0xFFu, fin_i = 0;
+            uint32_t walk_slot = 0;
+            bool walk = false;
             if (state == kLaneDone) {
                 const uint4 c = cold[threadIdx.x];
-                const SceneView &s = jt.jobs[job].scene;
                 const Hit &h = st.best;
-                const bool fused = (c.z & 1u) != 0;
-                const uint32_t key = c.z >> 1;
-                if (fused && key == 0 && h.inst != kNoHit && h.t < kExtTmin) {
+                const uint32_t key = c.z >> 3;
+                if (c.z & kColdShadow) {
+                    walk = shadow_finish(jt.jobs[job], ps, c.y, h);
+                    walk_slot = c.y;
+                    state = kLaneFree;
+                } else if ((c.z & kColdFused) && key == 0 && h.inst != kNoHit && h.t < kExtTmin) {
                     // the emitter ray's first candidate lies below the
                     // extension ray's tmin: the emitter ray takes the full
                     // candidate walk, and this lane goes on with the
                     // extension ray from its tmin
-                    cold[threadIdx.x].z = 1u | (4u << 1);
-                    trace_begin(st, s, st.o, st.d, kExtTmin, kExtTmax, no_hit());
+                    cold[threadIdx.x].z = kColdFused | (4u << 3);
+                    trace_begin(st, jt.jobs[job].scene, st.o, st.d, kExtTmin, kExtTmax, no_hit());
                     state = kLaneTracing;
                 } else {
                     ps.hit[c.y] = make_float4(h.t, h.u, h.v, __uint_as_float(h.prim));
                     ps.hit_inst[c.y] = h.inst;
-                    fin_slot = c.y;
-                    fin_i = c.x;
-                    fin_key = extend_key(s, h, fused, key);
+                    if (!(c.z & kColdEmitter))
+                        q.ext_key[c.x] = extend_key(jt.jobs[job].scene, h, (c.z & kColdFused) != 0, key);
                     state = kLaneFree;
                 }
             }
-#if VVPT_EXTEND_PARTITION
-            const uint32_t bin = fin_key & 3u;
-            uint32_t pos = warp_append_all(bin == 0, &q.counters[C_SHADE_L]);
-            if (bin == 0)
-                q.shade_l[pos] = fin_slot;
-            pos = warp_append_all(bin == 1, &q.counters[C_SHADE_P]);
-            if (bin == 1)
-                q.shade_p[pos] = fin_slot;
-            pos = warp_append_all(bin == 2, &q.counters[C_SHADE_M]);
-            if (bin == 2)
-                q.shade_m[pos] = fin_slot;
-            const bool walk = fin_key != 0xFFu && (fin_key & 4u);
-            pos = warp_append_all(walk, &q.counters[C_WALK]);
-            if (walk)
-                q.walk[pos] = fin_slot;
-#else
-            if (fin_key != 0xFFu)
-                q.ext_key[fin_i] = fin_key;
-#endif
+            if (__any_sync(0xFFFFFFFFu, walk)) {
+                const uint32_t pos = warp_append_all(walk, &q.counters[C_WALK]);
+                if (walk)
+                    q.walk[pos] = walk_slot;
+            }
             if (open) {
                 bool mine;
-                const uint32_t i = refill_take(state == kLaneFree, &q.counters[C_FETCH_EXT], n, open, mine);
+                const uint32_t i = refill_take(state == kLaneFree, &q.counters[C_FETCH], n, open, mine);
                 if (mine) {
-                    const uint32_t slot = queue[i];
+                    const bool ext = i < ne, shadow = !ext && i < ne + ns;
+                    const uint32_t slot = entry(i);
+                    const uint32_t flags = shadow ? 0u : ps.flags[slot];
                     job = ps.job[slot];
-                    // with an emitter ray riding on this ray, start at its tmin
-                    const bool fused = (ps.flags[slot] & F_NEE_FUSED) != 0;
-                    cold[threadIdx.x] = make_uint4(i, slot, fused ? 1u : 0u, 0u);
-                    trace_begin(st, jt.jobs[job].scene, f3(ps.o[slot]), f3(ps.d[slot]), fused ? kConnTmin : kExtTmin,
-                                kExtTmax, no_hit());
-                    state = kLaneTracing;
+                    // with an emitter ray riding on the extension ray, start at its tmin
+                    const bool fused = ext && (flags & F_NEE_FUSED) != 0;
+                    const float4 d = shadow ? ps.sh_dir[slot] : ps.d[slot];
+                    cold[threadIdx.x] =
+                        make_uint4(i, slot, shadow ? kColdShadow : (!ext ? kColdEmitter : (fused ? kColdFused : 0u)), 0u);
+                    const float tmax = ext ? kExtTmax : (shadow ? d.w - kConnTmin : jt.jobs[job].params.zfar);
+                    // the emitter ray of a path that goes on (zfar beyond the
+                    // extension rays' range) takes the walk as a whole: the
+                    // path's hit record belongs to its extension ray
+                    if (ext || shadow || (flags & F_DONE)) {
+                        trace_begin(st, jt.jobs[job].scene, f3(ps.o[slot]), f3(d),
+                                    ext && !fused ? kExtTmin : kConnTmin, tmax, no_hit());
+                        state = kLaneTracing;
+                    }
                 }
             }
             tr = __ballot_sync(0xFFFFFFFFu, state == kLaneTracing);
@@ -820,72 +814,21 @@ __global__ void __launch_bounds__(256, VVPT_EXTEND_MIN_BLOCKS) k_extend(JobTable
                 continue;
             }
         }
-#if VVPT_STEP_TURNS
         // triangle tests and node visits in separate warp steps: triangle
         // tests run when enough of the tracing lanes have one pending, the
         // other kinds of step otherwise (a lane whose kind is not this
         // step's waits; every lane's kind gets its turn, since the lanes
         // that step move on to a leaf, finish, or leave the tracing set)
-        const bool tri = state == kLaneTracing && st.leaf_count > 0;
+        const bool tri = state == kLaneTracing && trace_triangle_pending(st);
         const bool tri_turn =
             100 * __popc(__ballot_sync(0xFFFFFFFFu, tri)) >= VVPT_TRI_TURN_PCT * __popc(tr);
         if (state == kLaneTracing && tri == tri_turn && !trace_step(st, stack, jt.jobs[job].scene, no_hit(), err))
             state = kLaneDone;
-#else
-        if (state == kLaneTracing && !trace_step(st, stack, jt.jobs[job].scene, no_hit(), err))
-            state = kLaneDone;
-#endif
     }
-#else
-    if (first_ray() < n)
-        tlas_cache_fill(jt.jobs[ps.job[queue[first_ray()]]].scene);
-    else
-        tlas_cache_none();
-#if VVPT_BLAS_WIDE && VVPT_GROUP_TRAVERSAL
-    // One ray per group of eight lanes; the group's lanes share the
-    // traversal (trace_after_group) and lane 0 writes the result.
-    const LaneGroup g = lane_group();
-#endif
-    // A lane (group) takes its next ray as soon as its current one is done,
-    // so a warp is never held by its slowest ray. The shade bin is written
-    // per queue entry and compacted by k_partition.
-    for (uint32_t i = my_ray(); i < n; i += ray_stride()) {
-        const uint32_t slot = queue[i];
-        const SceneView &s = jt.jobs[ps.job[slot]].scene;
-        const float3 o = f3(ps.o[slot]);
-        const float3 d = f3(ps.d[slot]);
-        const uint32_t flags = ps.flags[slot];
-        // with an emitter ray riding on this ray, start at its tmin
-        const bool fused = (flags & F_NEE_FUSED) != 0;
-#if VVPT_BLAS_WIDE && VVPT_GROUP_TRAVERSAL
-        Hit h = trace_after_group(s, o, d, fused ? kConnTmin : kExtTmin, kExtTmax, no_hit(), err, g);
-#else
-        Hit h = trace_closest(s, o, d, fused ? kConnTmin : kExtTmin, kExtTmax, err);
-#endif
-        uint32_t key = 0;
-        if (fused && h.inst != kNoHit && h.t < kExtTmin) {
-            // the emitter ray's first candidate lies below the extension
-            // ray's tmin: the emitter ray takes the full candidate walk
-            key = 4;
-#if VVPT_BLAS_WIDE && VVPT_GROUP_TRAVERSAL
-            h = trace_after_group(s, o, d, kExtTmin, kExtTmax, no_hit(), err, g);
-#else
-            h = trace_closest(s, o, d, kExtTmin, kExtTmax, err);
-#endif
-        }
-        key = extend_key(s, h, fused, key);
-#if VVPT_BLAS_WIDE && VVPT_GROUP_TRAVERSAL
-        if (g.gl == 0)
-#endif
-        {
-            ps.hit[slot] = make_float4(h.t, h.u, h.v, __uint_as_float(h.prim));
-            ps.hit_inst[slot] = h.inst;
-            q.ext_key[i] = key;
-        }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        atomicAdd(&q.counters[C_SEGMENTS], ne);
+        atomicAdd(&q.counters[C_SHADOW], ns);
     }
-#endif
-    if (blockIdx.x == 0 && threadIdx.x == 0)
-        atomicAdd(&q.counters[C_SEGMENTS], n);
     if (err)
         atomicOr(&q.counters[C_ERR], err);
 }
@@ -896,6 +839,14 @@ __global__ void __launch_bounds__(256) k_partition(PathState ps, Queues q, int p
 {
     const uint32_t n = q.counters[C_EXT0 + pp];
     const uint32_t *queue = q.ext[pp];
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        // queues that are consumed by now and filled again by this
+        // iteration's k_shade; the emitter rays' entries stay for k_walk
+        q.counters[C_CONN] = 0u;
+        q.counters[C_REGEN0 + pp] = 0u;
+        q.counters[C_NEE_RUN] = q.counters[C_NEEQ];
+        q.counters[C_NEEQ] = 0u;
+    }
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
         const uint32_t i = base + threadIdx.x;
         uint32_t slot = 0, key = 0xFFu;
@@ -913,58 +864,17 @@ __global__ void __launch_bounds__(256) k_partition(PathState ps, Queues q, int p
         pos = warp_append_all(bin == 2, &q.counters[C_SHADE_M]);
         if (bin == 2)
             q.shade_m[pos] = slot;
-        const bool walk = key != 0xFFu && (key & 4u);
+        bool walk = key != 0xFFu && (key & 4u);
+        if (walk) {
+            // one entry per path: a shadow walk's entry serves both
+            const uint32_t flags = ps.flags[slot];
+            ps.flags[slot] = flags | F_NEE_FULL;
+            walk = !(flags & F_SHADOW_WALK);
+        }
         pos = warp_append_all(walk, &q.counters[C_WALK]);
         if (walk)
             q.walk[pos] = slot;
     }
-}
-
-template <class Tracer>
-__device__ __noinline__ void emitter_ray(const Tracer &trace, const SceneView &s, const RenderParams &p, float3 o,
-                                         const float3 &dir, bool inside, uint32_t vol, float3 &out_em_T,
-                                         float3 &out_T, float3 &out_em, float &out_pdf, uint32_t &err);
-
-// The pending emitter rays whose first candidate is transparent (or below the
-// extension ray's tmin): the full candidate walk, before shade adds this
-// iteration's contributions.
-__global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_walk(JobTable jt, PathState ps, Queues q)
-{
-    const uint32_t n = q.counters[C_WALK];
-    uint32_t err = 0;
-    if (first_ray() < n)
-        tlas_cache_fill(jt.jobs[ps.job[q.walk[first_ray()]]].scene);
-    else
-        tlas_cache_none();
-#if VVPT_BLAS_WIDE && VVPT_GROUP_TRAVERSAL
-    const GroupTracer trace{lane_group()};
-    const bool writer = trace.g.gl == 0;
-#else
-    const LaneTracer trace{};
-    const bool writer = true;
-#endif
-    for (uint32_t i = my_ray(); i < n; i += ray_stride()) {
-        const uint32_t slot = q.walk[i];
-        const JobView &J = jt.jobs[ps.job[slot]];
-        const SceneView &s = J.scene;
-        const RenderParams &p = J.params;
-        const uint32_t flags = ps.flags[slot];
-        const float4 nb = ps.nee_b[slot];
-        float3 emT, T, em;
-        float lpdf;
-        emitter_ray(trace, s, p, f3(ps.o[slot]), f3(ps.d[slot]), (flags & F_INSIDE) != 0, ps.vol[slot], emT, T, em,
-                    lpdf, err);
-        group_sync();
-        if (writer) {
-            if (!is_black(em))
-                ps.rad[slot] = f4(f3(ps.rad[slot]) + power_heuristic(nb.w, lpdf) * T * em * f3(nb), 0.0f);
-            ps.flags[slot] = flags & ~(F_NEE_FUSED | F_NEE_FULL);
-        }
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0 && n)
-        atomicAdd(&q.counters[C_NEE], n);
-    if (err)
-        atomicOr(&q.counters[C_ERR], err);
 }
 
 // Volume free flight on the current segment; returns true when the path
@@ -1041,6 +951,7 @@ __global__ void __launch_bounds__(256, KIND == 0 || KIND == 2 ? VVPT_SHADE_LM_MI
         const uint32_t i = base + threadIdx.x;
         uint32_t slot = 0;
         bool want_conn = false, want_nee = false, want_done = false, want_ext = false;
+        bool late = false; // an ended path with a ray still to trace: regen runs after it, an iteration later
         if (i < n) {
         slot = entry(i);
         const JobView &J = jt.jobs[ps.job[slot]];
@@ -1387,6 +1298,7 @@ __global__ void __launch_bounds__(256, KIND == 0 || KIND == 2 ? VVPT_SHADE_LM_MI
         want_conn = has_shadow;
         want_nee = has_nee && !fuse;
         want_done = done;
+        late = want_conn || want_nee;
         want_ext = !done;
         }
         uint32_t pos = warp_append_all(want_conn, &q.counters[C_CONN]);
@@ -1395,9 +1307,12 @@ __global__ void __launch_bounds__(256, KIND == 0 || KIND == 2 ? VVPT_SHADE_LM_MI
         pos = warp_append_all(want_nee, &q.counters[C_NEEQ]);
         if (want_nee)
             q.nee[pos] = slot;
-        pos = warp_append_all(want_done, &q.counters[C_REGEN0 + (1 - pp)]);
-        if (want_done)
+        pos = warp_append_all(want_done && !late, &q.counters[C_REGEN0 + (1 - pp)]);
+        if (want_done && !late)
             q.regen[1 - pp][pos] = slot;
+        pos = warp_append_all(want_done && late, &q.counters[C_REGEN0 + pp]);
+        if (want_done && late)
+            q.regen[pp][pos] = slot;
         pos = warp_append_all(want_ext, &q.counters[C_EXT0 + (1 - pp)]);
         if (want_ext)
             q.ext[1 - pp][pos] = slot;
@@ -1410,8 +1325,7 @@ __global__ void __launch_bounds__(256, KIND == 0 || KIND == 2 ? VVPT_SHADE_LM_MI
 // Shadow ray with transparent surfaces and media (lightSampling.glsl:108-144,
 // raySecondary.rahit.glsl:31-72, raySecondary.rchit.glsl:32-78,
 // raySecondary.rmiss.glsl:17-44). Candidates are processed nearest first.
-template <class Tracer>
-__device__ float3 shadow_transmittance(const Tracer &trace, const SceneView &s, const RenderParams &p, float3 o,
+__device__ float3 shadow_transmittance(const SceneView &s, const RenderParams &p, float3 o,
                                        const float3 &dir, float tmax_light, bool inside, uint32_t vol, uint32_t &err)
 {
     const float tmin = kConnTmin;
@@ -1426,7 +1340,7 @@ __device__ float3 shadow_transmittance(const Tracer &trace, const SceneView &s, 
         Hit acc;
         int guard = 0;
         for (;;) {
-            Hit h = trace(s, o, dir, tmin, distT, after, err);
+            Hit h = trace_after(s, o, dir, tmin, distT, after, err);
             if (h.inst == kNoHit)
                 break;
             if (++guard > kCandidateCap) {
@@ -1554,8 +1468,7 @@ __device__ __forceinline__ void emitter_eval(const SceneView &s, const RenderPar
 // BSDF-direction emitter ray (next_event_estimation.glsl:1-33,
 // rayNEE.rahit.glsl:32-132, rayNEE.rchit.glsl:33-82, rayNEE.rmiss.glsl:12-19).
 // Returns the emitter radiance times throughput and its light pdf.
-template <class Tracer>
-__device__ __noinline__ void emitter_ray(const Tracer &trace, const SceneView &s, const RenderParams &p, float3 o,
+__device__ __noinline__ void emitter_ray(const SceneView &s, const RenderParams &p, float3 o,
                                          const float3 &dir, bool inside, uint32_t vol, float3 &out_em_T,
                                          float3 &out_T, float3 &out_em, float &out_pdf, uint32_t &err)
 {
@@ -1572,7 +1485,7 @@ __device__ __noinline__ void emitter_ray(const Tracer &trace, const SceneView &s
         Hit acc;
         int guard = 0;
         for (;;) {
-            Hit h = trace(s, o, dir, tmin, tmax, after, err);
+            Hit h = trace_after(s, o, dir, tmin, tmax, after, err);
             if (h.inst == kNoHit)
                 break;
             if (++guard > kCandidateCap) {
@@ -1656,45 +1569,52 @@ __device__ __noinline__ void emitter_ray(const Tracer &trace, const SceneView &s
     out_em_T = T * em;
 }
 
+// The BSDF-direction emitter ray from its first candidate (the closest hit
+// along the ray from the emitter ray's tmin): true when that candidate is
+// transparent and the complete candidate walk of emitter_ray is needed,
+// otherwise T, em and pdf are the ray's. No candidate, or one beyond zfar, is
+// a miss.
+__device__ __forceinline__ bool emitter_first(const SceneView &s, const RenderParams &p, bool is_hit, uint32_t inst_id,
+                                              const float4 &hv, const float3 &o, const float3 &dir, bool inside,
+                                              uint32_t vol, float3 &T, float3 &em, float &pdf)
+{
+    if (!is_hit || !(hv.x <= p.zfar))
+        return false;
+    Hit h;
+    h.t = hv.x;
+    h.u = hv.y;
+    h.v = hv.z;
+    h.inst = inst_id;
+    h.prim = __float_as_uint(hv.w);
+    const DevInstance &inst = s.instances[inst_id];
+    const DevMaterial &m = s.materials[inst.material];
+    ShadeVertex a, b, c;
+    fetch_triangle(s, inst, h.prim, a, b, c);
+    const float bx = 1.0f - h.u - h.v;
+    float2 uv = make_float2(a.pos_u.w * bx + b.pos_u.w * h.u + c.pos_u.w * h.v,
+                            a.nrm_v.w * bx + b.nrm_v.w * h.u + c.nrm_v.w * h.v);
+    float2 tuv = make_float2(uv.x * m.uv_tiling.x, uv.y * m.uv_tiling.y);
+    float3 e = material_emissive(s, m, tuv);
+    if (is_black_eps(e, 0.05f))
+        return m.mrao.w >= 0.99f; // transparent: walk the candidates
+    emitter_eval(s, p, inst, a, b, c, h, e, o, dir, inside, vol, kConnTmin, T, em, pdf);
+    return false;
+}
+
 // The previous event's BSDF-direction emitter ray, resolved from this
 // iteration's extension hit: the two rays share origin and direction, and the
 // extension traversal starts at the emitter ray's tmin (1e-4) when one is
 // pending, so the extension hit is the emitter ray's first candidate unless
-// extend flagged a candidate below 1e-3 (`full`). Candidates beyond zfar are a
-// miss for the emitter ray; a transparent first candidate needs the complete
-// candidate walk of emitter_ray.
+// extend flagged a candidate below 1e-3 (`full`).
 __device__ __noinline__ float3 fused_nee(const SceneView &s, const RenderParams &p, bool full, bool is_hit,
                                          uint32_t inst_id, float4 hv, float3 o, float3 dir, bool inside, uint32_t vol,
                                          float4 nb, uint32_t &err, uint32_t &walks)
 {
     float3 T = f3(1.0f), em = f3(0.0f);
     float pdf = 0.0f;
-    if (!full && is_hit && hv.x <= p.zfar) {
-        Hit h;
-        h.t = hv.x;
-        h.u = hv.y;
-        h.v = hv.z;
-        h.inst = inst_id;
-        h.prim = __float_as_uint(hv.w);
-        const DevInstance &inst = s.instances[inst_id];
-        const DevMaterial &m = s.materials[inst.material];
-        ShadeVertex a, b, c;
-        fetch_triangle(s, inst, h.prim, a, b, c);
-        const float bx = 1.0f - h.u - h.v;
-        float2 uv = make_float2(a.pos_u.w * bx + b.pos_u.w * h.u + c.pos_u.w * h.v,
-                                a.nrm_v.w * bx + b.nrm_v.w * h.u + c.nrm_v.w * h.v);
-        float2 tuv = make_float2(uv.x * m.uv_tiling.x, uv.y * m.uv_tiling.y);
-        float3 e = material_emissive(s, m, tuv);
-        if (is_black_eps(e, 0.05f)) {
-            if (m.mrao.w >= 0.99f)
-                full = true; // transparent: walk the candidates
-        } else {
-            emitter_eval(s, p, inst, a, b, c, h, e, o, dir, inside, vol, kConnTmin, T, em, pdf);
-        }
-    }
-    if (full) {
+    if (full || emitter_first(s, p, is_hit, inst_id, hv, o, dir, inside, vol, T, em, pdf)) {
         float3 emT;
-        emitter_ray(LaneTracer{}, s, p, o, dir, inside, vol, emT, T, em, pdf, err);
+        emitter_ray(s, p, o, dir, inside, vol, emT, T, em, pdf, err);
         walks++;
     }
     if (is_black(em))
@@ -1702,283 +1622,69 @@ __device__ __noinline__ float3 fused_nee(const SceneView &s, const RenderParams 
     return power_heuristic(nb.w, pdf) * T * em * f3(nb);
 }
 
-// Shadow rays of the events shaded this iteration, then the BSDF-direction
-// emitter rays of the paths that end at this event (their own queue, after
-// the shadow entries, in the same launch: the few long emitter walks overlap
-// the shadow rays instead of forming a launch of their own). An emitter ray's
-// contribution goes to nee_c, so the two parts never write the same word;
-// regen (or shade, for a path that continues) adds it after the shadow ray's,
-// in the order of the reference's additions.
-// One shadow ray of shadow_transmittance as a resumable walk for the lane
-// refill loop of k_shadow: the candidate logic between two traversals, with
-// the same decisions in the same order. The walk's ray and traversal live in
-// the TraceState (st.o is the current segment's origin); the candidate loop
-// of a segment always starts at kConnTmin.
-struct ShadowWalk {
-    float3 T;
-    float distT;
-    uint32_t vol, seg, guard;
-    bool inside;
-};
-
-// The transparent-candidate part of the walk (alpha, volume boundaries), out
-// of line: it is rare on most scenes, and inline its registers would crowd
-// the traversal state of the refill loop. Returns 0 when T is final, 1 to go
-// on past the candidate, 2 to start the next segment at `next_o`.
-__device__ __noinline__ int shadow_walk_transparent(ShadowWalk &w, const SceneView &s, const RenderParams &p,
-                                                    const Hit h, const float3 dir, float3 &next_o)
+// The rays that need the full any-hit candidate walk, one lane each, before
+// shade adds this iteration's contributions: shadow rays whose nearest
+// candidate is transparent and fused emitter rays whose first candidate is
+// transparent or below the extension ray's tmin (one queue entry per path, the
+// shadow ray's contribution first, in the order of the reference's
+// additions), then the emitter rays traced on their own. Those of ended paths
+// have their first candidate from k_trace and walk only past a transparent
+// one. They write their contribution to nee_c, so the two parts never write
+// the same word; regen (or shade, for a path that continues) adds it after
+// the shadow ray's.
+__global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_walk(JobTable jt, PathState ps, Queues q)
 {
-    const float tmin = kConnTmin;
-    const DevInstance &inst = s.instances[h.inst];
-    const DevMaterial &m = s.materials[inst.material];
-    // alpha needs the hit's uv
-    ShadeVertex a, b, c;
-    fetch_triangle(s, inst, h.prim, a, b, c);
-    const float bx = 1.0f - h.u - h.v;
-    const float2 uv = make_float2(a.pos_u.w * bx + b.pos_u.w * h.u + c.pos_u.w * h.v,
-                                  a.nrm_v.w * bx + b.nrm_v.w * h.u + c.nrm_v.w * h.v);
-    const float alpha = material_alpha(s, m, make_float2(uv.x * m.uv_tiling.x, uv.y * m.uv_tiling.y));
-    w.T *= f3(1.0f - alpha);
-    if (inst.front_volume != inst.back_volume) {
-        // closest hit on a volume boundary: the segment ends here
-        const SurfaceHit sh = make_surface_hit(s, h.inst, h.prim, h.u, h.v, dir);
-        if (w.inside && w.vol < s.num_materials) {
-            w.T *= medium_transmittance(s, w.vol, tmin, h.t);
-            if (max3f(w.T) < kEps) {
-                w.T = f3(0.0f);
-                return 0;
-            }
-        }
-        w.inside = false;
-        const int nv = sh.flipped ? sh.front_volume : sh.back_volume;
-        if (nv != -1) {
-            w.inside = true;
-            w.vol = (uint32_t)nv;
-        }
-        w.distT -= h.t;
-        if (++w.seg >= p.depth)
-            return 0;
-        w.guard = 0;
-        next_o = sh.wpos;
-        return 2;
-    }
-    if (max3f(w.T) > kEps)
-        return 1;
-    w.T = f3(0.0f);
-    return 0;
-}
-
-// Result of one finished traversal of the walk: true while the walk goes on
-// (a new traversal has been begun, after the candidate `after`), false when
-// T is final (zero if shadowed).
-__device__ __forceinline__ bool shadow_walk_next(ShadowWalk &w, Hit &after, TraceState &st, const SceneView &s,
-                                                 const RenderParams &p, uint32_t &err)
-{
-    const float tmin = kConnTmin;
-    const Hit h = st.best;
-    if (h.inst == kNoHit) {
-        // miss shader
-        if (w.inside && w.vol < s.num_materials) {
-            w.T *= medium_transmittance(s, w.vol, tmin, fminf(p.zfar_trunc, w.distT));
-            if (!(max3f(w.T) > kEps))
-                w.T = f3(0.0f);
-        }
-        return false;
-    }
-    if (++w.guard > (uint32_t)kCandidateCap) {
-        err |= kErrLoopCap;
-        w.T = f3(0.0f);
-        return false;
-    }
-    if (!(s.materials[s.instances[h.inst].material].mrao.w >= 0.99f)) {
-        w.T = f3(0.0f);
-        return false;
-    }
-    float3 next_o;
-    const int r = shadow_walk_transparent(w, s, p, h, st.d, next_o);
-    if (r == 0)
-        return false;
-    if (r == 2) {
-        after = no_hit();
-        trace_begin(st, s, next_o, st.d, tmin, w.distT, after);
-    } else {
-        after = h;
-        trace_begin(st, s, st.o, st.d, tmin, w.distT, after);
-    }
-    return true;
-}
-
-// Lane refill for the shadow kernel (as in k_extend; binary BLAS only), a
-// build option, off: shadow rays aim at the same few lights, and the rays of
-// one warp taken together share their node fetches in L1; a warp of rays at
-// different stages does not. Measured on the 1080p medium scene at 64 spp:
-// shadow launch 37 % of the step with refill against 27 % without (L1 hit
-// rate 50 against 62 %, long-scoreboard stalls 18 against 4 cycles per
-// issued instruction), 137.6 against 160.4 M paths/s.
-#ifndef VVPT_SHADOW_REFILL
-#define VVPT_SHADOW_REFILL 0
-#endif
-#ifndef VVPT_SHADOW_REFILL_BELOW
-#define VVPT_SHADOW_REFILL_BELOW VVPT_REFILL_BELOW
-#endif
-
-__global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_shadow(JobTable jt, PathState ps, Queues q)
-{
-    const uint32_t nc = q.counters[C_CONN];
-    const uint32_t n = nc + q.counters[C_NEEQ];
-    uint32_t err = 0;
-    uint32_t nsh = 0, nnee = 0;
-#if VVPT_SHADOW_REFILL
-    // Shadow rays step by step with refill; an emitter ray (the entries past
-    // the connection queue, a few per cent) runs its whole walk when its lane
-    // takes it.
-    if (n > 0) {
-        const uint32_t b0 = min(first_ray(), n - 1u);
-        tlas_cache_fill(jt.jobs[ps.job[b0 < nc ? q.conn[b0] : q.nee[b0 - nc]]].scene);
-    } else {
-        tlas_cache_none();
-    }
-    // per lane: the walk's transmittance and remaining distance; slot,
-    // volume, segment, candidate count | inside << 31
-    __shared__ float4 cold_t[256];
-    __shared__ uint4 cold_w[256];
-    TraceState st;
-    TraceStack stack;
-    Hit after = no_hit();
-    uint32_t state = kLaneFree, job = 0;
-    bool open = true; // warp-uniform: the queues may still hold rays
-    for (;;) {
-        uint32_t tr = __ballot_sync(0xFFFFFFFFu, state == kLaneTracing);
-        if (__popc(tr) <= VVPT_SHADOW_REFILL_BELOW) {
-            if (state == kLaneDone) {
-                const JobView &J = jt.jobs[job];
-                const float4 ct = cold_t[threadIdx.x];
-                const uint4 cw = cold_w[threadIdx.x];
-                ShadowWalk w;
-                w.T = f3(ct);
-                w.distT = ct.w;
-                w.vol = cw.y;
-                w.seg = cw.z;
-                w.guard = cw.w & 0x7FFFFFFFu;
-                w.inside = (cw.w >> 31) != 0;
-                if (shadow_walk_next(w, after, st, J.scene, J.params, err)) {
-                    cold_t[threadIdx.x] = f4(w.T, w.distT);
-                    cold_w[threadIdx.x] = make_uint4(cw.x, w.vol, w.seg, w.guard | (w.inside ? 0x80000000u : 0u));
-                    state = kLaneTracing;
-                } else {
-                    const uint32_t slot = cw.x;
-                    if (!is_black(w.T))
-                        ps.rad[slot] = f4(f3(ps.rad[slot]) + f3(ps.sh_c[slot]) * w.T, 0.0f);
-                    ps.flags[slot] = ps.flags[slot] & ~F_SHADOW;
-                    nsh++;
-                    state = kLaneFree;
-                }
-            }
-            if (open) {
-                bool mine;
-                const uint32_t i = refill_take(state == kLaneFree, &q.counters[C_FETCH_SHADOW], n, open, mine);
-                if (mine && i < nc) {
-                    const uint32_t slot = q.conn[i];
-                    const uint32_t flags = ps.flags[slot];
-                    if (flags & F_SHADOW) {
-                        job = ps.job[slot];
-                        const JobView &J = jt.jobs[job];
-                        const float4 sd = ps.sh_dir[slot];
-                        const float distT = sd.w - kConnTmin;
-                        if (J.params.depth > 0) {
-                            cold_t[threadIdx.x] = make_float4(1.0f, 1.0f, 1.0f, distT);
-                            cold_w[threadIdx.x] =
-                                make_uint4(slot, ps.vol[slot], 0u, (flags & F_INSIDE) ? 0x80000000u : 0u);
-                            after = no_hit();
-                            trace_begin(st, J.scene, f3(ps.o[slot]), f3(sd), kConnTmin, distT, after);
-                            state = kLaneTracing;
-                        } else {
-                            // no segment to walk: the light is visible
-                            ps.rad[slot] = f4(f3(ps.rad[slot]) + f3(ps.sh_c[slot]), 0.0f);
-                            ps.flags[slot] = flags & ~F_SHADOW;
-                            nsh++;
-                        }
-                    }
-                } else if (mine) {
-                    const uint32_t eslot = q.nee[i - nc];
-                    const uint32_t flags = ps.flags[eslot]; // F_INSIDE; the shadow rays may clear F_SHADOW meanwhile
-                    const JobView &J = jt.jobs[ps.job[eslot]];
-                    const float4 nb = ps.nee_b[eslot];
-                    float3 emT, T, em;
-                    float lpdf;
-                    emitter_ray(LaneTracer{}, J.scene, J.params, f3(ps.o[eslot]), f3(ps.d[eslot]),
-                                (flags & F_INSIDE) != 0, ps.vol[eslot], emT, T, em, lpdf, err);
-                    float3 c = f3(0.0f);
-                    if (!is_black(em))
-                        c = power_heuristic(nb.w, lpdf) * T * em * f3(nb);
-                    ps.nee_c[eslot] = f4(c, 0.0f);
-                    nnee++;
-                }
-            }
-            tr = __ballot_sync(0xFFFFFFFFu, state == kLaneTracing);
-            if (tr == 0) {
-                if (!open)
-                    break;
-                continue;
-            }
-        }
-        if (state == kLaneTracing && !trace_step(st, stack, jt.jobs[job].scene, after, err))
-            state = kLaneDone;
-    }
-#else
-    const uint32_t b0 = first_ray();
+    const uint32_t nw = q.counters[C_WALK];
+    const uint32_t n = nw + q.counters[C_NEE_RUN];
+    uint32_t err = 0, nnee = 0;
+    // a short queue (the usual case) is spread over the grid's warps, so that
+    // few walks, or only one, share a warp and none waits for another's steps
+    // (1920 x 1080 x 32 medium scene, about 2300 entries a launch: 106 us a
+    // launch with 32 to a warp, 56 us spread)
+    uint32_t spread = 1;
+    while (spread < 32u && (unsigned long long)n * (2u * spread) <= gridDim.x * blockDim.x)
+        spread *= 2u;
+    const uint32_t b0 = first_ray() / spread;
     if (b0 < n)
-        tlas_cache_fill(jt.jobs[ps.job[b0 < nc ? q.conn[b0] : q.nee[b0 - nc]]].scene);
+        tlas_cache_fill(jt.jobs[ps.job[b0 < nw ? q.walk[b0] : q.nee[b0 - nw]]].scene);
     else
         tlas_cache_none();
-#if VVPT_BLAS_WIDE && VVPT_GROUP_TRAVERSAL
-    const GroupTracer trace{lane_group()};
-    const bool writer = trace.g.gl == 0;
-#else
-    const LaneTracer trace{};
-    const bool writer = true;
-#endif
-    for (uint32_t i = my_ray(); i < n; i += ray_stride()) {
-        if (i < nc) {
-            const uint32_t slot = q.conn[i];
-            const uint32_t flags = ps.flags[slot];
-            if (!(flags & F_SHADOW))
-                continue;
-            const JobView &J = jt.jobs[ps.job[slot]];
-            const SceneView &s = J.scene;
-            const RenderParams &p = J.params;
+    for (uint32_t i = my_ray() % spread ? n : my_ray() / spread; i < n; i += ray_stride() / spread) {
+        const uint32_t slot = i < nw ? q.walk[i] : q.nee[i - nw];
+        const JobView &J = jt.jobs[ps.job[slot]];
+        const SceneView &s = J.scene;
+        const RenderParams &p = J.params;
+        const uint32_t flags = ps.flags[slot]; // of an emitter ray's entry only F_INSIDE: the other part may write the rest
+        const bool inside = (flags & F_INSIDE) != 0;
+        if (i < nw && (flags & F_SHADOW_WALK)) {
             const float4 sd = ps.sh_dir[slot];
-            const float3 T = shadow_transmittance(trace, s, p, f3(ps.o[slot]), f3(sd), sd.w, (flags & F_INSIDE) != 0,
-                                                  ps.vol[slot], err);
-            group_sync();
-            if (writer) {
-                if (!is_black(T))
-                    ps.rad[slot] = f4(f3(ps.rad[slot]) + f3(ps.sh_c[slot]) * T, 0.0f);
-                ps.flags[slot] = flags & ~F_SHADOW;
-                nsh++;
-            }
-        } else {
-            const uint32_t slot = q.nee[i - nc];
-            const uint32_t flags = ps.flags[slot]; // F_INSIDE; the shadow part may clear F_SHADOW meanwhile
-            const JobView &J = jt.jobs[ps.job[slot]];
-            const SceneView &s = J.scene;
-            const RenderParams &p = J.params;
+            const float3 T = shadow_transmittance(s, p, f3(ps.o[slot]), f3(sd), sd.w, inside, ps.vol[slot], err);
+            if (!is_black(T))
+                ps.rad[slot] = f4(f3(ps.rad[slot]) + f3(ps.sh_c[slot]) * T, 0.0f);
+        }
+        if (i >= nw || (flags & F_NEE_FULL)) {
             const float4 nb = ps.nee_b[slot];
-            float3 emT, T, em;
-            float lpdf;
-            emitter_ray(trace, s, p, f3(ps.o[slot]), f3(ps.d[slot]), (flags & F_INSIDE) != 0, ps.vol[slot], emT, T,
-                        em, lpdf, err);
-            float3 c = f3(0.0f);
-            if (!is_black(em))
-                c = power_heuristic(nb.w, lpdf) * T * em * f3(nb);
-            if (writer) {
+            const float3 o = f3(ps.o[slot]), d = f3(ps.d[slot]);
+            const uint32_t vol = ps.vol[slot];
+            float3 emT, T = f3(1.0f), em = f3(0.0f);
+            float lpdf = 0.0f;
+            const uint32_t inst = ps.hit_inst[slot];
+            if (i < nw || !(flags & F_DONE) ||
+                emitter_first(s, p, inst != kNoHit, inst, ps.hit[slot], o, d, inside, vol, T, em, lpdf))
+                emitter_ray(s, p, o, d, inside, vol, emT, T, em, lpdf, err);
+            nnee++;
+            if (i < nw) {
+                if (!is_black(em))
+                    ps.rad[slot] = f4(f3(ps.rad[slot]) + power_heuristic(nb.w, lpdf) * T * em * f3(nb), 0.0f);
+                ps.flags[slot] = flags & ~(F_NEE_FUSED | F_NEE_FULL | F_SHADOW_WALK);
+            } else {
+                float3 c = f3(0.0f);
+                if (!is_black(em))
+                    c = power_heuristic(nb.w, lpdf) * T * em * f3(nb);
                 ps.nee_c[slot] = f4(c, 0.0f);
-                nnee++;
             }
         }
     }
-#endif
-    warp_add(&q.counters[C_SHADOW], nsh);
     warp_add(&q.counters[C_NEE], nnee);
     if (err)
         atomicOr(&q.counters[C_ERR], err);
@@ -2030,18 +1736,9 @@ __global__ void k_trace_closest(SceneView s, const float4 *rays, uint32_t n, flo
 {
     uint32_t err = 0;
     tlas_cache_fill(s);
-#if VVPT_BLAS_WIDE && VVPT_GROUP_TRAVERSAL
-    const LaneGroup g = lane_group();
-#endif
     for (uint32_t i = my_ray(); i < n; i += ray_stride()) {
         float4 a = rays[2 * i], b = rays[2 * i + 1];
-#if VVPT_BLAS_WIDE && VVPT_GROUP_TRAVERSAL
-        Hit h = trace_after_group(s, f3(a), f3(b), a.w, b.w, no_hit(), err, g);
-        if (g.gl != 0)
-            continue;
-#else
         Hit h = trace_closest(s, f3(a), f3(b), a.w, b.w, err);
-#endif
         tuv[i] = make_float4(h.t, h.u, h.v, 0.0f);
         ids[2 * i] = h.inst;
         ids[2 * i + 1] = h.prim;
@@ -2082,12 +1779,11 @@ void launch_kernel(KernelId k, const JobTable &jt, const PathState &ps, const Qu
     case K_REGEN:
         k_regen<<<shape.grid, shape.block, 0, stream>>>(jt, ps, q, pp);
         break;
-    case K_EXTEND:
-        k_extend<<<shape.grid, shape.block, kTlasCacheBytes, stream>>>(jt, ps, q, pp);
+    case K_TRACE:
+        k_trace<<<shape.grid, shape.block, kTlasCacheBytes, stream>>>(jt, ps, q, pp);
         break;
     case K_PARTITION:
-        if (kPartitionLaunches)
-            k_partition<<<shape.grid, shape.block, 0, stream>>>(ps, q, pp);
+        k_partition<<<shape.grid, shape.block, 0, stream>>>(ps, q, pp);
         break;
     case K_WALK:
         k_walk<<<shape.grid, shape.block, kTlasCacheBytes, stream>>>(jt, ps, q);
@@ -2100,9 +1796,6 @@ void launch_kernel(KernelId k, const JobTable &jt, const PathState &ps, const Qu
 #else
         k_shade<3><<<shape.grid, shape.block, kTlasCacheBytes, stream>>>(jt, ps, q, pp);
 #endif
-        break;
-    case K_SHADOW:
-        k_shadow<<<shape.grid, shape.block, kTlasCacheBytes, stream>>>(jt, ps, q);
         break;
     default:
         break;
@@ -2120,7 +1813,7 @@ void launch_reduce(const RenderParams &hp, const BatchResults &br, float4 *radia
 void launch_trace_closest(const SceneView &s, const float4 *rays, uint32_t n, float4 *tuv, uint32_t *ids, uint32_t *err,
                           cudaStream_t stream)
 {
-    int grid = (int)std::min<uint64_t>(((uint64_t)n * kLanesPerRay + 255) / 256, 65535u);
+    int grid = (int)std::min<uint64_t>(((uint64_t)n + 255) / 256, 65535u);
     if (grid < 1)
         grid = 1;
     k_trace_closest<<<grid, 256, kTlasCacheBytes, stream>>>(s, rays, n, tuv, ids, err);

@@ -78,8 +78,8 @@ enum CounterIndex {
     C_PATHS = 14,
     C_WALK = 15,
     C_NEEQ = 16,
-    C_FETCH_EXT = 17,    // extension rays handed out so far in this iteration (lane refill)
-    C_FETCH_SHADOW = 18, // shadow and emitter rays handed out so far in this iteration
+    C_FETCH = 17,   // rays k_trace has handed out so far in this iteration (lane refill)
+    C_NEE_RUN = 18, // emitter rays of this iteration's k_walk (C_NEEQ counts the next one's)
     C_COUNT = 19
 };
 
@@ -87,9 +87,9 @@ struct Queues {
     uint32_t *ext[2];
     uint32_t *ext_key;  // per extension-queue entry: shade bin (0 Lambert, 1 PBR, 2 miss) | 4 = emitter walk
     uint32_t *shade_l, *shade_p, *shade_m;
-    uint32_t *walk;     // paths whose pending emitter ray needs the full candidate walk
-    uint32_t *conn;     // paths with a shadow ray
-    uint32_t *nee;      // paths that end with an emitter ray (k_shadow, after the shadow rays)
+    uint32_t *walk;     // paths whose shadow ray or fused emitter ray needs the full candidate walk
+    uint32_t *conn;     // paths with a shadow ray (traced with the next iteration's extension rays)
+    uint32_t *nee;      // paths that end with an emitter ray (next iteration's k_walk)
     uint32_t *regen[2];
     uint32_t *counters; // CounterIndex
 };
@@ -155,12 +155,11 @@ void launch_trace_closest(const SceneView &s, const float4 *rays, uint32_t n, fl
 enum KernelId {
     K_BEGIN = 0,
     K_REGEN = 1,
-    K_EXTEND = 2,
+    K_TRACE = 2, // extension rays, then the shadow rays of the previous shading
     K_PARTITION = 3,
-    K_WALK = 4,
+    K_WALK = 4, // candidate walks, then the emitter rays of paths that ended
     K_SHADE = 5,
-    K_SHADOW = 6, // shadow rays, then the emitter rays of paths that end
-    K_NUM = 7
+    K_NUM = 6
 };
 // K_SHADE launches one kernel over the three material-sorted queues, or with
 // VVPT_SHADE_SPLIT = 1 (a build option) one kernel per queue, each compiled
@@ -171,25 +170,9 @@ enum KernelId {
 #ifndef VVPT_SHADE_SPLIT
 #define VVPT_SHADE_SPLIT 0
 #endif
-// Lane refill in the extension kernel (binary BLAS). With
-// VVPT_EXTEND_PARTITION = 1 (a build option, measured, not kept) the refill
-// kernel also appends its hits to the material-sorted shade queues and the
-// emitter-walk queue itself and k_partition is not launched: the extension
-// kernel grew by what the partition launch took (1920 x 1080 x 64 medium
-// scene: 174.3 against 174.5 M paths/s).
-#ifndef VVPT_EXTEND_REFILL
-#define VVPT_EXTEND_REFILL (!VVPT_BLAS_WIDE)
-#endif
-#ifndef VVPT_EXTEND_PARTITION
-#define VVPT_EXTEND_PARTITION 0
-#endif
 constexpr int kShadeLaunches = VVPT_SHADE_SPLIT ? 3 : 1;
-constexpr int kPartitionLaunches = (VVPT_EXTEND_REFILL && VVPT_EXTEND_PARTITION) ? 0 : 1;
-constexpr int launches_of(int k)
-{
-    return k == K_SHADE ? kShadeLaunches : (k == K_PARTITION ? kPartitionLaunches : 1);
-}
-constexpr int kKernelsPerIteration = K_NUM + kShadeLaunches - 1 + kPartitionLaunches - 1;
+constexpr int launches_of(int k) { return k == K_SHADE ? kShadeLaunches : 1; }
+constexpr int kKernelsPerIteration = K_NUM + kShadeLaunches - 1;
 void launch_kernel(KernelId k, const JobTable &jt, const PathState &ps, const Queues &q, int pingpong,
                    const LaunchShape &shape, cudaStream_t stream);
 
@@ -198,13 +181,14 @@ void launch_kernel(KernelId k, const JobTable &jt, const PathState &ps, const Qu
 // (nominal branch), plus the three shading vertices and their indices read by
 // shade. BVH nodes, triangles and textures are excluded.
 constexpr double kBytesRegen = 4 + 3 * 4 + 3 * sizeof(float4) + 3 * sizeof(float4) + 4 + 9 * sizeof(float4) + 5 * 4 + 4;
-constexpr double kBytesExtend = 4 + 4 /* flags */ + 2 * sizeof(float4) + sizeof(float4) + 4 + 4 /* key */;
+// an extension ray's or a shadow ray's entry (the larger of the two, a visible light's)
+constexpr double kBytesTrace = 4 + 4 + 4 /* job, flags */ + 2 * sizeof(float4) + 2 * sizeof(float4) /* rad sh_c */ +
+                               sizeof(float4);
 constexpr double kBytesPartition = 4 + 4 + 4;
 constexpr double kBytesWalk = 4 + 4 + 4 + 4 * sizeof(float4) /* o d nee_b rad */ + sizeof(float4) + 4;
 constexpr double kBytesShade = 4 + (4 + 4 + 4 + 4) + 5 * sizeof(float4) /* beta rad o d hit */ + 3 * 4 +
                                3 * sizeof(ShadeVertex) /* vertices */ + (4 + 4 + 4) + 4 * sizeof(float4) /* writes */ +
                                5 * sizeof(float4) /* alb nrm sh_dir sh_c nee_b */ + sizeof(float4) /* nee_b read */ +
                                2 * 4;
-constexpr double kBytesShadow = 4 + 4 + 4 + 4 * sizeof(float4) /* o sh_dir rad sh_c */ + sizeof(float4) + 4;
 
 }  // namespace vvpt
