@@ -209,8 +209,8 @@ public:
         float llo[3], lhi[3], rlo[3], rhi[3];
         box_or_empty(l, llo, lhi);
         box_or_empty(r, rlo, rhi);
-        nd.lxy = {llo[0], lhi[0], llo[1], lhi[1]};
-        nd.rxy = {rlo[0], rhi[0], rlo[1], rhi[1]};
+        nd.lxy = {llo[0], llo[1], lhi[0], lhi[1]};
+        nd.rxy = {rlo[0], rlo[1], rhi[0], rhi[1]};
         nd.lrz = {llo[2], lhi[2], rlo[2], rhi[2]};
         nd.c = {l.index, r.index, l.count, r.count};
         if (l.count == 0 && l.index < 0)

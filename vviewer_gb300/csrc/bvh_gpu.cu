@@ -403,8 +403,8 @@ __device__ void small_subtree(int b, int n, int depth, int *idx, const GBox *box
     small_subtree(b + best_k, n - best_k, depth + 1, idx, boxes, cent, nodes, counters, rl, rc, rb);
     atomicMax(&counters[2], depth + 1);
     BVHNode nd;
-    nd.lxy = make_float4(lb.lo[0], lb.hi[0], lb.lo[1], lb.hi[1]);
-    nd.rxy = make_float4(rb.lo[0], rb.hi[0], rb.lo[1], rb.hi[1]);
+    nd.lxy = make_float4(lb.lo[0], lb.lo[1], lb.hi[0], lb.hi[1]);
+    nd.rxy = make_float4(rb.lo[0], rb.lo[1], rb.hi[0], rb.hi[1]);
     nd.lrz = make_float4(lb.lo[2], lb.hi[2], rb.lo[2], rb.hi[2]);
     nd.c = make_int4(ll, rl, lc, rc);
     nodes[node] = nd;
@@ -471,8 +471,8 @@ __global__ void k_emit(const Task *tasks, int ntasks, Split *splits, const GBox 
     }
     atomicMax(&counters[2], T.depth + 1);
     BVHNode nd;
-    nd.lxy = make_float4(S.lbox.lo[0], S.lbox.hi[0], S.lbox.lo[1], S.lbox.hi[1]);
-    nd.rxy = make_float4(S.rbox.lo[0], S.rbox.hi[0], S.rbox.lo[1], S.rbox.hi[1]);
+    nd.lxy = make_float4(S.lbox.lo[0], S.lbox.lo[1], S.lbox.hi[0], S.lbox.hi[1]);
+    nd.rxy = make_float4(S.rbox.lo[0], S.rbox.lo[1], S.rbox.hi[0], S.rbox.hi[1]);
     nd.lrz = make_float4(S.lbox.lo[2], S.lbox.hi[2], S.rbox.lo[2], S.rbox.hi[2]);
     nd.c = make_int4(link[0], link[1], cnt[0], cnt[1]);
     nodes[T.node] = nd;

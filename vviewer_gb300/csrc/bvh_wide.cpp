@@ -120,8 +120,8 @@ private:
     void children_of(int n, std::vector<CRef> &out) const
     {
         const BVHNode &b = m_bin.nodes[n];
-        const float lo[2][3] = {{b.lxy.x, b.lxy.z, b.lrz.x}, {b.rxy.x, b.rxy.z, b.lrz.z}};
-        const float hi[2][3] = {{b.lxy.y, b.lxy.w, b.lrz.y}, {b.rxy.y, b.rxy.w, b.lrz.w}};
+        const float lo[2][3] = {{b.lxy.x, b.lxy.y, b.lrz.x}, {b.rxy.x, b.rxy.y, b.lrz.z}};
+        const float hi[2][3] = {{b.lxy.z, b.lxy.w, b.lrz.y}, {b.rxy.z, b.rxy.w, b.lrz.w}};
         const int idx[2] = {b.c.x, b.c.y}, cnt[2] = {b.c.z, b.c.w};
         for (int k = 0; k < 2; k++) {
             if (idx[k] < 0)

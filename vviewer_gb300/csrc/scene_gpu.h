@@ -13,8 +13,9 @@ namespace vvpt {
 constexpr int kTraversalStack = 128;
 
 // Binary BVH node, 64 bytes: both children's boxes plus child links, so one
-// node visit is four 128-bit loads. lxy = (l.lo.x, l.hi.x, l.lo.y, l.hi.y),
-// rxy likewise, lrz = (l.lo.z, l.hi.z, r.lo.z, r.hi.z).
+// node visit is four 128-bit loads. lxy = (l.lo.x, l.lo.y, l.hi.x, l.hi.y),
+// rxy likewise, lrz = (l.lo.z, l.hi.z, r.lo.z, r.hi.z): each half of a word is
+// a pair that the slab test takes in one two-float instruction.
 // c = (left, right, left_count, right_count): count > 0 -> leaf covering
 // primitives [index, index + count) of the leaf-ordered primitive array;
 // count == 0 -> internal node `index` (relative to the BVH's first node);
@@ -60,7 +61,8 @@ static_assert(sizeof(WideNode) == 80, "WideNode must be 80 bytes");
 // Triangle in leaf order for intersection: v0.w carries the original
 // primitive index (gl_PrimitiveID) as raw bits; v1.w is 0, or for the
 // baked world-space triangles of small instances (kFlattenMaxTriangles) the
-// instance slot + 1 as raw bits, the instance a hit on it reports.
+// instance slot + 1 as raw bits, the instance a hit on it reports; v2.w is
+// nonzero on the last triangle of a leaf.
 struct alignas(16) TriVerts {
     float4 v0, v1, v2;
 };
@@ -135,7 +137,7 @@ struct SceneView {
     const ShadeVertex *verts;
     const uint32_t *indices;   // 3 per triangle, original order
     const DevInstance *instances;
-    const uint32_t *tlas_order; // TLAS leaf order -> instance slot
+    const uint32_t *tlas_order; // TLAS leaf order -> instance slot (top bit: the last of its leaf)
     uint32_t tlas_root;        // node index of the TLAS root
     uint32_t tlas_count;       // TLAS nodes (from tlas_root to the end of `nodes`)
     uint32_t num_instances;

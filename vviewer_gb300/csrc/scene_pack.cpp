@@ -32,6 +32,27 @@ struct MeshBuild {
     Box3 root{};
 };
 
+// Calls mark(k) for the last entry k of every leaf of a tree.
+template <class F>
+void for_leaf_ends(const std::vector<BVHNode> &nodes, F mark)
+{
+    for (const BVHNode &n : nodes) {
+        if (n.c.x >= 0 && n.c.z > 0)
+            mark((size_t)n.c.x + (size_t)n.c.z - 1);
+        if (n.c.y >= 0 && n.c.w > 0)
+            mark((size_t)n.c.y + (size_t)n.c.w - 1);
+    }
+}
+
+// TriVerts::v2.w of a leaf's last triangle
+float last_mark()
+{
+    const uint32_t one = 1;
+    float f;
+    std::memcpy(&f, &one, 4);
+    return f;
+}
+
 }  // namespace
 
 // column-major 4x4 -> rows of the 3x4 affine part
@@ -341,6 +362,7 @@ vvpt_status pack_scene(const vvpt_scene_desc *desc, PackedScene &out, std::strin
             tv.v2 = make_float4(p2[0], p2[1], p2[2], 0.0f);
             tris.push_back(tv);
         }
+        for_leaf_ends(builds[m].bvh.nodes, [&](size_t k) { tris[mi.tri_offset + k].v2.w = last_mark(); });
         for (uint32_t v = 0; v < md.num_vertices; v++) {
             const vvpt_vertex &x = md.vertices[v];
             ShadeVertex sv;
@@ -554,6 +576,9 @@ vvpt_status pack_scene(const vvpt_scene_desc *desc, PackedScene &out, std::strin
 #endif
         for (uint32_t k = 0; k < (uint32_t)ft.size(); k++)
             tris.push_back(ft[forder[k]]);
+#if !VVPT_BLAS_WIDE
+        for_leaf_ends(fbvh.nodes, [&](size_t k) { tris[syn.tri_offset + k].v2.w = last_mark(); });
+#endif
         Box3 w;
         for (int a = 0; a < 3; a++) {
             w.lo[a] = INFINITY;
@@ -626,6 +651,7 @@ vvpt_status pack_scene(const vvpt_scene_desc *desc, PackedScene &out, std::strin
     tlas_order.resize(tlas.order.size());
     for (size_t k = 0; k < tlas.order.size(); k++)
         tlas_order[k] = tlas_ids[tlas.order[k]];
+    for_leaf_ends(tlas.nodes, [&](size_t k) { tlas_order[k] |= 0x80000000u; });
     {
         // the traversal stack holds at most two entries per TLAS level, the
         // instance return marker and one entry per BLAS level

@@ -743,8 +743,10 @@ __global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_trace(JobTable j
     } else {
         tlas_cache_none();
     }
-    // per lane: queue index, slot, kind of ray and shade-bin bits
+    // per lane: queue index, slot, kind of ray and shade-bin bits, job; the ray
     __shared__ uint4 cold[256];
+    __shared__ TraceRay rays[256];
+    TraceRay &ray = rays[threadIdx.x];
     TraceState st;
     TraceStack stack;
     uint32_t state = kLaneFree, job = 0;
@@ -768,7 +770,8 @@ __global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_trace(JobTable j
                     // candidate walk, and this lane goes on with the
                     // extension ray from its tmin
                     cold[threadIdx.x].z = kColdFused | (4u << 3);
-                    trace_begin(st, jt.jobs[job].scene, st.o, st.d, kExtTmin, kExtTmax, no_hit());
+                    const float3 o = ray.o, d = ray.d;
+                    trace_begin(st, ray, jt.jobs[job].scene, o, d, kExtTmin, kExtTmax, no_hit());
                     state = kLaneTracing;
                 } else {
                     ps.hit[c.y] = make_float4(h.t, h.u, h.v, __uint_as_float(h.prim));
@@ -801,7 +804,7 @@ __global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_trace(JobTable j
                     // extension rays' range) takes the walk as a whole: the
                     // path's hit record belongs to its extension ray
                     if (ext || shadow || (flags & F_DONE)) {
-                        trace_begin(st, jt.jobs[job].scene, f3(ps.o[slot]), f3(d),
+                        trace_begin(st, ray, jt.jobs[job].scene, f3(ps.o[slot]), f3(d),
                                     ext && !fused ? kExtTmin : kConnTmin, tmax, no_hit());
                         state = kLaneTracing;
                     }
@@ -822,7 +825,7 @@ __global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_trace(JobTable j
         const bool tri = state == kLaneTracing && trace_triangle_pending(st);
         const bool tri_turn =
             100 * __popc(__ballot_sync(0xFFFFFFFFu, tri)) >= VVPT_TRI_TURN_PCT * __popc(tr);
-        if (state == kLaneTracing && tri == tri_turn && !trace_step(st, stack, jt.jobs[job].scene, no_hit(), err))
+        if (state == kLaneTracing && tri == tri_turn && !trace_step(st, ray, stack, jt.jobs[job].scene, no_hit(), err))
             state = kLaneDone;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
