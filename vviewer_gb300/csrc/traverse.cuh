@@ -446,25 +446,24 @@ constexpr uint32_t kRefIndex = (1u << 30) - 1u;
 constexpr uint32_t kRefWide = 1u << 30; // wide children still to visit (its BLAS has no leaf references)
 #endif
 
-// What a step seldom reads: the world-space ray and its absolute culling
-// margin. The refill loop keeps it in shared memory.
-struct TraceRay {
-    float3 o;
-    float slack;
-    float3 d;
-    float pad;
+// What a node visit does not read: the world-space ray, the best hit so far
+// and the current instance. The refill loop keeps it in shared memory, one
+// array per member, and its registers for the visit.
+struct TraceCold {
+    float4 &o_slack; // origin, absolute culling margin
+    float4 &d_tmin;  // direction, tmin
+    float4 &best;    // best hit so far: t, u, v, primitive (bits)
+    uint2 &ids;      // its instance, the instance whose BLAS is traversed
 };
 
 struct TraceState {
-    float tmin, box_tmin;
-    float far_t;                 // culling distance of the best hit so far
-    LevelRay lr;                 // the level's ray (its shear is only set in a BLAS)
-    Hit best;
-    uint32_t inst_id;            // kNoHit: in the TLAS
-    uint32_t node_base, tri_base;
-    uint32_t cur;                // next reference
-    int cached;                  // TLAS nodes below this index come from shared memory
-    int sp, floor;               // stack entries; those of the level above
+    float box_tmin;
+    float far_t;         // culling distance of the best hit so far
+    LevelRay lr;         // the level's ray; in the TLAS its shear is not set and kz is kInTlas
+    uint32_t node_base;
+    uint32_t tri_base;   // in the TLAS: nodes below this index come from shared memory
+    uint32_t cur;        // next reference
+    int sp, floor;       // stack entries; those of the level above
 #if VVPT_BLAS_WIDE
     // BLAS level: the group of wide children still to visit (hits at bit
     // slot ^ oct, imask, first child) and the triangles still to test (mask
@@ -472,36 +471,50 @@ struct TraceState {
     uint32_t w_base, w_bits, w_imask, t_base, t_bits, oct;
 #endif
 };
+constexpr int kInTlas = 3;
 // The traversal stack (reference, entry distance), kept apart from the scalar
 // state so that the scalars stay in registers.
 typedef int2 TraceStack[kTraversalStack];
 
-__device__ __forceinline__ void trace_begin(TraceState &st, TraceRay &ray, const SceneView &s, const float3 &o,
-                                            const float3 &d, float tmin, float tmax, const Hit &after)
+__device__ __forceinline__ Hit trace_best(const TraceCold &c)
 {
-    ray.o = o;
-    ray.d = d;
-    ray.slack = cull_slack(s, o, d);
-    st.tmin = tmin;
-    st.best.t = tmax;
-    st.best.u = st.best.v = 0.0f;
-    st.best.inst = kNoHit;
-    st.best.prim = kNoHit;
-    st.far_t = cull_far(tmax, ray.slack);
-    st.box_tmin = cull_near(after.inst == kNoHit ? tmin : fmaxf(tmin, after.t), ray.slack);
+    Hit h;
+    h.t = c.best.x;
+    h.u = c.best.y;
+    h.v = c.best.z;
+    h.prim = __float_as_uint(c.best.w);
+    h.inst = c.ids.x;
+    return h;
+}
+
+// The world-space ray at the TLAS.
+__device__ __forceinline__ void trace_enter_tlas(TraceState &st, const SceneView &s, const float3 &o, const float3 &d)
+{
     st.lr.norg = -o;
     st.lr.invd = safe_inv(d);
-    st.lr.Sx = st.lr.Sy = st.lr.Sz = 0.0f;
-    st.lr.kz = 0;
-    st.inst_id = kNoHit;
+    st.lr.kz = kInTlas;
     st.node_base = s.tlas_root;
-    st.tri_base = 0;
+    st.tri_base = vvpt_tlas_cache_src == s.nodes + s.tlas_root ? (uint32_t)vvpt_tlas_cache_count : 0u;
+    st.floor = 0;
+}
+
+__device__ __forceinline__ void trace_begin(TraceState &st, const TraceCold &c, const SceneView &s, const float3 &o,
+                                            const float3 &d, float tmin, float tmax, const Hit &after)
+{
+    const float slack = cull_slack(s, o, d);
+    c.o_slack = make_float4(o.x, o.y, o.z, slack);
+    c.d_tmin = make_float4(d.x, d.y, d.z, tmin);
+    c.best = make_float4(tmax, 0.0f, 0.0f, __uint_as_float(kNoHit));
+    c.ids = make_uint2(kNoHit, kNoHit);
+    st.far_t = cull_far(tmax, slack);
+    st.box_tmin = cull_near(after.inst == kNoHit ? tmin : fmaxf(tmin, after.t), slack);
+    st.lr.Sx = st.lr.Sy = st.lr.Sz = 0.0f;
+    trace_enter_tlas(st, s, o, d);
     st.cur = 0;
-    st.cached = vvpt_tlas_cache_src == s.nodes + s.tlas_root ? vvpt_tlas_cache_count : 0;
 #if VVPT_BLAS_WIDE
     st.w_base = st.w_bits = st.w_imask = st.t_base = st.t_bits = st.oct = 0;
 #endif
-    st.sp = st.floor = 0;
+    st.sp = 0;
 }
 
 __device__ __forceinline__ void trace_push(TraceState &st, TraceStack &stack, uint32_t ref, float t, uint32_t &err)
@@ -529,69 +542,65 @@ __device__ __forceinline__ uint32_t trace_pop(TraceState &st, const TraceStack &
         if (__int_as_float(e.y) <= st.far_t)
             return (uint32_t)e.x;
     }
-    return st.inst_id != kNoHit ? kRefReturn : kRefDone;
+    return st.lr.kz != kInTlas ? kRefReturn : kRefDone;
 }
 
 // Tests one triangle of the current BLAS against the ray and keeps it when it
 // is the best candidate after `after`; whether it is its leaf's last.
-__device__ __forceinline__ bool trace_triangle(TraceState &st, const TraceRay &ray, const SceneView &s, uint32_t local,
+__device__ __forceinline__ bool trace_triangle(TraceState &st, const TraceCold &c, const SceneView &s, uint32_t local,
                                                const Hit &after)
 {
     const float4 *tp = reinterpret_cast<const float4 *>(s.tris + st.tri_base + local);
     const float4 p0 = ldg_scene(tp), p1 = ldg_scene(tp + 1), p2 = ldg_scene(tp + 2);
-    const uint32_t prim = __float_as_uint(p0.w);
-    const uint32_t tag = __float_as_uint(p1.w);
-    const uint32_t hinst = tag ? tag - 1u : st.inst_id; // baked triangles name their instance
     float t, u, v;
-    if (wt_intersect(st.lr, p0, p1, p2, st.tmin, st.best.t, t, u, v) && better(t, hinst, prim, st.best) &&
-        is_after(t, hinst, prim, after)) {
-        st.best.t = t;
-        st.best.u = u;
-        st.best.v = v;
-        st.best.inst = hinst;
-        st.best.prim = prim;
-        st.far_t = cull_far(t, ray.slack);
+    if (wt_intersect(st.lr, p0, p1, p2, c.d_tmin.w, c.best.x, t, u, v)) {
+        const uint32_t prim = __float_as_uint(p0.w);
+        const uint32_t tag = __float_as_uint(p1.w);
+        const uint32_t hinst = tag ? tag - 1u : c.ids.y; // baked triangles name their instance
+        if (better(t, hinst, prim, trace_best(c)) && is_after(t, hinst, prim, after)) {
+            c.best = make_float4(t, u, v, p0.w);
+            c.ids.x = hinst;
+            st.far_t = cull_far(t, c.o_slack.w);
+        }
     }
     return __float_as_uint(p2.w) != 0u;
 }
 
-// Whether the next step is a triangle test.
-__device__ __forceinline__ bool trace_triangle_pending(const TraceState &st)
+// The kind of a ray's next step: a node visit, a triangle test, or a
+// transition between the levels (enter or leave an instance).
+constexpr int kStepNode = 0, kStepTriangle = 1, kStepLevel = 2;
+__device__ __forceinline__ int trace_kind(const TraceState &st)
 {
 #if VVPT_BLAS_WIDE
-    return st.t_bits != 0;
+    if (st.t_bits)
+        return kStepTriangle;
+    if (st.cur == kRefWide)
+        return kStepNode;
+#endif
+    const uint32_t k = st.cur >> 30;
+    return k < 2u ? (int)k : kStepLevel;
+}
+
+__device__ __forceinline__ void trace_step_triangle(TraceState &st, const TraceCold &c, TraceStack &stack,
+                                                    const SceneView &s, const Hit &after)
+{
+    VVPT_TRAVERSAL_STAT(1);
+#if VVPT_BLAS_WIDE
+    const int b = __ffs((int)st.t_bits) - 1;
+    st.t_bits &= st.t_bits - 1u;
+    trace_triangle(st, c, s, st.t_base + (uint32_t)b, after);
+    if (!st.t_bits && !st.w_bits)
+        st.cur = trace_pop(st, stack);
 #else
-    return (st.cur >> 30) == 1u;
+    st.cur = trace_triangle(st, c, s, st.cur & kRefIndex, after) ? trace_pop(st, stack) : st.cur + 1u;
 #endif
 }
 
-// One loop step; false when the traversal is over (st.best holds the result).
-__device__ __forceinline__ bool trace_step(TraceState &st, const TraceRay &ray, TraceStack &stack, const SceneView &s,
-                                           const Hit &after, uint32_t &err)
+__device__ __forceinline__ void trace_step_level(TraceState &st, const TraceCold &c, TraceStack &stack,
+                                                 const SceneView &s, uint32_t &err)
 {
-#if VVPT_BLAS_WIDE
-    if (st.t_bits) {
-        const int b = __ffs((int)st.t_bits) - 1;
-        st.t_bits &= st.t_bits - 1u;
-        trace_triangle(st, ray, s, st.t_base + (uint32_t)b, after);
-        if (!st.t_bits && !st.w_bits)
-            st.cur = trace_pop(st, stack);
-        return st.cur != kRefDone;
-    }
-#else
-    if ((st.cur >> 30) == 1u) {
-        VVPT_TRAVERSAL_STAT(1);
-        st.cur = trace_triangle(st, ray, s, st.cur & kRefIndex, after) ? trace_pop(st, stack) : st.cur + 1u;
-        return st.cur != kRefDone;
-    }
-#endif
     if (st.cur == kRefReturn) {
-        // back to the TLAS
-        st.lr.norg = -ray.o;
-        st.lr.invd = safe_inv(ray.d);
-        st.node_base = s.tlas_root;
-        st.inst_id = kNoHit;
-        st.floor = 0;
+        trace_enter_tlas(st, s, f3(c.o_slack), f3(c.d_tmin));
         st.cur = trace_pop(st, stack);
     }
     if ((st.cur >> 30) == 2u) {
@@ -600,11 +609,11 @@ __device__ __forceinline__ bool trace_step(TraceState &st, const TraceRay &ray, 
         const uint32_t id = __ldg(s.tlas_order + at);
         if (!(id >> 31))
             trace_push(st, stack, kRefInst | (at + 1u), st.box_tmin, err);
-        st.inst_id = id & 0x7FFFFFFFu;
-        const DevInstance &inst = s.instances[st.inst_id];
+        c.ids.y = id & 0x7FFFFFFFu;
+        const DevInstance &inst = s.instances[id & 0x7FFFFFFFu];
         const float4 rows[3] = {inst.w2o[0], inst.w2o[1], inst.w2o[2]};
-        const float3 cd = wt_xform_vector(rows, ray.d);
-        st.lr.norg = -wt_xform_point(rows, ray.o);
+        const float3 cd = wt_xform_vector(rows, f3(c.d_tmin));
+        st.lr.norg = -wt_xform_point(rows, f3(c.o_slack));
         st.lr.invd = safe_inv(cd);
         level_shear(st.lr, cd);
         st.node_base = inst.node_offset;
@@ -622,6 +631,10 @@ __device__ __forceinline__ bool trace_step(TraceState &st, const TraceRay &ray, 
         st.cur = 0;
 #endif
     }
+}
+
+__device__ __forceinline__ void trace_step_node(TraceState &st, TraceStack &stack, const SceneView &s, uint32_t &err)
+{
 #if VVPT_BLAS_WIDE
     if (st.cur == kRefWide) {
         // nearest remaining child of the group (octant order)
@@ -637,27 +650,40 @@ __device__ __forceinline__ bool trace_step(TraceState &st, const TraceRay &ray, 
                    st.t_base, st.t_bits);
         if (!st.t_bits && !st.w_bits)
             st.cur = trace_pop(st, stack);
-        return st.cur != kRefDone;
+        return;
     }
 #endif
-    if ((st.cur >> 30) == 0u) {
-        VVPT_TRAVERSAL_STAT(st.inst_id != kNoHit ? 0 : 3);
-        const bool tlas = st.inst_id == kNoHit;
-        const BVHNode n = (tlas && (int)st.cur < st.cached) ? load_node_cached((int)st.cur)
-                                                            : load_node(s.nodes, (int)(st.node_base + st.cur));
-        bool hl, hr;
-        float tl, tr;
-        box2(n, st.lr, st.box_tmin, st.far_t, hl, hr, tl, tr);
-        const uint32_t leaf = tlas ? kRefInst : kRefLeaf;
-        const uint32_t lref = (uint32_t)n.c.x | (n.c.z ? leaf : 0u), rref = (uint32_t)n.c.y | (n.c.w ? leaf : 0u);
-        if (hl || hr) {
-            const bool both = hl && hr, right = both ? tr < tl : hr;
-            st.cur = right ? rref : lref;
-            if (both)
-                trace_push(st, stack, right ? lref : rref, right ? tl : tr, err);
-        } else {
-            st.cur = trace_pop(st, stack);
-        }
+    const bool tlas = st.lr.kz == kInTlas;
+    VVPT_TRAVERSAL_STAT(tlas ? 3 : 0);
+    const BVHNode n = (tlas && st.cur < st.tri_base) ? load_node_cached((int)st.cur)
+                                                        : load_node(s.nodes, (int)(st.node_base + st.cur));
+    bool hl, hr;
+    float tl, tr;
+    box2(n, st.lr, st.box_tmin, st.far_t, hl, hr, tl, tr);
+    const uint32_t leaf = tlas ? kRefInst : kRefLeaf;
+    const uint32_t lref = (uint32_t)n.c.x | (n.c.z ? leaf : 0u), rref = (uint32_t)n.c.y | (n.c.w ? leaf : 0u);
+    if (hl || hr) {
+        const bool both = hl && hr, right = both ? tr < tl : hr;
+        st.cur = right ? rref : lref;
+        if (both)
+            trace_push(st, stack, right ? lref : rref, right ? tl : tr, err);
+    } else {
+        st.cur = trace_pop(st, stack);
+    }
+}
+
+// One loop step of the one-ray loop, a transition together with the visit
+// that follows it; false when the traversal is over (trace_best is the result).
+__device__ __forceinline__ bool trace_step(TraceState &st, const TraceCold &c, TraceStack &stack, const SceneView &s,
+                                           const Hit &after, uint32_t &err)
+{
+    if (trace_kind(st) == kStepTriangle) {
+        trace_step_triangle(st, c, stack, s, after);
+    } else {
+        if (trace_kind(st) == kStepLevel)
+            trace_step_level(st, c, stack, s, err);
+        if (trace_kind(st) == kStepNode)
+            trace_step_node(st, stack, s, err);
     }
     return st.cur != kRefDone;
 }
@@ -666,12 +692,14 @@ __device__ __forceinline__ Hit trace_after(const SceneView &s, const float3 &o, 
                                            const Hit &after, uint32_t &err)
 {
     TraceState st;
-    TraceRay ray;
+    float4 o_slack, d_tmin, best;
+    uint2 ids;
+    const TraceCold c{o_slack, d_tmin, best, ids};
     TraceStack stack;
-    trace_begin(st, ray, s, o, d, tmin, tmax, after);
-    while (trace_step(st, ray, stack, s, after, err)) {
+    trace_begin(st, c, s, o, d, tmin, tmax, after);
+    while (trace_step(st, c, stack, s, after, err)) {
     }
-    return st.best;
+    return trace_best(c);
 }
 
 __device__ __forceinline__ Hit no_hit()

@@ -620,11 +620,16 @@ __global__ void __launch_bounds__(256, VVPT_REGEN_MIN_BLOCKS) k_regen(JobTable j
 }
 
 // Minimum resident blocks of 256 threads per SM requested for the traversal
-// kernels, which caps their registers (4: 64 registers, 50% occupancy); the
-// traversal is latency bound and gains more from resident warps than it
-// loses to the few spilled registers.
+// kernels, which caps their registers (k_trace 5: 48 registers; k_walk 4: 64).
+// What k_trace waits for most is its loads, and the fifth block, which the ray
+// state in shared memory makes room for without spills in the loop, covers
+// more of that: 161 -> 149 ms on the 1080p medium scene, 41.0 -> 38.9 ms on
+// the sky scene.
 #ifndef VVPT_TRACE_MIN_BLOCKS
-#define VVPT_TRACE_MIN_BLOCKS 4
+#define VVPT_TRACE_MIN_BLOCKS 5
+#endif
+#ifndef VVPT_WALK_MIN_BLOCKS
+#define VVPT_WALK_MIN_BLOCKS 4
 #endif
 #ifndef VVPT_SHADE_MIN_BLOCKS
 #define VVPT_SHADE_MIN_BLOCKS 2
@@ -661,15 +666,25 @@ __device__ __forceinline__ uint32_t extend_key(const SceneView &s, const Hit &h,
 // Per-lane values that only that code reads stay in shared memory (one entry
 // per thread), so the traversal state keeps the registers.
 #ifndef VVPT_REFILL_BELOW
-#define VVPT_REFILL_BELOW 16
+#define VVPT_REFILL_BELOW 20
 #endif
 constexpr uint32_t kLaneFree = 0, kLaneTracing = 1, kLaneDone = 2;
-// Step turns: triangle tests and the other kinds of step in separate warp
-// steps, triangle tests when at least VVPT_TRI_TURN_PCT % of the tracing
-// lanes have one pending.
+// Step turns: triangle tests, transitions between the levels and node visits
+// in separate warp steps. Triangle tests when at least VVPT_TRI_TURN_PCT % of
+// the tracing lanes have one pending, else transitions when at least
+// VVPT_LEVEL_TURN_PCT % have (or no lane has a node to visit). Entering an
+// instance is a hundred instructions that nearly every warp step executed for
+// one or two lanes: in turns of their own, trace launches of the 1080p medium
+// scene (32 spp) 167 -> 159 ms, of the sky scene 44.1 -> 40.7 ms (thresholds of
+// 10, 25 and 40 %: 163, 159, 159 ms).
 #ifndef VVPT_TRI_TURN_PCT
 #define VVPT_TRI_TURN_PCT 33
 #endif
+#ifndef VVPT_LEVEL_TURN_PCT
+#define VVPT_LEVEL_TURN_PCT 33
+#endif
+// (a turn always has a lane that steps, so the loop ends)
+static_assert(VVPT_TRI_TURN_PCT > 0 && VVPT_TRI_TURN_PCT <= 100, "share of the tracing lanes, in percent");
 
 // Hands the next queue entries to the free lanes of the warp: returns the
 // entry index of this lane (meaningful when `mine`), and clears `open` when
@@ -745,20 +760,27 @@ __global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_trace(JobTable j
     }
     // per lane: queue index, slot, kind of ray and shade-bin bits, job; the ray
     __shared__ uint4 cold[256];
-    __shared__ TraceRay rays[256];
-    TraceRay &ray = rays[threadIdx.x];
+    __shared__ float4 cold_o[256], cold_d[256], cold_best[256];
+    __shared__ uint2 cold_ids[256];
+    const TraceCold ray{cold_o[threadIdx.x], cold_d[threadIdx.x], cold_best[threadIdx.x], cold_ids[threadIdx.x]};
     TraceState st;
     TraceStack stack;
     uint32_t state = kLaneFree, job = 0;
     bool open = true; // warp-uniform: the queue may still hold rays
+    // fewer rays than the grid has lanes: every warp takes its share, on its
+    // first lanes, instead of some warps taking 32 and the rest none (256 x 256
+    // previews, about 100,000 rays a launch: 49 -> 41 us a launch)
+    const uint32_t warps = gridDim.x * blockDim.x / 32u;
+    const uint32_t lanes = min(n / warps + 1u, 32u);
+    const bool takes = (threadIdx.x & 31u) < lanes;
     for (;;) {
         uint32_t tr = __ballot_sync(0xFFFFFFFFu, state == kLaneTracing);
-        if (__popc(tr) <= VVPT_REFILL_BELOW) {
+        if (__popc(tr) <= (open ? (int)(lanes * VVPT_REFILL_BELOW / 32u) : 0)) {
             uint32_t walk_slot = 0;
             bool walk = false;
             if (state == kLaneDone) {
                 const uint4 c = cold[threadIdx.x];
-                const Hit &h = st.best;
+                const Hit h = trace_best(ray);
                 const uint32_t key = c.z >> 3;
                 if (c.z & kColdShadow) {
                     walk = shadow_finish(jt.jobs[job], ps, c.y, h);
@@ -770,7 +792,7 @@ __global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_trace(JobTable j
                     // candidate walk, and this lane goes on with the
                     // extension ray from its tmin
                     cold[threadIdx.x].z = kColdFused | (4u << 3);
-                    const float3 o = ray.o, d = ray.d;
+                    const float3 o = f3(ray.o_slack), d = f3(ray.d_tmin);
                     trace_begin(st, ray, jt.jobs[job].scene, o, d, kExtTmin, kExtTmax, no_hit());
                     state = kLaneTracing;
                 } else {
@@ -788,7 +810,7 @@ __global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_trace(JobTable j
             }
             if (open) {
                 bool mine;
-                const uint32_t i = refill_take(state == kLaneFree, &q.counters[C_FETCH], n, open, mine);
+                const uint32_t i = refill_take(takes && state == kLaneFree, &q.counters[C_FETCH], n, open, mine);
                 if (mine) {
                     const bool ext = i < ne, shadow = !ext && i < ne + ns;
                     const uint32_t slot = entry(i);
@@ -817,15 +839,23 @@ __global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_trace(JobTable j
                 continue;
             }
         }
-        // triangle tests and node visits in separate warp steps: triangle
-        // tests run when enough of the tracing lanes have one pending, the
-        // other kinds of step otherwise (a lane whose kind is not this
-        // step's waits; every lane's kind gets its turn, since the lanes
-        // that step move on to a leaf, finish, or leave the tracing set)
-        const bool tri = state == kLaneTracing && trace_triangle_pending(st);
-        const bool tri_turn =
-            100 * __popc(__ballot_sync(0xFFFFFFFFu, tri)) >= VVPT_TRI_TURN_PCT * __popc(tr);
-        if (state == kLaneTracing && tri == tri_turn && !trace_step(st, ray, stack, jt.jobs[job].scene, no_hit(), err))
+        // one kind of step at a time: a lane whose kind is not this step's
+        // waits (every kind gets its turn, since the lanes that step move on
+        // to another kind, finish, or leave the tracing set)
+        const int kind = state == kLaneTracing ? trace_kind(st) : -1;
+        const int ntri = 100 * __popc(__ballot_sync(0xFFFFFFFFu, kind == kStepTriangle));
+        const uint32_t lev = __ballot_sync(0xFFFFFFFFu, kind == kStepLevel);
+        const int all = __popc(tr);
+        if (ntri >= VVPT_TRI_TURN_PCT * all) {
+            if (kind == kStepTriangle)
+                trace_step_triangle(st, ray, stack, jt.jobs[job].scene, no_hit());
+        } else if (lev && (100 * __popc(lev) >= VVPT_LEVEL_TURN_PCT * all || 100 * __popc(lev) + ntri == 100 * all)) {
+            if (kind == kStepLevel)
+                trace_step_level(st, ray, stack, jt.jobs[job].scene, err);
+        } else if (kind == kStepNode) {
+            trace_step_node(st, stack, jt.jobs[job].scene, err);
+        }
+        if (kind >= 0 && st.cur == kRefDone)
             state = kLaneDone;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1635,7 +1665,7 @@ __device__ __noinline__ float3 fused_nee(const SceneView &s, const RenderParams 
 // one. They write their contribution to nee_c, so the two parts never write
 // the same word; regen (or shade, for a path that continues) adds it after
 // the shadow ray's.
-__global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_walk(JobTable jt, PathState ps, Queues q)
+__global__ void __launch_bounds__(256, VVPT_WALK_MIN_BLOCKS) k_walk(JobTable jt, PathState ps, Queues q)
 {
     const uint32_t nw = q.counters[C_WALK];
     const uint32_t n = nw + q.counters[C_NEE_RUN];
@@ -1783,7 +1813,8 @@ void launch_kernel(KernelId k, const JobTable &jt, const PathState &ps, const Qu
         k_regen<<<shape.grid, shape.block, 0, stream>>>(jt, ps, q, pp);
         break;
     case K_TRACE:
-        k_trace<<<shape.grid, shape.block, kTlasCacheBytes, stream>>>(jt, ps, q, pp);
+        // five blocks of k_trace fit an SM where the other kernels' shape counts four
+        k_trace<<<shape.grid + shape.grid / 4, shape.block, kTlasCacheBytes, stream>>>(jt, ps, q, pp);
         break;
     case K_PARTITION:
         k_partition<<<shape.grid, shape.block, 0, stream>>>(ps, q, pp);
