@@ -541,9 +541,8 @@ VVPT_API vvpt_status vvpt_render(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_sc
 
         if (info->flags & VVPT_RENDER_PROFILE_KERNELS) {
             // one kernel at a time with events around each launch
-            static const char *names[K_NUM] = {"k_begin", "k_regen", "k_trace", "k_partition", "k_walk", "k_shade"};
-            static const double bpu[K_NUM] = {0.0,        kBytesRegen, kBytesTrace, kBytesPartition,
-                                              kBytesWalk, kBytesShade};
+            static const char *names[K_NUM] = {"k_regen", "k_trace", "k_partition", "k_walk", "k_shade"};
+            static const double bpu[K_NUM] = {kBytesRegen, kBytesTrace, kBytesPartition, kBytesWalk, kBytesShade};
             vvpt_kernel_profile prof{};
             prof.count = K_NUM;
             for (int k = 0; k < K_NUM; k++) {

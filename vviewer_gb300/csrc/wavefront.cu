@@ -59,6 +59,30 @@ __device__ __forceinline__ uint32_t warp_append_all(bool want, uint32_t *counter
     return base + (uint32_t)__popc(mask & ((1u << lane) - 1u));
 }
 
+// K appends at once, in the same way: lane k makes the atomic of kind k, so a
+// warp waits for one atomic's latency instead of K one after the other.
+template <int K>
+__device__ __forceinline__ void warp_append_many(const bool (&want)[K], uint32_t *const (&counter)[K],
+                                                 uint32_t (&pos)[K])
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t mask[K], mine = 0, base = 0;
+    uint32_t *to = nullptr;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        mask[k] = __ballot_sync(0xFFFFFFFFu, want[k]);
+        if (lane == (uint32_t)k) {
+            mine = mask[k];
+            to = counter[k];
+        }
+    }
+    if (mine)
+        base = atomicAdd(to, (uint32_t)__popc(mine));
+#pragma unroll
+    for (int k = 0; k < K; k++)
+        pos[k] = __shfl_sync(0xFFFFFFFFu, base, k) + (uint32_t)__popc(mask[k] & ((1u << lane) - 1u));
+}
+
 __device__ __forceinline__ float4 mat4_mul(const float4 *cols, float x, float y, float z, float w)
 {
     return make_float4(cols[0].x * x + cols[1].x * y + cols[2].x * z + cols[3].x * w,
@@ -446,9 +470,21 @@ __device__ __forceinline__ uint32_t find_range(const JobTable &jt, uint32_t num_
     return lo;
 }
 
-__global__ void k_begin(Queues q, int pp)
+// Finalizes finished samples, hands out work items, and generates camera
+// rays (raygen.rgen.glsl:24-99, 126-129).
+// Bound by memory latency: a slot's state is loaded at once, before anything
+// depends on it, the counters take two rounds of atomics per warp, and what a
+// sample leaves as it is is not written back (246,000 paths: 108 -> 98 us; the
+// reset of the counters rides along instead of being a launch of its own).
+__global__ void __launch_bounds__(256) k_regen(JobTable jt, PathState ps, Queues q, int pp)
 {
-    if (threadIdx.x == 0) {
+    const uint32_t n = q.counters[C_REGEN0 + pp];
+    const uint32_t *queue = q.regen[pp];
+    const unsigned long long total_items = *jt.total_items;
+    const uint32_t num_ranges = *jt.num_ranges;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        // queues of the previous iteration, consumed by now, that this
+        // iteration's later kernels fill
         q.counters[C_SHADE_L] = 0u;
         q.counters[C_SHADE_P] = 0u;
         q.counters[C_SHADE_M] = 0u;
@@ -456,83 +492,6 @@ __global__ void k_begin(Queues q, int pp)
         q.counters[C_FETCH] = 0u;
         q.counters[C_EXT0 + (1 - pp)] = 0u;
     }
-}
-
-// Finalizes finished samples, hands out work items, and generates camera
-// rays (raygen.rgen.glsl:24-99, 126-129).
-#ifndef VVPT_REGEN_MIN_BLOCKS
-#define VVPT_REGEN_MIN_BLOCKS 1
-#endif
-__global__ void __launch_bounds__(256, VVPT_REGEN_MIN_BLOCKS) k_regen(JobTable jt, PathState ps, Queues q, int pp)
-{
-    const uint32_t n = q.counters[C_REGEN0 + pp];
-    const uint32_t *queue = q.regen[pp];
-    const unsigned long long total_items = *jt.total_items;
-    const uint32_t num_ranges = *jt.num_ranges;
-    // camera ray of a slot that holds a work item (fresh: a new item, its
-    // sums and RNG state start from zero)
-    auto body = [&](const uint32_t slot, uint32_t sample, uint32_t item, uint32_t job, bool fresh, float3 cr,
-                    float3 ca, float3 cn) -> bool {
-        const RenderParams &p = jt.jobs[job].params;
-        const uint32_t npix = p.width * p.height;
-        const uint32_t batch = item / npix;
-        const uint32_t pix = item - batch * npix;
-        const uint32_t px = pix % p.width, py = pix / p.width;
-        PathRng rng;
-        float3 alb, nrm;
-        if (fresh) {
-            rng.s = init_rng(px, py, p.width, batch);
-            alb = nrm = f3(0.0f);
-        } else {
-            rng.s = ps.rng[slot];
-            alb = f3(ps.alb[slot]);
-            nrm = f3(ps.nrm[slot]);
-        }
-        rng.pix = px | (py << 16);
-        rng.index = batch * p.batch_size + sample;
-        if (p.sampler)
-            rng.s = py * p.width + py; // dimension start of every sample, raygen.rgen.glsl:57-60
-        // camera ray, raygen.rgen.glsl:63-91
-        const float2 oxy = rnd2(p, rng);
-        const float ox = oxy.x, oy = oxy.y;
-        float uvx = ((float)px + ox) / (float)p.width;
-        float uvy = ((float)py + oy) / (float)p.height;
-        float dx = uvx * 2.0f - 1.0f, dy = uvy * 2.0f - 1.0f;
-        float4 target = mat4_mul(p.proj_inv, dx, dy, 1.0f, 1.0f);
-        float3 dcam = normalize3(f3(target.x, target.y, target.z));
-        float3 ocam = f3(0.0f);
-        if (p.lens_radius > 0.0f) {
-            const float2 lxy = rnd2(p, rng);
-            const float lx = lxy.x, ly = lxy.y;
-            float2 disk = concentric_sample_disk(lx, ly);
-            float2 lens = make_float2(p.lens_radius * disk.x, p.lens_radius * disk.y);
-            float ft = p.focal_distance / (-dcam.z);
-            float3 focus = dcam * ft;
-            ocam = f3(lens.x, lens.y, 0.0f);
-            dcam = normalize3(focus - ocam);
-        }
-        float4 wo = mat4_mul(p.view_inv, ocam.x, ocam.y, ocam.z, 1.0f);
-        float4 wd = mat4_mul(p.view_inv, dcam.x, dcam.y, dcam.z, 0.0f);
-        ps.o[slot] = make_float4(wo.x, wo.y, wo.z, 0.0f);
-        ps.d[slot] = make_float4(wd.x, wd.y, wd.z, 0.0f);
-        ps.beta[slot] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-        ps.rad[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        ps.alb[slot] = f4(alb, 0.0f);
-        ps.nrm[slot] = f4(nrm, 0.0f);
-        ps.cum_rad[slot] = f4(cr, 0.0f);
-        ps.cum_alb[slot] = f4(ca, 0.0f);
-        ps.cum_nrm[slot] = f4(cn, 0.0f);
-        ps.rng[slot] = rng.s;
-        uint32_t nf = F_ITEM;
-        if (p.cam_volume != -1)
-            nf |= F_INSIDE;
-        ps.flags[slot] = nf;
-        ps.vol[slot] = (uint32_t)p.cam_volume;
-        ps.item[slot] = item;
-        ps.sample[slot] = sample;
-        ps.job[slot] = job;
-        return true;
-    };
     // The loop bound is warp-uniform: the counters below take one atomic per
     // warp (one per job for finished items) instead of one per slot, as the
     // slots of a launch all update the same few addresses.
@@ -540,8 +499,8 @@ __global__ void __launch_bounds__(256, VVPT_REGEN_MIN_BLOCKS) k_regen(JobTable j
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
         const uint32_t i = base + threadIdx.x;
         const bool valid = i < n;
-        uint32_t slot = 0, flags = 0, sample = 0, item = 0, job = 0;
-        float3 cr = f3(0.0f), ca = f3(0.0f), cn = f3(0.0f);
+        uint32_t slot = 0, flags = 0, sample = 0, item = 0, job = 0, rng_state = 0;
+        float3 cr = f3(0.0f), ca = f3(0.0f), cn = f3(0.0f), rad = f3(0.0f), alb = f3(0.0f), nrm = f3(0.0f);
         bool path_done = false, item_done = false;
         if (valid) {
             slot = queue[i];
@@ -549,19 +508,21 @@ __global__ void __launch_bounds__(256, VVPT_REGEN_MIN_BLOCKS) k_regen(JobTable j
             sample = ps.sample[slot];
             item = ps.item[slot];
             job = ps.job[slot];
-            if (flags & F_ITEM) {
-                cr = f3(ps.cum_rad[slot]);
-                ca = f3(ps.cum_alb[slot]);
-                cn = f3(ps.cum_nrm[slot]);
-            }
+            rng_state = ps.rng[slot];
+            cr = f3(ps.cum_rad[slot]);
+            ca = f3(ps.cum_alb[slot]);
+            cn = f3(ps.cum_nrm[slot]);
+            rad = f3(ps.rad[slot]);
+            alb = f3(ps.alb[slot]);
+            nrm = f3(ps.nrm[slot]);
             if (flags & F_DONE) {
                 const float total = (float)jt.jobs[job].params.total_samples;
-                float3 r = f3(ps.rad[slot]);
+                float3 r = rad;
                 if (flags & F_NEE) // the emitter ray's contribution, after the shadow ray's
                     r = r + f3(ps.nee_c[slot]);
                 cr += r / total;
-                ca += f3(ps.alb[slot]) / total;
-                cn += f3(ps.nrm[slot]) / total;
+                ca += alb / total;
+                cn += nrm / total;
                 sample++;
                 path_done = true;
             }
@@ -589,33 +550,88 @@ __global__ void __launch_bounds__(256, VVPT_REGEN_MIN_BLOCKS) k_regen(JobTable j
         unsigned long long g0 = 0;
         if (lane == 0 && need_mask)
             g0 = atomicAdd(jt.next_item, (unsigned long long)__popc(need_mask));
+        if (lane == 1 && paths)
+            atomicAdd(&q.counters[C_PATHS], paths);
         g0 = __shfl_sync(0xFFFFFFFFu, g0, 0);
         const unsigned long long g = g0 + (unsigned long long)__popc(need_mask & ((1u << lane) - 1u));
         const bool got = need && g < total_items;
         const bool idle = need && !got;
         const uint32_t started = (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, got));
-        if (lane == 0) {
-            if (paths)
-                atomicAdd(&q.counters[C_PATHS], paths);
-            if (started != (uint32_t)__popc(fin))
-                atomicAdd(&q.counters[C_ACTIVE], started - (uint32_t)__popc(fin)); // mod 2^32
-        }
-        const uint32_t ipos = warp_append_all(idle, jt.idle_count);
-        bool emit = false;
+        if (lane == 2 && started != (uint32_t)__popc(fin))
+            atomicAdd(&q.counters[C_ACTIVE], started - (uint32_t)__popc(fin)); // mod 2^32
+        const bool emit = valid && !idle;
+        uint32_t pos[2];
+        warp_append_many<2>({idle, emit}, {jt.idle_count, &q.counters[C_EXT0 + pp]}, pos);
         if (idle) {
             ps.flags[slot] = 0u;
             ps.item[slot] = 0xFFFFFFFFu;
-            jt.idle[ipos] = slot;
-        } else if (got) {
-            const uint32_t r = find_range(jt, num_ranges, g);
-            emit = body(slot, 0u, (uint32_t)(g - jt.range_begin[r]), jt.range_job[r], true, f3(0.0f), f3(0.0f),
-                        f3(0.0f));
+            jt.idle[pos[0]] = slot;
         } else if (valid) {
-            emit = body(slot, sample, item, job, false, cr, ca, cn);
+            // camera ray of a slot that holds a work item (a new item's sums
+            // and RNG state start from zero)
+            q.ext[pp][pos[1]] = slot;
+            if (got) {
+                const uint32_t r = find_range(jt, num_ranges, g);
+                item = (uint32_t)(g - jt.range_begin[r]);
+                job = jt.range_job[r];
+                sample = 0;
+                cr = ca = cn = f3(0.0f);
+            }
+            const RenderParams &p = jt.jobs[job].params;
+            const uint32_t npix = p.width * p.height;
+            const uint32_t batch = item / npix;
+            const uint32_t pix = item - batch * npix;
+            const uint32_t px = pix % p.width, py = pix / p.width;
+            PathRng rng;
+            rng.s = got ? init_rng(px, py, p.width, batch) : rng_state;
+            rng.pix = px | (py << 16);
+            rng.index = batch * p.batch_size + sample;
+            if (p.sampler)
+                rng.s = py * p.width + py; // dimension start of every sample, raygen.rgen.glsl:57-60
+            // camera ray, raygen.rgen.glsl:63-91
+            const float2 oxy = rnd2(p, rng);
+            const float ox = oxy.x, oy = oxy.y;
+            float uvx = ((float)px + ox) / (float)p.width;
+            float uvy = ((float)py + oy) / (float)p.height;
+            float dx = uvx * 2.0f - 1.0f, dy = uvy * 2.0f - 1.0f;
+            float4 target = mat4_mul(p.proj_inv, dx, dy, 1.0f, 1.0f);
+            float3 dcam = normalize3(f3(target.x, target.y, target.z));
+            float3 ocam = f3(0.0f);
+            if (p.lens_radius > 0.0f) {
+                const float2 lxy = rnd2(p, rng);
+                const float lx = lxy.x, ly = lxy.y;
+                float2 disk = concentric_sample_disk(lx, ly);
+                float2 lens = make_float2(p.lens_radius * disk.x, p.lens_radius * disk.y);
+                float ft = p.focal_distance / (-dcam.z);
+                float3 focus = dcam * ft;
+                ocam = f3(lens.x, lens.y, 0.0f);
+                dcam = normalize3(focus - ocam);
+            }
+            float4 wo = mat4_mul(p.view_inv, ocam.x, ocam.y, ocam.z, 1.0f);
+            float4 wd = mat4_mul(p.view_inv, dcam.x, dcam.y, dcam.z, 0.0f);
+            ps.o[slot] = make_float4(wo.x, wo.y, wo.z, 0.0f);
+            ps.d[slot] = make_float4(wd.x, wd.y, wd.z, 0.0f);
+            ps.beta[slot] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+            ps.rad[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            ps.cum_rad[slot] = f4(cr, 0.0f);
+            ps.cum_alb[slot] = f4(ca, 0.0f);
+            ps.cum_nrm[slot] = f4(cn, 0.0f);
+            ps.rng[slot] = rng.s;
+            uint32_t nf = F_ITEM;
+            if (p.cam_volume != -1)
+                nf |= F_INSIDE;
+            ps.flags[slot] = nf;
+            ps.vol[slot] = (uint32_t)p.cam_volume;
+            ps.sample[slot] = sample;
+            if (got) {
+                // first-hit albedo and normal carry over from sample to
+                // sample of an item and start from zero
+                ps.alb[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                ps.nrm[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                ps.item[slot] = item;
+                ps.job[slot] = job;
+            }
         }
-        const uint32_t pos = warp_append_all(emit, &q.counters[C_EXT0 + pp]);
-        if (emit)
-            q.ext[pp][pos] = slot;
     }
 }
 
@@ -867,7 +883,10 @@ __global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_trace(JobTable j
 }
 
 // Compacts the extension queue into the material-sorted shade queues and the
-// emitter-walk queue (warp-uniform loop; uniform, cheap work per entry).
+// emitter-walk queue. Its work is a few bytes per entry; what it waits for is
+// its atomics, so a block takes four entries per thread and makes one atomic
+// per queue for all of them (875,000 entries, one atomic per warp and queue:
+// 47 us, per block of 1024: 14 us).
 __global__ void __launch_bounds__(256) k_partition(PathState ps, Queues q, int pp)
 {
     const uint32_t n = q.counters[C_EXT0 + pp];
@@ -880,33 +899,67 @@ __global__ void __launch_bounds__(256) k_partition(PathState ps, Queues q, int p
         q.counters[C_NEE_RUN] = q.counters[C_NEEQ];
         q.counters[C_NEEQ] = 0u;
     }
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-        const uint32_t i = base + threadIdx.x;
-        uint32_t slot = 0, key = 0xFFu;
-        if (i < n) {
-            slot = queue[i];
-            key = q.ext_key[i];
+    constexpr int kPer = 4, kBins = 4; // Lambert, PBR, miss, walk
+    __shared__ uint32_t at[8][kBins];  // per warp: entries, then its first position
+    uint32_t *const counters[kBins] = {&q.counters[C_SHADE_L], &q.counters[C_SHADE_P], &q.counters[C_SHADE_M],
+                                       &q.counters[C_WALK]};
+    uint32_t *const to[kBins] = {q.shade_l, q.shade_p, q.shade_m, q.walk};
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, below = (1u << lane) - 1u;
+    const uint32_t per_block = kPer * blockDim.x;
+    for (uint32_t base = blockIdx.x * per_block; base < n; base += gridDim.x * per_block) {
+        uint32_t slot[kPer], key[kPer];
+#pragma unroll
+        for (int k = 0; k < kPer; k++) {
+            const uint32_t i = base + (warp * kPer + k) * 32u + lane;
+            slot[k] = i < n ? queue[i] : 0u;
+            key[k] = i < n ? q.ext_key[i] : 3u;
         }
-        const uint32_t bin = key & 3u;
-        uint32_t pos = warp_append_all(bin == 0, &q.counters[C_SHADE_L]);
-        if (bin == 0)
-            q.shade_l[pos] = slot;
-        pos = warp_append_all(bin == 1, &q.counters[C_SHADE_P]);
-        if (bin == 1)
-            q.shade_p[pos] = slot;
-        pos = warp_append_all(bin == 2, &q.counters[C_SHADE_M]);
-        if (bin == 2)
-            q.shade_m[pos] = slot;
-        bool walk = key != 0xFFu && (key & 4u);
-        if (walk) {
-            // one entry per path: a shadow walk's entry serves both
-            const uint32_t flags = ps.flags[slot];
-            ps.flags[slot] = flags | F_NEE_FULL;
-            walk = !(flags & F_SHADOW_WALK);
+#pragma unroll
+        for (int k = 0; k < kPer; k++)
+            if (key[k] & 4u) {
+                // one walk entry per path: a shadow walk's entry serves both
+                const uint32_t flags = ps.flags[slot[k]];
+                ps.flags[slot[k]] = flags | F_NEE_FULL;
+                if (flags & F_SHADOW_WALK)
+                    key[k] &= 3u;
+            }
+        uint32_t count = 0; // lane b: the warp's entries of bin b
+#pragma unroll
+        for (int k = 0; k < kPer; k++)
+#pragma unroll
+            for (int b = 0; b < kBins; b++) {
+                const uint32_t m = __ballot_sync(0xFFFFFFFFu, b < 3 ? (key[k] & 3u) == (uint32_t)b : (key[k] & 4u) != 0);
+                if (lane == (uint32_t)b)
+                    count += (uint32_t)__popc(m);
+            }
+        if (lane < kBins)
+            at[warp][lane] = count;
+        __syncthreads();
+        if (threadIdx.x < kBins) {
+            uint32_t sum = 0;
+            for (uint32_t w = 0; w < blockDim.x / 32u; w++)
+                sum += at[w][lane];
+            uint32_t pos = sum ? atomicAdd(counters[lane], sum) : 0u;
+            for (uint32_t w = 0; w < blockDim.x / 32u; w++) {
+                const uint32_t c = at[w][lane];
+                at[w][lane] = pos;
+                pos += c;
+            }
         }
-        pos = warp_append_all(walk, &q.counters[C_WALK]);
-        if (walk)
-            q.walk[pos] = slot;
+        __syncthreads();
+#pragma unroll
+        for (int b = 0; b < kBins; b++) {
+            uint32_t pos = at[warp][b];
+#pragma unroll
+            for (int k = 0; k < kPer; k++) {
+                const bool in = b < 3 ? (key[k] & 3u) == (uint32_t)b : (key[k] & 4u) != 0;
+                const uint32_t m = __ballot_sync(0xFFFFFFFFu, in);
+                if (in)
+                    to[b][pos + (uint32_t)__popc(m & below)] = slot[k];
+                pos += (uint32_t)__popc(m);
+            }
+        }
+        __syncthreads(); // `at` is filled again
     }
 }
 
@@ -1334,21 +1387,22 @@ __global__ void __launch_bounds__(256, KIND == 0 || KIND == 2 ? VVPT_SHADE_LM_MI
         late = want_conn || want_nee;
         want_ext = !done;
         }
-        uint32_t pos = warp_append_all(want_conn, &q.counters[C_CONN]);
-        if (want_conn)
-            q.conn[pos] = slot;
-        pos = warp_append_all(want_nee, &q.counters[C_NEEQ]);
-        if (want_nee)
-            q.nee[pos] = slot;
-        pos = warp_append_all(want_done && !late, &q.counters[C_REGEN0 + (1 - pp)]);
-        if (want_done && !late)
-            q.regen[1 - pp][pos] = slot;
-        pos = warp_append_all(want_done && late, &q.counters[C_REGEN0 + pp]);
-        if (want_done && late)
-            q.regen[pp][pos] = slot;
-        pos = warp_append_all(want_ext, &q.counters[C_EXT0 + (1 - pp)]);
+        const bool now = want_done && !late, later = want_done && late;
+        uint32_t pos[5];
+        warp_append_many<5>({want_ext, want_conn, now, later, want_nee},
+                            {&q.counters[C_EXT0 + (1 - pp)], &q.counters[C_CONN], &q.counters[C_REGEN0 + (1 - pp)],
+                             &q.counters[C_REGEN0 + pp], &q.counters[C_NEEQ]},
+                            pos);
         if (want_ext)
-            q.ext[1 - pp][pos] = slot;
+            q.ext[1 - pp][pos[0]] = slot;
+        if (want_conn)
+            q.conn[pos[1]] = slot;
+        if (now)
+            q.regen[1 - pp][pos[2]] = slot;
+        if (later)
+            q.regen[pp][pos[3]] = slot;
+        if (want_nee)
+            q.nee[pos[4]] = slot;
     }
     warp_add(&q.counters[C_NEE], walks);
     if (err)
@@ -1806,9 +1860,6 @@ void launch_kernel(KernelId k, const JobTable &jt, const PathState &ps, const Qu
                    const LaunchShape &shape, cudaStream_t stream)
 {
     switch (k) {
-    case K_BEGIN:
-        k_begin<<<1, 32, 0, stream>>>(q, pp);
-        break;
     case K_REGEN:
         k_regen<<<shape.grid, shape.block, 0, stream>>>(jt, ps, q, pp);
         break;

@@ -153,13 +153,12 @@ void launch_trace_closest(const SceneView &s, const float4 *rays, uint32_t n, fl
 // One wavefront kernel, launched on its own (profiling mode); an iteration
 // launches all of them in this order.
 enum KernelId {
-    K_BEGIN = 0,
-    K_REGEN = 1,
-    K_TRACE = 2, // extension rays, then the shadow rays of the previous shading
-    K_PARTITION = 3,
-    K_WALK = 4, // candidate walks, then the emitter rays of paths that ended
-    K_SHADE = 5,
-    K_NUM = 6
+    K_REGEN = 0,
+    K_TRACE = 1, // extension rays, then the shadow rays of the previous shading
+    K_PARTITION = 2,
+    K_WALK = 3, // candidate walks, then the emitter rays of paths that ended
+    K_SHADE = 4,
+    K_NUM = 5
 };
 // K_SHADE launches one kernel over the three material-sorted queues, or with
 // VVPT_SHADE_SPLIT = 1 (a build option) one kernel per queue, each compiled
