@@ -422,9 +422,9 @@ VVPT_API vvpt_status vvpt_autotune(vvpt_ctx *ctx,
                                    double budget_ms,
                                    vvpt_tuning *out_tuning);
 
-/* BVH builder of vvpt_scene_upload: AUTO builds meshes of at least 65,536
- * triangles on the GPU (binned SAH, one tree level per round of kernels) and
- * the rest, the baked small instances and the TLAS on the host; HOST builds
+/* BVH builder of vvpt_scene_upload: AUTO builds meshes of at least 512
+ * triangles on the GPU (binned SAH, all meshes in the same launches) and the
+ * rest, the baked small instances and the TLAS on the host; HOST builds
  * every tree on the host (binned SAH with FP64 costs); GPU builds every BLAS,
  * the baked small instances' BLAS and the TLAS on the GPU (trees of at most
  * one leaf stay on the host). All give the same closest hits. */

@@ -159,13 +159,15 @@ Queues carve_queues(char *base, size_t n)
 
 namespace {
 
+// `front`: bytes left free before the uploaded array (what the device built)
 template <class T>
-vvpt_status upload(vvpt_ctx *ctx, DevBuf &buf, const std::vector<T> &v, uint64_t &bytes)
+vvpt_status upload(vvpt_ctx *ctx, DevBuf &buf, const std::vector<T> &v, uint64_t &bytes, size_t front = 0)
 {
     size_t n = v.size() * sizeof(T);
-    VV_CUDA(buf.alloc(n), "cudaMalloc scene buffer");
+    VV_CUDA(buf.alloc(front + n), "cudaMalloc scene buffer");
     if (n)
-        VV_CUDA(cudaMemcpyAsync(buf.ptr, v.data(), n, cudaMemcpyHostToDevice, vv_stream(ctx)), "upload scene buffer");
+        VV_CUDA(cudaMemcpyAsync(buf.as<char>() + front, v.data(), n, cudaMemcpyHostToDevice, vv_stream(ctx)),
+                "upload scene buffer");
     bytes += buf.bytes;
     return VVPT_OK;
 }
@@ -311,14 +313,31 @@ VVPT_API vvpt_status vvpt_scene_upload(vvpt_ctx *ctx, const vvpt_scene_desc *des
 
     PackedScene pk;
     std::string err;
-    BlasBuilder gpu_builder;
-    if (ctx->bvh_builder != VVPT_BVH_BUILDER_HOST) {
-        cudaStream_t bs = vv_stream(ctx);
-        gpu_builder = [bs](const std::vector<Box3> &boxes, const BVHBuildOptions &opt, BVHBuildResult &res,
-                           std::string &e) { return build_bvh2_gpu(boxes, opt, bs, res, e); };
+    const cudaStream_t bs = vv_stream(ctx);
+    DeviceMeshes dm;
+    OutsideMeshes outside;
+    outside.tree = [bs](const std::vector<Box3> &boxes, const BVHBuildOptions &opt, BVHBuildResult &res,
+                        std::string &e) { return build_bvh2_gpu(boxes, opt, bs, res, e); };
+    outside.build = [&](const std::vector<uint32_t> &meshes, std::vector<MeshPlace> &places, std::string &e) {
+        if (!build_meshes_gpu(desc, meshes, BVHBuildOptions(), bs, dm, e))
+            return false;
+        for (const DeviceMeshes::Placed &p : dm.placed) {
+            MeshPlace mp{p.node_offset, p.tri_offset, p.vertex_offset, 3u * p.tri_offset, {}, {}};
+            std::copy(p.root.lo, p.root.lo + 3, mp.lo);
+            std::copy(p.root.hi, p.root.hi + 3, mp.hi);
+            places.push_back(mp);
+        }
+        outside.nodes = dm.num_nodes;
+        outside.tris = dm.num_tris;
+        outside.verts = dm.num_verts;
+        outside.depth = dm.depth;
+        return true;
+    };
+    if (ctx->bvh_builder == VVPT_BVH_BUILDER_GPU) {
+        outside.min_triangles = 1;
+        outside.other_trees = true;
     }
-    const bool all_gpu = ctx->bvh_builder == VVPT_BVH_BUILDER_GPU;
-    vvpt_status st = pack_scene(desc, pk, err, 0, gpu_builder, all_gpu ? 1u : 65536u, all_gpu);
+    vvpt_status st = pack_scene(desc, pk, err, 0, ctx->bvh_builder != VVPT_BVH_BUILDER_HOST ? &outside : nullptr);
     if (st != VVPT_OK)
         return fail(ctx, st, err);
     auto scene = new vvpt_scene();
@@ -326,15 +345,15 @@ VVPT_API vvpt_status vvpt_scene_upload(vvpt_ctx *ctx, const vvpt_scene_desc *des
 
     // ---- upload
     uint64_t bytes = 0;
-    if ((st = upload(ctx, scene->nodes, pk.nodes, bytes)) != VVPT_OK)
+    if ((st = upload(ctx, scene->nodes, pk.nodes, bytes, dm.num_nodes * sizeof(BVHNode))) != VVPT_OK)
         return st;
     if ((st = upload(ctx, scene->wnodes, pk.wnodes, bytes)) != VVPT_OK)
         return st;
-    if ((st = upload(ctx, scene->tris, pk.tris, bytes)) != VVPT_OK)
+    if ((st = upload(ctx, scene->tris, pk.tris, bytes, dm.num_tris * sizeof(TriVerts))) != VVPT_OK)
         return st;
-    if ((st = upload(ctx, scene->verts, pk.verts, bytes)) != VVPT_OK)
+    if ((st = upload(ctx, scene->verts, pk.verts, bytes, dm.num_verts * sizeof(ShadeVertex))) != VVPT_OK)
         return st;
-    if ((st = upload(ctx, scene->indices, pk.indices, bytes)) != VVPT_OK)
+    if ((st = upload(ctx, scene->indices, pk.indices, bytes, dm.num_tris * 12ull)) != VVPT_OK)
         return st;
     if ((st = upload(ctx, scene->instances, pk.instances, bytes)) != VVPT_OK)
         return st;
@@ -352,6 +371,19 @@ VVPT_API vvpt_status vvpt_scene_upload(vvpt_ctx *ctx, const vvpt_scene_desc *des
         return st;
     if ((st = upload(ctx, scene->emit_boxes, pk.emit_boxes, bytes)) != VVPT_OK)
         return st;
+    if (dm.num_tris) {
+        auto copy = [&](void *to, const DevBuf &from, size_t n) {
+            return cudaMemcpyAsync(to, from.ptr, n, cudaMemcpyDeviceToDevice, bs);
+        };
+        char *to = scene->nodes.as<char>();
+        for (const auto &nb : dm.nodes) {
+            VV_CUDA(copy(to, *nb, nb->bytes), "place nodes");
+            to += nb->bytes;
+        }
+        VV_CUDA(copy(scene->tris.ptr, dm.tris, dm.num_tris * sizeof(TriVerts)), "place triangles");
+        VV_CUDA(copy(scene->verts.ptr, dm.verts, dm.num_verts * sizeof(ShadeVertex)), "place vertices");
+        VV_CUDA(copy(scene->indices.ptr, dm.indices, dm.num_tris * 12ull), "place indices");
+    }
     VV_CUDA(cudaStreamSynchronize(vv_stream(ctx)), "scene upload");
 
     SceneView &v = scene->view;
@@ -363,7 +395,7 @@ VVPT_API vvpt_status vvpt_scene_upload(vvpt_ctx *ctx, const vvpt_scene_desc *des
     v.instances = scene->instances.as<DevInstance>();
     v.tlas_order = scene->tlas_order.as<uint32_t>();
     v.tlas_root = pk.tlas_root;
-    v.tlas_count = (uint32_t)(pk.nodes.size() - pk.tlas_root);
+    v.tlas_count = (uint32_t)(dm.num_nodes + pk.nodes.size() - pk.tlas_root);
     v.num_instances = desc->num_instances;
     v.materials = scene->materials.as<DevMaterial>();
     v.num_materials = desc->num_materials;

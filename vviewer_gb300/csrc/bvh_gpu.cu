@@ -1,39 +1,50 @@
 // GPU binned-SAH BVH builder: the same binary BVH (BVHNode layout, leaf order)
-// as build_bvh2 in bvh_build.cpp, built top down one tree level per round of
-// kernels instead of one node at a time on the host.
+// as build_bvh2 in bvh_build.cpp, for a whole set of meshes at once (a forest:
+// one tree per mesh, all in the same launches), built top down one tree level
+// per round of kernels, and the meshes' device arrays.
 //
 // A task is an inner node to split: a range of positions in the primitive
 // order array and its primitives' centroid bounds. Per level:
 //   k_bin        every primitive of every task adds its box and centroid to
 //                32 bins per axis of its task (shared-memory bins when a whole
 //                block of positions belongs to one task, global atomics else)
-//   k_split      one thread per task: SAH over the 31 candidate planes per
-//                axis (surface area x count on both sides), or the median when
-//                all centroids coincide
+//   k_split      one warp per task, one lane per bin: SAH over the 31
+//                candidate planes per axis (surface area x count on both
+//                sides), or the median when all centroids coincide
 //   k_partition  every primitive moves to its side (per-task cursors)
 //   k_emit       the task's node is written (both children's boxes and links);
-//                children above the leaf size become next-level tasks, smaller
-//                ones are finished by the same thread (split while the SAH
-//                says so, as the host builder does)
-// The host only reads the task count per level. Positions inside a leaf keep
-// the order the partition left them in, so the build is not deterministic
-// across runs; traversal results do not depend on it (exact closest hit under
-// the (t, instance, primitive) order).
+//                children of more than 32 primitives become next-level tasks
+// Ranges of at most 32 primitives are left to one launch at the end (k_small:
+// a warp per range, a lane per primitive, every split of the sorted centroids
+// tried), which also ends the levels early: binning 96 bins per task pays for
+// hundreds of primitives, not for a few. The host only reads the task count
+// per level. Positions inside a leaf keep the order the partition left them
+// in, so the build is not deterministic across runs; traversal results do not
+// depend on it (exact closest hit under the (t, instance, primitive) order).
+//
+// Bound by atomics and latency at the top levels (few tasks, all primitives in
+// one) and by launches below. Building eight meshes of 124,820 triangles one
+// after the other, a thread per split, took 60 ms; together, with the boxes
+// and the packing on the device, the whole scene uploads in 7.5 ms instead
+// of 97 (k_bin 1.7 ms in all, k_small 1.1).
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cfloat>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "bvh_build.h"
+#include "internal.h"
 
 namespace vvpt {
 
 namespace {
 
 constexpr int kBins = 32;
+constexpr int kSmall = 32; // ranges up to this size are finished by one warp
 
 struct GBox {
     float lo[3], hi[3];
@@ -41,8 +52,17 @@ struct GBox {
 
 struct Task {
     int begin, end, node, depth;
+    int mesh; // its root's node index; links are relative to it
     float cmin[3], cmax[3];
 };
+
+// A range for k_small: link and count go to node `parent`, child `side`; side
+// -1: the range is a whole tree and `parent` its root.
+struct SmallTask {
+    int begin, n, parent, side, depth, mesh;
+};
+
+enum { kNodes = 0, kNextTasks = 1, kMaxDepth = 2, kSmallTasks = 3, kCounters = 4 };
 
 // per task, axis, bin: count, box lo/hi, centroid lo/hi (float bits as
 // order-preserving ints for atomic min/max)
@@ -75,13 +95,99 @@ __device__ __forceinline__ int bin_of(float c, float lo, float hi)
     return min(max(b, 0), kBins - 1);
 }
 
-__global__ void k_init(const GBox *boxes, int n, int *idx, int *task_of, float4 *cent)
+// Per mesh: bounds of the centroids, then of the boxes (lo, hi; ordered ints).
+constexpr int kBoundInts = 12;
+__global__ void k_clear_bounds(int *bounds, int meshes)
 {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kBoundInts * meshes; i += gridDim.x * blockDim.x)
+        bounds[i] = i % 6 < 3 ? f2o(FLT_MAX) : f2o(-FLT_MAX);
+}
+
+// The primitives of one mesh: boxes (of its triangles, or given), centroids,
+// start order, the mesh's bounds.
+__global__ void __launch_bounds__(256) k_primitives(const vvpt_vertex *verts, const uint32_t *tri, const GBox *given,
+                                                    int n, int begin, int mesh, GBox *boxes, float4 *cent, int *idx,
+                                                    int *side, int *bounds)
+{
+    __shared__ int sb[kBoundInts];
+    if (threadIdx.x < kBoundInts)
+        sb[threadIdx.x] = threadIdx.x % 6 < 3 ? f2o(FLT_MAX) : f2o(-FLT_MAX);
+    __syncthreads();
+    int mine[kBoundInts];
+    for (int k = 0; k < kBoundInts; k++)
+        mine[k] = k % 6 < 3 ? f2o(FLT_MAX) : f2o(-FLT_MAX);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        idx[i] = i;
-        task_of[i] = 0;
-        const GBox &b = boxes[i];
-        cent[i] = make_float4(0.5f * (b.lo[0] + b.hi[0]), 0.5f * (b.lo[1] + b.hi[1]), 0.5f * (b.lo[2] + b.hi[2]), 0.0f);
+        GBox b;
+        if (given) {
+            b = given[i];
+        } else {
+            for (int a = 0; a < 3; a++) {
+                b.lo[a] = INFINITY;
+                b.hi[a] = -INFINITY;
+            }
+            for (int c = 0; c < 3; c++) {
+                const float *p = verts[tri[3 * (size_t)i + c]].position;
+                for (int a = 0; a < 3; a++) { // a NaN coordinate leaves the box as it is
+                    b.lo[a] = fminf(b.lo[a], p[a]);
+                    b.hi[a] = fmaxf(b.hi[a], p[a]);
+                }
+            }
+        }
+        const float c[3] = {0.5f * (b.lo[0] + b.hi[0]), 0.5f * (b.lo[1] + b.hi[1]), 0.5f * (b.lo[2] + b.hi[2])};
+        boxes[begin + i] = b;
+        cent[begin + i] = make_float4(c[0], c[1], c[2], 0.0f);
+        idx[begin + i] = begin + i;
+        side[begin + i] = mesh;
+        for (int a = 0; a < 3; a++) {
+            if (c[a] == c[a]) {
+                mine[a] = min(mine[a], f2o(c[a]));
+                mine[3 + a] = max(mine[3 + a], f2o(c[a]));
+            }
+            mine[6 + a] = min(mine[6 + a], f2o(b.lo[a]));
+            mine[9 + a] = max(mine[9 + a], f2o(b.hi[a]));
+        }
+    }
+    for (int k = 0; k < kBoundInts; k++) {
+        const int v = k % 6 < 3 ? __reduce_min_sync(0xFFFFFFFFu, mine[k]) : __reduce_max_sync(0xFFFFFFFFu, mine[k]);
+        if ((threadIdx.x & 31u) == 0) {
+            if (k % 6 < 3)
+                atomicMin(&sb[k], v);
+            else
+                atomicMax(&sb[k], v);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < kBoundInts) {
+        if (threadIdx.x % 6 < 3)
+            atomicMin(&bounds[kBoundInts * mesh + threadIdx.x], sb[threadIdx.x]);
+        else
+            atomicMax(&bounds[kBoundInts * mesh + threadIdx.x], sb[threadIdx.x]);
+    }
+}
+
+// The root task of every mesh (node index = mesh index).
+__global__ void k_roots(const int2 *ranges, int meshes, const int *bounds, Task *tasks, SmallTask *small, int *counters,
+                        int *child_task)
+{
+    for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < meshes; m += gridDim.x * blockDim.x) {
+        const int begin = ranges[m].x, n = ranges[m].y;
+        child_task[m] = -1;
+        if (n <= kSmall) {
+            small[atomicAdd(&counters[kSmallTasks], 1)] = SmallTask{begin, n, m, -1, 0, m};
+            continue;
+        }
+        Task t;
+        t.begin = begin;
+        t.end = begin + n;
+        t.node = t.mesh = m;
+        t.depth = 0;
+        for (int j = 0; j < 3; j++) {
+            t.cmin[j] = o2f(bounds[kBoundInts * m + j]);
+            t.cmax[j] = o2f(bounds[kBoundInts * m + 3 + j]);
+        }
+        const int id = atomicAdd(&counters[kNextTasks], 1);
+        tasks[id] = t;
+        child_task[m] = id;
     }
 }
 
@@ -97,20 +203,18 @@ __global__ void k_clear_bins(BinStat *bins, int nstats)
     }
 }
 
-__device__ __forceinline__ void add_to_bin(BinStat &s, const GBox &b, const float4 &c, bool shared_mem)
+__device__ __forceinline__ void add_to_bin(BinStat &s, const GBox &b, const float4 &c)
 {
-    (void)shared_mem;
     atomicAdd(&s.count, 1);
+    const float cc[3] = {c.x, c.y, c.z};
     for (int a = 0; a < 3; a++) {
         atomicMin(&s.blo[a], f2o(b.lo[a]));
         atomicMax(&s.bhi[a], f2o(b.hi[a]));
+        if (cc[a] == cc[a]) {
+            atomicMin(&s.clo[a], f2o(cc[a]));
+            atomicMax(&s.chi[a], f2o(cc[a]));
+        }
     }
-    atomicMin(&s.clo[0], f2o(c.x));
-    atomicMax(&s.chi[0], f2o(c.x));
-    atomicMin(&s.clo[1], f2o(c.y));
-    atomicMax(&s.chi[1], f2o(c.y));
-    atomicMin(&s.clo[2], f2o(c.z));
-    atomicMax(&s.chi[2], f2o(c.z));
 }
 
 // Blocks of 256 positions; a block whose positions all belong to one task
@@ -150,7 +254,7 @@ __global__ void __launch_bounds__(256) k_bin(const GBox *boxes, const float4 *ce
         const float cc[3] = {c.x, c.y, c.z};
         for (int a = 0; a < 3; a++) {
             const int k = a * kBins + bin_of(cc[a], T.cmin[a], T.cmax[a]);
-            add_to_bin(use_shared ? sb[k] : bins[(size_t)t * 3 * kBins + k], b, c, use_shared);
+            add_to_bin(use_shared ? sb[k] : bins[(size_t)t * 3 * kBins + k], b, c);
         }
     }
     if (use_shared) {
@@ -177,81 +281,96 @@ __device__ __forceinline__ float half_area(const float lo[3], const float hi[3])
     return dx * dy + dy * dz + dz * dx;
 }
 
-__global__ void k_split(const Task *tasks, int ntasks, const BinStat *bins, Split *splits)
+// Inclusive min / max scans over the lanes, from the first lane up (UP) or
+// from the last one down; `from` and `to` bound the lanes that take part.
+template <bool UP>
+__device__ __forceinline__ void scan_box(float (&lo)[3], float (&hi)[3], int from, int to)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = (int)(threadIdx.x & 31u);
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const bool ok = UP ? lane - d >= from : lane + d < to;
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const float l = UP ? __shfl_up_sync(0xFFFFFFFFu, lo[j], d) : __shfl_down_sync(0xFFFFFFFFu, lo[j], d);
+            const float h = UP ? __shfl_up_sync(0xFFFFFFFFu, hi[j], d) : __shfl_down_sync(0xFFFFFFFFu, hi[j], d);
+            if (ok) {
+                lo[j] = fminf(lo[j], l);
+                hi[j] = fmaxf(hi[j], h);
+            }
+        }
+    }
+}
+
+// Cost of the cut after this lane, the left box scanned up and the right one
+// down: area x count on both sides.
+__device__ __forceinline__ float cut_cost(const float (&llo)[3], const float (&lhi)[3], int lc, const float (&rlo)[3],
+                                          const float (&rhi)[3], int rc)
+{
+    float nlo[3], nhi[3];
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        nlo[j] = __shfl_down_sync(0xFFFFFFFFu, rlo[j], 1);
+        nhi[j] = __shfl_down_sync(0xFFFFFFFFu, rhi[j], 1);
+    }
+    return half_area(llo, lhi) * (float)lc + half_area(nlo, nhi) * (float)rc;
+}
+
+__global__ void __launch_bounds__(256) k_split(const Task *tasks, int ntasks, const BinStat *bins, Split *splits)
+{
+    const int t = (int)((blockIdx.x * blockDim.x + threadIdx.x) / 32u), lane = (int)(threadIdx.x & 31u);
     if (t >= ntasks)
         return;
     const BinStat *B = bins + (size_t)t * 3 * kBins;
-    Split best;
-    best.axis = -1;
-    best.bin = 0;
-    best.nl = (tasks[t].end - tasks[t].begin) / 2;
-    double best_cost = 1e300;
+    const int total = tasks[t].end - tasks[t].begin;
+    float best = INFINITY;
+    int best_axis = -1, best_left = 0;
     for (int a = 0; a < 3; a++) {
         if (!(tasks[t].cmax[a] > tasks[t].cmin[a]))
             continue;
-        // right-to-left sweep: area x count of the right side of plane k
-        double rcost[kBins];
-        float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-        int cnt = 0;
-        for (int k = kBins - 1; k > 0; k--) {
-            const BinStat &s = B[a * kBins + k];
-            if (s.count) {
-                for (int j = 0; j < 3; j++) {
-                    lo[j] = fminf(lo[j], o2f(s.blo[j]));
-                    hi[j] = fmaxf(hi[j], o2f(s.bhi[j]));
-                }
-                cnt += s.count;
-            }
-            rcost[k] = cnt ? (double)half_area(lo, hi) * cnt : 0.0;
+        const BinStat s = B[a * kBins + lane];
+        float llo[3], lhi[3], rlo[3], rhi[3];
+        for (int j = 0; j < 3; j++) {
+            llo[j] = rlo[j] = o2f(s.blo[j]);
+            lhi[j] = rhi[j] = o2f(s.bhi[j]);
         }
-        float llo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, lhi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-        int lc = 0;
-        for (int k = 0; k < kBins - 1; k++) {
-            const BinStat &s = B[a * kBins + k];
-            if (s.count) {
-                for (int j = 0; j < 3; j++) {
-                    llo[j] = fminf(llo[j], o2f(s.blo[j]));
-                    lhi[j] = fmaxf(lhi[j], o2f(s.bhi[j]));
-                }
-                lc += s.count;
-            }
-            const int rc = tasks[t].end - tasks[t].begin - lc;
-            if (lc == 0 || rc == 0)
-                continue;
-            const double cost = (double)half_area(llo, lhi) * lc + rcost[k + 1];
-            if (cost < best_cost) {
-                best_cost = cost;
-                best.axis = a;
-                best.bin = k;
-                best.nl = lc;
-            }
+        int lc = s.count;
+        for (int d = 1; d < 32; d <<= 1) {
+            const int o = __shfl_up_sync(0xFFFFFFFFu, lc, d);
+            lc += lane >= d ? o : 0;
+        }
+        scan_box<true>(llo, lhi, 0, 32);
+        scan_box<false>(rlo, rhi, 0, 32);
+        const float cost = cut_cost(llo, lhi, lc, rlo, rhi, total - lc);
+        if (lc > 0 && lc < total && lane < kBins - 1 && cost < best) {
+            best = cost;
+            best_axis = a;
+            best_left = lc;
         }
     }
-    // children's boxes and centroid bounds from the bins (median split: from
-    // the task's bounds; k_emit recomputes nothing for it)
-    for (int j = 0; j < 3; j++) {
-        best.lbox.lo[j] = best.rbox.lo[j] = best.lcmin[j] = best.rcmin[j] = FLT_MAX;
-        best.lbox.hi[j] = best.rbox.hi[j] = best.lcmax[j] = best.rcmax[j] = -FLT_MAX;
-    }
-    if (best.axis >= 0) {
-        for (int k = 0; k < kBins; k++) {
-            const BinStat &s = B[best.axis * kBins + k];
-            if (!s.count)
-                continue;
-            GBox &bx = k <= best.bin ? best.lbox : best.rbox;
-            float *cl = k <= best.bin ? best.lcmin : best.rcmin;
-            float *ch = k <= best.bin ? best.lcmax : best.rcmax;
-            for (int j = 0; j < 3; j++) {
-                bx.lo[j] = fminf(bx.lo[j], o2f(s.blo[j]));
-                bx.hi[j] = fmaxf(bx.hi[j], o2f(s.bhi[j]));
-                cl[j] = fminf(cl[j], o2f(s.clo[j]));
-                ch[j] = fmaxf(ch[j], o2f(s.chi[j]));
-            }
+    const int low = __reduce_min_sync(0xFFFFFFFFu, best_axis >= 0 ? f2o(best) : 0x7FFFFFFF);
+    const uint32_t at = __ballot_sync(0xFFFFFFFFu, best_axis >= 0 && f2o(best) == low);
+    const int from = at ? __ffs((int)at) - 1 : 0;
+    Split S;
+    S.axis = at ? __shfl_sync(0xFFFFFFFFu, best_axis, from) : -1;
+    S.bin = from;
+    S.nl = at ? __shfl_sync(0xFFFFFFFFu, best_left, from) : total / 2;
+    // children's boxes and centroid bounds from the bins (for a median split
+    // k_partition and k_emit fill them in)
+    const BinStat s = B[(S.axis < 0 ? 0 : S.axis) * kBins + lane];
+    for (int side = 0; side < 2; side++) {
+        const bool in = S.axis >= 0 && s.count && (lane <= S.bin) == (side == 0);
+        GBox &bx = side == 0 ? S.lbox : S.rbox;
+        float *cl = side == 0 ? S.lcmin : S.rcmin, *ch = side == 0 ? S.lcmax : S.rcmax;
+        for (int j = 0; j < 3; j++) {
+            bx.lo[j] = o2f(__reduce_min_sync(0xFFFFFFFFu, in ? s.blo[j] : f2o(FLT_MAX)));
+            bx.hi[j] = o2f(__reduce_max_sync(0xFFFFFFFFu, in ? s.bhi[j] : f2o(-FLT_MAX)));
+            cl[j] = o2f(__reduce_min_sync(0xFFFFFFFFu, in ? s.clo[j] : f2o(FLT_MAX)));
+            ch[j] = o2f(__reduce_max_sync(0xFFFFFFFFu, in ? s.chi[j] : f2o(-FLT_MAX)));
         }
     }
-    splits[t] = best;
+    if (lane == 0)
+        splits[t] = S;
 }
 
 // Median splits (all centroids equal) keep the order: the first nl
@@ -260,38 +379,49 @@ __global__ void k_partition(const GBox *boxes, const float4 *cent, const int *id
                             const Task *tasks, const Split *splits, int *cursors, int *idx_out, int *side_out,
                             GBox *median_boxes)
 {
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
-        const int t = task_of_in[p];
-        if (t < 0) {
-            idx_out[p] = idx_in[p];
+    const uint32_t lane = threadIdx.x & 31u;
+    for (int base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+        const int p = base + (int)threadIdx.x;
+        const int t = p < n ? task_of_in[p] : -1;
+        const int prim = p < n ? idx_in[p] : 0;
+        bool left = false;
+        if (t >= 0) {
+            const Task &T = tasks[t];
+            const Split &S = splits[t];
+            if (S.axis < 0) {
+                left = p - T.begin < S.nl;
+            } else {
+                const float4 c = cent[prim];
+                const float cc = S.axis == 0 ? c.x : (S.axis == 1 ? c.y : c.z);
+                left = bin_of(cc, T.cmin[S.axis], T.cmax[S.axis]) <= S.bin;
+            }
+        }
+        // one atomic per warp for the primitives of a task and side
+        const int key = t >= 0 ? 2 * t + (left ? 0 : 1) : -1;
+        const uint32_t same = __match_any_sync(0xFFFFFFFFu, key);
+        const int leader = __ffs((int)same) - 1;
+        int at = 0;
+        if (key >= 0 && (int)lane == leader)
+            at = atomicAdd(&cursors[key], __popc(same));
+        at = __shfl_sync(0xFFFFFFFFu, at, leader) + __popc(same & ((1u << lane) - 1u));
+        if (p >= n)
+            continue;
+        if (key < 0) {
+            idx_out[p] = prim;
             side_out[p] = -1;
             continue;
         }
-        const Task &T = tasks[t];
-        const Split &S = splits[t];
-        const int prim = idx_in[p];
-        bool left;
-        if (S.axis < 0) {
-            left = p - T.begin < S.nl;
-        } else {
-            const float4 c = cent[prim];
-            const float cc = S.axis == 0 ? c.x : (S.axis == 1 ? c.y : c.z);
-            left = bin_of(cc, T.cmin[S.axis], T.cmax[S.axis]) <= S.bin;
-        }
-        const int dst = left ? T.begin + atomicAdd(&cursors[2 * t], 1) : T.begin + S.nl + atomicAdd(&cursors[2 * t + 1], 1);
+        const int dst = tasks[t].begin + (left ? 0 : splits[t].nl) + at;
         idx_out[dst] = prim;
-        side_out[dst] = 2 * t + (left ? 0 : 1);
-        if (S.axis < 0) {
+        side_out[dst] = key;
+        if (splits[t].axis < 0) {
             // median split: children boxes accumulated here
             const GBox b = boxes[prim];
-            const float4 c = cent[prim];
-            GBox &m = median_boxes[2 * t + (left ? 0 : 1)];
-            int *mi = reinterpret_cast<int *>(&m);
+            int *mi = reinterpret_cast<int *>(&median_boxes[key]);
             for (int j = 0; j < 3; j++) {
                 atomicMin(&mi[j], f2o(b.lo[j]));
                 atomicMax(&mi[3 + j], f2o(b.hi[j]));
             }
-            (void)c;
         }
     }
 }
@@ -307,117 +437,12 @@ __global__ void k_clear_median(GBox *m, int n)
     }
 }
 
-// A child of at most max_leaf primitives is finished by its parent's thread
-// with the same rule as the host builder: split while the SAH says a split
-// is cheaper than the leaf (traversal cost 1, intersection cost 1 per
-// primitive); with so few primitives the candidate planes are the gaps
-// between the sorted centroids. Returns the parent's link and count.
-__device__ void small_subtree(int b, int n, int depth, int *idx, const GBox *boxes, const float4 *cent,
-                              BVHNode *nodes, int *counters, int &link, int &count, GBox &box)
-{
-    float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-    for (int i = 0; i < n; i++) {
-        const GBox g = boxes[idx[b + i]];
-        for (int j = 0; j < 3; j++) {
-            lo[j] = fminf(lo[j], g.lo[j]);
-            hi[j] = fmaxf(hi[j], g.hi[j]);
-        }
-    }
-    for (int j = 0; j < 3; j++) {
-        box.lo[j] = lo[j];
-        box.hi[j] = hi[j];
-    }
-    link = b;
-    count = n;
-    if (n <= 1)
-        return;
-    const double parent_area = (double)half_area(lo, hi);
-    double best = 1e300;
-    int best_axis = -1, best_k = 0;
-    int order[8];
-    for (int a = 0; a < 3; a++) {
-        // sort this range's positions by centroid on axis a (n <= 8)
-        for (int i = 0; i < n; i++)
-            order[i] = idx[b + i];
-        for (int i = 1; i < n; i++) {
-            const int x = order[i];
-            const float4 cx = cent[x];
-            const float vx = a == 0 ? cx.x : (a == 1 ? cx.y : cx.z);
-            int j = i - 1;
-            while (j >= 0) {
-                const float4 cj = cent[order[j]];
-                const float vj = a == 0 ? cj.x : (a == 1 ? cj.y : cj.z);
-                if (vj <= vx)
-                    break;
-                order[j + 1] = order[j];
-                j--;
-            }
-            order[j + 1] = x;
-        }
-        for (int k = 1; k < n; k++) {
-            float llo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, lhi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-            float rlo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, rhi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-            for (int i = 0; i < n; i++) {
-                const GBox g = boxes[order[i]];
-                float *l = i < k ? llo : rlo, *h = i < k ? lhi : rhi;
-                for (int j = 0; j < 3; j++) {
-                    l[j] = fminf(l[j], g.lo[j]);
-                    h[j] = fmaxf(h[j], g.hi[j]);
-                }
-            }
-            const double cost = (double)half_area(llo, lhi) * k + (double)half_area(rlo, rhi) * (n - k);
-            if (cost < best) {
-                best = cost;
-                best_axis = a;
-                best_k = k;
-            }
-        }
-    }
-    const double split_cost = 1.0 + (parent_area > 0.0 ? best / parent_area : (double)n);
-    if (best_axis < 0 || (double)n <= split_cost)
-        return; // leaf
-    // reorder the range by the best axis and build both sides
-    for (int i = 0; i < n; i++)
-        order[i] = idx[b + i];
-    for (int i = 1; i < n; i++) {
-        const int x = order[i];
-        const float4 cx = cent[x];
-        const float vx = best_axis == 0 ? cx.x : (best_axis == 1 ? cx.y : cx.z);
-        int j = i - 1;
-        while (j >= 0) {
-            const float4 cj = cent[order[j]];
-            const float vj = best_axis == 0 ? cj.x : (best_axis == 1 ? cj.y : cj.z);
-            if (vj <= vx)
-                break;
-            order[j + 1] = order[j];
-            j--;
-        }
-        order[j + 1] = x;
-    }
-    for (int i = 0; i < n; i++)
-        idx[b + i] = order[i];
-    const int node = atomicAdd(&counters[0], 1);
-    int ll, lc, rl, rc;
-    GBox lb, rb;
-    small_subtree(b, best_k, depth + 1, idx, boxes, cent, nodes, counters, ll, lc, lb);
-    small_subtree(b + best_k, n - best_k, depth + 1, idx, boxes, cent, nodes, counters, rl, rc, rb);
-    atomicMax(&counters[2], depth + 1);
-    BVHNode nd;
-    nd.lxy = make_float4(lb.lo[0], lb.lo[1], lb.hi[0], lb.hi[1]);
-    nd.rxy = make_float4(rb.lo[0], rb.lo[1], rb.hi[0], rb.hi[1]);
-    nd.lrz = make_float4(lb.lo[2], lb.hi[2], rb.lo[2], rb.hi[2]);
-    nd.c = make_int4(ll, rl, lc, rc);
-    nodes[node] = nd;
-    link = node;
-    count = 0;
-}
-
-// One thread per task: the node record, child tasks for children above the
-// leaf size (small children finished here); child task ids go to
+// One thread per task: the node record, child tasks for children of more than
+// kSmall primitives, entries for k_small for the others; child task ids go to
 // child_task[2t + side].
 __global__ void k_emit(const Task *tasks, int ntasks, Split *splits, const GBox *median_boxes, BVHNode *nodes,
-                       int *counters /* [0] nodes, [1] next tasks, [2] max depth */, Task *next, int *child_task,
-                       int max_leaf, int max_depth, int *idx, const GBox *boxes, const float4 *cent)
+                       int *counters, Task *next, SmallTask *small, int *child_task, int max_depth,
+                       const int2 *ranges, uint8_t *last)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= ntasks)
@@ -439,43 +464,180 @@ __global__ void k_emit(const Task *tasks, int ntasks, Split *splits, const GBox 
             S.lcmax[j] = S.rcmax[j] = T.cmax[j];
         }
     }
-    int link[2], cnt[2];
+    int link[2] = {0, 0}, cnt[2] = {0, 0};
     for (int side = 0; side < 2; side++) {
         const int b = side == 0 ? T.begin : T.begin + S.nl;
         const int e = side == 0 ? T.begin + S.nl : T.end;
         const int n = e - b;
         child_task[2 * t + side] = -1;
         if (T.depth + 1 >= max_depth) {
-            link[side] = b;
+            link[side] = b - ranges[T.mesh].x;
             cnt[side] = n;
-        } else if (n <= max_leaf && n <= 8) {
-            GBox bx;
-            small_subtree(b, n, T.depth + 1, idx, boxes, cent, nodes, counters, link[side], cnt[side], bx);
+            last[e - 1] = 1;
+        } else if (n <= kSmall) {
+            // link and count: k_small
+            small[atomicAdd(&counters[kSmallTasks], 1)] = SmallTask{b, n, T.node, side, T.depth + 1, T.mesh};
         } else {
-            const int node = atomicAdd(&counters[0], 1);
-            const int nt = atomicAdd(&counters[1], 1);
+            const int node = atomicAdd(&counters[kNodes], 1);
+            const int nt = atomicAdd(&counters[kNextTasks], 1);
             Task c;
             c.begin = b;
             c.end = e;
             c.node = node;
+            c.mesh = T.mesh;
             c.depth = T.depth + 1;
             for (int j = 0; j < 3; j++) {
                 c.cmin[j] = side == 0 ? S.lcmin[j] : S.rcmin[j];
                 c.cmax[j] = side == 0 ? S.lcmax[j] : S.rcmax[j];
             }
             next[nt] = c;
-            link[side] = node;
-            cnt[side] = 0;
+            link[side] = node - T.mesh;
             child_task[2 * t + side] = nt;
         }
     }
-    atomicMax(&counters[2], T.depth + 1);
+    atomicMax(&counters[kMaxDepth], T.depth + 1);
     BVHNode nd;
     nd.lxy = make_float4(S.lbox.lo[0], S.lbox.lo[1], S.lbox.hi[0], S.lbox.hi[1]);
     nd.rxy = make_float4(S.rbox.lo[0], S.rbox.lo[1], S.rbox.hi[0], S.rbox.hi[1]);
     nd.lrz = make_float4(S.lbox.lo[2], S.lbox.hi[2], S.rbox.lo[2], S.rbox.hi[2]);
     nd.c = make_int4(link[0], link[1], cnt[0], cnt[1]);
     nodes[T.node] = nd;
+}
+
+// The rest of the tree over at most 32 primitives: a warp, one lane per
+// primitive. Every cut of the centroids sorted along each axis is a candidate
+// plane; a range of at most max_leaf primitives stays a leaf unless the SAH
+// says a split is cheaper (traversal cost 1, intersection cost 1 per
+// primitive), the host builder's rule.
+constexpr int kSmallWarps = 4;
+__global__ void __launch_bounds__(32 * kSmallWarps)
+    k_small(const SmallTask *tasks, int ntasks, int *idx, const GBox *boxes, const float4 *cent, BVHNode *nodes,
+            int *counters, int max_leaf, int max_depth, const int2 *ranges, uint8_t *last)
+{
+    struct Seg {
+        int off, n, parent, side, depth;
+    };
+    __shared__ Seg segs[kSmallWarps][kSmall + 1];
+    __shared__ int source[kSmallWarps][32];
+    const uint32_t all = 0xFFFFFFFFu;
+    const int lane = (int)(threadIdx.x & 31u), w = (int)(threadIdx.x >> 5);
+    const int t = (int)(blockIdx.x * kSmallWarps) + w;
+    if (t >= ntasks)
+        return;
+    const SmallTask T = tasks[t];
+    const int mesh_begin = ranges[T.mesh].x;
+    int prim = lane < T.n ? idx[T.begin + lane] : 0;
+    GBox b = boxes[prim];
+    float c[3];
+    {
+        const float4 c4 = cent[prim];
+        c[0] = c4.x;
+        c[1] = c4.y;
+        c[2] = c4.z;
+    }
+    int sp = 0;
+    if (lane == 0)
+        segs[w][0] = Seg{0, T.n, T.parent, T.side, T.depth};
+    sp = 1;
+    __syncwarp();
+    while (sp > 0) {
+        const Seg g = segs[w][--sp];
+        const int end = g.off + g.n;
+        const bool in = lane >= g.off && lane < end;
+        int node = -1; // this range's inner node, -1: a leaf
+        int cut = g.n / 2, order = lane;
+        if (g.side < 0 || g.n > max_leaf || g.n > 1) {
+            float best = INFINITY, area = 0.0f;
+            int best_k = 0;
+            for (int a = 0; a < 3; a++) {
+                int rank = 0;
+                for (int k = g.off; k < end; k++) {
+                    const float o = __shfl_sync(all, c[a], k);
+                    rank += o < c[a] || (!(c[a] < o) && k < lane) ? 1 : 0;
+                }
+                // NaN centroids compare as equal to everything: keep a permutation
+                const uint32_t seen = __reduce_or_sync(all, in && rank < g.n ? 1u << rank : 0u);
+                if (seen != (g.n == 32 ? all : (1u << g.n) - 1u))
+                    rank = lane - g.off;
+                if (in)
+                    source[w][g.off + rank] = lane;
+                __syncwarp();
+                const int from = in ? source[w][lane] : lane;
+                __syncwarp();
+                float llo[3], lhi[3], rlo[3], rhi[3];
+                for (int j = 0; j < 3; j++) {
+                    llo[j] = rlo[j] = __shfl_sync(all, b.lo[j], from);
+                    lhi[j] = rhi[j] = __shfl_sync(all, b.hi[j], from);
+                }
+                scan_box<true>(llo, lhi, g.off, end);
+                scan_box<false>(rlo, rhi, g.off, end);
+                const int k = lane - g.off + 1;
+                const float cost = cut_cost(llo, lhi, k, rlo, rhi, g.n - k);
+                area = half_area(llo, lhi); // of the whole range on its last lane
+                const bool ok = in && k < g.n && cost < INFINITY;
+                const int low = __reduce_min_sync(all, ok ? f2o(cost) : 0x7FFFFFFF);
+                const uint32_t at = __ballot_sync(all, ok && f2o(cost) == low);
+                if (at && o2f(low) < best) {
+                    best = o2f(low);
+                    best_k = __ffs((int)at) - g.off;
+                    order = from;
+                }
+            }
+            area = __shfl_sync(all, area, end - 1);
+            if (best_k > 0)
+                cut = best_k;
+            const float split_cost = 1.0f + (area > 0.0f ? best / area : (float)g.n);
+            const bool leaf = g.side >= 0 && (g.depth >= max_depth ||
+                                              (g.n <= max_leaf && (best_k == 0 || (float)g.n <= split_cost)));
+            if (!leaf) {
+                if (g.side < 0) {
+                    node = g.parent; // the root's node is given
+                } else {
+                    if (lane == 0)
+                        node = atomicAdd(&counters[kNodes], 1);
+                    node = __shfl_sync(all, node, 0);
+                }
+            }
+        }
+        if (g.side >= 0 && lane == 0) {
+            int *link = reinterpret_cast<int *>(&nodes[g.parent].c);
+            link[g.side] = node >= 0 ? node - T.mesh : T.begin + g.off - mesh_begin;
+            link[2 + g.side] = node >= 0 ? 0 : g.n;
+        }
+        if (node < 0) {
+            if (lane == 0)
+                last[T.begin + end - 1] = 1;
+            continue;
+        }
+        // the range in the order of the best axis, its children's boxes
+        prim = __shfl_sync(all, prim, order);
+        for (int j = 0; j < 3; j++) {
+            b.lo[j] = __shfl_sync(all, b.lo[j], order);
+            b.hi[j] = __shfl_sync(all, b.hi[j], order);
+            c[j] = __shfl_sync(all, c[j], order);
+        }
+        float box[2][6];
+        for (int side = 0; side < 2; side++) {
+            const bool mine = in && (lane < g.off + cut) == (side == 0);
+            for (int j = 0; j < 3; j++) {
+                box[side][j] = o2f(__reduce_min_sync(all, mine ? f2o(b.lo[j]) : f2o(FLT_MAX)));
+                box[side][3 + j] = o2f(__reduce_max_sync(all, mine ? f2o(b.hi[j]) : f2o(-FLT_MAX)));
+            }
+        }
+        if (lane == 0) {
+            BVHNode &nd = nodes[node];
+            nd.lxy = make_float4(box[0][0], box[0][1], box[0][3], box[0][4]);
+            nd.rxy = make_float4(box[1][0], box[1][1], box[1][3], box[1][4]);
+            nd.lrz = make_float4(box[0][2], box[0][5], box[1][2], box[1][5]);
+            segs[w][sp] = Seg{g.off, cut, node, 0, g.depth + 1};
+            segs[w][sp + 1] = Seg{g.off + cut, g.n - cut, node, 1, g.depth + 1};
+            atomicMax(&counters[kMaxDepth], g.depth + 1);
+        }
+        sp += 2;
+        __syncwarp();
+    }
+    if (lane < T.n)
+        idx[T.begin + lane] = prim;
 }
 
 // positions of child tasks get their new task id; leaf positions -1
@@ -487,21 +649,172 @@ __global__ void k_retask(const int *side_in, const int *child_task, int n, int *
     }
 }
 
-struct DevMem {
-    void *p = nullptr;
-    ~DevMem()
-    {
-        if (p)
-            cudaFree(p);
+// One mesh's triangles in leaf order.
+__global__ void k_gather(const vvpt_vertex *verts, const uint32_t *tri, const int *idx, const uint8_t *last, int n,
+                         int begin, TriVerts *out)
+{
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const int prim = idx[begin + k] - begin;
+        float4 v[3];
+        for (int c = 0; c < 3; c++) {
+            const float *p = verts[tri[3 * (size_t)prim + c]].position;
+            v[c] = make_float4(p[0], p[1], p[2], 0.0f);
+        }
+        v[0].w = __int_as_float(prim);
+        v[2].w = __int_as_float((int)last[begin + k]);
+        out[begin + k] = TriVerts{v[0], v[1], v[2]};
     }
-    template <class T>
-    T *as() const
-    {
-        return reinterpret_cast<T *>(p);
+}
+
+__global__ void k_shade_verts(const vvpt_vertex *verts, size_t n, ShadeVertex *out)
+{
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const vvpt_vertex &x = verts[i];
+        ShadeVertex v;
+        v.pos_u = make_float4(x.position[0], x.position[1], x.position[2], x.uv[0]);
+        v.nrm_v = make_float4(x.normal[0], x.normal[1], x.normal[2], x.uv[1]);
+        v.tan_ = make_float4(x.tangent[0], x.tangent[1], x.tangent[2], 0.0f);
+        out[i] = v;
     }
-};
+}
 
 int grid_of(long n) { return (int)std::max<long>(1, std::min<long>((n + 255) / 256, 152L * 32)); }
+
+bool ck(std::string &err, cudaError_t e, const char *what)
+{
+    if (e == cudaSuccess)
+        return true;
+    cudaGetLastError();
+    err = std::string("GPU BVH build: ") + what + ": " + cudaGetErrorString(e);
+    return false;
+}
+
+// The device arrays of a forest build, carved from one allocation.
+struct Forest {
+    int n = 0, meshes = 0, cap = 0; // primitives, trees, tasks of a level
+    DevBuf mem;
+    GBox *boxes = nullptr, *median = nullptr;
+    float4 *cent = nullptr;
+    int *idx[2] = {}, *task_of[2] = {}, *side = nullptr, *cursors = nullptr, *child = nullptr, *counters = nullptr;
+    int *bounds = nullptr;
+    int2 *ranges = nullptr;
+    uint8_t *last = nullptr;
+    BVHNode *nodes = nullptr;
+    Task *tasks[2] = {};
+    SmallTask *small = nullptr;
+    BinStat *bins = nullptr;
+    Split *splits = nullptr;
+    std::vector<int2> ranges_h;
+    int counters_h[kCounters] = {};
+
+    size_t carve(char *base)
+    {
+        size_t off = 0;
+        auto take = [&](auto *&p, size_t count) {
+            p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + off);
+            off += aligned256(count * sizeof(*p));
+        };
+        take(boxes, n);
+        take(cent, n);
+        for (int k = 0; k < 2; k++) {
+            take(idx[k], n);
+            take(task_of[k], n);
+            take(tasks[k], cap);
+        }
+        take(side, n);
+        take(last, n);
+        take(nodes, (size_t)n + meshes); // a tree whose leaves hold >= 1 primitive has < n inner nodes
+        take(small, (size_t)n + meshes);
+        take(bins, (size_t)3 * kBins * cap);
+        take(splits, cap);
+        take(cursors, (size_t)2 * cap);
+        take(child, std::max<size_t>((size_t)2 * cap, meshes));
+        take(median, (size_t)2 * cap);
+        take(bounds, (size_t)kBoundInts * meshes);
+        take(ranges, meshes);
+        take(counters, kCounters);
+        return off;
+    }
+
+    bool begin(const std::vector<int> &counts, cudaStream_t s, std::string &err)
+    {
+        n = 0;
+        meshes = (int)counts.size();
+        ranges_h.clear();
+        for (int c : counts) {
+            ranges_h.push_back(make_int2(n, c));
+            n += c;
+        }
+        cap = n / (kSmall + 1) + 1; // a task has more than kSmall primitives
+        if (!ck(err, mem.alloc(carve(nullptr)), "alloc"))
+            return false;
+        carve(mem.as<char>());
+        const int start[kCounters] = {meshes, 0, 0, 0};
+        if (!ck(err, cudaMemcpyAsync(ranges, ranges_h.data(), sizeof(int2) * meshes, cudaMemcpyHostToDevice, s),
+                "upload") ||
+            !ck(err, cudaMemcpyAsync(counters, start, sizeof(start), cudaMemcpyHostToDevice, s), "upload") ||
+            !ck(err, cudaMemsetAsync(last, 0, n, s), "clear"))
+            return false;
+        k_clear_bounds<<<grid_of((long)kBoundInts * meshes), 256, 0, s>>>(bounds, meshes);
+        return true;
+    }
+
+    void add(int mesh, const vvpt_vertex *verts, const uint32_t *tri, const GBox *given, cudaStream_t s)
+    {
+        const int2 r = ranges_h[mesh];
+        k_primitives<<<std::min(grid_of(r.y), 304), 256, 0, s>>>(verts, tri, given, r.y, r.x, mesh, boxes, cent, idx[0],
+                                                                 side, bounds);
+    }
+
+    // Builds every tree: nodes (roots first), idx[0] the leaf order.
+    bool build(int max_leaf, int max_depth, cudaStream_t s, std::string &err)
+    {
+        auto counters_back = [&] {
+            return ck(err, cudaGetLastError(), "launch") &&
+                   ck(err, cudaMemcpyAsync(counters_h, counters, sizeof(counters_h), cudaMemcpyDeviceToHost, s),
+                      "download") &&
+                   ck(err, cudaStreamSynchronize(s), "sync");
+        };
+        k_roots<<<grid_of(meshes), 256, 0, s>>>(ranges, meshes, bounds, tasks[0], small, counters, child);
+        k_retask<<<grid_of(n), 256, 0, s>>>(side, child, n, task_of[0]);
+        if (!counters_back())
+            return false;
+        int ntasks = counters_h[kNextTasks];
+        for (int level = 0, cur = 0; ntasks > 0; level++, cur ^= 1) {
+            if (level > max_depth + 1) {
+                err = "GPU BVH build: depth bound exceeded";
+                return false;
+            }
+            k_clear_bins<<<grid_of(3L * kBins * ntasks), 256, 0, s>>>(bins, 3 * kBins * ntasks);
+            k_bin<<<(n + 255) / 256, 256, 0, s>>>(boxes, cent, idx[0], task_of[0], n, tasks[cur], bins);
+            k_split<<<(ntasks + 7) / 8, 256, 0, s>>>(tasks[cur], ntasks, bins, splits);
+            cudaMemsetAsync(cursors, 0, 8ull * ntasks, s);
+            k_clear_median<<<grid_of(2L * ntasks), 256, 0, s>>>(median, 2 * ntasks);
+            k_partition<<<grid_of(n), 256, 0, s>>>(boxes, cent, idx[0], task_of[0], n, tasks[cur], splits, cursors,
+                                                   idx[1], side, median);
+            cudaMemsetAsync(counters + kNextTasks, 0, 4, s);
+            k_emit<<<(ntasks + 127) / 128, 128, 0, s>>>(tasks[cur], ntasks, splits, median, nodes, counters,
+                                                        tasks[cur ^ 1], small, child, max_depth, ranges, last);
+            k_retask<<<grid_of(n), 256, 0, s>>>(side, child, n, task_of[1]);
+            std::swap(idx[0], idx[1]);
+            std::swap(task_of[0], task_of[1]);
+            if (!counters_back())
+                return false;
+            ntasks = counters_h[kNextTasks];
+        }
+        const int ns = counters_h[kSmallTasks];
+        if (ns > 0)
+            k_small<<<(ns + kSmallWarps - 1) / kSmallWarps, 32 * kSmallWarps, 0, s>>>(
+                small, ns, idx[0], boxes, cent, nodes, counters, max_leaf, max_depth, ranges, last);
+        if (!counters_back())
+            return false;
+        if (counters_h[kNodes] > n + meshes) {
+            err = "GPU BVH build: node bound exceeded";
+            return false;
+        }
+        return true;
+    }
+};
 
 }  // namespace
 
@@ -511,136 +824,113 @@ bool build_bvh2_gpu(const std::vector<Box3> &boxes, const BVHBuildOptions &opt, 
     const int n = (int)boxes.size();
     if (n <= opt.max_leaf)
         return false; // the host builder handles trivial trees
-    auto ck = [&](cudaError_t e, const char *what) {
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            err = std::string("GPU BVH build: ") + what + ": " + cudaGetErrorString(e);
-            return false;
-        }
-        return true;
-    };
-    const int max_nodes = std::max(1, n); // a binary tree whose leaves hold >= 1 primitive has < n inner nodes
-    DevMem d_boxes, d_cent, d_idx[2], d_task_of[2], d_side, d_tasks[2], d_bins, d_splits, d_cursors, d_nodes,
-        d_counters, d_child, d_median;
-    if (!ck(cudaMalloc(&d_boxes.p, sizeof(GBox) * n), "alloc") || !ck(cudaMalloc(&d_cent.p, sizeof(float4) * n), "alloc") ||
-        !ck(cudaMalloc(&d_idx[0].p, 4ull * n), "alloc") || !ck(cudaMalloc(&d_idx[1].p, 4ull * n), "alloc") ||
-        !ck(cudaMalloc(&d_task_of[0].p, 4ull * n), "alloc") || !ck(cudaMalloc(&d_task_of[1].p, 4ull * n), "alloc") ||
-        !ck(cudaMalloc(&d_side.p, 4ull * n), "alloc") || !ck(cudaMalloc(&d_nodes.p, sizeof(BVHNode) * max_nodes), "alloc") ||
-        !ck(cudaMalloc(&d_counters.p, 16), "alloc"))
-        return false;
     static_assert(sizeof(GBox) == sizeof(Box3), "box layout");
-    if (!ck(cudaMemcpyAsync(d_boxes.p, boxes.data(), sizeof(GBox) * n, cudaMemcpyHostToDevice, s), "upload"))
+    Forest f;
+    DevBuf given;
+    if (!f.begin({n}, s, err) || !ck(err, given.alloc(sizeof(GBox) * n), "alloc") ||
+        !ck(err, cudaMemcpyAsync(given.ptr, boxes.data(), sizeof(GBox) * n, cudaMemcpyHostToDevice, s), "upload"))
         return false;
-    k_init<<<grid_of(n), 256, 0, s>>>(d_boxes.as<GBox>(), n, d_idx[0].as<int>(), d_task_of[0].as<int>(),
-                                      d_cent.as<float4>());
-    // root task: centroid bounds on the host (one pass over the boxes)
-    Task root{};
-    root.begin = 0;
-    root.end = n;
-    root.node = 0;
-    root.depth = 0;
-    for (int j = 0; j < 3; j++) {
-        root.cmin[j] = FLT_MAX;
-        root.cmax[j] = -FLT_MAX;
-    }
-    for (const Box3 &b : boxes)
-        for (int j = 0; j < 3; j++) {
-            const float c = 0.5f * (b.lo[j] + b.hi[j]);
-            root.cmin[j] = std::min(root.cmin[j], c);
-            root.cmax[j] = std::max(root.cmax[j], c);
-        }
-    int ntasks = 1, cap = 1;
-    auto ensure_tasks = [&](int need) {
-        if (need <= cap && d_tasks[0].p)
-            return true;
-        cap = std::max(need, cap * 2);
-        for (auto *m : {&d_tasks[0], &d_tasks[1]}) {
-            if (m->p)
-                cudaFree(m->p);
-            m->p = nullptr;
-        }
-        for (auto *m : {&d_bins, &d_splits, &d_cursors, &d_child, &d_median}) {
-            if (m->p)
-                cudaFree(m->p);
-            m->p = nullptr;
-        }
-        return ck(cudaMalloc(&d_tasks[0].p, sizeof(Task) * cap), "alloc") &&
-               ck(cudaMalloc(&d_tasks[1].p, sizeof(Task) * 2 * cap), "alloc") &&
-               ck(cudaMalloc(&d_bins.p, sizeof(BinStat) * 3 * kBins * (size_t)cap), "alloc") &&
-               ck(cudaMalloc(&d_splits.p, sizeof(Split) * cap), "alloc") &&
-               ck(cudaMalloc(&d_cursors.p, 8ull * cap), "alloc") && ck(cudaMalloc(&d_child.p, 8ull * cap), "alloc") &&
-               ck(cudaMalloc(&d_median.p, sizeof(GBox) * 2 * cap), "alloc");
-    };
-    if (!ensure_tasks(1024))
+    f.add(0, nullptr, nullptr, given.as<GBox>(), s);
+    if (!f.build(opt.max_leaf, opt.max_depth, s, err))
         return false;
-    if (!ck(cudaMemcpyAsync(d_tasks[0].p, &root, sizeof(Task), cudaMemcpyHostToDevice, s), "upload"))
-        return false;
-    int counters_h[4] = {1, 0, 0, 0};
-    if (!ck(cudaMemcpyAsync(d_counters.p, counters_h, 16, cudaMemcpyHostToDevice, s), "upload"))
-        return false;
-    int cur = 0;
-    int depth = 0;
-    for (int level = 0; ntasks > 0; level++) {
-        if (level > opt.max_depth + 1) {
-            err = "GPU BVH build: depth bound exceeded";
-            return false;
-        }
-        // the next level holds at most 2 tasks per task
-        if (2 * ntasks > cap) {
-            // grow while keeping the current tasks
-            std::vector<Task> keep(ntasks);
-            if (!ck(cudaMemcpyAsync(keep.data(), d_tasks[cur].p, sizeof(Task) * ntasks, cudaMemcpyDeviceToHost, s),
-                    "download") ||
-                !ck(cudaStreamSynchronize(s), "sync"))
-                return false;
-            if (!ensure_tasks(2 * ntasks))
-                return false;
-            cur = 0;
-            if (!ck(cudaMemcpyAsync(d_tasks[0].p, keep.data(), sizeof(Task) * ntasks, cudaMemcpyHostToDevice, s),
-                    "upload"))
-                return false;
-        }
-        Task *tasks = d_tasks[cur].as<Task>();
-        Task *next = d_tasks[cur ^ 1].as<Task>();
-        k_clear_bins<<<grid_of(3L * kBins * ntasks), 256, 0, s>>>(d_bins.as<BinStat>(), 3 * kBins * ntasks);
-        k_bin<<<(n + 255) / 256, 256, 0, s>>>(d_boxes.as<GBox>(), d_cent.as<float4>(), d_idx[0].as<int>(),
-                                              d_task_of[0].as<int>(), n, tasks, d_bins.as<BinStat>());
-        k_split<<<(ntasks + 127) / 128, 128, 0, s>>>(tasks, ntasks, d_bins.as<BinStat>(), d_splits.as<Split>());
-        cudaMemsetAsync(d_cursors.p, 0, 8ull * ntasks, s);
-        k_clear_median<<<grid_of(2L * ntasks), 256, 0, s>>>(d_median.as<GBox>(), 2 * ntasks);
-        k_partition<<<grid_of(n), 256, 0, s>>>(d_boxes.as<GBox>(), d_cent.as<float4>(), d_idx[0].as<int>(),
-                                               d_task_of[0].as<int>(), n, tasks, d_splits.as<Split>(),
-                                               d_cursors.as<int>(), d_idx[1].as<int>(), d_side.as<int>(),
-                                               d_median.as<GBox>());
-        cudaMemsetAsync(d_counters.as<int>() + 1, 0, 4, s);
-        k_emit<<<(ntasks + 127) / 128, 128, 0, s>>>(tasks, ntasks, d_splits.as<Split>(), d_median.as<GBox>(),
-                                                    d_nodes.as<BVHNode>(), d_counters.as<int>(), next,
-                                                    d_child.as<int>(), opt.max_leaf, opt.max_depth,
-                                                    d_idx[1].as<int>(), d_boxes.as<GBox>(), d_cent.as<float4>());
-        k_retask<<<grid_of(n), 256, 0, s>>>(d_side.as<int>(), d_child.as<int>(), n, d_task_of[1].as<int>());
-        std::swap(d_idx[0].p, d_idx[1].p);
-        std::swap(d_task_of[0].p, d_task_of[1].p);
-        if (!ck(cudaGetLastError(), "launch") ||
-            !ck(cudaMemcpyAsync(counters_h, d_counters.p, 16, cudaMemcpyDeviceToHost, s), "download") ||
-            !ck(cudaStreamSynchronize(s), "sync"))
-            return false;
-        ntasks = counters_h[1];
-        depth = std::max(depth, counters_h[2]);
-        cur ^= 1;
-        if (counters_h[0] > max_nodes) {
-            err = "GPU BVH build: node bound exceeded";
-            return false;
-        }
-    }
-    const int nnodes = counters_h[0];
+    const int nnodes = f.counters_h[kNodes];
     out.nodes.resize(nnodes);
     out.order.resize(n);
-    out.depth = depth;
-    if (!ck(cudaMemcpyAsync(out.nodes.data(), d_nodes.p, sizeof(BVHNode) * nnodes, cudaMemcpyDeviceToHost, s),
-            "download") ||
-        !ck(cudaMemcpyAsync(out.order.data(), d_idx[0].p, 4ull * n, cudaMemcpyDeviceToHost, s), "download") ||
-        !ck(cudaStreamSynchronize(s), "sync"))
+    out.depth = f.counters_h[kMaxDepth];
+    return ck(err, cudaMemcpyAsync(out.nodes.data(), f.nodes, sizeof(BVHNode) * nnodes, cudaMemcpyDeviceToHost, s),
+              "download") &&
+           ck(err, cudaMemcpyAsync(out.order.data(), f.idx[0], 4ull * n, cudaMemcpyDeviceToHost, s), "download") &&
+           ck(err, cudaStreamSynchronize(s), "sync");
+}
+
+// The device part of a scene. Meshes are taken in groups of at most
+// kGroupTriangles triangles (or one mesh), which bounds the working memory to
+// a few gigabytes however large the scene is.
+bool build_meshes_gpu(const vvpt_scene_desc *desc, const std::vector<uint32_t> &meshes, const BVHBuildOptions &opt,
+                      cudaStream_t s, DeviceMeshes &out, std::string &err)
+{
+    constexpr uint64_t kGroupTriangles = 16u << 20;
+    out.placed.assign(meshes.size(), DeviceMeshes::Placed{});
+    uint64_t nt = 0, nv = 0;
+    for (size_t k = 0; k < meshes.size(); k++) {
+        const vvpt_mesh_desc &md = desc->meshes[meshes[k]];
+        out.placed[k].tri_offset = (uint32_t)nt;
+        out.placed[k].vertex_offset = (uint32_t)nv;
+        nt += md.num_triangles;
+        nv += md.num_vertices;
+    }
+    out.num_tris = (uint32_t)nt;
+    out.num_verts = (uint32_t)nv;
+    if (!ck(err, out.tris.alloc(sizeof(TriVerts) * nt), "alloc") ||
+        !ck(err, out.verts.alloc(sizeof(ShadeVertex) * nv), "alloc") ||
+        !ck(err, out.indices.alloc(12ull * nt), "alloc"))
         return false;
+    for (size_t first = 0; first < meshes.size();) {
+        size_t end = first;
+        std::vector<int> counts;
+        uint64_t tris = 0, verts = 0;
+        while (end < meshes.size()) {
+            const vvpt_mesh_desc &md = desc->meshes[meshes[end]];
+            if (end > first && tris + md.num_triangles > kGroupTriangles)
+                break;
+            tris += md.num_triangles;
+            verts += md.num_vertices;
+            counts.push_back((int)md.num_triangles);
+            end++;
+        }
+        Forest f;
+        DevBuf raw;
+        if (!f.begin(counts, s, err) || !ck(err, raw.alloc(sizeof(vvpt_vertex) * verts), "alloc"))
+            return false;
+        vvpt_vertex *rv = raw.as<vvpt_vertex>();
+        const uint32_t t0 = out.placed[first].tri_offset, v0 = out.placed[first].vertex_offset;
+        auto mesh_verts = [&](size_t k) { return rv + (out.placed[k].vertex_offset - v0); };
+        auto mesh_tris = [&](size_t k) { return out.indices.as<uint32_t>() + 3ull * out.placed[k].tri_offset; };
+        for (size_t k = first; k < end; k++) {
+            const vvpt_mesh_desc &md = desc->meshes[meshes[k]];
+            if (!ck(err, cudaMemcpyAsync(mesh_verts(k), md.vertices, sizeof(vvpt_vertex) * (size_t)md.num_vertices,
+                                         cudaMemcpyHostToDevice, s), "upload") ||
+                !ck(err, cudaMemcpyAsync(mesh_tris(k), md.indices, 12ull * md.num_triangles, cudaMemcpyHostToDevice, s),
+                    "upload"))
+                return false;
+            f.add((int)(k - first), mesh_verts(k), mesh_tris(k), nullptr, s);
+        }
+        k_shade_verts<<<grid_of((long)verts), 256, 0, s>>>(rv, verts, out.verts.as<ShadeVertex>() + v0);
+        if (!f.build(opt.max_leaf, opt.max_depth, s, err))
+            return false;
+        for (size_t k = first; k < end; k++) {
+            const int2 r = f.ranges_h[k - first];
+            k_gather<<<grid_of(r.y), 256, 0, s>>>(mesh_verts(k), mesh_tris(k), f.idx[0], f.last, r.y, r.x,
+                                                  out.tris.as<TriVerts>() + t0);
+        }
+        const int nnodes = f.counters_h[kNodes];
+        out.nodes.emplace_back(new DevBuf());
+        DevBuf &nb = *out.nodes.back();
+        std::vector<int> bounds((size_t)kBoundInts * f.meshes);
+        if (!ck(err, nb.alloc(sizeof(BVHNode) * (size_t)nnodes), "alloc") ||
+            !ck(err, cudaMemcpyAsync(nb.ptr, f.nodes, sizeof(BVHNode) * (size_t)nnodes, cudaMemcpyDeviceToDevice, s),
+                "copy") ||
+            !ck(err, cudaMemcpyAsync(bounds.data(), f.bounds, 4 * bounds.size(), cudaMemcpyDeviceToHost, s), "download") ||
+            !ck(err, cudaStreamSynchronize(s), "sync"))
+            return false;
+        auto back = [](int i) {
+            const int b = i >= 0 ? i : i ^ 0x7FFFFFFF;
+            float x;
+            std::memcpy(&x, &b, 4);
+            return x;
+        };
+        for (size_t k = first; k < end; k++) {
+            DeviceMeshes::Placed &p = out.placed[k];
+            p.node_offset = out.num_nodes + (uint32_t)(k - first);
+            for (int a = 0; a < 3; a++) {
+                p.root.lo[a] = back(bounds[kBoundInts * (k - first) + 6 + a]);
+                p.root.hi[a] = back(bounds[kBoundInts * (k - first) + 9 + a]);
+            }
+        }
+        out.num_nodes += (uint32_t)nnodes;
+        out.depth = std::max(out.depth, f.counters_h[kMaxDepth]);
+        first = end;
+    }
     return true;
 }
 

@@ -7,10 +7,12 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <vector>
 
 #include <cuda_runtime.h>
 
 #include "../../include/vvpt.h"
+#include "bvh_build.h"
 #include "scene_gpu.h"
 #include "wavefront.cuh"
 
@@ -57,6 +59,23 @@ struct DevBuf {
 };
 
 struct Engine; // engine.cu
+
+// Meshes built and packed on the device (bvh_gpu.cu): the first part of the
+// scene's node, triangle, vertex and index arrays. Each mesh's links are
+// relative to its root node.
+struct DeviceMeshes {
+    struct Placed {
+        uint32_t node_offset = 0, tri_offset = 0, vertex_offset = 0; // its index triples start at tri_offset too
+        Box3 root{};
+    };
+    std::vector<Placed> placed;                 // per mesh, in the order given
+    std::vector<std::unique_ptr<DevBuf>> nodes; // in order, num_nodes in all
+    DevBuf tris, verts, indices;
+    uint32_t num_nodes = 0, num_tris = 0, num_verts = 0;
+    int depth = 0;
+};
+bool build_meshes_gpu(const vvpt_scene_desc *desc, const std::vector<uint32_t> &meshes, const BVHBuildOptions &opt,
+                      cudaStream_t stream, DeviceMeshes &out, std::string &err);
 
 }  // namespace vvpt
 

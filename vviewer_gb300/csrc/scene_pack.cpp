@@ -149,15 +149,15 @@ float build_env_distribution(const float *rgba, uint32_t w, uint32_t h, std::vec
 }
 
 vvpt_status pack_scene(const vvpt_scene_desc *desc, PackedScene &out, std::string &err, unsigned threads,
-                       const BlasBuilder &large_builder, uint32_t large_min, bool builder_for_all)
+                       OutsideMeshes *outside)
 {
     // a tree for the TLAS or the baked small instances: on the given builder
     // when it takes every tree, else (or when it declines) on the host
     auto build_other = [&](const std::vector<Box3> &boxes, const BVHBuildOptions &opt,
                            BVHBuildResult &res) -> bool {
-        if (builder_for_all && large_builder) {
+        if (outside && outside->other_trees) {
             std::string e;
-            if (large_builder(boxes, opt, res, e))
+            if (outside->tree(boxes, opt, res, e))
                 return true;
             if (!e.empty()) {
                 err = e;
@@ -244,15 +244,41 @@ vvpt_status pack_scene(const vvpt_scene_desc *desc, PackedScene &out, std::strin
     std::sort(order.begin(), order.end(),
               [&](uint32_t a, uint32_t b) { return desc->meshes[a].num_triangles > desc->meshes[b].num_triangles; });
     std::atomic<uint32_t> next{0};
-    std::mutex large_mu;
-    std::string large_err; // a failed large build falls back to the host builder
+    const BVHBuildOptions blas_opt;
+    std::vector<uint32_t> away; // meshes built outside
+    std::vector<MeshPlace> places;
+    std::vector<uint8_t> is_away(nm, 0);
+#if !VVPT_BLAS_WIDE
+    if (outside)
+        for (uint32_t m = 0; m < nm; m++)
+            if (desc->meshes[m].num_triangles >= outside->min_triangles &&
+                desc->meshes[m].num_triangles > (uint32_t)blas_opt.max_leaf) {
+                is_away[m] = 1;
+                away.push_back(m);
+            }
+#endif
     const unsigned hw = threads ? threads : std::max(1u, std::thread::hardware_concurrency());
+#if VVPT_BLAS_WIDE
+    // the wide layout is collapsed on the host: a large mesh's tree comes back
+    std::mutex outside_mu;
+    std::string outside_err;
+    auto outside_tree = [&](const std::vector<Box3> &boxes, const BVHBuildOptions &opt, BVHBuildResult &res) {
+        std::lock_guard<std::mutex> lk(outside_mu);
+        std::string e;
+        const bool built = outside->tree(boxes, opt, res, e);
+        if (!built && !e.empty() && outside_err.empty())
+            outside_err = e;
+        return built;
+    };
+#endif
     auto worker = [&]() {
         for (;;) {
             uint32_t k = next.fetch_add(1);
             if (k >= nm)
                 break;
             uint32_t m = order[k];
+            if (is_away[m])
+                continue;
             const vvpt_mesh_desc &md = desc->meshes[m];
             std::vector<Box3> boxes(md.num_triangles);
             for (uint32_t t = 0; t < md.num_triangles; t++) {
@@ -269,17 +295,11 @@ vvpt_status pack_scene(const vvpt_scene_desc *desc, PackedScene &out, std::strin
                     }
                 }
             }
-            BVHBuildOptions opt;
+            BVHBuildOptions opt = blas_opt;
             opt.threads = (k == 0 && md.num_triangles > 100000) ? (int)hw : 1;
-            bool built = false;
-            if (large_builder && md.num_triangles >= large_min) {
-                std::lock_guard<std::mutex> lk(large_mu);
-                std::string e;
-                built = large_builder(boxes, opt, builds[m].bvh, e);
-                if (!built && !e.empty() && large_err.empty())
-                    large_err = e;
-            }
-            if (!built)
+#if VVPT_BLAS_WIDE
+            if (!(outside && md.num_triangles >= outside->min_triangles && outside_tree(boxes, opt, builds[m].bvh)))
+#endif
                 builds[m].bvh = build_bvh2(boxes, opt);
 #if VVPT_BLAS_WIDE
             builds[m].wide = collapse_to_wide(builds[m].bvh, boxes);
@@ -300,15 +320,25 @@ vvpt_status pack_scene(const vvpt_scene_desc *desc, PackedScene &out, std::strin
     };
     {
         std::vector<std::thread> th;
-        unsigned nth = std::min<unsigned>(hw, std::max<uint32_t>(nm, 1));
+        unsigned nth = std::min<unsigned>(hw, std::max<uint32_t>(nm - (uint32_t)away.size(), 1));
         for (unsigned i = 0; i < nth; i++)
             th.emplace_back(worker);
+        bool ok = true;
+        std::string e;
+        if (!away.empty())
+            ok = outside->build(away, places, e);
         for (auto &t : th)
             t.join();
+        if (!ok)
+            return fail(err, VVPT_ERR_DEVICE, e);
     }
-
-    if (!large_err.empty())
-        return fail(err, VVPT_ERR_DEVICE, large_err);
+#if VVPT_BLAS_WIDE
+    if (!outside_err.empty())
+        return fail(err, VVPT_ERR_DEVICE, outside_err);
+#endif
+    // elements in front of the arrays packed here
+    const uint32_t nodes0 = away.empty() ? 0u : outside->nodes, tris0 = away.empty() ? 0u : outside->tris,
+                   verts0 = away.empty() ? 0u : outside->verts;
 
     std::vector<MeshInfo> minfo(nm);
     std::vector<BVHNode> &nodes = out.nodes;
@@ -318,6 +348,8 @@ vvpt_status pack_scene(const vvpt_scene_desc *desc, PackedScene &out, std::strin
     std::vector<uint32_t> &indices = out.indices;
     size_t total_nodes = 0, total_tris = 0, total_verts = 0;
     for (uint32_t m = 0; m < nm; m++) {
+        if (is_away[m])
+            continue;
         total_nodes += builds[m].bvh.nodes.size() + builds[m].wide.nodes.size();
         total_tris += desc->meshes[m].num_triangles;
         total_verts += desc->meshes[m].num_vertices;
@@ -326,17 +358,33 @@ vvpt_status pack_scene(const vvpt_scene_desc *desc, PackedScene &out, std::strin
     wnodes.reserve(total_nodes);
     nodes.reserve(2 * desc->num_instances + 2);
 #else
-    nodes.reserve(total_nodes + 2 * desc->num_instances + 2);
+    // the small instances' BLAS and the TLAS follow
+    nodes.reserve(total_nodes + (2 + kFlattenMaxTriangles) * (size_t)desc->num_instances + 2);
 #endif
     tris.reserve(total_tris);
     verts.reserve(total_verts);
     indices.reserve(3 * total_tris);
+    for (size_t k = 0; k < away.size(); k++) {
+        MeshInfo &mi = minfo[away[k]];
+        mi.node_offset = places[k].node_offset;
+        mi.tri_offset = places[k].tri_offset;
+        mi.vertex_offset = places[k].vertex_offset;
+        mi.index_offset = places[k].index_offset;
+        mi.num_triangles = desc->meshes[away[k]].num_triangles;
+        for (int a = 0; a < 3; a++) {
+            builds[away[k]].root.lo[a] = places[k].lo[a];
+            builds[away[k]].root.hi[a] = places[k].hi[a];
+        }
+        builds[away[k]].bvh.depth = outside->depth;
+    }
     for (uint32_t m = 0; m < nm; m++) {
+        if (is_away[m])
+            continue;
         const vvpt_mesh_desc &md = desc->meshes[m];
         MeshInfo &mi = minfo[m];
-        mi.tri_offset = (uint32_t)tris.size();
-        mi.vertex_offset = (uint32_t)verts.size();
-        mi.index_offset = (uint32_t)indices.size();
+        mi.tri_offset = tris0 + (uint32_t)tris.size();
+        mi.vertex_offset = verts0 + (uint32_t)verts.size();
+        mi.index_offset = 3u * tris0 + (uint32_t)indices.size();
         mi.num_triangles = md.num_triangles;
 #if VVPT_BLAS_WIDE
         mi.node_offset = (uint32_t)wnodes.size();
@@ -344,7 +392,7 @@ vvpt_status pack_scene(const vvpt_scene_desc *desc, PackedScene &out, std::strin
         wnodes.insert(wnodes.end(), builds[m].wide.nodes.begin(), builds[m].wide.nodes.end());
         const std::vector<uint32_t> &leaf_order = builds[m].wide.order;
 #else
-        mi.node_offset = (uint32_t)nodes.size();
+        mi.node_offset = nodes0 + (uint32_t)nodes.size();
         mi.num_nodes = (uint32_t)builds[m].bvh.nodes.size();
         nodes.insert(nodes.end(), builds[m].bvh.nodes.begin(), builds[m].bvh.nodes.end());
         const std::vector<uint32_t> &leaf_order = builds[m].bvh.order;
@@ -362,7 +410,7 @@ vvpt_status pack_scene(const vvpt_scene_desc *desc, PackedScene &out, std::strin
             tv.v2 = make_float4(p2[0], p2[1], p2[2], 0.0f);
             tris.push_back(tv);
         }
-        for_leaf_ends(builds[m].bvh.nodes, [&](size_t k) { tris[mi.tri_offset + k].v2.w = last_mark(); });
+        for_leaf_ends(builds[m].bvh.nodes, [&](size_t k) { tris[mi.tri_offset - tris0 + k].v2.w = last_mark(); });
         for (uint32_t v = 0; v < md.num_vertices; v++) {
             const vvpt_vertex &x = md.vertices[v];
             ShadeVertex sv;
@@ -561,7 +609,7 @@ vvpt_status pack_scene(const vvpt_scene_desc *desc, PackedScene &out, std::strin
         const float ident[16] = {1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1};
         affine_rows(ident, syn.o2w);
         affine_rows(ident, syn.w2o);
-        syn.tri_offset = (uint32_t)tris.size();
+        syn.tri_offset = tris0 + (uint32_t)tris.size();
         syn.num_triangles = (uint32_t)ft.size();
         syn.front_volume = syn.back_volume = -1;
 #if VVPT_BLAS_WIDE
@@ -570,14 +618,14 @@ vvpt_status pack_scene(const vvpt_scene_desc *desc, PackedScene &out, std::strin
         wnodes.insert(wnodes.end(), fw.nodes.begin(), fw.nodes.end());
         const std::vector<uint32_t> &forder = fw.order;
 #else
-        syn.node_offset = (uint32_t)nodes.size();
+        syn.node_offset = nodes0 + (uint32_t)nodes.size();
         nodes.insert(nodes.end(), fbvh.nodes.begin(), fbvh.nodes.end());
         const std::vector<uint32_t> &forder = fbvh.order;
 #endif
         for (uint32_t k = 0; k < (uint32_t)ft.size(); k++)
             tris.push_back(ft[forder[k]]);
 #if !VVPT_BLAS_WIDE
-        for_leaf_ends(fbvh.nodes, [&](size_t k) { tris[syn.tri_offset + k].v2.w = last_mark(); });
+        for_leaf_ends(fbvh.nodes, [&](size_t k) { tris[syn.tri_offset - tris0 + k].v2.w = last_mark(); });
 #endif
         Box3 w;
         for (int a = 0; a < 3; a++) {
@@ -645,7 +693,7 @@ vvpt_status pack_scene(const vvpt_scene_desc *desc, PackedScene &out, std::strin
     BVHBuildResult tlas;
     if (!build_other(tlas_boxes, tlas_opt, tlas))
         return VVPT_ERR_DEVICE;
-    out.tlas_root = (uint32_t)nodes.size();
+    out.tlas_root = nodes0 + (uint32_t)nodes.size();
     nodes.insert(nodes.end(), tlas.nodes.begin(), tlas.nodes.end());
     std::vector<uint32_t> &tlas_order = out.tlas_order;
     tlas_order.resize(tlas.order.size());

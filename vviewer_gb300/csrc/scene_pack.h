@@ -41,21 +41,42 @@ struct PackedScene {
     std::vector<float4> emit_boxes;   // SceneView::emit_boxes (lo, hi pairs)
 };
 
-// Builder for large BLAS (e.g. the GPU builder): fills `out` and returns true,
-// or returns false to leave the mesh to the host builder (err set on failure).
 struct Box3;
 struct BVHBuildOptions;
 struct BVHBuildResult;
+// Builder for a tree over given boxes (e.g. the GPU builder): fills `out` and
+// returns true, or returns false to leave it to the host builder (err set on
+// failure).
 using BlasBuilder = std::function<bool(const std::vector<Box3> &, const BVHBuildOptions &, BVHBuildResult &,
                                        std::string &)>;
 
+// Meshes that are built and packed elsewhere (on the GPU): their nodes,
+// triangles, vertices and indices precede those of PackedScene's arrays, and
+// every offset in the packed scene counts from the first of them.
+struct MeshPlace {
+    uint32_t node_offset, tri_offset, vertex_offset, index_offset;
+    float lo[3], hi[3]; // box of its triangles
+};
+struct OutsideMeshes {
+    // Meshes of at least so many (and more than a leaf's) triangles. All of
+    // them are one set of launches outside, of about a millisecond; a host
+    // thread takes that long for 500 triangles (uploads with one such mesh:
+    // 320 triangles 0.95 ms on the host against 1.03 outside, 1280 2.5 / 1.2,
+    // 50,000 84 / 2.3).
+    uint32_t min_triangles = 512;
+    bool other_trees = false;       // the baked small instances' BLAS and the TLAS go to `tree` too
+    BlasBuilder tree;
+    // builds the given meshes; false with err set on failure
+    std::function<bool(const std::vector<uint32_t> &meshes, std::vector<MeshPlace> &places, std::string &err)> build;
+    uint32_t nodes = 0, tris = 0, verts = 0; // set by build: elements in front of the packed arrays
+    int depth = 0;
+};
+
 // Returns VVPT_OK or an error status with `err` set. `threads` = 0 uses every
-// hardware thread for the BLAS builds. Meshes of at least `large_min`
-// triangles go to `large_builder` when one is given (one at a time); with
-// `builder_for_all` the baked small instances' BLAS and the TLAS go to it too.
+// hardware thread for the BLAS builds. The meshes that `outside` asks for are
+// left to it; with the wide BLAS layout all are built here.
 vvpt_status pack_scene(const vvpt_scene_desc *desc, PackedScene &out, std::string &err, unsigned threads = 0,
-                       const BlasBuilder &large_builder = BlasBuilder(), uint32_t large_min = 65536,
-                       bool builder_for_all = false);
+                       OutsideMeshes *outside = nullptr);
 
 // Piecewise-constant sampling tables of an RGBA32F equirect environment
 // (PackedScene::env_dist layout): function = luminance dilated over the 3x3
