@@ -841,32 +841,23 @@ VVPT_API vvpt_status vvpt_trace_closest(vvpt_ctx *ctx, vvpt_scene *scene, const 
         VV_CUDA(cudaMemcpyAsync(ctx->rays.ptr, rays, (size_t)n * 32, cudaMemcpyHostToDevice, vv_stream(ctx)), "upload rays");
         d_rays = ctx->rays.as<float4>();
     }
-    VV_CUDA(ctx->hits_tuv.reserve((size_t)n * 16), "cudaMalloc hits");
-    VV_CUDA(ctx->hits_ids.reserve((size_t)n * 8), "cudaMalloc hits");
+    // hits of a caller on the host come back in one copy, straight into its array
+    vvpt_hit *d_hits = hits;
+    if (!on_device) {
+        VV_CUDA(ctx->hits.reserve((size_t)n * sizeof(vvpt_hit)), "cudaMalloc hits");
+        d_hits = ctx->hits.as<vvpt_hit>();
+    }
     VV_CUDA(ctx->err_word.reserve(16), "cudaMalloc err");
-    VV_CUDA(cudaMemsetAsync(ctx->err_word.ptr, 0, 4, vv_stream(ctx)), "clear err");
-    launch_trace_closest(scene->view, d_rays, n, ctx->hits_tuv.as<float4>(), ctx->hits_ids.as<uint32_t>(),
-                         ctx->err_word.as<uint32_t>(), vv_stream(ctx));
+    VV_CUDA(cudaMemsetAsync(ctx->err_word.ptr, 0, 8, vv_stream(ctx)), "clear err");
+    launch_trace_closest(scene->view, d_rays, n, d_hits, ctx->err_word.as<uint32_t>(), ctx->num_sms,
+                         vv_stream(ctx));
     VV_CUDA(cudaGetLastError(), "launch trace");
-    std::vector<float4> tuv(n);
-    std::vector<uint32_t> ids(2 * (size_t)n);
     uint32_t err = 0;
-    VV_CUDA(cudaMemcpyAsync(tuv.data(), ctx->hits_tuv.ptr, (size_t)n * 16, cudaMemcpyDeviceToHost, vv_stream(ctx)), "d2h");
-    VV_CUDA(cudaMemcpyAsync(ids.data(), ctx->hits_ids.ptr, (size_t)n * 8, cudaMemcpyDeviceToHost, vv_stream(ctx)), "d2h");
+    if (!on_device)
+        VV_CUDA(cudaMemcpyAsync(hits, d_hits, (size_t)n * sizeof(vvpt_hit), cudaMemcpyDeviceToHost, vv_stream(ctx)),
+                "d2h");
     VV_CUDA(cudaMemcpyAsync(&err, ctx->err_word.ptr, 4, cudaMemcpyDeviceToHost, vv_stream(ctx)), "d2h");
     VV_CUDA(cudaStreamSynchronize(vv_stream(ctx)), "trace");
-    std::vector<vvpt_hit> hv(n);
-    for (uint32_t i = 0; i < n; i++) {
-        hv[i].t = tuv[i].x;
-        hv[i].u = tuv[i].y;
-        hv[i].v = tuv[i].z;
-        hv[i].instance = ids[2 * i];
-        hv[i].primitive = ids[2 * i + 1];
-    }
-    if (on_device)
-        VV_CUDA(cudaMemcpy(hits, hv.data(), (size_t)n * sizeof(vvpt_hit), cudaMemcpyHostToDevice), "store hits");
-    else
-        std::memcpy(hits, hv.data(), (size_t)n * sizeof(vvpt_hit));
     if (err)
         return fail(ctx, VVPT_ERR_DEVICE, "traversal status word set: " + std::to_string(err));
     return VVPT_OK;

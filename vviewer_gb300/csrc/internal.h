@@ -100,7 +100,7 @@ struct vvpt_ctx {
     // render buffers (grow-only, reused across renders)
     vvpt::DevBuf state, queues, results, params, outputs;
     uint32_t *counters_pinned = nullptr;
-    vvpt::DevBuf rays, hits_tuv, hits_ids, err_word;
+    vvpt::DevBuf rays, hits, err_word;
     cudaStream_t user_stream = nullptr;
     vvpt_kernel_profile profile{};
     // job engine (vvpt_submit ...), created on first use

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "../../include/vvpt.h"
 #include "scene_gpu.h"
 
 namespace vvpt {
@@ -148,8 +149,9 @@ void launch_init_slots(const Queues &q, const PathState &ps, const JobTable &jt,
 // the range arrays were written.
 void launch_admit(const Queues &q, const JobTable &jt, unsigned long long total_items, uint32_t num_ranges,
                   cudaStream_t stream);
-void launch_trace_closest(const SceneView &s, const float4 *rays, uint32_t n, float4 *hits_tuv, uint32_t *hits_ids,
-                          uint32_t *err, cudaStream_t stream);
+// `status`: error bits and a hand-out counter, both zero before the launch.
+void launch_trace_closest(const SceneView &s, const float4 *rays, uint32_t n, vvpt_hit *hits, uint32_t *status,
+                          int num_sms, cudaStream_t stream);
 // One wavefront kernel, launched on its own (profiling mode); an iteration
 // launches all of them in this order.
 enum KernelId {
