@@ -101,7 +101,7 @@ struct vvpt_denoiser {
     // shape-dependent buffers
     int n = 0, h = 0, w = 0;
     bool with_grads = false;
-    DevBuf acts, gacts, out_f32, target3, dout, loss, err;
+    DevBuf acts, gacts, out_f32, dout, loss, err;
     bool mma_sync = false; // warp-level mma.sync convolutions instead of tcgen05
     vvdn::ConvKernels conv_kind = vvdn::kConvAuto;
     // tensors: x[l], a[l], e[l]; u[l], b[l], d[l] (l < 4)
@@ -148,7 +148,6 @@ vvpt_status ensure_shape(vvpt_denoiser *dn, int n, int h, int w, bool with_grads
     VV_CUDA(dn->out_f32.reserve(p0 * kOutCh * sizeof(float)), "cudaMalloc denoiser output");
     if (dn->with_grads) {
         VV_CUDA(dn->gacts.reserve(off * sizeof(bf16)), "cudaMalloc denoiser gradients");
-        VV_CUDA(dn->target3.reserve(p0 * 3 * sizeof(float)), "cudaMalloc denoiser target");
         VV_CUDA(dn->dout.reserve(p0 * kOutCh * sizeof(bf16)), "cudaMalloc denoiser output gradient");
         VV_CUDA(dn->loss.reserve(sizeof(float)), "cudaMalloc loss");
     }
@@ -162,10 +161,18 @@ void refresh_weights(vvpt_denoiser *dn, cudaStream_t s)
 {
     if (!dn->weights_dirty)
         return;
-    for (const Layer &L : dn->layers) {
-        vvdn::to_bf16(dn->params.as<float>() + L.w_off, dn->w16.as<bf16>() + L.w16_off, (size_t)L.cout * 9 * L.cin, s);
-        vvdn::transform_weights(dn->w16.as<bf16>() + L.w16_off, dn->wt16.as<bf16>() + L.w16_off, L.cout, L.cin, s);
+    vvdn::WeightTable t{};
+    t.layers = (int)dn->layers.size();
+    static_assert(kLayers <= vvdn::kMaxLayers, "layer table");
+    for (int l = 0; l < t.layers; l++) {
+        const Layer &L = dn->layers[l];
+        t.start[l] = (unsigned)L.w16_off;
+        t.param[l] = (unsigned)L.w_off;
+        t.cin[l] = (unsigned short)L.cin;
+        t.cout[l] = (unsigned short)L.cout;
     }
+    t.start[t.layers] = (unsigned)dn->nw16;
+    vvdn::prepare_weights(dn->params.as<float>(), t, dn->w16.as<bf16>(), dn->wt16.as<bf16>(), s);
     dn->weights_dirty = false;
 }
 
@@ -345,10 +352,8 @@ vvpt_status loss_and_grads(vvpt_denoiser *dn, const vvpt_denoise_batch *bt, floa
     cudaStream_t s = vv_stream(ctx);
     const int p0 = (int)level_pixels(dn, 0);
     forward(dn, bt->radiance, bt->albedo, bt->normal, s);
-    vvdn::pack_target(bt->target, dn->target3.as<float>(), p0, s);
     VV_CUDA(cudaMemsetAsync(dn->loss.ptr, 0, sizeof(float), s), "clear loss");
-    vvdn::l1_loss(dn->out_f32.as<float>(), kOutCh, dn->target3.as<float>(), dn->dout.as<bf16>(), dn->loss.as<float>(),
-                  p0, s);
+    vvdn::l1_loss(dn->out_f32.as<float>(), kOutCh, bt->target, dn->dout.as<bf16>(), dn->loss.as<float>(), p0, s);
     VV_CUDA(cudaMemsetAsync(dn->grads.ptr, 0, dn->nparams * sizeof(float), s), "clear gradients");
     backward(dn, s);
     VV_CUDA(cudaGetLastError(), "denoiser kernels");

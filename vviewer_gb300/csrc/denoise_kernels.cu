@@ -15,8 +15,6 @@ namespace vvdn {
 
 namespace {
 
-constexpr int kTileC = 64;  // channels per weight-gradient block tile
-
 __device__ __forceinline__ uint32_t smem_addr(const void *p)
 {
     return (uint32_t)__cvta_generic_to_shared(p);
@@ -197,108 +195,178 @@ __global__ void __launch_bounds__(256) k_conv3x3(ConvArgs a)
         }
 }
 
-// Weight gradient for one tap: block tile BM output channels x 64 input
-// channels, K = a slice of pixels in steps of 32 through a 3-stage cp.async
-// pipeline. BM = 64: warp w owns output channels [16w, 16w + 16) and all 64
-// input channels; BM = 32 (layers of at most 32 output channels): warp w
-// owns output channels 16 (w & 1) and input channels 32 (w >> 1). Partial
-// sums are added to dw with atomics.
-constexpr int kWgK = 32, kWgStages = 3;
-template <int BM>
-__global__ void __launch_bounds__(128) k_conv3x3_wgrad(const bf16 *__restrict__ dout, int cout,
-                                                       const bf16 *__restrict__ in, int cin, int n, int h, int w,
-                                                       float *dw, long slice)
+// Weight (and bias) gradient, all nine taps in one pass over the pixels:
+// dW_tap[co][ci] = sum_p dout[p][co] * in[p shifted by the tap][ci] on the
+// warp-level mma.sync m16n8k16. A block owns 32 output x BN input channels and
+// a set of units, a unit being a 64-pixel column of one image and a run of
+// rows; warp t owns tap t and keeps its 32 x BN sums in registers over all
+// units. Rows arrive by cp.async, two ahead: output row y reads input rows
+// y - 1, y, y + 1 from a ring of five and its dout row, so a row of either is
+// staged once for the nine taps. A tap's operand is the staged row shifted by
+// a pixel or two, which ldmatrix takes as it is. The warp of the middle tap
+// also multiplies dout by ones: the bias gradient. Partial sums are added to
+// dw and dbias with atomics.
+// Bound by shared-memory reads and MMA issue of the nine warps. Against one
+// launch per layer that staged both tensors again for every tap (and a launch
+// for the bias): 32 x 32 channels over 8 x 256 x 256 pixels 45 us, 157 + 10
+// before; 80 x 32 channels 136 us, 314 + 10 before.
+constexpr int kWgPx = 64, kWgM = 32, kWgThreads = 288, kWgRing = 5, kWgDRing = 3, kWgDRow = kWgM + 8;
+template <int BN>
+constexpr int wg_smem()
 {
-    constexpr int NT = BM == 64 ? 8 : 4; // n-tiles of 8 input channels per warp
-    __shared__ __align__(16) bf16 Ds[kWgStages][kWgK][kTileC + 8]; // [pixel][cout]
-    __shared__ __align__(16) bf16 Xs[kWgStages][kWgK][kTileC + 8]; // [pixel][cin]
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int tap = blockIdx.y % 9;
-    const int tiles_ci = (cin + kTileC - 1) / kTileC;
-    const int ct = blockIdx.y / 9;
-    const int co0 = (ct / tiles_ci) * BM, ci0 = (ct % tiles_ci) * kTileC;
-    const long P = (long)n * h * w;
-    const long pbeg = (long)blockIdx.x * slice, pend = min(P, pbeg + slice);
-    const int dy = tap / 3 - 1, dx = tap % 3 - 1;
-    const int wm = BM == 64 ? warp * 16 : (warp & 1) * 16; // warp's output-channel offset in the tile
-    const int wn = BM == 64 ? 0 : (warp >> 1) * 32;        // warp's input-channel offset in the tile
-    // load mapping: row = tid / 4 (pixel), group = (tid % 4) * 16 channels
-    const int lr = tid >> 2, lg = (tid & 3) * 16;
-    float acc[NT][4];
-#pragma unroll
-    for (int j = 0; j < NT; j++)
-        acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
-    const int nsteps = (int)((pend - pbeg + kWgK - 1) / kWgK);
-    auto load = [&](int step) {
-        const int st = step % kWgStages;
-        const long p = pbeg + (long)step * kWgK + lr;
-        const bool ok = p < pend;
-        int pn = 0, py = 0, px = 0;
-        if (ok) {
-            pn = (int)(p / ((long)h * w));
-            const int rem = (int)(p - (long)pn * h * w);
-            py = rem / w;
-            px = rem - py * w;
-        }
-        const int co = co0 + lg, ci = ci0 + lg;
-        const bool dok = ok && co < cout && lg < BM;
-        const bf16 *ds = dok ? dout + p * cout + co : dout;
-        cp_async16(&Ds[st][lr][lg], ds, dok);
-        cp_async16(&Ds[st][lr][lg + 8], dok ? ds + 8 : dout, dok);
-        const int yy = py + dy, xx = px + dx;
-        const bool xok = ok && yy >= 0 && yy < h && xx >= 0 && xx < w && ci < cin;
-        const bf16 *xs = xok ? in + (((long)pn * h + yy) * w + xx) * cin + ci : in;
-        cp_async16(&Xs[st][lr][lg], xs, xok);
-        cp_async16(&Xs[st][lr][lg + 8], xok ? xs + 8 : in, xok);
+    return (kWgRing * (kWgPx + 2) * (BN + 8) + kWgDRing * kWgPx * kWgDRow) * (int)sizeof(bf16);
+}
+
+template <int BN>
+__global__ void __launch_bounds__(kWgThreads, BN == 32 ? 3 : 2) k_conv3x3_wgrad(const bf16 *__restrict__ dout, int cout,
+                                                              const bf16 *__restrict__ in, int cin, int n, int h,
+                                                              int w, float *dw, float *dbias, int segs, int seg_rows)
+{
+    constexpr int G = BN / 8, XRow = BN + 8, XSlot = (kWgPx + 2) * XRow, DSlot = kWgPx * kWgDRow, NT = BN / 8;
+    extern __shared__ __align__(16) uint8_t wg_raw[];
+    bf16 *Xs = reinterpret_cast<bf16 *>(wg_raw); // [ring][pixel][BN + 8]
+    bf16 *Ds = Xs + kWgRing * XSlot;             // [ring][pixel][kWgDRow]
+    const int tid = threadIdx.x, tap = tid >> 5, lane = tid & 31;
+    const int tiles_ci = (cin + BN - 1) / BN;
+    const int co0 = ((int)blockIdx.y / tiles_ci) * kWgM, ci0 = ((int)blockIdx.y % tiles_ci) * BN;
+    const int cols = (w + kWgPx - 1) / kWgPx, units = n * cols * segs;
+    const int dy = tap / 3, dx = tap % 3;
+    const bool bias = dbias && tap == 4 && ci0 == 0;
+
+    // A unit's copies: what a thread copies of a row is fixed within a unit
+    // (element offsets within the row, -1: zeros), so a row costs it no
+    // index arithmetic beyond the row's address.
+    constexpr int NV = ((kWgPx + 2) * G + kWgThreads - 1) / kWgThreads;
+    struct Unit {
+        int u, x0, ya, nout;
+        long row0; // the unit's first output row among all images' rows
+        int xoff[NV], doff;
     };
-    for (int st = 0; st < kWgStages - 1; st++) {
-        if (st < nsteps)
-            load(st);
-        cp_async_commit();
-    }
-    for (int step = 0; step < nsteps; step++) {
-        cp_async_wait<kWgStages - 2>();
-        __syncthreads();
-        const int st = step % kWgStages;
+    const int dpx = tid >> 2, dg = tid & 3;
+    auto unit = [&](int u) {
+        Unit t;
+        t.u = u;
+        const int sg = u % segs, c = (u / segs) % cols, nb = u / (segs * cols);
+        t.x0 = c * kWgPx;
+        t.ya = sg * seg_rows;
+        t.nout = u < units ? min(h, t.ya + seg_rows) - t.ya : 0;
+        t.row0 = (long)nb * h + t.ya;
 #pragma unroll
-        for (int ks = 0; ks < kWgK; ks += 16) {
-            // A[m = cout][k = pixel] from Ds[k][m] (transposed load)
-            uint32_t a0, a1, a2, a3;
-            ldsm_x4_t(smem_addr(&Ds[st][ks + (lane & 7) + ((lane >> 4) << 3)][wm + ((lane >> 3) & 1) * 8]), a0, a1,
-                      a2, a3);
+        for (int k = 0; k < NV; k++) {
+            const int v = tid + k * kWgThreads, px = v / G, g = v % G, xx = t.x0 - 1 + px, ci = ci0 + 8 * g;
+            t.xoff[k] = xx >= 0 && xx < w && ci < cin ? xx * cin + ci : -1;
+        }
+        const int x = t.x0 + dpx, co = co0 + 8 * dg;
+        t.doff = x < w && co < cout ? x * cout + co : -1;
+        return t;
+    };
+    // rows of a unit: nout + 2 input rows; with input row r >= 2 comes the
+    // dout row of output row r - 2
+    auto load = [&](const Unit &t, int r, int at) {
+        bf16 *xd = Xs + (at % kWgRing) * XSlot;
+        const int yy = t.ya - 1 + r;
+        const bool row_ok = yy >= 0 && yy < h;
+        const bf16 *xrow = in + (t.row0 - 1 + r) * w * cin;
 #pragma unroll
-            for (int j = 0; j < NT / 2; j++) {
-                // B[k = pixel][n = cin] from Xs[k][n] (transposed load): two n-tiles
-                uint32_t b0, b1, b2, b3;
-                ldsm_x4_t(smem_addr(&Xs[st][ks + (lane & 7) + ((lane >> 3) & 1) * 8][wn + 16 * j + (lane >> 4) * 8]),
-                          b0, b1, b2, b3);
-                mma_bf16(acc[2 * j], a0, a1, a2, a3, b0, b1);
-                mma_bf16(acc[2 * j + 1], a0, a1, a2, a3, b2, b3);
+        for (int k = 0; k < NV; k++) {
+            const int v = tid + k * kWgThreads;
+            if (v < (kWgPx + 2) * G) {
+                const bool ok = row_ok && t.xoff[k] >= 0;
+                cp_async16(xd + (v / G) * XRow + 8 * (v % G), ok ? xrow + t.xoff[k] : in, ok);
             }
         }
-        // the stage refilled next was read two steps ago; the barrier above
-        // ordered those reads
-        if (step + kWgStages - 1 < nsteps)
-            load(step + kWgStages - 1);
+        if (r >= 2 && tid < kWgPx * (kWgM / 8)) {
+            const bool ok = t.doff >= 0;
+            cp_async16(Ds + (at % kWgDRing) * DSlot + dpx * kWgDRow + 8 * dg,
+                       ok ? dout + (t.row0 + r - 2) * w * cout + t.doff : dout, ok);
+        }
+    };
+    auto advance = [&](Unit &t, int &r) {
+        if (++r == t.nout + 2) {
+            t = unit(t.u + (int)gridDim.x);
+            r = 0;
+        }
+    };
+
+    float acc[2][NT][4] = {}, sum[2][2] = {}; // sum: output channels g and g + 8 of both halves
+    Unit cu = unit((int)blockIdx.x), lu = cu;
+    int cr = 0, lr = 0;
+    for (int k = 0; k < 2; k++) {
+        if (lu.u < units) {
+            load(lu, lr, k);
+            advance(lu, lr);
+        }
         cp_async_commit();
+    }
+    for (int at = 0; cu.u < units; at++) {
+        cp_async_wait<1>(); // this thread's copies of row `at` landed
+        __syncthreads();    // everyone's; and the ring slots of row at - 3 are read
+        if (lu.u < units) {
+            load(lu, lr, at + 2);
+            advance(lu, lr);
+        }
+        cp_async_commit();
+        if (cr >= 2) {
+            const bf16 *D = Ds + (at % kWgDRing) * DSlot;
+            const bf16 *X = Xs + ((at - 2 + dy) % kWgRing) * XSlot + dx * XRow;
+            const int steps = (min(kWgPx, w - cu.x0) + 15) >> 4;
+            float row_sum[2][4] = {};
+            for (int ks = 0; ks < 16 * steps; ks += 16) {
+                // A[m = cout][k = pixel] from D[k][m], B[k = pixel][n = cin]
+                // from X[k][n] (transposed loads)
+                uint32_t a[2][4];
+#pragma unroll
+                for (int m = 0; m < 2; m++)
+                    ldsm_x4_t(smem_addr(D + (ks + (lane & 7) + ((lane >> 4) << 3)) * kWgDRow + 16 * m +
+                                        ((lane >> 3) & 1) * 8),
+                              a[m][0], a[m][1], a[m][2], a[m][3]);
+#pragma unroll
+                for (int j = 0; j < NT / 2; j++) {
+                    uint32_t b0, b1, b2, b3;
+                    ldsm_x4_t(smem_addr(X + (ks + (lane & 7) + ((lane >> 3) & 1) * 8) * XRow + 16 * j +
+                                        (lane >> 4) * 8),
+                              b0, b1, b2, b3);
+#pragma unroll
+                    for (int m = 0; m < 2; m++) {
+                        mma_bf16(acc[m][2 * j], a[m][0], a[m][1], a[m][2], a[m][3], b0, b1);
+                        mma_bf16(acc[m][2 * j + 1], a[m][0], a[m][1], a[m][2], a[m][3], b2, b3);
+                    }
+                }
+                if (bias) {
+                    constexpr uint32_t kOnes = 0x3F803F80u; // two bf16 ones
+#pragma unroll
+                    for (int m = 0; m < 2; m++)
+                        mma_bf16(row_sum[m], a[m][0], a[m][1], a[m][2], a[m][3], kOnes, kOnes);
+                }
+            }
+            if (bias) // row by row, so that the sums over all rows round to nearest
+#pragma unroll
+                for (int m = 0; m < 2; m++) {
+                    sum[m][0] += row_sum[m][0];
+                    sum[m][1] += row_sum[m][2];
+                }
+        }
+        advance(cu, cr);
     }
     cp_async_wait<0>();
     const int g = lane >> 2, t = lane & 3;
 #pragma unroll
-    for (int half = 0; half < 2; half++) {
-        const int co = co0 + wm + g + half * 8;
-        if (co >= cout)
-            continue;
+    for (int m = 0; m < 2; m++)
 #pragma unroll
-        for (int j = 0; j < NT; j++) {
-            const int ci = ci0 + wn + 8 * j + 2 * t;
-            if (ci >= cin)
+        for (int half = 0; half < 2; half++) {
+            const int co = co0 + 16 * m + g + half * 8;
+            if (co >= cout)
                 continue;
-            float *d = dw + ((long)co * 9 + tap) * cin + ci;
-            atomicAdd(d, acc[j][2 * half]);
-            atomicAdd(d + 1, acc[j][2 * half + 1]);
+#pragma unroll
+            for (int j = 0; j < NT; j++) {
+                const int ci = ci0 + 8 * j + 2 * t;
+                if (ci < cin)
+                    atomicAdd(reinterpret_cast<float2 *>(dw + ((long)co * 9 + tap) * cin + ci),
+                              make_float2(acc[m][j][2 * half], acc[m][j][2 * half + 1]));
+            }
+            if (bias && t == 0)
+                atomicAdd(dbias + co, sum[m][half]);
         }
-    }
 }
 
 // The layout kernels below move 8 channels (16 bytes) per thread: channel
@@ -360,21 +428,20 @@ __global__ void __launch_bounds__(kBiasThreads) k_bias_grad(const bf16 *dout, in
     }
 }
 
-__global__ void k_transform_weights(const bf16 *w, bf16 *wt, int cout, int cin)
+// bf16 copies of all layers' weights, w16 as they are and wt16 transposed for
+// the input gradients (wt[ci][8 - tap][co] = w[co][tap][ci]), in one launch.
+__global__ void k_prepare_weights(const float *params, WeightTable t, bf16 *w16, bf16 *wt16)
 {
-    const long total = (long)cout * 9 * cin;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-        const int ci = (int)(i % cin);
-        const int tap = (int)((i / cin) % 9);
-        const int co = (int)(i / ((long)cin * 9));
-        wt[((long)ci * 9 + (8 - tap)) * cout + co] = w[i];
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < t.start[t.layers]; i += gridDim.x * blockDim.x) {
+        int l = 0;
+        while (i >= t.start[l + 1])
+            l++;
+        const unsigned k = i - t.start[l], cin = t.cin[l], cout = t.cout[l];
+        const bf16 v = __float2bfloat16_rn(params[t.param[l] + k]);
+        w16[i] = v;
+        const unsigned ci = k % cin, tap = (k / cin) % 9, co = k / (9 * cin);
+        wt16[t.start[l] + (ci * 9 + (8 - tap)) * cout + co] = v;
     }
-}
-
-__global__ void k_to_bf16(const float *src, bf16 *dst, size_t n)
-{
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        dst[i] = __float2bfloat16_rn(src[i]);
 }
 
 __global__ void k_pack_features(const float4 *rad, const float4 *alb, const float4 *nrm, bf16 *x, int npix)
@@ -397,16 +464,6 @@ __global__ void k_pack_features(const float4 *rad, const float4 *alb, const floa
         uint4 *dst = reinterpret_cast<uint4 *>(x + (long)p * 16);
         dst[0] = *reinterpret_cast<const uint4 *>(&v[0]);
         dst[1] = *reinterpret_cast<const uint4 *>(&v[8]);
-    }
-}
-
-__global__ void k_pack_target(const float4 *t, float *t3, int npix)
-{
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += gridDim.x * blockDim.x) {
-        const float4 v = t[p];
-        t3[3 * p] = log1pf(fmaxf(v.x, 0.0f));
-        t3[3 * p + 1] = log1pf(fmaxf(v.y, 0.0f));
-        t3[3 * p + 2] = log1pf(fmaxf(v.z, 0.0f));
     }
 }
 
@@ -518,25 +575,41 @@ __global__ void k_pool_backward_combine(const bf16 *dskip, const bf16 *dpooled, 
     }
 }
 
-__global__ void k_l1_loss(const float *out, int cout, const float *t3, bf16 *dout, float *loss_sum, int npix)
+// Loss and its gradient from the output layer (`cout` f32 channels, the first 3
+// used) and the target frame in one pass over the pixels.
+__global__ void __launch_bounds__(256) k_l1_loss(const float *out, int cout, const float4 *target, bf16 *dout,
+                                                 float *loss_sum, int npix)
 {
+    __shared__ float part[8];
     float local = 0.0f;
     const float scale = 1.0f / (3.0f * (float)npix);
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += gridDim.x * blockDim.x) {
-        for (int c = 0; c < cout; c++) {
-            float g = 0.0f;
-            if (c < 3) {
-                const float d = out[(long)p * cout + c] - t3[3 * p + c];
-                local += fabsf(d);
-                g = d > 0.0f ? scale : (d < 0.0f ? -scale : 0.0f);
-            }
-            dout[(long)p * cout + c] = __float2bfloat16_rn(g);
+        const float4 y = *reinterpret_cast<const float4 *>(out + (long)p * cout);
+        const float4 v = target[p];
+        const float t[3] = {log1pf(fmaxf(v.x, 0.0f)), log1pf(fmaxf(v.y, 0.0f)), log1pf(fmaxf(v.z, 0.0f))};
+        const float d[3] = {y.x - t[0], y.y - t[1], y.z - t[2]};
+        float g[8] = {};
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            local += fabsf(d[c]);
+            g[c] = d[c] > 0.0f ? scale : (d[c] < 0.0f ? -scale : 0.0f);
         }
+        bf16 *o = dout + (long)p * cout;
+        st16(o, pack8(g));
+        for (int c = 8; c < cout; c += 8)
+            st16(o + c, make_uint4(0u, 0u, 0u, 0u));
     }
     for (int o = 16; o > 0; o >>= 1)
         local += __shfl_xor_sync(0xffffffffu, local, o);
     if ((threadIdx.x & 31) == 0)
-        atomicAdd(loss_sum, local);
+        part[threadIdx.x >> 5] = local;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float sum = 0.0f;
+        for (int k = 0; k < 8; k++)
+            sum += part[k];
+        atomicAdd(loss_sum, sum);
+    }
 }
 
 __global__ void k_adam(float *p, const float *g, float *m, float *v, size_t n, float lr, float b1, float b2, float eps,
@@ -1737,9 +1810,9 @@ void conv3x3_wgrad(const bf16 *dout, int cout, const bf16 *in, int cin, int n, i
         dim3 grid((unsigned)slices, (unsigned)(9 * tiles));
         k_conv3x3_wgrad_tc<<<grid, 128, smem, s>>>(dout, cout, in, cin, n, h, w, dw, slice, ntile, ncols, err);
     } else {
-        wgrad_mma_sync(dout, cout, in, cin, n, h, w, dw, s);
+        wgrad_mma_sync(dout, cout, in, cin, n, h, w, dw, dbias, s);
     }
-    if (dbias) {
+    if (err && dbias) {
         // channel counts are multiples of 8 up to 256: 1-32 groups per pixel lane
         const int lanes = kBiasThreads / (cout / 8);
         const long blocks = std::min<long>(152L * 4, (P + 16L * lanes - 1) / (16L * lanes));
@@ -1747,33 +1820,40 @@ void conv3x3_wgrad(const bf16 *dout, int cout, const bf16 *in, int cin, int n, i
     }
 }
 
-void wgrad_mma_sync(const bf16 *dout, int cout, const bf16 *in, int cin, int n, int h, int w, float *dw,
+template <int BN>
+static void launch_wgrad(const bf16 *dout, int cout, const bf16 *in, int cin, int n, int h, int w, float *dw,
+                         float *dbias, cudaStream_t s)
+{
+    static bool attr_set = false;
+    if (!attr_set) {
+        cudaFuncSetAttribute(k_conv3x3_wgrad<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, wg_smem<BN>());
+        attr_set = true;
+    }
+    // three (BN = 32) or two blocks fit an SM: about one unit per block over
+    // all channel tiles
+    const int tiles = ((cout + kWgM - 1) / kWgM) * ((cin + BN - 1) / BN);
+    const long cols = (long)n * ((w + kWgPx - 1) / kWgPx), blocks = std::max<long>(1, 152L * (BN == 32 ? 3 : 2) / tiles);
+    int segs = (int)std::max<long>(1, std::min<long>(h, blocks / cols));
+    const int seg_rows = (h + segs - 1) / segs;
+    segs = (h + seg_rows - 1) / seg_rows;
+    dim3 grid((unsigned)std::min<long>(cols * segs, blocks), (unsigned)tiles);
+    k_conv3x3_wgrad<BN><<<grid, kWgThreads, wg_smem<BN>(), s>>>(dout, cout, in, cin, n, h, w, dw, dbias, segs, seg_rows);
+}
+
+void wgrad_mma_sync(const bf16 *dout, int cout, const bf16 *in, int cin, int n, int h, int w, float *dw, float *dbias,
                     cudaStream_t s)
 {
-    const long P = (long)n * h * w;
-    const int bm = cout <= 32 ? 32 : 64;
-    const int tiles = ((cout + bm - 1) / bm) * ((cin + kTileC - 1) / kTileC);
-    // about 8 blocks per SM over all taps and tiles (each block's K loop is
-    // latency-bound; more blocks keep more copies and MMAs in flight)
-    long slices = std::max<long>(1, (152L * 8) / (9L * tiles));
-    long slice = (P + slices - 1) / slices;
-    slice = std::max<long>(kWgK, (slice + kWgK - 1) / kWgK * kWgK);
-    slices = (P + slice - 1) / slice;
-    dim3 grid((unsigned)slices, (unsigned)(9 * tiles));
-    if (bm == 32)
-        k_conv3x3_wgrad<32><<<grid, 128, 0, s>>>(dout, cout, in, cin, n, h, w, dw, slice);
+    // 64 input channels per block where that leaves no more of them empty
+    // than 32 would (64, 112, 128 channels)
+    if ((cin + 63) / 64 * 64 == (cin + 31) / 32 * 32)
+        launch_wgrad<64>(dout, cout, in, cin, n, h, w, dw, dbias, s);
     else
-        k_conv3x3_wgrad<64><<<grid, 128, 0, s>>>(dout, cout, in, cin, n, h, w, dw, slice);
+        launch_wgrad<32>(dout, cout, in, cin, n, h, w, dw, dbias, s);
 }
 
-void transform_weights(const bf16 *w, bf16 *wt, int cout, int cin, cudaStream_t s)
+void prepare_weights(const float *params, const WeightTable &t, bf16 *w16, bf16 *wt16, cudaStream_t s)
 {
-    k_transform_weights<<<grid_for((long)cout * 9 * cin), 256, 0, s>>>(w, wt, cout, cin);
-}
-
-void to_bf16(const float *src, bf16 *dst, size_t n, cudaStream_t s)
-{
-    k_to_bf16<<<grid_for((long)n), 256, 0, s>>>(src, dst, n);
+    k_prepare_weights<<<grid_for((long)t.start[t.layers]), 256, 0, s>>>(params, t, w16, wt16);
 }
 
 void pack_features(const float *radiance, const float *albedo, const float *normal, bf16 *x, int npix, cudaStream_t s)
@@ -1781,11 +1861,6 @@ void pack_features(const float *radiance, const float *albedo, const float *norm
     k_pack_features<<<grid_for(npix), 256, 0, s>>>(reinterpret_cast<const float4 *>(radiance),
                                                    reinterpret_cast<const float4 *>(albedo),
                                                    reinterpret_cast<const float4 *>(normal), x, npix);
-}
-
-void pack_target(const float *target, float *t3, int npix, cudaStream_t s)
-{
-    k_pack_target<<<grid_for(npix), 256, 0, s>>>(reinterpret_cast<const float4 *>(target), t3, npix);
 }
 
 // 8-channel groups of a layout kernel, indexed in 32 bits by the kernels: the
@@ -1818,9 +1893,10 @@ void pool_backward_combine(const bf16 *dskip, const bf16 *dpooled, const bf16 *e
     k_pool_backward_combine<<<grid_for(groups8((long)n * h * w, c)), 256, 0, s>>>(dskip, dpooled, e, de, n, h, w, c);
 }
 
-void l1_loss(const float *out, int cout, const float *t3, bf16 *dout, float *loss_sum, int npix, cudaStream_t s)
+void l1_loss(const float *out, int cout, const float *target, bf16 *dout, float *loss_sum, int npix, cudaStream_t s)
 {
-    k_l1_loss<<<grid_for(npix), 256, 0, s>>>(out, cout, t3, dout, loss_sum, npix);
+    k_l1_loss<<<std::min(grid_for(npix), 152 * 8), 256, 0, s>>>(out, cout, reinterpret_cast<const float4 *>(target),
+                                                                dout, loss_sum, npix);
 }
 
 void adam(float *p, const float *g, float *m, float *v, size_t n, float lr, float b1, float b2, float eps, int t,

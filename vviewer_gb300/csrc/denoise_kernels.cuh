@@ -63,25 +63,30 @@ void inject_wait_timeout();
 // dbias[co] += sum_p dout[p][co] (dbias may be null).
 // With `err` set it runs on the tcgen05 tensor cores (err receives a status
 // bit if a wait timed out), with err null on the warp-level mma.sync kernel
-// (the faster of the two for this network: training step 3.2 vs 4.1 ms).
+// (the faster of the two for this network: gradients of 8 x 256 x 256
+// pixels 2.25 vs 4.1 ms).
 void conv3x3_wgrad(const bf16 *dout, int cout, const bf16 *in, int cin, int n, int h, int w, float *dw,
                    float *dbias, cudaStream_t s, uint32_t *err = nullptr);
-// the mma.sync weight gradient (dw only)
-void wgrad_mma_sync(const bf16 *dout, int cout, const bf16 *in, int cin, int n, int h, int w, float *dw,
+// the mma.sync weight and bias gradient
+void wgrad_mma_sync(const bf16 *dout, int cout, const bf16 *in, int cin, int n, int h, int w, float *dw, float *dbias,
                     cudaStream_t s);
 
-// w_t[ci][8 - tap][co] = w[co][tap][ci]
-void transform_weights(const bf16 *w, bf16 *wt, int cout, int cin, cudaStream_t s);
-
-// f32 master weights -> bf16 copy
-void to_bf16(const float *src, bf16 *dst, size_t n, cudaStream_t s);
+// The layers' weights: first element in the bf16 copies (start[layers]: their
+// end) and in the f32 parameters.
+constexpr int kMaxLayers = 24;
+struct WeightTable {
+    int layers;
+    unsigned start[kMaxLayers + 1], param[kMaxLayers];
+    unsigned short cin[kMaxLayers], cout[kMaxLayers];
+};
+// f32 master weights -> bf16 copies, as they are and transposed
+// (w_t[ci][8 - tap][co] = w[co][tap][ci]), every layer in one launch
+void prepare_weights(const float *params, const WeightTable &t, bf16 *w16, bf16 *wt16, cudaStream_t s);
 
 // Input features from RGBA32F buffers: log(1 + max(radiance, 0)), albedo,
-// normal, zeros to 16 channels. `target` (optional) -> log(1 + max(t, 0)),
-// 3 floats per pixel.
+// normal, zeros to 16 channels.
 void pack_features(const float *radiance, const float *albedo, const float *normal, bf16 *x, int npix,
                    cudaStream_t s);
-void pack_target(const float *target, float *t3, int npix, cudaStream_t s);
 
 void avgpool2(const bf16 *in, bf16 *out, int n, int h, int w, int c, cudaStream_t s);
 // out[.., 0:cc] = nearest-upsampled coarse (h/2 x w/2), out[.., cc:cc+cs] = skip
@@ -93,9 +98,10 @@ void upcat_backward(const bf16 *dcat, int cc, int cs, bf16 *dcoarse, bf16 *dskip
 // de = (dskip + dpooled[p / 2] / 4) * (e > 0); dskip may be null
 void pool_backward_combine(const bf16 *dskip, const bf16 *dpooled, const bf16 *e, bf16 *de, int n, int h, int w,
                            int c, cudaStream_t s);
-// L1 loss between out[.., 0:3] (f32, stride cout) and t3; dout (bf16, stride
-// cout, zero beyond channel 3) = sign(out - t) / (3 * npix); loss_sum += |diff|
-void l1_loss(const float *out, int cout, const float *t3, bf16 *dout, float *loss_sum, int npix, cudaStream_t s);
+// L1 loss between out[.., 0:3] (f32, stride cout, a multiple of 8) and
+// log(1 + max(target, 0)) of the RGBA32F target; dout (bf16, stride cout, zero
+// beyond channel 3) = sign(out - t) / (3 * npix); loss_sum += |diff|
+void l1_loss(const float *out, int cout, const float *target, bf16 *dout, float *loss_sum, int npix, cudaStream_t s);
 // Adam (Kingma and Ba 2015) with bias correction; t = step number from 1
 void adam(float *p, const float *g, float *m, float *v, size_t n, float lr, float b1, float b2, float eps, int t,
           cudaStream_t s);
