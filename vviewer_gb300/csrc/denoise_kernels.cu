@@ -43,6 +43,17 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// Programmatic dependent launch: the network's launches follow each other
+// closely, so each one starts while the previous one still runs, up to its
+// first access to what earlier launches write (weights excepted, which a
+// launch at least two back wrote): 12 us of launch and start-up per
+// convolution are mostly hidden (a 256 x 256 frame, 27 launches: 289 us of
+// kernel time one by one, 249 us as they run). pdl_wait returns when the previous launch
+// is complete and its writes are visible; pdl_start, issued after it, lets the
+// next launch begin.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Asynchronous 16-byte global -> shared copy; src_bytes = 0 writes zeros
 // (padding, channels past cin, rows past cout).
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, bool valid)
@@ -446,6 +457,8 @@ __global__ void k_prepare_weights(const float *params, WeightTable t, bf16 *w16,
 
 __global__ void k_pack_features(const float4 *rad, const float4 *alb, const float4 *nrm, bf16 *x, int npix)
 {
+    pdl_wait();
+    pdl_start();
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += gridDim.x * blockDim.x) {
         const float4 r = rad[p], a = alb[p], q = nrm[p];
         __align__(16) bf16 v[16];
@@ -469,6 +482,8 @@ __global__ void k_pack_features(const float4 *rad, const float4 *alb, const floa
 
 __global__ void k_avgpool2(const bf16 *in, bf16 *out, int n, int h, int w, int c)
 {
+    pdl_wait();
+    pdl_start();
     const unsigned ho = h / 2, wo = w / 2, g = c / 8;
     const unsigned total = (unsigned)n * ho * wo * g;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
@@ -495,6 +510,8 @@ __global__ void k_avgpool2(const bf16 *in, bf16 *out, int n, int h, int w, int c
 
 __global__ void k_upcat(const bf16 *coarse, int cc, const bf16 *skip, int cs, bf16 *out, int n, int h, int w)
 {
+    pdl_wait();
+    pdl_start();
     const unsigned gc = cc / 8, gt = (cc + cs) / 8;
     const unsigned total = (unsigned)n * h * w * gt;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
@@ -512,6 +529,8 @@ __global__ void k_upcat(const bf16 *coarse, int cc, const bf16 *skip, int cs, bf
 
 __global__ void k_upcat_backward_coarse(const bf16 *dcat, int cc, int cs, bf16 *dcoarse, int n, int h, int w)
 {
+    pdl_wait();
+    pdl_start();
     const int ct = cc + cs;
     const unsigned ho = h / 2, wo = w / 2, g = cc / 8;
     const unsigned total = (unsigned)n * ho * wo * g;
@@ -539,6 +558,8 @@ __global__ void k_upcat_backward_coarse(const bf16 *dcat, int cc, int cs, bf16 *
 
 __global__ void k_upcat_backward_skip(const bf16 *dcat, int cc, int cs, bf16 *dskip, unsigned npix)
 {
+    pdl_wait();
+    pdl_start();
     const unsigned g = cs / 8, gt = (cc + cs) / 8, gc = cc / 8;
     const unsigned total = npix * g;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
@@ -550,6 +571,8 @@ __global__ void k_upcat_backward_skip(const bf16 *dcat, int cc, int cs, bf16 *ds
 __global__ void k_pool_backward_combine(const bf16 *dskip, const bf16 *dpooled, const bf16 *e, bf16 *de, int n, int h,
                                         int w, int c)
 {
+    pdl_wait();
+    pdl_start();
     const unsigned g = c / 8;
     const unsigned total = (unsigned)n * h * w * g;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
@@ -642,7 +665,7 @@ int grid_for(long n, int block = 256)
 // ---------------------------------------------------------------------------
 // tcgen05 convolution (5th-generation tensor cores, accumulator in TMEM).
 //
-// CTA = 128 threads, tile = 128 consecutive pixels of one image row (UMMA
+// CTA = kTcThreads threads, tile = 128 consecutive pixels of one image row (UMMA
 // M = 128: pixel i of the tile is TMEM lane i) x all output channels (N =
 // cout <= 256, one accumulator of N f32 columns). For each 32-channel chunk
 // of the input the CTA stages a halo of 3 rows x 130 pixels once in shared
@@ -661,6 +684,10 @@ constexpr int kTcM = 128, kTcBK = 32, kTcKC = kTcBK / 8, kTcBStages = 4, kTcHalo
 constexpr int kTcHaloRow = kTcKC * kTcHaloPx * 16;  // one halo row: 4 channel groups x 130 pixels x 16 B
 constexpr int kTcHaloAlloc = 25088;                 // rounded up to 1 KB multiples
 constexpr unsigned long long kTcWaitNs = 2000000000ull;
+// threads of the per-tile kernels: what bounds a chunk is the index arithmetic
+// of its copies, so 16 warps share them (and the drain): 160 to 64 channels at
+// 960 x 540 274 us with 4 warps, 220 us with 16
+constexpr int kTcThreads = 512;
 
 __host__ __device__ constexpr int tc_smem_bytes(int N) { return 2 * kTcHaloAlloc + kTcBStages * N * kTcBK * 2; }
 
@@ -753,7 +780,7 @@ __device__ __forceinline__ void store_row16(const ConvArgs &a, long p, int c, co
     }
 }
 
-__global__ void __launch_bounds__(128) k_conv3x3_tc(ConvArgs a, int ncols, uint32_t *err)
+__global__ void __launch_bounds__(kTcThreads) k_conv3x3_tc(ConvArgs a, int ncols, uint32_t *err)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint32_t tmem_holder;
@@ -786,6 +813,8 @@ __global__ void __launch_bounds__(128) k_conv3x3_tc(ConvArgs a, int ncols, uint3
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
+    pdl_wait();
+    pdl_start();
     const uint32_t tmem = tmem_holder;
     // D f32, A/B bf16, both K-major, N >> 3, M >> 4
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kTcM >> 4) << 24);
@@ -795,7 +824,7 @@ __global__ void __launch_bounds__(128) k_conv3x3_tc(ConvArgs a, int ncols, uint3
         if (tap == 0) {
             // halo of chunk c: 3 rows x 130 pixels x 4 channel groups
             uint8_t *h = halo[c & 1];
-            for (int i = tid; i < 3 * kTcKC * kTcHaloPx; i += 128) {
+            for (int i = tid; i < 3 * kTcKC * kTcHaloPx; i += kTcThreads) {
                 const int px = i % kTcHaloPx, kc = (i / kTcHaloPx) % kTcKC, hr = i / (kTcHaloPx * kTcKC);
                 const int yy = y + hr - 1, xx = x0 - 1 + px, ci = ci0 + 8 * kc;
                 const bool ok = yy >= 0 && yy < a.h && xx >= 0 && xx < a.wd && ci < a.cin;
@@ -804,7 +833,7 @@ __global__ void __launch_bounds__(128) k_conv3x3_tc(ConvArgs a, int ncols, uint3
             }
         }
         uint8_t *b = bst + (st % kTcBStages) * bstage_bytes;
-        for (int i = tid; i < N * kTcKC; i += 128) {
+        for (int i = tid; i < N * kTcKC; i += kTcThreads) {
             const int n = i / kTcKC, kc = i - n * kTcKC, ci = ci0 + 8 * kc;
             const bool ok = n < a.cout && ci < a.cin;
             const bf16 *src = ok ? a.wgt + ((long)n * 9 + tap) * a.cin + ci : a.wgt;
@@ -864,17 +893,11 @@ __global__ void __launch_bounds__(128) k_conv3x3_tc(ConvArgs a, int ncols, uint3
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     if (!abort_flag) {
-        const int x = x0 + warp * 32 + lane;
+        const int q = warp & 3, x = x0 + q * 32 + lane;
         const long p = ((long)nb * a.h + y) * a.wd + x;
-        for (int c = 0; c < N; c += 16) {
+        for (int c = 16 * (warp >> 2); c < N; c += 16 * (kTcThreads / 128)) {
             uint32_t r[16];
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
-                         "%12, %13, %14, %15}, [%16];"
-                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                           "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-                           "=r"(r[14]), "=r"(r[15])
-                         : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c));
-            asm volatile("tcgen05.wait::ld.sync.aligned;");
+            tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c, r);
             if (x >= a.wd || c >= a.cout)
                 continue;
             store_row16(a, p, c, r);
@@ -907,7 +930,8 @@ __host__ __device__ constexpr int tc_chunk_smem_bytes(int N, int nchunks, int ro
 // for all of them (4 rows up to 64 output channels, else 2: two stages fit)
 inline int tc_chunk_rows(int N) { return N <= 64 ? 4 : 2; }
 
-__global__ void __launch_bounds__(128) k_conv3x3_tc_chunk(ConvArgs a, int ncols, int nacc, int rows, uint32_t *err)
+__global__ void __launch_bounds__(kTcThreads) k_conv3x3_tc_chunk(ConvArgs a, int ncols, int nacc, int rows, int ntile,
+                                                                 uint32_t *err)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint32_t tmem_holder;
@@ -920,7 +944,7 @@ __global__ void __launch_bounds__(128) k_conv3x3_tc_chunk(ConvArgs a, int ncols,
     const int y0 = (blockIdx.x / tiles_x) % yblocks * rows;
     const int nb = blockIdx.x / (tiles_x * yblocks);
     const int x0 = tx * kTcM;
-    const int N = (a.cout + 15) & ~15;
+    const int N = ntile, n0 = (int)blockIdx.y * ntile; // this CTA's output channels
     const int tap_bytes = N * kTcBK * 2;
     const int halo_alloc = tc_chunk_halo_bytes(rows);
     const int stage_bytes = halo_alloc + 9 * tap_bytes;
@@ -943,26 +967,32 @@ __global__ void __launch_bounds__(128) k_conv3x3_tc_chunk(ConvArgs a, int ncols,
     const uint32_t tmem = tmem_holder;
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kTcM >> 4) << 24);
 
-    auto load_chunk = [&](int c) {
+    auto load_halo = [&](int c) {
         uint8_t *h = smem + (c & 1) * stage_bytes;
-        uint8_t *bw = h + halo_alloc;
         const int ci0 = c * kTcBK;
-        for (int i = tid; i < (rows + 2) * kTcKC * kTcHaloPx; i += 128) {
+        for (int i = tid; i < (rows + 2) * kTcKC * kTcHaloPx; i += kTcThreads) {
             const int px = i % kTcHaloPx, kc = (i / kTcHaloPx) % kTcKC, hr = i / (kTcHaloPx * kTcKC);
             const int yy = y0 + hr - 1, xx = x0 - 1 + px, ci = ci0 + 8 * kc;
             const bool ok = yy >= 0 && yy < a.h && xx >= 0 && xx < a.wd && ci < a.cin;
             const bf16 *src = ok ? a.in + (((long)nb * a.h + yy) * a.wd + xx) * a.cin + ci : a.in;
             cp_async16(h + ((hr * kTcKC + kc) * kTcHaloPx + px) * 16, src, ok);
         }
-        for (int i = tid; i < 9 * N * kTcKC; i += 128) {
+    };
+    auto load_weights = [&](int c) {
+        uint8_t *bw = smem + (c & 1) * stage_bytes + halo_alloc;
+        const int ci0 = c * kTcBK;
+        for (int i = tid; i < 9 * N * kTcKC; i += kTcThreads) {
             const int kc = i % kTcKC, n = (i / kTcKC) % N, tap = i / (kTcKC * N), ci = ci0 + 8 * kc;
-            const bool ok = n < a.cout && ci < a.cin;
-            const bf16 *src = ok ? a.wgt + ((long)n * 9 + tap) * a.cin + ci : a.wgt;
+            const bool ok = n0 + n < a.cout && ci < a.cin;
+            const bf16 *src = ok ? a.wgt + ((long)(n0 + n) * 9 + tap) * a.cin + ci : a.wgt;
             cp_async16(bw + tap * tap_bytes + (n >> 3) * (kTcKC * 128) + kc * 128 + (n & 7) * 16, src, ok);
         }
     };
 
-    load_chunk(0);
+    load_weights(0);
+    pdl_wait();
+    pdl_start();
+    load_halo(0);
     cp_async_commit();
     for (int c = 0; c < nchunks; c++) {
         cp_async_wait<0>(); // this thread's copies of chunk c landed
@@ -1001,7 +1031,8 @@ __global__ void __launch_bounds__(128) k_conv3x3_tc_chunk(ConvArgs a, int ncols,
         if (c + 1 < nchunks) {
             if (c >= 1 && !mbar_wait(smem_addr(&mbar[(c - 1) & 1]), ((c - 1) >> 1) & 1))
                 atomicOr(&abort_flag, 1);
-            load_chunk(c + 1);
+            load_weights(c + 1);
+            load_halo(c + 1);
         }
         cp_async_commit();
     }
@@ -1014,24 +1045,26 @@ __global__ void __launch_bounds__(128) k_conv3x3_tc_chunk(ConvArgs a, int ncols,
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     if (!abort_flag) {
-        const int x = x0 + warp * 32 + lane;
-        for (int rr = 0; rr < rows && y0 + rr < a.h; rr++) {
+        // warps w, w + 4, ... read the same 32 pixels, each its share of
+        // (row, 16 channels)
+        const int quarter = warp & 3, x = x0 + quarter * 32 + lane, groups = N / 16;
+        for (int k = warp >> 2; k < rows * groups; k += kTcThreads / 128) {
+            const int rr = k / groups, c = 16 * (k - rr * groups);
+            if (y0 + rr >= a.h)
+                break;
             const long p = ((long)nb * a.h + y0 + rr) * a.wd + x;
-            const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(rr * nacc * N);
-            for (int c = 0; c < N; c += 16) {
-                uint32_t r[16];
-                tmem_ld16(lane_base + (uint32_t)c, r);
-                for (int q = 1; q < nacc; q++) {
-                    uint32_t t[16];
-                    tmem_ld16(lane_base + (uint32_t)(q * N + c), t);
+            const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(rr * nacc * N);
+            uint32_t r[16];
+            tmem_ld16(lane_base + (uint32_t)c, r);
+            for (int q = 1; q < nacc; q++) {
+                uint32_t t[16];
+                tmem_ld16(lane_base + (uint32_t)(q * N + c), t);
 #pragma unroll
-                    for (int k = 0; k < 16; k++)
-                        r[k] = __float_as_uint(__uint_as_float(r[k]) + __uint_as_float(t[k]));
-                }
-                if (x >= a.wd || c >= a.cout)
-                    continue;
-                store_row16(a, p, c, r);
+                for (int m = 0; m < 16; m++)
+                    r[m] = __float_as_uint(__uint_as_float(r[m]) + __uint_as_float(t[m]));
             }
+            if (x < a.wd && n0 + c < a.cout)
+                store_row16(a, p, n0 + c, r);
         }
     } else if (tid == 0) {
         atomicOr(err, 1u);
@@ -1104,32 +1137,35 @@ __device__ __forceinline__ void umma_commit(uint32_t bar)
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar));
 }
 
-// 224 threads: warps 0-3 drain accumulators (TMEM lane quarter = warp),
-// warp 4 loads halo rows by TMA, warp 5 issues the MMAs, warp 6 fills the
-// upsampled channels of a fused upsample + concat input (a.coarse). The roles
-// run ahead of each other as far as the ring (`ring` halo-row slots) and the
+// Warps 0-3 drain accumulators (TMEM lane quarter = warp), warp 4 loads halo
+// rows by TMA, warp 5 issues the MMAs, warps 6-9 (launched for it only) fill
+// the upsampled channels of a fused upsample + concat input (a.coarse). The
+// warps other than 4 and 5 first copy the weights, which the MMA warp waits
+// for; the first rows are on their way meanwhile. (One warp for the upsampled
+// channels bounded the full-resolution decoder input: 1037 us at 3840 x 2160,
+// 782 us with four.) The roles run ahead of each other as far as the ring (`ring` halo-row slots) and the
 // two accumulators allow, synchronised only by mbarriers:
 //   full[s]   the halo row in slot s is complete: TMA bytes landed (producer)
-//             and, fused, the upsampled channels stored (warp 6) -> MMA
+//             and, fused, the upsampled channels stored (warps 6-9) -> MMA
 //   empty[s]  the MMAs that read slot s completed (MMA commit -> producer)
 //   acc_full[b]  row accumulator b is complete (MMA commit -> drain)
 //   acc_empty[b] the four drain warps have read accumulator b (drain -> MMA)
-constexpr int kStThreads = 224;
+constexpr int kStThreads = 192, kStUpWarps = 4;
 
-__global__ void __launch_bounds__(kStThreads) k_conv3x3_strip(ConvArgs a, const __grid_constant__ CUtensorMap tmap,
-                                                              int ncols, int nacc, int ring, int segs, int seg_rows,
-                                                              uint32_t *err, int withhold_acc_full)
+__global__ void __launch_bounds__(kStThreads + 32 * kStUpWarps)
+    k_conv3x3_strip(ConvArgs a, const __grid_constant__ CUtensorMap tmap, int ncols, int nacc, int ring, int segs,
+                    int seg_rows, int ntile, uint32_t *err, int withhold_acc_full)
 {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     __shared__ uint32_t tmem_holder;
     __shared__ __align__(8) uint64_t full[kStMaxRing], empty[kStMaxRing];
-    __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2];
+    __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], weights_full;
     __shared__ int abort_flag;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tiles_x = (a.wd + kTcM - 1) / kTcM;
     const int units = a.n * tiles_x * segs;
     const int KC = a.cin >> 3;
-    const int N = (a.cout + 15) & ~15;
+    const int N = ntile, n0 = (int)blockIdx.y * ntile; // this CTA's output channels
     const int slot_bytes = KC * kStKCBytes;
     const int tap_bytes = N * a.cin * 2;
     const uint32_t half_cols = (uint32_t)ncols >> 1;
@@ -1139,49 +1175,61 @@ __global__ void __launch_bounds__(kStThreads) k_conv3x3_strip(ConvArgs a, const 
     uint8_t *w_ptr = smem_raw + (w_base - raw);
     const volatile int *abort_v = &abort_flag;
 
-    const int CG = a.cc >> 3;  // channel groups filled by warp 6 (upsampled coarse input)
+    const int CG = a.cc >> 3;  // channel groups filled by warps 6-9 (upsampled coarse input)
     if (tid == 0) {
         for (int r = 0; r < ring; r++) {
-            mbar_init(&full[r], CG ? 2 : 1);
+            mbar_init(&full[r], CG ? 1 + kStUpWarps : 1);
             mbar_init(&empty[r], 1);
         }
         for (int k = 0; k < 2; k++) {
             mbar_init(&acc_full[k], 1);
             mbar_init(&acc_empty[k], 4);
         }
+        mbar_init(&weights_full, blockDim.x - 64u); // every thread of the warps that copy them
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    const bool copies = warp != 4 && warp != 5;
+    if (copies) {
+        const int ct = warp < 4 ? tid : tid - 64, cn = (int)blockDim.x - 64;
+        for (int i = ct; i < 9 * N * KC; i += cn) {
+            const int kc = i % KC, n = (i / KC) % N, tap = i / (KC * N);
+            const bool ok = n0 + n < a.cout;
+            const bf16 *src = ok ? a.wgt + ((long)(n0 + n) * 9 + tap) * a.cin + 8 * kc : a.wgt;
+            cp_async16(w_ptr + tap * tap_bytes + (n >> 3) * (KC * 128) + kc * 128 + (n & 7) * 16, src, ok);
+        }
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_holder)),
                      "r"(ncols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
-    for (int i = tid; i < 9 * N * KC; i += kStThreads) {
-        const int kc = i % KC, n = (i / KC) % N, tap = i / (KC * N);
-        const bool ok = n < a.cout;
-        const bf16 *src = ok ? a.wgt + ((long)n * 9 + tap) * a.cin + 8 * kc : a.wgt;
-        cp_async16(w_ptr + tap * tap_bytes + (n >> 3) * (KC * 128) + kc * 128 + (n & 7) * 16, src, ok);
-    }
-    cp_async_commit();
-    cp_async_wait<0>();
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = tmem_holder;
+    if (copies) {
+        cp_async_commit();
+        cp_async_wait<0>();
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        mbar_arrive(smem_addr(&weights_full));
+    }
+    pdl_wait();
+    if (tid == 0)
+        pdl_start();
 
-    if (warp == 6) {
+    if (warp >= 6) {
         // ---- upsampled channels of a fused concat input: fine pixel x of
         // halo row y reads coarse pixel (x >> 1, y >> 1). 16-byte cp.async
         // copies (consecutive lanes on consecutive channel groups of a coarse
-        // pixel), one commit group per row; a row is published (fence to the
-        // async proxy, arrive on its full barrier) once `lag` newer rows are
-        // in flight, lag <= ring - 3 so the MMA warp can always release the
-        // slot this warp waits for.
+        // pixel), the warps taking every fourth run of 32, one commit group per
+        // row; a row is published (fence to the async proxy, arrive on its full
+        // barrier) once `lag` newer rows are in flight, lag <= ring - 3 so the
+        // MMA warp can always release the slot a warp waits for.
         if (CG) {
             const int hc = a.h >> 1, wc = a.wd >> 1;
-            const int npc = kStHaloPx * CG, dp = 32 / CG, dg = 32 % CG;
+            constexpr int kUp = 32 * kStUpWarps;
+            const int npc = kStHaloPx * CG, dp = kUp / CG, dg = kUp % CG, first = 32 * (warp - 6) + lane;
             const int lag = min(2, ring - 3);
             int slot = 0, phase = 0, pub_slot = 0, pending = 0;
             auto publish = [&]() {
@@ -1210,8 +1258,8 @@ __global__ void __launch_bounds__(kStThreads) k_conv3x3_strip(ConvArgs a, const 
                     const bool row_ok = yy >= 0 && yy < a.h;
                     const bf16 *crow = a.coarse + ((long)nb * hc + (row_ok ? yy >> 1 : 0)) * wc * a.cc;
                     uint8_t *dst = smem_raw + (ring_base - raw) + slot * slot_bytes;
-                    int pp = lane / CG, g = lane - (lane / CG) * CG;
-                    for (int idx = lane; idx < npc; idx += 32) {
+                    int pp = first / CG, g = first - (first / CG) * CG;
+                    for (int idx = first; idx < npc; idx += kUp) {
                         const int xx = x0 - 1 + pp;
                         const bool in = row_ok && xx >= 0 && xx < a.wd;
                         cp_async16(dst + g * kStKCBytes + pp * 16, in ? crow + (long)(xx >> 1) * a.cc + 8 * g : a.coarse,
@@ -1302,7 +1350,7 @@ __global__ void __launch_bounds__(kStThreads) k_conv3x3_strip(ConvArgs a, const 
             int wait_slot = 0, wait_phase = 0, waited = 0; // next halo row to see complete
             int gi = 0;                  // output rows so far
             int halo = 0;                // halo rows of earlier units
-            bool ok = true;
+            bool ok = mbar_wait_role(smem_addr(&weights_full), 0, abort_v);
             for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
                 const int sg = u % segs;
                 const int ya = sg * seg_rows;
@@ -1409,8 +1457,8 @@ __global__ void __launch_bounds__(kStThreads) k_conv3x3_strip(ConvArgs a, const 
                         if (lane == 0)
                             mbar_arrive(smem_addr(&acc_empty[b]));
                     }
-                    if (x < a.wd && c < a.cout)
-                        store_row16(a, p, c, r);
+                    if (x < a.wd && n0 + c < a.cout)
+                        store_row16(a, p, n0 + c, r);
                 }
             }
         }
@@ -1606,7 +1654,36 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
     return fn;
 }
 
+// Launch that may start while the previous one runs (see pdl_wait).
+template <class... P, class... A>
+void launch_pdl(void (*kernel)(P...), dim3 grid, int threads, int smem, cudaStream_t s, A... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
+// Output channels per CTA where `ctas` CTAs with all N leave SMs idle: the
+// smallest share (a divisor of N, a multiple of 16) for which one CTA per SM
+// still takes them all at once.
+int split_channels(int N, long ctas)
+{
+    for (int nt = 16; nt < N; nt += 16)
+        if (N % nt == 0 && ctas * (N / nt) <= 152)
+            return nt;
+    return N;
+}
+
 struct StripPlan {
+    int ntile = 0; // output channels per CTA
     int ring = 0, smem = 0, grid = 0, segs = 0, seg_rows = 0, ncols = 0, nacc = 1, per_sm = 1;
 };
 
@@ -1665,14 +1742,22 @@ bool plan_strip(const ConvArgs &a, StripPlan &pl)
                 break;
             }
         }
-        pl.ring = ring;
-        pl.smem = dyn;
+        // a small image: fewer output channels per CTA (the accumulators, and
+        // with them the order of the sums, stay as planned for all of them)
+        pl.grid = (int)std::min<long>(cols * segs, ctas);
+        pl.ntile = split_channels(N, pl.grid);
+        if (pl.ntile != N)
+            for (tcols = 32; tcols < 2 * nacc * pl.ntile;)
+                tcols <<= 1;
+        // no more shared memory than the rows of a CTA's run need, so that the
+        // next launch can begin beside this one
+        pl.ring = std::min<long>(ring, cols * segs <= ctas ? std::max(kStMinRing, seg_rows + 2) : kStMaxRing);
+        pl.smem = 1024 + 9 * pl.ntile * a.cin * 2 + pl.ring * slot;
         pl.segs = segs;
         pl.seg_rows = seg_rows;
         pl.ncols = tcols;
         pl.nacc = nacc;
         pl.per_sm = c;
-        pl.grid = (int)std::min<long>(cols * segs, ctas);
         return true;
     }
     return false;
@@ -1722,8 +1807,9 @@ bool launch_strip(const ConvArgs &a, cudaStream_t s, uint32_t *err, ConvKernels 
         attr_smem = pl.smem;
     }
     const int withhold = g_inject_wait_timeout.exchange(false) ? 1 : 0;
-    k_conv3x3_strip<<<pl.grid, kStThreads, pl.smem, s>>>(a, tmap, pl.ncols, pl.nacc, pl.ring, pl.segs, pl.seg_rows,
-                                                         err, withhold);
+    launch_pdl(k_conv3x3_strip, dim3((unsigned)pl.grid, (unsigned)(((a.cout + 15) & ~15) / pl.ntile)),
+               kStThreads + (a.cc ? 32 * kStUpWarps : 0), pl.smem, s, a, tmap, pl.ncols, pl.nacc, pl.ring, pl.segs,
+               pl.seg_rows, pl.ntile, err, withhold);
     return true;
 }
 
@@ -1761,16 +1847,26 @@ void conv3x3(const ConvArgs &a_in, cudaStream_t s, uint32_t *err, ConvKernels ki
         if (N <= 128) {
             // several output rows per CTA, one accumulator (one MMA chain)
             // per row
-            const int rows = tc_chunk_rows(N);
-            const int smem = tc_chunk_smem_bytes(N, (a.cin + kTcBK - 1) / kTcBK, rows);
+            const long columns = (long)a.n * ((a.wd + kTcM - 1) / kTcM);
+            int rows = tc_chunk_rows(N);
+            // a small image leaves SMs idle: fewer rows per CTA while the
+            // CTAs still run at once, one per SM (224 to 96 channels at 32 x 32:
+            // 28 us on 32 CTAs, 19 us on 96)
+            while (rows > 1 && 2 * columns * ((a.h + rows - 1) / rows) <= 152)
+                rows /= 2;
+            const long blocks = columns * ((a.h + rows - 1) / rows);
+            // ... and then fewer output channels per CTA, which share the
+            // staging of the weights
+            const int nt = split_channels(N, blocks);
+            const int smem = tc_chunk_smem_bytes(nt, (a.cin + kTcBK - 1) / kTcBK, rows);
             int cols = 32;
-            while (cols < rows * N)
+            while (cols < rows * nt)
                 cols <<= 1;
-            const long blocks = (long)a.n * ((a.h + rows - 1) / rows) * ((a.wd + kTcM - 1) / kTcM);
-            k_conv3x3_tc_chunk<<<(unsigned)blocks, 128, smem, s>>>(a, cols, 1, rows, err);
+            launch_pdl(k_conv3x3_tc_chunk, dim3((unsigned)blocks, (unsigned)(N / nt)), kTcThreads, smem, s, a, cols, 1,
+                       rows, nt, err);
         }
         else
-            k_conv3x3_tc<<<(unsigned)tiles, 128, tc_smem_bytes(N), s>>>(a, ncols, err);
+            launch_pdl(k_conv3x3_tc, dim3((unsigned)tiles), kTcThreads, tc_smem_bytes(N), s, a, ncols, err);
         return;
     }
     // 32-wide channel tiles where they leave fewer channels of the last tile
@@ -1858,9 +1954,8 @@ void prepare_weights(const float *params, const WeightTable &t, bf16 *w16, bf16 
 
 void pack_features(const float *radiance, const float *albedo, const float *normal, bf16 *x, int npix, cudaStream_t s)
 {
-    k_pack_features<<<grid_for(npix), 256, 0, s>>>(reinterpret_cast<const float4 *>(radiance),
-                                                   reinterpret_cast<const float4 *>(albedo),
-                                                   reinterpret_cast<const float4 *>(normal), x, npix);
+    launch_pdl(k_pack_features, dim3(grid_for(npix)), 256, 0, s, reinterpret_cast<const float4 *>(radiance),
+               reinterpret_cast<const float4 *>(albedo), reinterpret_cast<const float4 *>(normal), x, npix);
 }
 
 // 8-channel groups of a layout kernel, indexed in 32 bits by the kernels: the
@@ -1870,27 +1965,28 @@ static long groups8(long pixels, int c) { return pixels * (c / 8); }
 
 void avgpool2(const bf16 *in, bf16 *out, int n, int h, int w, int c, cudaStream_t s)
 {
-    k_avgpool2<<<grid_for(groups8((long)n * (h / 2) * (w / 2), c)), 256, 0, s>>>(in, out, n, h, w, c);
+    launch_pdl(k_avgpool2, dim3(grid_for(groups8((long)n * (h / 2) * (w / 2), c))), 256, 0, s, in, out, n, h, w, c);
 }
 
 void upcat(const bf16 *coarse, int cc, const bf16 *skip, int cs, bf16 *out, int n, int h, int w, cudaStream_t s)
 {
-    k_upcat<<<grid_for(groups8((long)n * h * w, cc + cs)), 256, 0, s>>>(coarse, cc, skip, cs, out, n, h, w);
+    launch_pdl(k_upcat, dim3(grid_for(groups8((long)n * h * w, cc + cs))), 256, 0, s, coarse, cc, skip, cs, out, n, h, w);
 }
 
 void upcat_backward(const bf16 *dcat, int cc, int cs, bf16 *dcoarse, bf16 *dskip, int n, int h, int w, cudaStream_t s)
 {
-    k_upcat_backward_coarse<<<grid_for(groups8((long)n * (h / 2) * (w / 2), cc)), 256, 0, s>>>(dcat, cc, cs, dcoarse,
-                                                                                                n, h, w);
+    launch_pdl(k_upcat_backward_coarse, dim3(grid_for(groups8((long)n * (h / 2) * (w / 2), cc))), 256, 0, s, dcat, cc,
+               cs, dcoarse, n, h, w);
     if (dskip)
-        k_upcat_backward_skip<<<grid_for(groups8((long)n * h * w, cs + cc)), 256, 0, s>>>(dcat, cc, cs, dskip,
-                                                                                          (unsigned)((long)n * h * w));
+        launch_pdl(k_upcat_backward_skip, dim3(grid_for(groups8((long)n * h * w, cs + cc))), 256, 0, s, dcat, cc, cs,
+                   dskip, (unsigned)((long)n * h * w));
 }
 
 void pool_backward_combine(const bf16 *dskip, const bf16 *dpooled, const bf16 *e, bf16 *de, int n, int h, int w, int c,
                            cudaStream_t s)
 {
-    k_pool_backward_combine<<<grid_for(groups8((long)n * h * w, c)), 256, 0, s>>>(dskip, dpooled, e, de, n, h, w, c);
+    launch_pdl(k_pool_backward_combine, dim3(grid_for(groups8((long)n * h * w, c))), 256, 0, s, dskip, dpooled, e, de, n,
+               h, w, c);
 }
 
 void l1_loss(const float *out, int cout, const float *target, bf16 *dout, float *loss_sum, int npix, cudaStream_t s)
