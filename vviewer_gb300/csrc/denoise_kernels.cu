@@ -715,6 +715,31 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
     }
 }
 
+// The MMAs are issued by one elected lane, but by code that the whole warp runs
+// with the same values: descriptors, instruction word and accumulator address
+// of a tcgen05.mma are uniform registers, and code of a single lane moves each
+// of them there for every MMA. Measured, MMAs of M 128, K 16 one after the
+// other: 55 clocks each from a lane's own code whatever N, 32 + N / 4 (the
+// operands' shared-memory reads) from the warp's.
+__device__ __forceinline__ uint32_t elect_one()
+{
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(e));
+    return e;
+}
+__device__ __forceinline__ void umma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate,
+                                     uint32_t elected)
+{
+    asm volatile("{\n\t.reg .pred p, e;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+                 "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+                 "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)accumulate), "r"(elected));
+}
+
+__device__ __forceinline__ void umma_commit(uint32_t bar)
+{
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar));
+}
+
 // shared-memory matrix descriptor: start, LBO, SBO (16-byte units),
 // version 1, no swizzle
 __device__ __forceinline__ uint64_t umma_desc(uint32_t addr, uint32_t lbo, uint32_t sbo)
@@ -734,17 +759,115 @@ __device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&r)[16])
     asm volatile("tcgen05.wait::ld.sync.aligned;");
 }
 
+__device__ __forceinline__ void tmem_ld8_issue(uint32_t addr, uint32_t (&r)[8])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(addr));
+}
+
+__device__ __forceinline__ void tmem_ld16_issue(uint32_t addr, uint32_t (&r)[16])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+                 "%14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
+                   "=r"(r[15])
+                 : "r"(addr));
+}
+// Every use of the loaded values depends on a value that passes through here.
+__device__ __forceinline__ void tmem_wait8(uint32_t *r)
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])::
+                     "memory");
+}
+
+// 16 channels of a row accumulator of `nacc` (1, 2 or 4) partial sums, ncol
+// columns apart, added in their order: as many loads in flight before a wait
+// as fit 32 registers.
+template <int nacc>
+__device__ __forceinline__ void tmem_sum16(uint32_t addr, uint32_t ncol, uint32_t (&r)[16])
+{
+    static_assert(nacc == 1 || nacc == 2 || nacc == 4, "partial sums");
+    if constexpr (nacc <= 2) {
+        uint32_t t[16];
+        tmem_ld16_issue(addr, r);
+        if constexpr (nacc > 1)
+            tmem_ld16_issue(addr + ncol, t);
+        tmem_wait8(r);
+        tmem_wait8(r + 8);
+        if constexpr (nacc > 1)
+#pragma unroll
+            for (int k = 0; k < 16; k++)
+                r[k] = __float_as_uint(__uint_as_float(r[k]) + __uint_as_float(t[k]));
+    } else {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            uint32_t t[3][8];
+            tmem_ld8_issue(addr + 8 * h, *reinterpret_cast<uint32_t(*)[8]>(r + 8 * h));
+#pragma unroll
+            for (int q = 1; q < 4; q++)
+                tmem_ld8_issue(addr + 8 * h + q * ncol, t[q - 1]);
+            tmem_wait8(r + 8 * h);
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                float v = __uint_as_float(r[8 * h + k]) + __uint_as_float(t[0][k]);
+                v += __uint_as_float(t[1][k]);
+                v += __uint_as_float(t[2][k]);
+                r[8 * h + k] = __float_as_uint(v);
+            }
+        }
+    }
+}
+
+// 32 bytes per lane in one instruction (sm_100 and later): a whole sector. The
+// operand reads of the MMAs take the same path, so what the epilogue saves
+// there the MMAs get.
+__device__ __forceinline__ void st32(void *p, const uint32_t (&v)[8])
+{
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+                 "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+__device__ __forceinline__ void ld32(const void *p, uint32_t (&v)[8])
+{
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "l"(p));
+}
+
 // Epilogue of one pixel row x 16 channels: bias, ReLU, mask, store (bf16, or
-// f32 for the output layer).
-__device__ __forceinline__ void store_row16(const ConvArgs &a, long p, int c, const uint32_t (&r)[16])
+// f32 for the output layer). Channel counts are multiples of 16 and the arrays
+// 32-byte aligned, so 16 bf16 channels are one sector.
+struct Bias16 {
+    float4 b[4];
+};
+__device__ __forceinline__ void load_bias(const ConvArgs &a, int c, Bias16 &b)
+{
+    if (a.bias && c < a.cout)
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            b.b[k] = __ldg(reinterpret_cast<const float4 *>(a.bias + c) + k);
+}
+__device__ __forceinline__ void store_row16(const ConvArgs &a, long p, int c, const uint32_t (&r)[16], const Bias16 &b)
 {
     float v[16];
 #pragma unroll
-    for (int k = 0; k < 16; k++) {
+    for (int k = 0; k < 16; k++)
         v[k] = __uint_as_float(r[k]);
-        if (a.bias)
-            v[k] += a.bias[c + k];
-        if (a.relu)
+    if (a.bias) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            v[4 * k] += b.b[k].x;
+            v[4 * k + 1] += b.b[k].y;
+            v[4 * k + 2] += b.b[k].z;
+            v[4 * k + 3] += b.b[k].w;
+        }
+    }
+    if (a.relu) {
+#pragma unroll
+        for (int k = 0; k < 16; k++)
             v[k] = fmaxf(v[k], 0.0f);
     }
     if (a.rgba) {
@@ -756,13 +879,16 @@ __device__ __forceinline__ void store_row16(const ConvArgs &a, long p, int c, co
     }
     const long o = p * a.cout + c;
     if (a.mask) {
-        __align__(16) bf16 m[16];
-        *reinterpret_cast<uint4 *>(&m[0]) = *reinterpret_cast<const uint4 *>(a.mask + o);
-        *reinterpret_cast<uint4 *>(&m[8]) = *reinterpret_cast<const uint4 *>(a.mask + o + 8);
+        uint32_t m[8];
+        ld32(a.mask + o, m);
 #pragma unroll
-        for (int k = 0; k < 16; k++)
-            if (!(__bfloat162float(m[k]) > 0.0f))
-                v[k] = 0.0f;
+        for (int k = 0; k < 8; k++) {
+            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&m[k]));
+            if (!(f.x > 0.0f))
+                v[2 * k] = 0.0f;
+            if (!(f.y > 0.0f))
+                v[2 * k + 1] = 0.0f;
+        }
     }
     if (a.out_f32) {
         float4 *dst = reinterpret_cast<float4 *>(reinterpret_cast<float *>(a.out) + o);
@@ -770,13 +896,13 @@ __device__ __forceinline__ void store_row16(const ConvArgs &a, long p, int c, co
         for (int k = 0; k < 4; k++)
             dst[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
     } else {
-        __align__(16) __nv_bfloat162 hh[8];
+        uint32_t h[8];
 #pragma unroll
-        for (int k = 0; k < 8; k++)
-            hh[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
-        uint4 *dst = reinterpret_cast<uint4 *>(reinterpret_cast<bf16 *>(a.out) + o);
-        dst[0] = *reinterpret_cast<const uint4 *>(&hh[0]);
-        dst[1] = *reinterpret_cast<const uint4 *>(&hh[4]);
+        for (int k = 0; k < 8; k++) {
+            const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
+            h[k] = *reinterpret_cast<const uint32_t *>(&b);
+        }
+        st32(reinterpret_cast<bf16 *>(a.out) + o, h);
     }
 }
 
@@ -786,7 +912,7 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3x3_tc(ConvArgs a, int ncols
     __shared__ uint32_t tmem_holder;
     __shared__ __align__(8) uint64_t mbar[kTcBStages];
     __shared__ int abort_flag;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int tiles_x = (a.wd + kTcM - 1) / kTcM;
     const int tx = blockIdx.x % tiles_x;
     const int y = (blockIdx.x / tiles_x) % a.h;
@@ -815,7 +941,7 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3x3_tc(ConvArgs a, int ncols
     asm volatile("tcgen05.fence::after_thread_sync;");
     pdl_wait();
     pdl_start();
-    const uint32_t tmem = tmem_holder;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_holder, 0), elected = elect_one();
     // D f32, A/B bf16, both K-major, N >> 3, M >> 4
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kTcM >> 4) << 24);
 
@@ -853,22 +979,17 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3x3_tc(ConvArgs a, int ncols
         __syncthreads();
         if (abort_flag)
             break;
-        if (tid == 0) {
+        if (warp == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;");
             const int c = st / 9, tap = st - c * 9, dy = tap / 3, dx = tap % 3;
             const uint32_t a_addr = sbase + (c & 1) * kTcHaloAlloc + dy * kTcHaloRow + dx * 16;
             const uint32_t b_addr = sbase + 2 * kTcHaloAlloc + (st % kTcBStages) * bstage_bytes;
 #pragma unroll
-            for (int j = 0; j < kTcBK / 16; j++) {
-                const uint64_t ad = umma_desc(a_addr + j * 2 * kTcHaloPx * 16, kTcHaloPx * 16, 128);
-                const uint64_t bd = umma_desc(b_addr + j * 2 * 128, 128, kTcKC * 128);
-                const uint32_t accumulate = (st > 0 || j > 0) ? 1u : 0u;
-                asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                             "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
-                             "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate));
-            }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                smem_addr(&mbar[st % kTcBStages])));
+            for (int j = 0; j < kTcBK / 16; j++)
+                umma(tmem, umma_desc(a_addr + j * 2 * kTcHaloPx * 16, kTcHaloPx * 16, 128),
+                     umma_desc(b_addr + j * 2 * 128, 128, kTcKC * 128), idesc, st > 0 || j > 0, elected);
+            if (elected)
+                umma_commit(smem_addr(&mbar[st % kTcBStages]));
         }
         // step st + 2 reuses the weight stage of step st - 2 and, at a chunk
         // start, the halo of chunk (st + 2) / 9 - 2: both done once step st - 2
@@ -897,10 +1018,12 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3x3_tc(ConvArgs a, int ncols
         const long p = ((long)nb * a.h + y) * a.wd + x;
         for (int c = 16 * (warp >> 2); c < N; c += 16 * (kTcThreads / 128)) {
             uint32_t r[16];
+            Bias16 bias;
+            load_bias(a, c, bias);
             tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c, r);
             if (x >= a.wd || c >= a.cout)
                 continue;
-            store_row16(a, p, c, r);
+            store_row16(a, p, c, r, bias);
         }
     } else if (tid == 0) {
         atomicOr(err, 1u);
@@ -930,14 +1053,14 @@ __host__ __device__ constexpr int tc_chunk_smem_bytes(int N, int nchunks, int ro
 // for all of them (4 rows up to 64 output channels, else 2: two stages fit)
 inline int tc_chunk_rows(int N) { return N <= 64 ? 4 : 2; }
 
-__global__ void __launch_bounds__(kTcThreads) k_conv3x3_tc_chunk(ConvArgs a, int ncols, int nacc, int rows, int ntile,
+__global__ void __launch_bounds__(kTcThreads) k_conv3x3_tc_chunk(ConvArgs a, int ncols, int rows, int ntile,
                                                                  uint32_t *err)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint32_t tmem_holder;
     __shared__ __align__(8) uint64_t mbar[2];
     __shared__ int abort_flag;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int tiles_x = (a.wd + kTcM - 1) / kTcM;
     const int yblocks = (a.h + rows - 1) / rows;
     const int tx = blockIdx.x % tiles_x;
@@ -964,7 +1087,7 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3x3_tc_chunk(ConvArgs a, int
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
-    const uint32_t tmem = tmem_holder;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_holder, 0), elected = elect_one();
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kTcM >> 4) << 24);
 
     auto load_halo = [&](int c) {
@@ -1000,31 +1123,27 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3x3_tc_chunk(ConvArgs a, int
         __syncthreads();
         if (abort_flag)
             break;
-        if (tid == 0) {
+        if (warp == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;");
             const uint32_t h_addr = sbase + (c & 1) * stage_bytes, b_addr = h_addr + halo_alloc;
-            // output row r of the block, tap t: accumulator r * nacc + t % nacc
-            // (independent chains); the chunk's weights serve all rows
+            // output row r of the block: accumulator r; the chunk's weights
+            // serve all rows
             for (int r = 0; r < rows; r++) {
 #pragma unroll
                 for (int j = 0; j < kTcBK / 16; j++) {
 #pragma unroll
                     for (int tap = 0; tap < 9; tap++) {
                         const int dy = tap / 3, dx = tap % 3;
-                        const uint64_t ad = umma_desc(h_addr + (r + dy) * kTcHaloRow + dx * 16 +
-                                                          j * 2 * kTcHaloPx * 16,
-                                                      kTcHaloPx * 16, 128);
-                        const uint64_t bd = umma_desc(b_addr + tap * tap_bytes + j * 2 * 128, 128, kTcKC * 128);
-                        const uint32_t accumulate = (c > 0 || j > 0 || tap >= nacc) ? 1u : 0u;
-                        const uint32_t dst = tmem + (uint32_t)((r * nacc + (tap & (nacc - 1))) * N);
-                        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                                     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(dst),
-                                     "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate));
+                        umma(tmem + (uint32_t)(r * N),
+                             umma_desc(h_addr + (r + dy) * kTcHaloRow + dx * 16 + j * 2 * kTcHaloPx * 16,
+                                       kTcHaloPx * 16, 128),
+                             umma_desc(b_addr + tap * tap_bytes + j * 2 * 128, 128, kTcKC * 128), idesc,
+                             c > 0 || j > 0 || tap > 0, elected);
                     }
                 }
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                smem_addr(&mbar[c & 1])));
+            if (elected)
+                umma_commit(smem_addr(&mbar[c & 1]));
         }
         // chunk c + 1 goes to the stage chunk c - 1 was read from; the MMAs of
         // chunk c are queued behind it meanwhile
@@ -1053,18 +1172,13 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3x3_tc_chunk(ConvArgs a, int
             if (y0 + rr >= a.h)
                 break;
             const long p = ((long)nb * a.h + y0 + rr) * a.wd + x;
-            const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(rr * nacc * N);
+            const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(rr * N);
             uint32_t r[16];
-            tmem_ld16(lane_base + (uint32_t)c, r);
-            for (int q = 1; q < nacc; q++) {
-                uint32_t t[16];
-                tmem_ld16(lane_base + (uint32_t)(q * N + c), t);
-#pragma unroll
-                for (int m = 0; m < 16; m++)
-                    r[m] = __float_as_uint(__uint_as_float(r[m]) + __uint_as_float(t[m]));
-            }
+            Bias16 bias;
+            load_bias(a, n0 + c, bias);
+            tmem_sum16<1>(lane_base + (uint32_t)c, 0u, r);
             if (x < a.wd && n0 + c < a.cout)
-                store_row16(a, p, n0 + c, r);
+                store_row16(a, p, n0 + c, r, bias);
         }
     } else if (tid == 0) {
         atomicOr(err, 1u);
@@ -1085,11 +1199,17 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3x3_tc_chunk(ConvArgs a, int
 // pixels and rows outside the image, which is the convolution's zero padding.
 // Output row i of a segment reads halo rows i, i + 1, i + 2, so every output
 // row needs one new halo row (the input is read once, not three times).
-// Slot layout (K-major, no swizzle): per 8-channel group the 130 pixels are
-// consecutive 16-byte rows (one TMA box of 8 channels x 130 pixels), groups
-// kStKCBytes apart; a tap (dy, dx) of output row i is the operand starting at
-// slot(i + dy) + 16 dx (SBO 128 B between 8-pixel groups, LBO kStKCBytes
-// between channel groups). Two TMEM accumulators alternate between output
+// Slot layout (K-major, 32-byte swizzle): per 16 channels a plane of kStPlane
+// bytes in which the 130 pixels are consecutive 32-byte rows (one TMA box of
+// 16 channels x 130 pixels; boxes of 8 channels without swizzle copied 16
+// bytes a pixel and took twice the requests); a tap (dy, dx) of output row i
+// is the operand starting at slot(i + dy) + 32 dx (256 B between 8-pixel
+// groups; the swizzle follows address bits, so a start inside a group of 8
+// reads the pixels where they were stored). What bounds it: an MMA of M = 128,
+// K = 16 and N <= 64 takes 32 + N / 4 clocks, the time to read its pixels from
+// shared memory, if a whole warp reaches it and one elected lane issues it (55
+// clocks when the code is one lane's own); layers with few channels are bound
+// by memory instead. Two TMEM accumulators alternate between output
 // rows; each holds `nacc` partial sums (taps spread over independent MMA
 // chains) that the drain adds. The roles (k_conv3x3_strip below) are warp
 // specialised: a producer warp, an MMA warp and four drain warps, linked by
@@ -1098,8 +1218,14 @@ __global__ void __launch_bounds__(kTcThreads) k_conv3x3_tc_chunk(ConvArgs a, int
 // bounded by the global timer; on a timeout the kernel records an error, the
 // other roles stop at their next wait, copies and MMAs in flight are waited
 // for (bounded) and the TMEM is freed.
-constexpr int kStKCBytes = 2176; // 130 pixels x 16 B, padded to a multiple of 128 B
+constexpr int kStPlane = 4352; // 130 pixels x 32 B, padded to a multiple of the swizzle's 256 B
 constexpr int kStHaloPx = kTcM + 2;
+// byte of channel group g (8 channels) of pixel px in a ring slot: the 32-byte
+// swizzle exchanges the two halves of a pixel where address bit 7 is set
+__device__ __forceinline__ int st_chunk(int g, int px)
+{
+    return (g >> 1) * kStPlane + px * 32 + (((g & 1) ^ ((px >> 2) & 1)) << 4);
+}
 // at least the three halo rows one output row reads; three slots (no row
 // prefetched ahead) are taken when they let more CTAs share an SM
 constexpr int kStMaxRing = 8, kStMinRing = 3;
@@ -1132,41 +1258,40 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar)
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-__device__ __forceinline__ void umma_commit(uint32_t bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar));
-}
-
-// Warps 0-3 drain accumulators (TMEM lane quarter = warp), warp 4 loads halo
-// rows by TMA, warp 5 issues the MMAs, warps 6-9 (launched for it only) fill
-// the upsampled channels of a fused upsample + concat input (a.coarse). The
-// warps other than 4 and 5 first copy the weights, which the MMA warp waits
-// for; the first rows are on their way meanwhile. (One warp for the upsampled
-// channels bounded the full-resolution decoder input: 1037 us at 3840 x 2160,
-// 782 us with four.) The roles run ahead of each other as far as the ring (`ring` halo-row slots) and the
-// two accumulators allow, synchronised only by mbarriers:
+// Warps 0-3 drain accumulators, and with two drain sets warps 6-9 too (TMEM
+// lane quarter = warp % 4; the sets share a row's channels), warp 4 loads halo
+// rows by TMA, warp 5 issues the MMAs, the last four warps (launched for it
+// only) fill the upsampled channels of a fused upsample + concat input
+// (a.coarse). The warps other than 4 and 5 first copy the weights, which the
+// MMA warp waits for; the first rows are on their way meanwhile. (One warp for
+// the upsampled channels bounded the full-resolution decoder input: 1037 us at
+// 3840 x 2160, 782 us with four.) The roles run ahead of each other as far as
+// the ring (`ring` halo-row slots) and the two accumulators allow, synchronised
+// only by mbarriers:
 //   full[s]   the halo row in slot s is complete: TMA bytes landed (producer)
-//             and, fused, the upsampled channels stored (warps 6-9) -> MMA
+//             and, fused, the upsampled channels stored -> MMA
 //   empty[s]  the MMAs that read slot s completed (MMA commit -> producer)
 //   acc_full[b]  row accumulator b is complete (MMA commit -> drain)
-//   acc_empty[b] the four drain warps have read accumulator b (drain -> MMA)
+//   acc_empty[b] the drain warps have read accumulator b (drain -> MMA)
 constexpr int kStThreads = 192, kStUpWarps = 4;
 
-__global__ void __launch_bounds__(kStThreads + 32 * kStUpWarps)
-    k_conv3x3_strip(ConvArgs a, const __grid_constant__ CUtensorMap tmap, int ncols, int nacc, int ring, int segs,
-                    int seg_rows, int ntile, uint32_t *err, int withhold_acc_full)
+// (80 registers let four CTAs of 192 threads share an SM.)
+template <int nacc>
+__global__ void __maxnreg__(80)
+    k_conv3x3_strip(ConvArgs a, const __grid_constant__ CUtensorMap tmap, int ncols, int ring, int segs, int seg_rows,
+                    int ntile, int dsets, uint32_t *err, int withhold_acc_full)
 {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     __shared__ uint32_t tmem_holder;
     __shared__ __align__(8) uint64_t full[kStMaxRing], empty[kStMaxRing];
     __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], weights_full;
     __shared__ int abort_flag;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int tiles_x = (a.wd + kTcM - 1) / kTcM;
     const int units = a.n * tiles_x * segs;
     const int KC = a.cin >> 3;
     const int N = ntile, n0 = (int)blockIdx.y * ntile; // this CTA's output channels
-    const int slot_bytes = KC * kStKCBytes;
+    const int slot_bytes = (KC / 2) * kStPlane;
     const int tap_bytes = N * a.cin * 2;
     const uint32_t half_cols = (uint32_t)ncols >> 1;
     const uint32_t raw = smem_addr(smem_raw);
@@ -1175,7 +1300,8 @@ __global__ void __launch_bounds__(kStThreads + 32 * kStUpWarps)
     uint8_t *w_ptr = smem_raw + (w_base - raw);
     const volatile int *abort_v = &abort_flag;
 
-    const int CG = a.cc >> 3;  // channel groups filled by warps 6-9 (upsampled coarse input)
+    const int CG = a.cc >> 3;  // channel groups filled by the last warps (upsampled coarse input)
+    const int up_warp = 2 + 4 * dsets;
     if (tid == 0) {
         for (int r = 0; r < ring; r++) {
             mbar_init(&full[r], CG ? 1 + kStUpWarps : 1);
@@ -1183,7 +1309,7 @@ __global__ void __launch_bounds__(kStThreads + 32 * kStUpWarps)
         }
         for (int k = 0; k < 2; k++) {
             mbar_init(&acc_full[k], 1);
-            mbar_init(&acc_empty[k], 4);
+            mbar_init(&acc_empty[k], 4 * dsets);
         }
         mbar_init(&weights_full, blockDim.x - 64u); // every thread of the warps that copy them
         abort_flag = 0;
@@ -1207,7 +1333,7 @@ __global__ void __launch_bounds__(kStThreads + 32 * kStUpWarps)
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
-    const uint32_t tmem = tmem_holder;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_holder, 0);
     if (copies) {
         cp_async_commit();
         cp_async_wait<0>();
@@ -1218,18 +1344,17 @@ __global__ void __launch_bounds__(kStThreads + 32 * kStUpWarps)
     if (tid == 0)
         pdl_start();
 
-    if (warp >= 6) {
+    if (warp >= up_warp) {
         // ---- upsampled channels of a fused concat input: fine pixel x of
         // halo row y reads coarse pixel (x >> 1, y >> 1). 16-byte cp.async
-        // copies (consecutive lanes on consecutive channel groups of a coarse
-        // pixel), the warps taking every fourth run of 32, one commit group per
-        // row; a row is published (fence to the async proxy, arrive on its full
+        // copies (consecutive lanes on consecutive pixels, a lane all channel
+        // groups of its pixel), one commit group per row; a row is published (fence to the async proxy, arrive on its full
         // barrier) once `lag` newer rows are in flight, lag <= ring - 3 so the
         // MMA warp can always release the slot a warp waits for.
         if (CG) {
             const int hc = a.h >> 1, wc = a.wd >> 1;
             constexpr int kUp = 32 * kStUpWarps;
-            const int npc = kStHaloPx * CG, dp = kUp / CG, dg = kUp % CG, first = 32 * (warp - 6) + lane;
+            const int first = 32 * (warp - up_warp) + lane;
             const int lag = min(2, ring - 3);
             int slot = 0, phase = 0, pub_slot = 0, pending = 0;
             auto publish = [&]() {
@@ -1258,18 +1383,12 @@ __global__ void __launch_bounds__(kStThreads + 32 * kStUpWarps)
                     const bool row_ok = yy >= 0 && yy < a.h;
                     const bf16 *crow = a.coarse + ((long)nb * hc + (row_ok ? yy >> 1 : 0)) * wc * a.cc;
                     uint8_t *dst = smem_raw + (ring_base - raw) + slot * slot_bytes;
-                    int pp = first / CG, g = first - (first / CG) * CG;
-                    for (int idx = first; idx < npc; idx += kUp) {
+                    for (int pp = first; pp < kStHaloPx; pp += kUp) {
                         const int xx = x0 - 1 + pp;
                         const bool in = row_ok && xx >= 0 && xx < a.wd;
-                        cp_async16(dst + g * kStKCBytes + pp * 16, in ? crow + (long)(xx >> 1) * a.cc + 8 * g : a.coarse,
-                                   in);
-                        g += dg;
-                        pp += dp;
-                        if (g >= CG) {
-                            g -= CG;
-                            pp++;
-                        }
+                        const bf16 *src = in ? crow + (long)(xx >> 1) * a.cc : a.coarse;
+                        for (int g = 0; g < CG; g++)
+                            cp_async16(dst + st_chunk(g, pp), src + (in ? 8 * g : 0), in);
                     }
                     cp_async_commit();
                     pending++;
@@ -1295,7 +1414,7 @@ __global__ void __launch_bounds__(kStThreads + 32 * kStUpWarps)
                 abort_flag = 1;
         }
     } else if (warp == 4) {
-        // ---- producer: one TMA row (the KC - CG boxes of 8 channels x 130
+        // ---- producer: one TMA row ((KC - CG) / 2 boxes of 16 channels x 130
         // pixels of `in`) per halo row
         if (lane == 0) {
             const uint64_t tmap_ptr = reinterpret_cast<uint64_t>(&tmap);
@@ -1319,10 +1438,10 @@ __global__ void __launch_bounds__(kStThreads + 32 * kStUpWarps)
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(row_tx)
                                  : "memory");
                     const uint32_t dst = ring_base + (uint32_t)(slot * slot_bytes);
-                    for (int kc = CG; kc < KC; kc++)
+                    for (int kp = CG / 2; kp < KC / 2; kp++)
                         asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-                                     "[%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst + (uint32_t)(kc * kStKCBytes)),
-                                     "l"(tmap_ptr), "r"(8 * (kc - CG)), "r"(x0 - 1), "r"(ya - 1 + h), "r"(nb),
+                                     "[%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst + (uint32_t)(kp * kStPlane)),
+                                     "l"(tmap_ptr), "r"(16 * kp - 8 * CG), "r"(x0 - 1), "r"(ya - 1 + h), "r"(nb),
                                      "r"(bar)
                                      : "memory");
                     last_phase[slot] = phase;
@@ -1340,90 +1459,101 @@ __global__ void __launch_bounds__(kStThreads + 32 * kStUpWarps)
         }
     } else if (warp == 5) {
         // ---- MMA issue: 9 taps x cin / 16 steps per output row
-        if (lane == 0) {
-            const uint32_t idesc =
-                (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kTcM >> 4) << 24);
-            const uint64_t a_hi = umma_desc(0, kStKCBytes, 128), b_hi = umma_desc(0, 128, (uint32_t)(KC * 128));
-            const uint32_t a_lo_base = ring_base >> 4, a_lo_slot = (uint32_t)slot_bytes >> 4;
-            const uint32_t b_lo_base = w_base >> 4, b_lo_tap = (uint32_t)tap_bytes >> 4;
-            int row_slot = 0;            // slot of the unit's halo row i
-            int wait_slot = 0, wait_phase = 0, waited = 0; // next halo row to see complete
-            int gi = 0;                  // output rows so far
-            int halo = 0;                // halo rows of earlier units
-            bool ok = mbar_wait_role(smem_addr(&weights_full), 0, abort_v);
-            for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
-                const int sg = u % segs;
-                const int ya = sg * seg_rows;
-                const int nout = min(a.h, ya + seg_rows) - ya;
-                if (nout <= 0)
-                    continue;
-                for (int i = 0; i < nout && ok; i++, gi++) {
-                    while (ok && waited < halo + i + 3) {
-                        ok = mbar_wait_role(smem_addr(&full[wait_slot]), (uint32_t)wait_phase, abort_v);
-                        if (ok) {
-                            waited++;
-                            if (++wait_slot == ring) {
-                                wait_slot = 0;
-                                wait_phase ^= 1;
-                            }
+        const uint32_t elected = elect_one();
+        const uint32_t idesc =
+            (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kTcM >> 4) << 24);
+        const uint64_t a_hi = umma_desc(0, 16, 256) | (6ull << 61), b_hi = umma_desc(0, 128, (uint32_t)(KC * 128));
+        const uint32_t a_lo_base = ring_base >> 4, a_lo_slot = (uint32_t)slot_bytes >> 4;
+        const uint32_t b_lo_base = w_base >> 4, b_lo_tap = (uint32_t)tap_bytes >> 4;
+        // the whole warp waits, and goes on or gives up together
+        auto wait = [&](uint64_t &bar, int phase) {
+            return __all_sync(0xffffffffu, mbar_wait_role(smem_addr(&bar), (uint32_t)phase, abort_v)) != 0;
+        };
+        int row_slot = 0;            // slot of the unit's halo row i
+        int wait_slot = 0, wait_phase = 0, waited = 0; // next halo row to see complete
+        int gi = 0;                  // output rows so far
+        int halo = 0;                // halo rows of earlier units
+        bool ok = wait(weights_full, 0);
+        for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
+            const int sg = u % segs;
+            const int ya = sg * seg_rows;
+            const int nout = min(a.h, ya + seg_rows) - ya;
+            if (nout <= 0)
+                continue;
+            for (int i = 0; i < nout && ok; i++, gi++) {
+                while (ok && waited < halo + i + 3) {
+                    ok = wait(full[wait_slot], wait_phase);
+                    if (ok) {
+                        waited++;
+                        if (++wait_slot == ring) {
+                            wait_slot = 0;
+                            wait_phase ^= 1;
                         }
                     }
-                    const int b = gi & 1;
-                    if (ok)
-                        ok = mbar_wait_role(smem_addr(&acc_empty[b]), (uint32_t)(((gi >> 1) & 1) ^ 1), abort_v);
-                    if (!ok)
-                        break;
-                    asm volatile("tcgen05.fence::after_thread_sync;");
-                    const uint32_t acc = tmem + (uint32_t)b * half_cols;
-                    uint32_t slot_lo[3];
+                }
+                const int b = gi & 1;
+                if (ok)
+                    ok = wait(acc_empty[b], ((gi >> 1) & 1) ^ 1);
+                if (!ok)
+                    break;
+                asm volatile("tcgen05.fence::after_thread_sync;");
+                const uint32_t acc = tmem + (uint32_t)b * half_cols;
+                uint32_t slot_lo[3];
 #pragma unroll
-                    for (int dy = 0; dy < 3; dy++) {
-                        int sl = row_slot + dy;
-                        sl = sl >= ring ? sl - ring : sl;
-                        slot_lo[dy] = a_lo_base + (uint32_t)sl * a_lo_slot;
-                    }
-                    for (int j = 0; j < KC / 2; j++) {
+                for (int dy = 0; dy < 3; dy++) {
+                    int sl = row_slot + dy;
+                    sl = sl >= ring ? sl - ring : sl;
+                    slot_lo[dy] = a_lo_base + (uint32_t)sl * a_lo_slot;
+                }
+                for (int j = 0; j < KC / 2; j++) {
 #pragma unroll
-                        for (int tap = 0; tap < 9; tap++) {
-                            const int dy = tap / 3, dx = tap % 3;
-                            const uint64_t ad =
-                                a_hi | (uint64_t)(slot_lo[dy] + (uint32_t)dx + (uint32_t)j * (2 * kStKCBytes / 16));
-                            const uint64_t bd =
-                                b_hi | (uint64_t)(b_lo_base + (uint32_t)tap * b_lo_tap + (uint32_t)j * (2 * 128 / 16));
-                            const uint32_t accumulate = (j > 0 || tap >= nacc) ? 1u : 0u;
-                            const uint32_t dst = acc + (uint32_t)((tap & (nacc - 1)) * N);
-                            asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                                         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(dst),
-                                         "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate));
-                        }
+                    for (int tap = 0; tap < 9; tap++) {
+                        const int dy = tap / 3, dx = tap % 3;
+                        umma(acc + (uint32_t)((tap & (nacc - 1)) * N),
+                             a_hi | (uint64_t)(slot_lo[dy] + (uint32_t)(2 * dx) + (uint32_t)j * (kStPlane / 16)),
+                             b_hi | (uint64_t)(b_lo_base + (uint32_t)tap * b_lo_tap + (uint32_t)j * (2 * 128 / 16)),
+                             idesc, j > 0 || tap >= nacc, elected);
                     }
+                }
+                if (elected) {
                     // (withhold_acc_full: a diagnostic launch that never signals
                     // the drain warps, whose bounded waits then run out)
                     if (!withhold_acc_full)
                         umma_commit(smem_addr(&acc_full[b]));
                     // halo row i is not read by later rows of the unit
                     umma_commit(smem_addr(&empty[row_slot]));
-                    row_slot = row_slot + 1 == ring ? 0 : row_slot + 1;
                 }
-                if (!ok)
-                    break;
-                // the unit's last two halo rows
-                for (int k = 0; k < 2; k++) {
-                    umma_commit(smem_addr(&empty[row_slot]));
-                    row_slot = row_slot + 1 == ring ? 0 : row_slot + 1;
-                }
-                halo += nout + 2;
+                __syncwarp();
+                row_slot = row_slot + 1 == ring ? 0 : row_slot + 1;
             }
             if (!ok)
-                abort_flag = 1;
-            // the MMAs of the last row issued are complete before TMEM is freed
-            if (gi > 0 && !mbar_wait(smem_addr(&acc_full[(gi - 1) & 1]), (uint32_t)(((gi - 1) >> 1) & 1)))
-                abort_flag = 1;
+                break;
+            // the unit's last two halo rows
+            for (int k = 0; k < 2; k++) {
+                if (elected)
+                    umma_commit(smem_addr(&empty[row_slot]));
+                __syncwarp();
+                row_slot = row_slot + 1 == ring ? 0 : row_slot + 1;
+            }
+            halo += nout + 2;
         }
+        if (!ok)
+            abort_flag = 1;
+        // the MMAs of the last row issued are complete before TMEM is freed
+        if (lane == 0 && gi > 0 && !mbar_wait(smem_addr(&acc_full[(gi - 1) & 1]), (uint32_t)(((gi - 1) >> 1) & 1)))
+            abort_flag = 1;
     } else {
-        // ---- drain: warp w reads TMEM lanes 32w..32w+31 (pixels x0 + 32w + lane)
+        // ---- drain: warp w reads TMEM lanes 32 (w % 4) .. + 31 (pixels x0 +
+        // 32 (w % 4) + lane), 16 channels at a time, a set every `dsets`th 16.
+        // A row's drain has to keep up with its MMAs, which hold the path that
+        // loads and stores take, so what it loads is asked for early: the bias
+        // one group ahead (loaded when it was needed, it made a drain of 64
+        // channels 4000 clocks long against 1760 of MMAs).
         int gi = 0;
         bool ok = true;
+        const int set = warp < 4 ? 0 : 1, quarter = warp & 3;
+        Bias16 bias;
+        load_bias(a, n0 + 16 * set, bias);
         for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
             const int sg = u % segs, tx = (u / segs) % tiles_x, nb = u / (segs * tiles_x);
             const int x0 = tx * kTcM, ya = sg * seg_rows;
@@ -1437,20 +1567,14 @@ __global__ void __launch_bounds__(kStThreads + 32 * kStUpWarps)
                 if (!ok)
                     break;
                 asm volatile("tcgen05.fence::after_thread_sync;");
-                const int x = x0 + warp * 32 + lane;
+                const int x = x0 + quarter * 32 + lane;
                 const long p = ((long)nb * a.h + ya + i) * a.wd + x;
-                const uint32_t acc = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)b * half_cols;
-                for (int c = 0; c < N; c += 16) {
+                const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)b * half_cols;
+                for (int c = 16 * set; c < N; c += 16 * dsets) {
                     uint32_t r[16];
-                    tmem_ld16(acc + (uint32_t)c, r);
-                    for (int q = 1; q < nacc; q++) {
-                        uint32_t t[16];
-                        tmem_ld16(acc + (uint32_t)(q * N + c), t);
-#pragma unroll
-                        for (int k = 0; k < 16; k++)
-                            r[k] = __float_as_uint(__uint_as_float(r[k]) + __uint_as_float(t[k]));
-                    }
-                    if (c + 16 >= N) {
+                    tmem_sum16<nacc>(acc + (uint32_t)c, (uint32_t)N, r);
+                    const bool last = c + 16 * dsets >= N;
+                    if (last) {
                         // the accumulator is read: hand it back to the MMA warp
                         asm volatile("tcgen05.fence::before_thread_sync;");
                         __syncwarp();
@@ -1458,7 +1582,9 @@ __global__ void __launch_bounds__(kStThreads + 32 * kStUpWarps)
                             mbar_arrive(smem_addr(&acc_empty[b]));
                     }
                     if (x < a.wd && n0 + c < a.cout)
-                        store_row16(a, p, n0 + c, r);
+                        store_row16(a, p, n0 + c, r, bias);
+                    if (dsets * 16 < N)
+                        load_bias(a, n0 + (last ? 16 * set : c + 16 * dsets), bias);
                 }
             }
         }
@@ -1684,6 +1810,7 @@ int split_channels(int N, long ctas)
 
 struct StripPlan {
     int ntile = 0; // output channels per CTA
+    int dsets = 1; // drain sets of four warps
     int ring = 0, smem = 0, grid = 0, segs = 0, seg_rows = 0, ncols = 0, nacc = 1, per_sm = 1;
 };
 
@@ -1691,14 +1818,11 @@ struct StripPlan {
 // 512 TMEM columns of an SM), then the deepest ring that fits; the rows of
 // every 128-pixel column are cut into segments so that one wave of CTAs
 // covers the layer.
-#ifndef VVPT_STRIP_FUSED_ONE_CTA
-#define VVPT_STRIP_FUSED_ONE_CTA 0
-#endif
 bool plan_strip(const ConvArgs &a, StripPlan &pl)
 {
     if (a.cin % 16 || a.cin < 16 || a.cout > 256 || a.cout < 1 || (reinterpret_cast<uintptr_t>(a.in) & 15))
         return false;
-    if (a.cc && (a.cc % 8 || a.cc >= a.cin || a.h % 2 || a.wd % 2 || (reinterpret_cast<uintptr_t>(a.coarse) & 15)))
+    if (a.cc && (a.cc % 16 || a.cc >= a.cin || a.h % 2 || a.wd % 2 || (reinterpret_cast<uintptr_t>(a.coarse) & 15)))
         return false;
     static int nsm = 0, sm_smem = 0, optin = 0, reserved = 0;
     if (!nsm) {
@@ -1712,68 +1836,84 @@ bool plan_strip(const ConvArgs &a, StripPlan &pl)
     if (!tensor_map_encoder())
         return false;
     const int N = (a.cout + 15) & ~15;
-    const int wbytes = 9 * N * a.cin * 2, slot = (a.cin / 8) * kStKCBytes;
+    const int wbytes = 9 * N * a.cin * 2, slot = (a.cin / 16) * kStPlane;
     int ncols = 32;
     while (ncols < 2 * N)
         ncols <<= 1;
     constexpr int kStatic = 2048; // mbarriers, TMEM address, flags (1 KB aligned)
-    for (int c = (a.cc && VVPT_STRIP_FUSED_ONE_CTA) ? 1 : 4; c >= 1; c--) {
-        if (c * ncols > 512)
-            continue;
+    auto ring_of = [&](int c) {
         const int dyn = std::min(optin - kStatic, sm_smem / c - reserved - kStatic);
-        const int ring = std::min(kStMaxRing, (dyn - 1024 - wbytes) / slot);
-        if (ring < kStMinRing)
-            continue;
-        const long cols = (long)a.n * ((a.wd + kTcM - 1) / kTcM);
-        const long ctas = (long)nsm * c;
-        int segs = (int)std::max<long>(1, std::min<long>(a.h, ctas / std::max<long>(1, cols)));
-        const int seg_rows = (a.h + segs - 1) / segs;
-        segs = (a.h + seg_rows - 1) / seg_rows;
-        // accumulators per row: as many independent MMA chains (1, 2 or 4) as
-        // the SM's TMEM leaves room for at this occupancy
-        int nacc = 1, tcols = ncols;
-        for (int q = 4; q >= 2; q >>= 1) {
-            int cq = 32;
-            while (cq < 2 * q * N)
-                cq <<= 1;
-            if (c * cq <= 512) {
-                nacc = q;
-                tcols = cq;
-                break;
-            }
-        }
-        // a small image: fewer output channels per CTA (the accumulators, and
-        // with them the order of the sums, stay as planned for all of them)
-        pl.grid = (int)std::min<long>(cols * segs, ctas);
-        pl.ntile = split_channels(N, pl.grid);
-        if (pl.ntile != N)
-            for (tcols = 32; tcols < 2 * nacc * pl.ntile;)
-                tcols <<= 1;
-        // no more shared memory than the rows of a CTA's run need, so that the
-        // next launch can begin beside this one
-        pl.ring = std::min<long>(ring, cols * segs <= ctas ? std::max(kStMinRing, seg_rows + 2) : kStMaxRing);
-        pl.smem = 1024 + 9 * pl.ntile * a.cin * 2 + pl.ring * slot;
-        pl.segs = segs;
-        pl.seg_rows = seg_rows;
-        pl.ncols = tcols;
-        pl.nacc = nacc;
-        pl.per_sm = c;
-        return true;
+        return std::min(kStMaxRing, (dyn - 1024 - wbytes) / slot);
+    };
+    // accumulators per row (independent MMA chains, whose sums the drain adds):
+    // 1, 2 or 4, as many as the TMEM of an SM holds beside the other CTAs of
+    // the most that fit there with a ring of at most eight rows. This fixes
+    // the order of the sums, whatever occupancy and ring are chosen below.
+    int most = 0, nacc = 1;
+    for (int c = 4; c >= 1 && !most; c--)
+        if (c * ncols <= 512 && std::min(8, ring_of(c)) >= kStMinRing)
+            most = c;
+    if (!most)
+        return false;
+    for (int q = 4; q >= 2 && nacc == 1; q >>= 1) {
+        int cq = 32;
+        while (cq < 2 * q * N)
+            cq <<= 1;
+        if (most * cq <= 512)
+            nacc = q;
     }
-    return false;
+    int tcols = 32;
+    while (tcols < 2 * nacc * N)
+        tcols <<= 1;
+    // CTAs per SM. A fused upsample + concat input takes one, with the deepest
+    // ring: its upsample warps then run rows ahead of the MMAs (the
+    // half-resolution decoder input at 3840 x 2160, 192 to 64 channels: 324 us,
+    // against 450 us for upsampling, concatenating and convolving it
+    // separately; the full-resolution one 583 against 650 with two per SM).
+    const int c = a.cc ? 1 : most;
+    const int ring = ring_of(c);
+    const long cols = (long)a.n * ((a.wd + kTcM - 1) / kTcM);
+    const long ctas = (long)nsm * c;
+    int segs = (int)std::max<long>(1, std::min<long>(a.h, ctas / std::max<long>(1, cols)));
+    const int seg_rows = (a.h + segs - 1) / segs;
+    segs = (a.h + seg_rows - 1) / seg_rows;
+    // a small image: fewer output channels per CTA (the accumulators stay as
+    // planned for all of them)
+    pl.grid = (int)std::min<long>(cols * segs, ctas);
+    pl.ntile = split_channels(N, pl.grid);
+    if (pl.ntile != N)
+        for (tcols = 32; tcols < 2 * nacc * pl.ntile;)
+            tcols <<= 1;
+    // no more shared memory than the rows of a CTA's run need, so that the
+    // next launch can begin beside this one
+    pl.ring = (int)std::min<long>(ring, cols * segs <= ctas ? std::max(kStMinRing, seg_rows + 2) : kStMaxRing);
+    pl.smem = 1024 + 9 * pl.ntile * a.cin * 2 + pl.ring * slot;
+    pl.segs = segs;
+    pl.seg_rows = seg_rows;
+    pl.ncols = tcols;
+    pl.nacc = nacc;
+    pl.per_sm = c;
+    // A second set of drain warps where the registers of the CTAs of an SM
+    // leave room for it and there are channels to share (64 channels at
+    // 960 x 540: 72 to 52 us; 32 to 64 at 1920 x 1080: 114 to 95). A fused
+    // input keeps one: its MMAs bound it, and a second set only takes
+    // shared-memory and issue slots from them (96 to 32 channels at
+    // 3840 x 2160: 583 us with one, 615 with two).
+    pl.dsets = c <= 2 && pl.ntile >= 32 && !a.cc ? 2 : 1;
+    return true;
 }
 
 // rank-4 map over the NHWC input {C, W, H, N} (the cin - cc channels of `in`);
-// box = 8 channels x 130 pixels
+// box = 16 channels x 130 pixels, stored with the 32-byte swizzle (st_chunk)
 bool encode_input_map(const ConvArgs &a, CUtensorMap &m)
 {
     const int c = a.cin - a.cc;
     const cuuint64_t dims[4] = {(cuuint64_t)c, (cuuint64_t)a.wd, (cuuint64_t)a.h, (cuuint64_t)a.n};
     const cuuint64_t strides[3] = {(cuuint64_t)c * 2, (cuuint64_t)a.wd * c * 2, (cuuint64_t)a.h * a.wd * c * 2};
-    const cuuint32_t box[4] = {8, (cuuint32_t)kStHaloPx, 1, 1};
+    const cuuint32_t box[4] = {16, (cuuint32_t)kStHaloPx, 1, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     return tensor_map_encoder()(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16 *>(a.in), dims, strides, box,
-                                estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B,
                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -1781,35 +1921,39 @@ bool encode_input_map(const ConvArgs &a, CUtensorMap &m)
 
 namespace {
 
+template <int nacc>
+void launch_strip_nacc(const ConvArgs &a, const CUtensorMap &tmap, const StripPlan &pl, int withhold, cudaStream_t s,
+                       uint32_t *err)
+{
+    static int attr_smem = 0;
+    if (pl.smem > attr_smem) {
+        cudaFuncSetAttribute(k_conv3x3_strip<nacc>, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem);
+        cudaFuncSetAttribute(k_conv3x3_strip<nacc>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             cudaSharedmemCarveoutMaxShared);
+        attr_smem = pl.smem;
+    }
+    launch_pdl(k_conv3x3_strip<nacc>, dim3((unsigned)pl.grid, (unsigned)(((a.cout + 15) & ~15) / pl.ntile)),
+               kStThreads + 128 * (pl.dsets - 1) + (a.cc ? 32 * kStUpWarps : 0), pl.smem, s, a, tmap, pl.ncols, pl.ring,
+               pl.segs, pl.seg_rows, pl.ntile, pl.dsets, err, withhold);
+}
+
 // The strip kernel for `a` when it takes the layer; false (nothing launched)
-// otherwise. A fused upsample + concat input is taken only where two or more
-// CTAs share an SM: the warp that copies the upsampled channels keeps up
-// there, while with one CTA per SM (level 1, 219 KB of weights and ring) the
-// unfused path measured faster (0.47 vs 0.57 ms at 1920 x 1080).
+// otherwise.
 bool launch_strip(const ConvArgs &a, cudaStream_t s, uint32_t *err, ConvKernels kind)
 {
     StripPlan pl;
     CUtensorMap tmap;
-    // A fused layer (upsample + concat in the kernel) needs two CTAs per SM
-    // to pay: at one (the half-resolution decoder input, whose weights leave
-    // room for one) it took 581 us against 450 us for the separate
-    // upsample-concat and convolution at 3840 x 2160.
-    if (!err || kind == kConvTiles || !plan_strip(a, pl) || (a.cc && pl.per_sm < 2 && !VVPT_STRIP_FUSED_ONE_CTA) ||
-        !encode_input_map(a, tmap))
+    if (!err || kind == kConvTiles || !plan_strip(a, pl) || !encode_input_map(a, tmap))
         return false;
     if (kind == kConvPersistent)
         pl.grid = std::min(pl.grid, 16);
-    static int attr_smem = 0;
-    if (pl.smem > attr_smem) {
-        cudaFuncSetAttribute(k_conv3x3_strip, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem);
-        cudaFuncSetAttribute(k_conv3x3_strip, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared);
-        attr_smem = pl.smem;
-    }
     const int withhold = g_inject_wait_timeout.exchange(false) ? 1 : 0;
-    launch_pdl(k_conv3x3_strip, dim3((unsigned)pl.grid, (unsigned)(((a.cout + 15) & ~15) / pl.ntile)),
-               kStThreads + (a.cc ? 32 * kStUpWarps : 0), pl.smem, s, a, tmap, pl.ncols, pl.nacc, pl.ring, pl.segs,
-               pl.seg_rows, pl.ntile, err, withhold);
+    if (pl.nacc == 4)
+        launch_strip_nacc<4>(a, tmap, pl, withhold, s, err);
+    else if (pl.nacc == 2)
+        launch_strip_nacc<2>(a, tmap, pl, withhold, s, err);
+    else
+        launch_strip_nacc<1>(a, tmap, pl, withhold, s, err);
     return true;
 }
 
@@ -1862,8 +2006,8 @@ void conv3x3(const ConvArgs &a_in, cudaStream_t s, uint32_t *err, ConvKernels ki
             int cols = 32;
             while (cols < rows * nt)
                 cols <<= 1;
-            launch_pdl(k_conv3x3_tc_chunk, dim3((unsigned)blocks, (unsigned)(N / nt)), kTcThreads, smem, s, a, cols, 1,
-                       rows, nt, err);
+            launch_pdl(k_conv3x3_tc_chunk, dim3((unsigned)blocks, (unsigned)(N / nt)), kTcThreads, smem, s, a, cols, rows,
+                       nt, err);
         }
         else
             launch_pdl(k_conv3x3_tc, dim3((unsigned)tiles), kTcThreads, tc_smem_bytes(N), s, a, ncols, err);
