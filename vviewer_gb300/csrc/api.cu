@@ -87,6 +87,16 @@ vvpt_status make_render_params(vvpt_ctx *ctx, const vvpt_scene *scene, const vvp
     return VVPT_OK;
 }
 
+// Path slots of a render whose tuning leaves them open. More slots mean fewer,
+// larger launches, and paths that start together: their rays stay neighbours
+// on the image for longer, and less of the time goes by waiting for a launch's
+// last rays. 2^20 slots (0.3 GB with their queues), 2^22 and 2^24 (4.8 GB):
+// 225, 196 and 184 ms on the 1080p x 32 medium scene, 62, 52 and 51 ms on the
+// 1919 x 1079 x 16 sky scene. A render has at most one slot per work item. (The
+// job engine keeps 2^20: with several jobs in flight a larger pool only mixes
+// their scenes, 180 ms against 219 with 2^22 for twelve previews.)
+constexpr uint32_t kDefaultSlots = 1u << 24, kSmallPoolSlots = 1u << 20;
+
 // seven 32-byte and one 16-byte member per slot
 size_t path_state_bytes(size_t slots)
 {
@@ -514,8 +524,19 @@ VVPT_API vvpt_status vvpt_render(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_sc
                 VV_CUDA(cudaMemsetAsync(d_out[k], 0, img_bytes, vv_stream(ctx)), "clear outputs");
     } else {
         // ---- path state and queues
-        uint32_t slots = ctx->tuning.slots ? ctx->tuning.slots : (1u << 20);
+        uint32_t slots = ctx->tuning.slots ? ctx->tuning.slots : kDefaultSlots;
         slots = std::max<uint32_t>(32u, std::min<uint32_t>(slots, hp.total_items));
+        const size_t rb = (size_t)hp.total_items * sizeof(float4);
+        VV_CUDA(ctx->results.reserve(3 * aligned256(rb)), "cudaMalloc batch results");
+        if (!ctx->tuning.slots && slots > kSmallPoolSlots &&
+            (ctx->state.reserve(path_state_bytes(slots)) != cudaSuccess ||
+             ctx->queues.reserve(queue_bytes(slots)) != cudaSuccess)) {
+            // no room for the default pool
+            cudaGetLastError();
+            ctx->state.release();
+            ctx->queues.release();
+            slots = kSmallPoolSlots;
+        }
         const size_t n = slots;
         const size_t u4 = n * sizeof(uint32_t);
         auto aligned = [](size_t b) { return aligned256(b); };
@@ -530,9 +551,6 @@ VVPT_API vvpt_status vvpt_render(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_sc
         VV_CUDA(ctx->queues.reserve(queue_bytes(n)), "cudaMalloc queues");
         const Queues q = carve_queues(ctx->queues.as<char>(), n);
 
-        const size_t rb = (size_t)hp.total_items * sizeof(float4);
-        size_t rneed = 3 * aligned(rb);
-        VV_CUDA(ctx->results.reserve(rneed), "cudaMalloc batch results");
         base = ctx->results.as<char>();
         BatchResults br;
         br.rad = (float4 *)take(rb);
@@ -551,7 +569,11 @@ VVPT_API vvpt_status vvpt_render(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_sc
         shape.block = ctx->tuning.threads_per_block ? (int)ctx->tuning.threads_per_block : 256;
         int bps = ctx->tuning.blocks_per_sm ? (int)ctx->tuning.blocks_per_sm : 4;
         shape.grid = std::max(1, ctx->num_sms * bps);
-        const int K = ctx->tuning.iterations_per_graph ? (int)ctx->tuning.iterations_per_graph : 8;
+        // Iterations between checks of the counters. Up to this many and as
+        // many again in flight run empty once the last path has ended: 8 took
+        // 48 iterations, 4 takes 40, where a 256 x 256 preview needs 34
+        // (3.22 and 3.07 ms)
+        const int K = ctx->tuning.iterations_per_graph ? (int)ctx->tuning.iterations_per_graph : 4;
 
         cudaEvent_t tev[2];
         cudaEventCreate(&tev[0]);
@@ -571,6 +593,7 @@ VVPT_API vvpt_status vvpt_render(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_sc
         const uint64_t max_iters =
             (uint64_t)hp.batch_size * (hp.depth + 2) * ((hp.total_items + slots - 1) / slots + 1) + 64;
 
+        bool reduced = false; // launch_reduce already queued
         if (info->flags & VVPT_RENDER_PROFILE_KERNELS) {
             // one kernel at a time with events around each launch
             static const char *names[K_NUM] = {"k_regen", "k_trace", "k_partition", "k_walk", "k_shade"};
@@ -635,8 +658,13 @@ VVPT_API vvpt_status vvpt_render(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_sc
             ctx->profile = prof;
             stats.iterations = it + 1;
         } else {
-        // capture K iterations (K even keeps the ping-pong phase aligned)
+        // The first K iterations go out as they are, and run while the graph of
+        // K iterations is captured and instantiated (K even keeps the ping-pong
+        // phase aligned).
         const int Ke = (K + 1) & ~1;
+        for (int it = 0; it < Ke; it++)
+            launch_iteration(jt, ps, q, it & 1, shape, vv_stream(ctx));
+        VV_CUDA(cudaGetLastError(), "launch iteration");
         cudaGraph_t graph;
         cudaGraphExec_t exec;
         VV_CUDA(cudaStreamBeginCapture(vv_stream(ctx), cudaStreamCaptureModeThreadLocal), "begin capture");
@@ -661,7 +689,6 @@ VVPT_API vvpt_status vvpt_render(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_sc
         bool done = false;
         vvpt_status loop_status = VVPT_OK;
         // keep one graph in flight ahead of the counter check
-        VV_CUDA(cudaGraphLaunch(exec, vv_stream(ctx)), "graph launch");
         VV_CUDA(cudaEventRecord(ev[0], vv_stream(ctx)), "event");
         launched = 1;
         iters += Ke;
@@ -693,17 +720,26 @@ VVPT_API vvpt_status vvpt_render(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_sc
                 break;
             }
         }
-        VV_CUDA(cudaStreamSynchronize(vv_stream(ctx)), "render");
+        // every item is done: the last graph finds nothing to do, and the
+        // counters just read are final
+        if (loop_status == VVPT_OK) {
+            launch_reduce(hp, br, d_out[0], d_out[1], d_out[2], d_out[3], vv_stream(ctx));
+            cudaEventRecord(tev[1], vv_stream(ctx));
+        }
+        const cudaError_t se = cudaStreamSynchronize(vv_stream(ctx));
         cudaGraphExecDestroy(exec);
         cudaEventDestroy(ev[0]);
         cudaEventDestroy(ev[1]);
+        VV_CUDA(se, "render");
         if (loop_status != VVPT_OK)
             return loop_status;
+        reduced = true;
         stats.iterations = iters;
         stats.kernel_launches += (uint64_t)iters * kKernelsPerIteration;
         }
-        VV_CUDA(cudaMemcpy(ctx->counters_pinned, q.counters, C_COUNT * sizeof(uint32_t), cudaMemcpyDeviceToHost),
-                "final counters");
+        if (!reduced)
+            VV_CUDA(cudaMemcpy(ctx->counters_pinned, q.counters, C_COUNT * sizeof(uint32_t), cudaMemcpyDeviceToHost),
+                    "final counters");
         stats.segments = ctx->counters_pinned[C_SEGMENTS];
         stats.shadow_rays = ctx->counters_pinned[C_SHADOW];
         stats.emitter_rays = ctx->counters_pinned[C_NEE];
@@ -711,10 +747,12 @@ VVPT_API vvpt_status vvpt_render(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_sc
         if (ctx->counters_pinned[C_ERR])
             return fail(ctx, VVPT_ERR_DEVICE, "device status word set: " + std::to_string(ctx->counters_pinned[C_ERR]));
 
-        launch_reduce(hp, br, d_out[0], d_out[1], d_out[2], d_out[3], vv_stream(ctx));
+        if (!reduced) {
+            launch_reduce(hp, br, d_out[0], d_out[1], d_out[2], d_out[3], vv_stream(ctx));
+            VV_CUDA(cudaEventRecord(tev[1], vv_stream(ctx)), "event");
+        }
         stats.kernel_launches += 1;
         VV_CUDA(cudaGetLastError(), "launch reduce");
-        VV_CUDA(cudaEventRecord(tev[1], vv_stream(ctx)), "event");
         VV_CUDA(cudaEventSynchronize(tev[1]), "render");
         float ms = 0.0f;
         cudaEventElapsedTime(&ms, tev[0], tev[1]);
