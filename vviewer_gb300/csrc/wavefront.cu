@@ -693,14 +693,22 @@ __device__ __forceinline__ uint32_t extend_key(const SceneView &s, const Hit &h,
 #define VVPT_REFILL_BELOW 20
 #endif
 constexpr uint32_t kLaneFree = 0, kLaneTracing = 1, kLaneDone = 2;
-// Step turns: triangle tests, transitions between the levels and node visits
-// in separate warp steps. Triangle tests when at least VVPT_TRI_TURN_PCT % of
+// Step turns: triangle tests and transitions between the levels wait until
+// enough lanes share them. Triangle tests when at least VVPT_TRI_TURN_PCT % of
 // the tracing lanes have one pending, else transitions when at least
 // VVPT_LEVEL_TURN_PCT % have (or no lane has a node to visit). Entering an
 // instance is a hundred instructions that nearly every warp step executed for
 // one or two lanes: in turns of their own, trace launches of the 1080p medium
 // scene (32 spp) 167 -> 159 ms, of the sky scene 44.1 -> 40.7 ms (thresholds of
 // 10, 25 and 40 %: 163, 159, 159 ms).
+// Within a turn a lane takes up to kTriSteps triangles and then up to
+// kNodeSteps nodes, without another vote: the two ballots and the comparisons
+// of a vote cost about half as much as a node visit, and most lanes that visit
+// a node visit another. One step a turn, one kind of step a turn: 185 ms on the
+// 1080p x 32 medium scene, 50.8 ms on the sky scene, 9.6 ms on the 64-sample
+// Cornell box; these: 170, 48.8 and 9.0 ms (two nodes 178, 49.4 and 9.4; eight
+// 178, 49.1 and 9.2; three triangles 175, 48.9 and 9.1).
+constexpr int kTriSteps = 2, kNodeSteps = 4;
 #ifndef VVPT_TRI_TURN_PCT
 #define VVPT_TRI_TURN_PCT 33
 #endif
@@ -729,9 +737,9 @@ __device__ __forceinline__ uint32_t refill_take(bool free, uint32_t *counter, ui
     return idx;
 }
 
-// One warp step of the refill loops over their `all` tracing lanes, one kind of
-// step at a time: a lane whose kind is not this step's waits (every kind gets
-// its turn, since the lanes that step move on to another kind, finish, or
+// One turn of the refill loops over their `all` tracing lanes: triangle tests or
+// transitions where enough lanes wait for them, then node visits (every kind
+// gets its turn, since the lanes that step move on to another kind, finish, or
 // leave the tracing set). True when this lane's traversal ended.
 __device__ __forceinline__ bool trace_turn(TraceState &st, const TraceCold &ray, TraceStack &stack, const SceneView &s,
                                            bool tracing, int all, uint32_t &err)
@@ -740,14 +748,18 @@ __device__ __forceinline__ bool trace_turn(TraceState &st, const TraceCold &ray,
     const int ntri = 100 * __popc(__ballot_sync(0xFFFFFFFFu, kind == kStepTriangle));
     const int nlev = 100 * __popc(__ballot_sync(0xFFFFFFFFu, kind == kStepLevel));
     if (ntri >= VVPT_TRI_TURN_PCT * all) {
-        if (kind == kStepTriangle)
-            trace_step_triangle(st, ray, stack, s, no_hit());
+#pragma unroll
+        for (int r = 0; r < kTriSteps; r++)
+            if (tracing && trace_kind(st) == kStepTriangle)
+                trace_step_triangle(st, ray, stack, s, no_hit());
     } else if (nlev && (nlev >= VVPT_LEVEL_TURN_PCT * all || nlev + ntri == 100 * all)) {
         if (kind == kStepLevel)
             trace_step_level(st, ray, stack, s, err);
-    } else if (kind == kStepNode) {
-        trace_step_node(st, stack, s, err);
     }
+#pragma unroll
+    for (int r = 0; r < kNodeSteps; r++)
+        if (tracing && trace_kind(st) == kStepNode)
+            trace_step_node(st, stack, s, err);
     return tracing && st.cur == kRefDone;
 }
 
