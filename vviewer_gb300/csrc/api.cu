@@ -97,48 +97,11 @@ vvpt_status make_render_params(vvpt_ctx *ctx, const vvpt_scene *scene, const vvp
 // their scenes, 180 ms against 219 with 2^22 for twelve previews.)
 constexpr uint32_t kDefaultSlots = 1u << 24, kSmallPoolSlots = 1u << 20;
 
-// seven 32-byte and one 16-byte member per slot
-size_t path_state_bytes(size_t slots)
-{
-    return 7 * aligned256(slots * 2 * sizeof(float4)) + aligned256(slots * sizeof(float4));
-}
+size_t path_state_bytes(size_t slots) { return slots * sizeof(PathRecord); }
 
 size_t queue_bytes(size_t slots)
 {
     return 11 * aligned256(slots * sizeof(uint32_t)) + aligned256(C_COUNT * sizeof(uint32_t));
-}
-
-PathState carve_path_state(char *base, size_t n)
-{
-    const size_t pair_bytes = aligned256(n * 2 * sizeof(float4));
-    auto take = [&](size_t b) {
-        char *p = base;
-        base += b;
-        return p;
-    };
-    PathState ps;
-    auto pair = [&](SlotField<float4, 2> &a, SlotField<float4, 2> &b) {
-        a.p = (float4 *)take(pair_bytes);
-        b.p = a.p + 1;
-    };
-    SlotField<float4, 2> meta;
-    pair(ps.hit, meta);
-    ps.meta.p = (uint4 *)meta.p;
-    ps.flags.p = (uint32_t *)meta.p;
-    ps.vol.p = ps.flags.p + 1;
-    ps.job.p = ps.flags.p + 2;
-    ps.hit_inst.p = ps.flags.p + 3;
-    pair(ps.o, ps.d);
-    pair(ps.beta, ps.rad);
-    ps.rng.p = (uint32_t *)ps.beta.p + 3;
-    pair(ps.sh_dir, ps.sh_c);
-    pair(ps.nee_b, ps.nee_c);
-    pair(ps.alb, ps.nrm);
-    pair(ps.cum_rad, ps.cum_alb);
-    ps.item.p = (uint32_t *)ps.cum_rad.p + 3;
-    ps.sample.p = (uint32_t *)ps.cum_alb.p + 3;
-    ps.cum_nrm.p = (float4 *)take(aligned256(n * sizeof(float4)));
-    return ps;
 }
 
 Queues carve_queues(char *base, size_t n)
@@ -547,7 +510,7 @@ VVPT_API vvpt_status vvpt_render(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_sc
             return p;
         };
         VV_CUDA(ctx->state.reserve(path_state_bytes(n)), "cudaMalloc path state");
-        const PathState ps = carve_path_state(ctx->state.as<char>(), n);
+        const PathState ps{ctx->state.as<PathRecord>()};
         VV_CUDA(ctx->queues.reserve(queue_bytes(n)), "cudaMalloc queues");
         const Queues q = carve_queues(ctx->queues.as<char>(), n);
 
@@ -974,11 +937,13 @@ VVPT_API vvpt_status vvpt_render_noalloc(vvpt_ctx *ctx, vvpt_scene *scene, const
     const uint64_t slots64 = std::max<uint64_t>(32, std::min<uint64_t>(items64, kNoAllocMaxSlots));
     auto aligned = [](uint64_t b) { return (b + 255) & ~uint64_t(255); };
     const uint64_t f4 = slots64 * sizeof(float4), u4 = slots64 * sizeof(uint32_t);
-    // (path state counted as 14 f4 and 7 u4 arrays, which sets the renders that
-    // are refused; it takes a little less)
+    // (path state counted as 14 f4 and 7 u4 arrays, 252 bytes a slot, which sets
+    // the renders that are refused; a record takes 256, so one slot in 32 stays
+    // unused)
     const uint64_t need = aligned(sizeof(SingleJobBlock)) + aligned(C_COUNT * sizeof(uint32_t)) + 14 * aligned(f4) +
                           7 * aligned(u4) + aligned(u4) /* idle slots */ + 11 * aligned(u4) +
                           3 * aligned(items64 * sizeof(float4));
+    const uint32_t slots = (uint32_t)std::max<uint64_t>(32, slots64 - slots64 / 32);
     if (need > kNoAllocScratchBytes)
         return fail(ctx, VVPT_ERR_INVALID_ARG,
                     "render needs " + std::to_string(need) + " bytes of scratch; vvpt_render_noalloc has " +
@@ -1016,7 +981,7 @@ VVPT_API vvpt_status vvpt_render_noalloc(vvpt_ctx *ctx, vvpt_scene *scene, const
     SingleJobBlock *djob = reinterpret_cast<SingleJobBlock *>(take(sizeof(SingleJobBlock)));
     Queues q;
     q.counters = reinterpret_cast<uint32_t *>(take(C_COUNT * sizeof(uint32_t)));
-    const PathState ps = carve_path_state(reinterpret_cast<char *>(take(path_state_bytes(slots64))), slots64);
+    const PathState ps{reinterpret_cast<PathRecord *>(take(path_state_bytes(slots)))};
     const JobTable jt = single_job_table(djob, reinterpret_cast<uint32_t *>(take(u4)));
     uint32_t **qs[11] = {&q.ext[0], &q.ext[1],  &q.shade_l, &q.shade_p,  &q.shade_m, &q.conn,
                          &q.nee,    &q.ext_key, &q.walk,    &q.regen[0], &q.regen[1]};
@@ -1032,7 +997,6 @@ VVPT_API vvpt_status vvpt_render_noalloc(vvpt_ctx *ctx, vvpt_scene *scene, const
     LaunchShape shape;
     shape.block = 256;
     shape.grid = std::max(1, ctx->num_sms * 4);
-    const uint32_t slots = (uint32_t)slots64;
     launch_init_slots(q, ps, jt, slots, stream);
     VV_CUDA(cudaGetLastError(), "launch init");
     const uint64_t max_iters =

@@ -173,7 +173,7 @@ bool Engine::init_device(std::string &err)
     if (!ck(state_buf.alloc(path_state_bytes(slots)), "cudaMalloc path state") ||
         !ck(queue_buf.alloc(queue_bytes(slots)), "cudaMalloc queues"))
         return false;
-    ps = carve_path_state(state_buf.as<char>(), slots);
+    ps.slots = state_buf.as<PathRecord>();
     q = carve_queues(queue_buf.as<char>(), slots);
     const size_t tb = aligned256(kMaxJobSlots * sizeof(JobView)) + aligned256(kMaxRanges * 8) +
                       aligned256(kMaxRanges * 4) + aligned256(kMaxJobSlots * 4) + aligned256(sizeof(TableCounters)) +

@@ -150,7 +150,6 @@ vvpt_status make_render_params(vvpt_ctx *ctx, const vvpt_scene *scene, const vvp
 // Path state and queues for `slots` paths carved from one allocation each.
 size_t path_state_bytes(size_t slots);
 size_t queue_bytes(size_t slots);
-PathState carve_path_state(char *base, size_t slots);
 Queues carve_queues(char *base, size_t slots);
 
 // Engine teardown (vvpt_destroy): stops the worker, fails unfinished jobs.

@@ -34,57 +34,50 @@ struct RenderParams {
     const float *blue_noise; // [48][128][128] (sampler 1)
 };
 
-// One member of the path state: element `slot` lies `stride` elements after
-// the first.
-template <class T, int stride>
-struct SlotField {
-    T *p;
-#ifdef __CUDACC__
-    __device__ __forceinline__ T &operator[](uint32_t slot) const { return p[(size_t)slot * stride]; }
-#endif
-};
-
-// Path state, one entry per slot. A slot runs one (pixel, batch) work item:
-// its batch_size samples in order, because the RTGEMS state carries from one
-// sample to the next (raygen.rgen.glsl:36-55).
+// Path state of one slot. A slot runs one (pixel, batch) work item: its
+// batch_size samples in order, because the RTGEMS state carries from one sample
+// to the next (raygen.rgen.glsl:36-55).
 // The queues hold slots in the order in which atomics handed out their places,
-// so a warp's 32 slots lie all over the pool, and what a kernel touches of a
-// slot costs whole 32-byte sectors. Members that are used together therefore
-// share one: a lane reads or writes both with one 32-byte access. (As an array
-// per member, 16 or 4 bytes each, a shading event touched 10 sectors to load
-// and up to 12 to store; 3 and 6 now. 1080p x 32 medium scene: shading 74 to
-// 57 ms, regeneration 26 to 15 ms, a render 255 to 225 ms.)
-struct PathState {
-    // hit record | flags, medium, job index, hit instance
-    SlotField<float4, 2> hit; // t, u, v, prim bits
-    SlotField<uint4, 2> meta; // the next four in one access
-    SlotField<uint32_t, 8> flags;
-    SlotField<uint32_t, 8> vol;
-    SlotField<uint32_t, 8> job; // index into the job table
-    SlotField<uint32_t, 8> hit_inst;
-    // ray
-    SlotField<float4, 2> o; // ray origin (xyz)
-    SlotField<float4, 2> d; // ray direction (xyz)
-    // throughput and radiance
-    SlotField<float4, 2> beta; // throughput (xyz), sampler state (w bits)
-    SlotField<uint32_t, 8> rng;
-    SlotField<float4, 2> rad; // sample radiance (xyz)
-    // shadow ray
-    SlotField<float4, 2> sh_dir; // shadow direction (xyz), tmax (w)
-    SlotField<float4, 2> sh_c;   // unoccluded light contribution (xyz)
-    // emitter ray
-    SlotField<float4, 2> nee_b; // beta for the emitter-ray contribution (xyz), BSDF pdf (w)
-    SlotField<float4, 2> nee_c; // emitter-ray contribution of a path flagged F_NEE (xyz), added by regen or shade
+// so a warp's 32 slots lie all over the pool. What a kernel touches of a slot
+// costs whole 32-byte sectors: members that are used together share one, and a
+// lane reads or writes both with one 32-byte access. What it touches in memory
+// costs more again where it is spread over more lines: tracing and shading keep
+// to the first 128 bytes, regeneration mostly to the second.
+// (1080p x 32 medium scene, an array per member: shading 74 ms, regeneration 26,
+// a render 255; an array per pair of members: 57, 15 and 225; with more slots
+// 54, 14.6 and 170; records: 48, 14.2 and 164. The sky scene, whose paths stay
+// in order for longer, 47.9 and 48.5.)
+struct alignas(128) PathRecord {
+    float4 hit; // t, u, v, prim bits
+    union {
+        struct {
+            uint32_t flags, vol;
+            uint32_t job; // index into the job table
+            uint32_t hit_inst;
+        };
+        uint4 meta; // the four in one access
+    };
+    float4 o, d;   // ray origin, direction (xyz)
+    float4 beta;   // throughput (xyz), sampler state (w bits)
+    float4 rad;    // sample radiance (xyz)
+    float4 sh_dir; // shadow direction (xyz), tmax (w)
+    float4 sh_c;   // unoccluded light contribution (xyz)
+    float4 nee_b;  // beta for the emitter-ray contribution (xyz), BSDF pdf (w)
+    float4 nee_c;  // emitter-ray contribution of a path flagged F_NEE (xyz), added by regen or shade
     // first hit, carried across samples (payload semantics)
-    SlotField<float4, 2> alb;
-    SlotField<float4, 2> nrm;
+    float4 alb, nrm;
     // per-batch sums (cumRadiance/cumAlbedo/cumNormal), and in two of their w:
     // work item within its job (batch * width * height + pixel), sample
-    SlotField<float4, 2> cum_rad;
-    SlotField<uint32_t, 8> item;
-    SlotField<float4, 2> cum_alb;
-    SlotField<uint32_t, 8> sample;
-    SlotField<float4, 1> cum_nrm;
+    float4 cum_rad, cum_alb, cum_nrm;
+    float4 unused;
+};
+static_assert(sizeof(PathRecord) == 256, "path record");
+
+struct PathState {
+    PathRecord *slots;
+#ifdef __CUDACC__
+    __device__ __forceinline__ PathRecord &operator[](uint32_t slot) const { return slots[slot]; }
+#endif
 };
 
 enum CounterIndex {
