@@ -1348,23 +1348,17 @@ __global__ void __maxnreg__(80)
         // ---- upsampled channels of a fused concat input: fine pixel x of
         // halo row y reads coarse pixel (x >> 1, y >> 1). 16-byte cp.async
         // copies (consecutive lanes on consecutive pixels, a lane all channel
-        // groups of its pixel), one commit group per row; a row is published (fence to the async proxy, arrive on its full
-        // barrier) once `lag` newer rows are in flight, lag <= ring - 3 so the
-        // MMA warp can always release the slot a warp waits for.
+        // groups of its pixel); a row is published (fence to the async proxy,
+        // arrive on its full barrier) as soon as its copies have landed. (Held
+        // back until two newer rows were on their way, it had to wait for the
+        // slots of those: with the four slots of the half-resolution decoder
+        // input the MMAs then waited for every row, 324 us at 3840 x 2160
+        // against 211. The full-resolution one: 583 and 578 us.)
         if (CG) {
             const int hc = a.h >> 1, wc = a.wd >> 1;
             constexpr int kUp = 32 * kStUpWarps;
             const int first = 32 * (warp - up_warp) + lane;
-            const int lag = min(2, ring - 3);
-            int slot = 0, phase = 0, pub_slot = 0, pending = 0;
-            auto publish = [&]() {
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-                if (lane == 0)
-                    mbar_arrive(smem_addr(&full[pub_slot]));
-                pub_slot = pub_slot + 1 == ring ? 0 : pub_slot + 1;
-                pending--;
-            };
+            int slot = 0, phase = 0;
             bool ok = true;
             for (int u = blockIdx.x; u < units && ok; u += gridDim.x) {
                 const int sg = u % segs, tx = (u / segs) % tiles_x, nb = u / (segs * tiles_x);
@@ -1391,25 +1385,17 @@ __global__ void __maxnreg__(80)
                             cp_async16(dst + st_chunk(g, pp), src + (in ? 8 * g : 0), in);
                     }
                     cp_async_commit();
-                    pending++;
+                    cp_async_wait<0>();
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0)
+                        mbar_arrive(smem_addr(&full[slot]));
                     if (++slot == ring) {
                         slot = 0;
                         phase ^= 1;
                     }
-                    if (pending > lag) {
-                        if (lag <= 0)
-                            cp_async_wait<0>();
-                        else if (lag == 1)
-                            cp_async_wait<1>();
-                        else
-                            cp_async_wait<2>();
-                        publish();
-                    }
                 }
             }
-            cp_async_wait<0>();
-            while (pending > 0)
-                publish();
             if (!ok)
                 abort_flag = 1;
         }
@@ -1867,9 +1853,9 @@ bool plan_strip(const ConvArgs &a, StripPlan &pl)
         tcols <<= 1;
     // CTAs per SM. A fused upsample + concat input takes one, with the deepest
     // ring: its upsample warps then run rows ahead of the MMAs (the
-    // half-resolution decoder input at 3840 x 2160, 192 to 64 channels: 324 us,
+    // half-resolution decoder input at 3840 x 2160, 112 to 48 channels: 211 us,
     // against 450 us for upsampling, concatenating and convolving it
-    // separately; the full-resolution one 583 against 650 with two per SM).
+    // separately; the full-resolution one 578 against 650 with two per SM).
     const int c = a.cc ? 1 : most;
     const int ring = ring_of(c);
     const long cols = (long)a.n * ((a.wd + kTcM - 1) / kTcM);
@@ -1895,9 +1881,9 @@ bool plan_strip(const ConvArgs &a, StripPlan &pl)
     pl.per_sm = c;
     // A second set of drain warps where the registers of the CTAs of an SM
     // leave room for it and there are channels to share (64 channels at
-    // 960 x 540: 72 to 52 us; 32 to 64 at 1920 x 1080: 114 to 95). A fused
+    // 960 x 540: 72 to 52 us; 48 at 1920 x 1080: 114 to 95). A fused
     // input keeps one: its MMAs bound it, and a second set only takes
-    // shared-memory and issue slots from them (96 to 32 channels at
+    // shared-memory and issue slots from them (80 to 32 channels at
     // 3840 x 2160: 583 us with one, 615 with two).
     pl.dsets = c <= 2 && pl.ntile >= 32 && !a.cc ? 2 : 1;
     return true;
