@@ -1,7 +1,8 @@
 """The denoiser's convolutions over image sizes that change how a layer is
 split: all output channels in a CTA or a share of them (small images), one or
 two sets of drain warps, fused upsample + concat inputs at one CTA per SM,
-segments shorter and longer than the ring, partial 128-pixel columns. The split
+segments shorter and longer than the ring, partial 128-pixel columns, layers
+whose weights are shared out over two CTAs (from one row of 128 pixels per SM). The split
 changes which CTA adds up an output element, not the order of its sum: the
 image is bit-identical between the strip kernel's plans and with the unfused
 inputs. Against the mma.sync kernels, whose sums run in another order before
@@ -16,7 +17,7 @@ from vviewer_gb300.denoiser import Denoiser
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("h,w", [(16, 16), (16, 272), (144, 16), (128, 128), (256, 256), (272, 400), (544, 976)])
+@pytest.mark.parametrize("h,w", [(16, 16), (16, 272), (144, 16), (128, 128), (256, 256), (272, 400), (544, 976), (1072, 1104)])
 def test_split_does_not_change_the_image(ctx, h, w):
     import torch
     rng = np.random.default_rng(h * 10000 + w)

@@ -1822,14 +1822,15 @@ bool plan_strip(const ConvArgs &a, StripPlan &pl)
     if (!tensor_map_encoder())
         return false;
     const int N = (a.cout + 15) & ~15;
-    const int wbytes = 9 * N * a.cin * 2, slot = (a.cin / 16) * kStPlane;
+    const int slot = (a.cin / 16) * kStPlane;
+    int share = N; // output channels whose weights a CTA holds
     int ncols = 32;
     while (ncols < 2 * N)
         ncols <<= 1;
     constexpr int kStatic = 2048; // mbarriers, TMEM address, flags (1 KB aligned)
     auto ring_of = [&](int c) {
         const int dyn = std::min(optin - kStatic, sm_smem / c - reserved - kStatic);
-        return std::min(kStMaxRing, (dyn - 1024 - wbytes) / slot);
+        return std::min(kStMaxRing, (dyn - 1024 - 9 * share * a.cin * 2) / slot);
     };
     // accumulators per row (independent MMA chains, whose sums the drain adds):
     // 1, 2 or 4, as many as the TMEM of an SM holds beside the other CTAs of
@@ -1839,9 +1840,26 @@ bool plan_strip(const ConvArgs &a, StripPlan &pl)
     for (int c = 4; c >= 1 && !most; c--)
         if (c * ncols <= 512 && std::min(8, ring_of(c)) >= kStMinRing)
             most = c;
-    if (!most)
-        return false;
-    for (int q = 4; q >= 2 && nacc == 1; q >>= 1) {
+    const long cols = (long)a.n * ((a.wd + kTcM - 1) / kTcM);
+    if (!most) {
+        // The weights of all channels leave no room for three rows: shares of
+        // them, one CTA per SM, each of which reads the whole input. The sums
+        // are the per-tile kernel's (one accumulator, channels in the same
+        // order), which keeps the layer where the image has less than a row of
+        // 128 pixels per SM. 96 to 96 channels at 480 x 270: 65 to 35 us; 160 to
+        // 64 at 960 x 540, fused: 249 to 238; whole images of 1024 x 512,
+        // 1280 x 720 and 2560 x 1440: 383 to 378, 514 to 509 and 1378 to 1341.
+        if (N > 128)
+            return false;
+        for (share = N - 16; share >= 16 && !most; share -= 16)
+            if (N % share == 0 && ring_of(1) >= kStMinRing) {
+                most = 1;
+                break;
+            }
+        if (!most || cols * a.h * (N / share) < nsm)
+            return false;
+    }
+    for (int q = 4; q >= 2 && nacc == 1 && share == N; q >>= 1) {
         int cq = 32;
         while (cq < 2 * q * N)
             cq <<= 1;
@@ -1858,15 +1876,14 @@ bool plan_strip(const ConvArgs &a, StripPlan &pl)
     // separately; the full-resolution one 578 against 650 with two per SM).
     const int c = a.cc ? 1 : most;
     const int ring = ring_of(c);
-    const long cols = (long)a.n * ((a.wd + kTcM - 1) / kTcM);
-    const long ctas = (long)nsm * c;
+    const long ctas = (long)nsm * c / (N / share);
     int segs = (int)std::max<long>(1, std::min<long>(a.h, ctas / std::max<long>(1, cols)));
     const int seg_rows = (a.h + segs - 1) / segs;
     segs = (a.h + seg_rows - 1) / seg_rows;
     // a small image: fewer output channels per CTA (the accumulators stay as
     // planned for all of them)
     pl.grid = (int)std::min<long>(cols * segs, ctas);
-    pl.ntile = split_channels(N, pl.grid);
+    pl.ntile = std::min(split_channels(N, pl.grid), share);
     if (pl.ntile != N)
         for (tcols = 32; tcols < 2 * nacc * pl.ntile;)
             tcols <<= 1;
