@@ -532,6 +532,8 @@ VVPT_API vvpt_status vvpt_render(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_sc
         shape.block = ctx->tuning.threads_per_block ? (int)ctx->tuning.threads_per_block : 256;
         int bps = ctx->tuning.blocks_per_sm ? (int)ctx->tuning.blocks_per_sm : 4;
         shape.grid = std::max(1, ctx->num_sms * bps);
+        shape.num_sms = ctx->num_sms;
+        shape.slots = slots;
         // Iterations between checks of the counters. Up to this many and as
         // many again in flight run empty once the last path has ended: 8 took
         // 48 iterations, 4 takes 40, where a 256 x 256 preview needs 34
@@ -997,6 +999,8 @@ VVPT_API vvpt_status vvpt_render_noalloc(vvpt_ctx *ctx, vvpt_scene *scene, const
     LaunchShape shape;
     shape.block = 256;
     shape.grid = std::max(1, ctx->num_sms * 4);
+    shape.num_sms = ctx->num_sms;
+    shape.slots = slots;
     launch_init_slots(q, ps, jt, slots, stream);
     VV_CUDA(cudaGetLastError(), "launch init");
     const uint64_t max_iters =

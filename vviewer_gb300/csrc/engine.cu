@@ -216,6 +216,8 @@ bool Engine::init_device(std::string &err)
     LaunchShape shape;
     shape.block = t.threads_per_block ? (int)t.threads_per_block : 256;
     shape.grid = std::max(1, ctx->num_sms * (t.blocks_per_sm ? (int)t.blocks_per_sm : 4));
+    shape.num_sms = ctx->num_sms;
+    shape.slots = slots;
     cudaGraph_t graph;
     if (!ck(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture"))
         return false;

@@ -809,15 +809,13 @@ __global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_trace(JobTable j
 {
     const uint32_t ne = q.counters[C_EXT0 + pp], ns = q.counters[C_CONN];
     const uint32_t n = ne + ns + q.counters[C_NEEQ];
+    if (n == 0)
+        return;
     uint32_t err = 0;
     auto entry = [&](uint32_t i) {
         return i < ne ? q.ext[pp][i] : (i < ne + ns ? q.conn[i - ne] : q.nee[i - ne - ns]);
     };
-    if (n > 0) {
-        tlas_cache_fill(jt.jobs[ps[entry(min(first_ray(), n - 1u))].job].scene);
-    } else {
-        tlas_cache_none();
-    }
+    tlas_cache_fill(jt.jobs[ps[entry(min(first_ray(), n - 1u))].job].scene);
     // per lane: queue index, slot, kind of ray and shade-bin bits, job; the ray
     __shared__ uint4 cold[256];
     __shared__ float4 cold_o[256], cold_d[256], cold_best[256];
@@ -1935,16 +1933,31 @@ void launch_iteration(const JobTable &jt, const PathState &ps, const Queues &q, 
 void launch_kernel(KernelId k, const JobTable &jt, const PathState &ps, const Queues &q, int pp,
                    const LaunchShape &shape, cudaStream_t stream)
 {
+    // At most `grid` blocks. Those past what the slots can occupy (`per_block`
+    // each), or past what fits at once, only cost their launch: the loops
+    // stride over the grid. k_shade's 128 registers let two blocks of 256 share
+    // an SM, and two also serve k_regen best, whose accesses get in each other's
+    // way beyond that (1080p x 32 medium scene, four and two per SM: shading 47.7
+    // and 46.9 ms, regeneration 14.3 and 13.6 ms). With all limits 256 x 256
+    // previews, 131,072 slots, went from 2.63 to 2.37 ms on the device.
+    auto blocks = [&](int grid, int per_sm, uint32_t per_block) {
+        const uint64_t fit = (uint64_t)shape.num_sms * per_sm * 256 / shape.block;
+        const uint64_t full = ((uint64_t)shape.slots + per_block - 1) / per_block;
+        return (int)std::max<uint64_t>(1, std::min(std::min((uint64_t)grid, fit), full));
+    };
+    const uint32_t block = (uint32_t)shape.block;
     switch (k) {
     case K_REGEN:
-        k_regen<<<shape.grid, shape.block, 0, stream>>>(jt, ps, q, pp);
+        k_regen<<<blocks(shape.grid, 2, block), shape.block, 0, stream>>>(jt, ps, q, pp);
         break;
     case K_TRACE:
-        // five blocks of k_trace fit an SM where the other kernels' shape counts four
-        k_trace<<<shape.grid + shape.grid / 4, shape.block, kTlasCacheBytes, stream>>>(jt, ps, q, pp);
+        // five blocks of k_trace fit an SM where the other kernels' shape counts
+        // four; two per SM stay even for few slots, whose rays are spread thin
+        k_trace<<<blocks(shape.grid + shape.grid / 4, 8, std::min(block, shape.slots / (2u * shape.num_sms) + 1u)),
+                  shape.block, kTlasCacheBytes, stream>>>(jt, ps, q, pp);
         break;
     case K_PARTITION:
-        k_partition<<<shape.grid, shape.block, 0, stream>>>(ps, q, pp);
+        k_partition<<<blocks(shape.grid, 8, 4 * block), shape.block, 0, stream>>>(ps, q, pp);
         break;
     case K_WALK:
         k_walk<<<shape.grid, shape.block, kTlasCacheBytes, stream>>>(jt, ps, q);
@@ -1955,7 +1968,7 @@ void launch_kernel(KernelId k, const JobTable &jt, const PathState &ps, const Qu
         k_shade<1><<<shape.grid, shape.block, kTlasCacheBytes, stream>>>(jt, ps, q, pp);
         k_shade<2><<<shape.grid, shape.block, kTlasCacheBytes, stream>>>(jt, ps, q, pp);
 #else
-        k_shade<3><<<shape.grid, shape.block, kTlasCacheBytes, stream>>>(jt, ps, q, pp);
+        k_shade<3><<<blocks(shape.grid, VVPT_SHADE_MIN_BLOCKS, block), shape.block, kTlasCacheBytes, stream>>>(jt, ps, q, pp);
 #endif
         break;
     default:

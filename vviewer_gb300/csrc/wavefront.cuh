@@ -150,6 +150,8 @@ struct JobTable {
 struct LaunchShape {
     int grid;
     int block;
+    int num_sms;
+    uint32_t slots; // path slots: the most entries a queue can hold
 };
 
 // Kernel launchers (wavefront.cu). Each reads its work count from `counters`,
