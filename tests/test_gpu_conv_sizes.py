@@ -1,8 +1,8 @@
 """The denoiser's convolutions over image sizes that change how a layer is
 split: all output channels in a CTA or a share of them (small images), one or
 two sets of drain warps, fused upsample + concat inputs at one CTA per SM,
-segments shorter and longer than the ring, partial 128-pixel columns, layers
-whose weights are shared out over two CTAs (from one row of 128 pixels per SM). The split
+segments shorter and longer than the ring, partial 128-pixel columns, 2x2 averages written by
+the drains, layers whose weights are shared out over two CTAs (from one row of 128 pixels per SM). The split
 changes which CTA adds up an output element, not the order of its sum: the
 image is bit-identical between the strip kernel's plans and with the unfused
 inputs. Against the mma.sync kernels, whose sums run in another order before

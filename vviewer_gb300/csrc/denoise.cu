@@ -176,8 +176,9 @@ void refresh_weights(vvpt_denoiser *dn, cudaStream_t s)
     dn->weights_dirty = false;
 }
 
+// pool: the 2x2 average of the output, for the next level
 void conv_fwd(vvpt_denoiser *dn, int li, const bf16 *in, void *out, int level, bool out_f32, cudaStream_t s,
-              float4 *rgba = nullptr)
+              float4 *rgba = nullptr, bf16 *pool = nullptr)
 {
     const Layer &L = dn->layers[li];
     vvdn::ConvArgs a{};
@@ -194,7 +195,9 @@ void conv_fwd(vvpt_denoiser *dn, int li, const bf16 *in, void *out, int level, b
     a.h = dn->h >> level;
     a.wd = dn->w >> level;
     a.rgba = rgba;
-    vvdn::conv3x3(a, s, dn->mma_sync ? nullptr : dn->err.as<uint32_t>(), dn->conv_kind);
+    a.pool = pool;
+    if (!vvdn::conv3x3(a, s, dn->mma_sync ? nullptr : dn->err.as<uint32_t>(), dn->conv_kind) && pool)
+        vvdn::avgpool2((const bf16 *)out, pool, a.n, a.h, a.wd, a.cout, s);
 }
 
 // layer li over concat(upsample2(coarse), skip) without the concatenated
@@ -262,11 +265,9 @@ void forward(vvpt_denoiser *dn, const float *rad, const float *alb, const float 
     const int n = dn->n;
     vvdn::pack_features(rad, alb, nrm, act(dn, dn->x[0]), (int)level_pixels(dn, 0), s);
     for (int l = 0; l < kLevels; l++) {
-        if (l > 0)
-            vvdn::avgpool2(act(dn, dn->e[l - 1]), act(dn, dn->x[l]), n, dn->h >> (l - 1), dn->w >> (l - 1),
-                           kCh[l - 1], s);
         conv_fwd(dn, 2 * l, act(dn, dn->x[l]), act(dn, dn->a[l]), l, false, s);
-        conv_fwd(dn, 2 * l + 1, act(dn, dn->a[l]), act(dn, dn->e[l]), l, false, s);
+        conv_fwd(dn, 2 * l + 1, act(dn, dn->a[l]), act(dn, dn->e[l]), l, false, s, nullptr,
+                 l + 1 < kLevels ? act(dn, dn->x[l + 1]) : nullptr);
     }
     for (int l = kLevels - 2; l >= 0; l--) {
         const Tensor &coarse = l == kLevels - 2 ? dn->e[kLevels - 1] : dn->d[l + 1];

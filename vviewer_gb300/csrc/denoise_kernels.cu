@@ -850,7 +850,9 @@ __device__ __forceinline__ void load_bias(const ConvArgs &a, int c, Bias16 &b)
         for (int k = 0; k < 4; k++)
             b.b[k] = __ldg(reinterpret_cast<const float4 *>(a.bias + c) + k);
 }
-__device__ __forceinline__ void store_row16(const ConvArgs &a, long p, int c, const uint32_t (&r)[16], const Bias16 &b)
+// (h: the 16 channels as stored, where they are stored as bf16.)
+__device__ __forceinline__ void store_row16(const ConvArgs &a, long p, int c, const uint32_t (&r)[16], const Bias16 &b,
+                                            uint32_t (&h)[8])
 {
     float v[16];
 #pragma unroll
@@ -896,7 +898,6 @@ __device__ __forceinline__ void store_row16(const ConvArgs &a, long p, int c, co
         for (int k = 0; k < 4; k++)
             dst[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
     } else {
-        uint32_t h[8];
 #pragma unroll
         for (int k = 0; k < 8; k++) {
             const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
@@ -904,6 +905,38 @@ __device__ __forceinline__ void store_row16(const ConvArgs &a, long p, int c, co
         }
         st32(reinterpret_cast<bf16 *>(a.out) + o, h);
     }
+}
+__device__ __forceinline__ void store_row16(const ConvArgs &a, long p, int c, const uint32_t (&r)[16], const Bias16 &b)
+{
+    uint32_t h[8];
+    store_row16(a, p, c, r, b, h);
+}
+
+// 2x2 averages of 16 channels, of the row just stored (h) and the one above it,
+// which the same thread stored: the lanes of an even and an odd pixel exchange
+// halves, and each averages eight channels in the order of k_avgpool2. The
+// whole warp calls it; `ok`: the lane's pixel and channels exist.
+__device__ __forceinline__ void pool_row16(const ConvArgs &a, long p, long pool_p, int c, const uint32_t (&h)[8], bool ok)
+{
+    uint32_t up[8] = {};
+    if (ok)
+        ld32(reinterpret_cast<const bf16 *>(a.out) + (p - a.wd) * a.cout + c, up);
+    const bool odd = threadIdx.x & 1;
+    uint4 res;
+    uint32_t *out = reinterpret_cast<uint32_t *>(&res);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const uint32_t mu = odd ? up[4 + k] : up[k], mc = odd ? h[4 + k] : h[k];
+        const uint32_t ou = __shfl_xor_sync(0xffffffffu, odd ? up[k] : up[4 + k], 1);
+        const uint32_t oc = __shfl_xor_sync(0xffffffffu, odd ? h[k] : h[4 + k], 1);
+        auto f = [](uint32_t w) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&w)); };
+        const float2 f00 = f(odd ? ou : mu), f01 = f(odd ? mu : ou), f10 = f(odd ? oc : mc), f11 = f(odd ? mc : oc);
+        const __nv_bfloat162 b = __floats2bfloat162_rn(0.25f * (((f00.x + f01.x) + f10.x) + f11.x),
+                                                       0.25f * (((f00.y + f01.y) + f10.y) + f11.y));
+        out[k] = *reinterpret_cast<const uint32_t *>(&b);
+    }
+    if (ok)
+        *reinterpret_cast<uint4 *>(a.pool + pool_p * a.cout + c + (odd ? 8 : 0)) = res;
 }
 
 __global__ void __launch_bounds__(kTcThreads) k_conv3x3_tc(ConvArgs a, int ncols, uint32_t *err)
@@ -1276,7 +1309,11 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar)
 constexpr int kStThreads = 192, kStUpWarps = 4;
 
 // (80 registers let four CTAs of 192 threads share an SM.)
-template <int nacc>
+// pool: the 2x2 averages are written in the drain of every odd row (rows start
+// even in every unit). As a pass of their own they read the whole output again:
+// 207 + 97 us for the second layer at 3840 x 2160, 262 together; 95 + 35 and 113
+// a level down.
+template <int nacc, bool pool>
 __global__ void __maxnreg__(80)
     k_conv3x3_strip(ConvArgs a, const __grid_constant__ CUtensorMap tmap, int ncols, int ring, int segs, int seg_rows,
                     int ntile, int dsets, uint32_t *err, int withhold_acc_full)
@@ -1567,8 +1604,14 @@ __global__ void __maxnreg__(80)
                         if (lane == 0)
                             mbar_arrive(smem_addr(&acc_empty[b]));
                     }
-                    if (x < a.wd && n0 + c < a.cout)
-                        store_row16(a, p, n0 + c, r, bias);
+                    const bool ok_px = x < a.wd && n0 + c < a.cout;
+                    uint32_t h[8] = {};
+                    if (ok_px)
+                        store_row16(a, p, n0 + c, r, bias, h);
+                    if constexpr (pool)
+                        if (i & 1)
+                            pool_row16(a, p, ((long)nb * (a.h >> 1) + ((ya + i) >> 1)) * (a.wd >> 1) + (x >> 1), n0 + c, h,
+                                       ok_px);
                     if (dsets * 16 < N)
                         load_bias(a, n0 + (last ? 16 * set : c + 16 * dsets), bias);
                 }
@@ -1878,7 +1921,9 @@ bool plan_strip(const ConvArgs &a, StripPlan &pl)
     const int ring = ring_of(c);
     const long ctas = (long)nsm * c / (N / share);
     int segs = (int)std::max<long>(1, std::min<long>(a.h, ctas / std::max<long>(1, cols)));
-    const int seg_rows = (a.h + segs - 1) / segs;
+    int seg_rows = (a.h + segs - 1) / segs;
+    if (a.pool)
+        seg_rows = (seg_rows + 1) & ~1; // rows that are averaged together in one unit
     segs = (a.h + seg_rows - 1) / seg_rows;
     // a small image: fewer output channels per CTA (the accumulators stay as
     // planned for all of them)
@@ -1924,18 +1969,18 @@ bool encode_input_map(const ConvArgs &a, CUtensorMap &m)
 
 namespace {
 
-template <int nacc>
-void launch_strip_nacc(const ConvArgs &a, const CUtensorMap &tmap, const StripPlan &pl, int withhold, cudaStream_t s,
+template <int nacc, bool pool>
+void launch_strip_as(const ConvArgs &a, const CUtensorMap &tmap, const StripPlan &pl, int withhold, cudaStream_t s,
                        uint32_t *err)
 {
     static int attr_smem = 0;
     if (pl.smem > attr_smem) {
-        cudaFuncSetAttribute(k_conv3x3_strip<nacc>, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem);
-        cudaFuncSetAttribute(k_conv3x3_strip<nacc>, cudaFuncAttributePreferredSharedMemoryCarveout,
+        cudaFuncSetAttribute(k_conv3x3_strip<nacc, pool>, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem);
+        cudaFuncSetAttribute(k_conv3x3_strip<nacc, pool>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared);
         attr_smem = pl.smem;
     }
-    launch_pdl(k_conv3x3_strip<nacc>, dim3((unsigned)pl.grid, (unsigned)(((a.cout + 15) & ~15) / pl.ntile)),
+    launch_pdl(k_conv3x3_strip<nacc, pool>, dim3((unsigned)pl.grid, (unsigned)(((a.cout + 15) & ~15) / pl.ntile)),
                kStThreads + 128 * (pl.dsets - 1) + (a.cc ? 32 * kStUpWarps : 0), pl.smem, s, a, tmap, pl.ncols, pl.ring,
                pl.segs, pl.seg_rows, pl.ntile, pl.dsets, err, withhold);
 }
@@ -1952,11 +1997,14 @@ bool launch_strip(const ConvArgs &a, cudaStream_t s, uint32_t *err, ConvKernels 
         pl.grid = std::min(pl.grid, 16);
     const int withhold = g_inject_wait_timeout.exchange(false) ? 1 : 0;
     if (pl.nacc == 4)
-        launch_strip_nacc<4>(a, tmap, pl, withhold, s, err);
+        a.pool ? launch_strip_as<4, true>(a, tmap, pl, withhold, s, err)
+               : launch_strip_as<4, false>(a, tmap, pl, withhold, s, err);
     else if (pl.nacc == 2)
-        launch_strip_nacc<2>(a, tmap, pl, withhold, s, err);
+        a.pool ? launch_strip_as<2, true>(a, tmap, pl, withhold, s, err)
+               : launch_strip_as<2, false>(a, tmap, pl, withhold, s, err);
     else
-        launch_strip_nacc<1>(a, tmap, pl, withhold, s, err);
+        a.pool ? launch_strip_as<1, true>(a, tmap, pl, withhold, s, err)
+               : launch_strip_as<1, false>(a, tmap, pl, withhold, s, err);
     return true;
 }
 
@@ -1969,14 +2017,15 @@ bool conv3x3_concat(const ConvArgs &a, cudaStream_t s, uint32_t *err, ConvKernel
     return kind != kConvNoFusion && a.coarse && a.cc > 0 && launch_strip(a, s, err, kind);
 }
 
-void conv3x3(const ConvArgs &a_in, cudaStream_t s, uint32_t *err, ConvKernels kind)
+bool conv3x3(const ConvArgs &a_in, cudaStream_t s, uint32_t *err, ConvKernels kind)
 {
     ConvArgs a = a_in;
     a.coarse = nullptr;
     a.cc = 0;
     const long P = (long)a.n * a.h * a.wd;
     if (launch_strip(a, s, err, kind))
-        return;
+        return a.pool != nullptr;
+    a.pool = nullptr;
     if (err && a.cout <= 256) {
         static bool attr_set = false;
         if (!attr_set) {
@@ -2014,7 +2063,7 @@ void conv3x3(const ConvArgs &a_in, cudaStream_t s, uint32_t *err, ConvKernels ki
         }
         else
             launch_pdl(k_conv3x3_tc, dim3((unsigned)tiles), kTcThreads, tc_smem_bytes(N), s, a, ncols, err);
-        return;
+        return false;
     }
     // 32-wide channel tiles where they leave fewer channels of the last tile
     // empty than 64-wide ones (16, 32, 80, 96, 160, 224 channels)
@@ -2026,6 +2075,7 @@ void conv3x3(const ConvArgs &a_in, cudaStream_t s, uint32_t *err, ConvKernels ki
         dim3 grid((unsigned)((P + kBM - 1) / kBM), (unsigned)((a.cout + 63) / 64));
         k_conv3x3<64, 32><<<grid, 256, 0, s>>>(a);
     }
+    return false;
 }
 
 void conv3x3_wgrad(const bf16 *dout, int cout, const bf16 *in, int cin, int n, int h, int w, float *dw, float *dbias,

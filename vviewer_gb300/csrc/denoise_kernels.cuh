@@ -32,6 +32,9 @@ struct ConvArgs {
     // Output layer at inference (tcgen05 kernels): the frame written as RGBA
     // f32, expm1(max(y, 0)) of channels 0-2 and alpha 1, instead of `out`.
     float4 *rgba;
+    // The 2x2 average of the output ([n][h/2][wd/2][cout]; h and wd even), or
+    // null: written beside it where the kernel that takes the layer can.
+    bf16 *pool;
 };
 
 enum ConvKernels {
@@ -47,7 +50,8 @@ enum ConvKernels {
 // With `err` set (and cout <= 256) it runs on the tcgen05 tensor cores and
 // `err` receives a status bit if one of its waits timed out; with err null
 // it runs the warp-level mma.sync kernel.
-void conv3x3(const ConvArgs &a, cudaStream_t s, uint32_t *err, ConvKernels kind = kConvAuto);
+// True when it has written a.pool as well.
+bool conv3x3(const ConvArgs &a, cudaStream_t s, uint32_t *err, ConvKernels kind = kConvAuto);
 
 // The same convolution over concat(upsample2(coarse), in) without writing the
 // concatenated tensor (a.coarse, a.cc set): runs only on the strip kernel and
