@@ -159,10 +159,11 @@ struct SingleJobBlock {
     uint32_t item_done;
 };
 
-JobTable single_job_table(SingleJobBlock *d, uint32_t *idle)
+JobTable single_job_table(SingleJobBlock *d, const SingleJobBlock *host, uint32_t *idle)
 {
     JobTable jt;
     jt.jobs = &d->job;
+    jt.only = &host->job;
     jt.range_begin = &d->range_begin;
     jt.range_job = &d->range_job;
     jt.item_done = &d->item_done;
@@ -523,8 +524,8 @@ VVPT_API vvpt_status vvpt_render(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_sc
         VV_CUDA(ctx->params.reserve(aligned(sizeof(SingleJobBlock)) + u4), "cudaMalloc job table");
         base = ctx->params.as<char>();
         SingleJobBlock *djob = (SingleJobBlock *)take(sizeof(SingleJobBlock));
-        const JobTable jt = single_job_table(djob, (uint32_t *)take(u4));
         const SingleJobBlock hjob = single_job_host(scene->view, hp, br);
+        const JobTable jt = single_job_table(djob, &hjob, (uint32_t *)take(u4));
         VV_CUDA(cudaMemcpyAsync(djob, &hjob, sizeof(hjob), cudaMemcpyHostToDevice, vv_stream(ctx)), "upload job");
         uint32_t *d_item_done = &djob->item_done;
 
@@ -984,7 +985,8 @@ VVPT_API vvpt_status vvpt_render_noalloc(vvpt_ctx *ctx, vvpt_scene *scene, const
     Queues q;
     q.counters = reinterpret_cast<uint32_t *>(take(C_COUNT * sizeof(uint32_t)));
     const PathState ps{reinterpret_cast<PathRecord *>(take(path_state_bytes(slots)))};
-    const JobTable jt = single_job_table(djob, reinterpret_cast<uint32_t *>(take(u4)));
+    SingleJobBlock hjob;
+    const JobTable jt = single_job_table(djob, &hjob, reinterpret_cast<uint32_t *>(take(u4)));
     uint32_t **qs[11] = {&q.ext[0], &q.ext[1],  &q.shade_l, &q.shade_p,  &q.shade_m, &q.conn,
                          &q.nee,    &q.ext_key, &q.walk,    &q.regen[0], &q.regen[1]};
     for (uint32_t **p : qs)
@@ -994,7 +996,7 @@ VVPT_API vvpt_status vvpt_render_noalloc(vvpt_ctx *ctx, vvpt_scene *scene, const
     br.alb = reinterpret_cast<float4 *>(take(items64 * sizeof(float4)));
     br.nrm = reinterpret_cast<float4 *>(take(items64 * sizeof(float4)));
 
-    const SingleJobBlock hjob = single_job_host(scene->view, hp, br);
+    hjob = single_job_host(scene->view, hp, br);
     VV_CUDA(cudaMemcpyAsync(djob, &hjob, sizeof(hjob), cudaMemcpyHostToDevice, stream), "upload job");
     LaunchShape shape;
     shape.block = 256;

@@ -429,6 +429,17 @@ __device__ __forceinline__ float3 medium_transmittance(const SceneView &s, uint3
 // ---------------------------------------------------------------------------
 // Kernels
 
+// The job of a path. A render has one, which its kernels get as a parameter
+// (kOne): its fields are then operands in constant memory instead of loads
+// through the table, of which every traversal step needs one before its node
+// and a shading event dozens (1080p x 32 medium scene 162.1 to 156.2 ms, 64-sample
+// Cornell box 8.44 to 8.07, 256 x 256 preview 2.37 to 2.25).
+template <bool kOne>
+__device__ __forceinline__ const JobView &job_view(const JobTable &jt, const JobView &one, uint32_t job)
+{
+    return kOne ? one : jt.jobs[job];
+}
+
 __global__ void k_init_slots(Queues q, PathState ps, JobTable jt, uint32_t slots)
 {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < slots; i += gridDim.x * blockDim.x) {
@@ -490,7 +501,9 @@ __device__ __forceinline__ uint32_t find_range(const JobTable &jt, uint32_t num_
 // depends on it, the counters take two rounds of atomics per warp, and what a
 // sample leaves as it is is not written back (246,000 paths: 108 -> 98 us; the
 // reset of the counters rides along instead of being a launch of its own).
-__global__ void __launch_bounds__(256) k_regen(JobTable jt, PathState ps, Queues q, int pp)
+template <bool kOne>
+__global__ void __launch_bounds__(256)
+    k_regen(JobTable jt, PathState ps, Queues q, int pp, const __grid_constant__ JobView one)
 {
     const uint32_t n = q.counters[C_REGEN0 + pp];
     const uint32_t *queue = q.regen[pp];
@@ -539,7 +552,7 @@ __global__ void __launch_bounds__(256) k_regen(JobTable jt, PathState ps, Queues
             alb = f3(e);
             nrm = f3(f);
             if (flags & F_DONE) {
-                const float total = (float)jt.jobs[job].params.total_samples;
+                const float total = (float)job_view<kOne>(jt, one, job).params.total_samples;
                 float3 r = rad;
                 if (flags & F_NEE) // the emitter ray's contribution, after the shadow ray's
                     r = r + f3(ps[slot].nee_c);
@@ -549,10 +562,10 @@ __global__ void __launch_bounds__(256) k_regen(JobTable jt, PathState ps, Queues
                 sample++;
                 path_done = true;
             }
-            if ((flags & F_ITEM) && sample >= jt.jobs[job].params.batch_size) {
+            if ((flags & F_ITEM) && sample >= job_view<kOne>(jt, one, job).params.batch_size) {
                 // the item's batch sums; the host and k_reduce read them after
                 // this launch, in stream order
-                const BatchResults br = jt.jobs[job].results;
+                const BatchResults br = job_view<kOne>(jt, one, job).results;
                 br.rad[item] = f4(cr, 1.0f);
                 br.alb[item] = f4(ca, 1.0f);
                 br.nrm[item] = f4(cn, 1.0f);
@@ -596,7 +609,7 @@ __global__ void __launch_bounds__(256) k_regen(JobTable jt, PathState ps, Queues
                 sample = 0;
                 cr = ca = cn = f3(0.0f);
             }
-            const RenderParams &p = jt.jobs[job].params;
+            const RenderParams &p = job_view<kOne>(jt, one, job).params;
             const uint32_t npix = p.width * p.height;
             const uint32_t batch = item / npix;
             const uint32_t pix = item - batch * npix;
@@ -805,7 +818,9 @@ __device__ __forceinline__ bool shadow_finish(const JobView &J, const PathState 
 // the open sky (512 instances) took 215 us a launch, nearly all of it the
 // tail, and now disappear behind the extension rays: 106 -> 92 ms.
 constexpr uint32_t kColdFused = 1u, kColdShadow = 2u, kColdEmitter = 4u; // cold[].z; shade-bin bits above them
-__global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_trace(JobTable jt, PathState ps, Queues q, int pp)
+template <bool kOne>
+__global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS)
+    k_trace(JobTable jt, PathState ps, Queues q, int pp, const __grid_constant__ JobView one)
 {
     const uint32_t ne = q.counters[C_EXT0 + pp], ns = q.counters[C_CONN];
     const uint32_t n = ne + ns + q.counters[C_NEEQ];
@@ -815,7 +830,7 @@ __global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_trace(JobTable j
     auto entry = [&](uint32_t i) {
         return i < ne ? q.ext[pp][i] : (i < ne + ns ? q.conn[i - ne] : q.nee[i - ne - ns]);
     };
-    tlas_cache_fill(jt.jobs[ps[entry(min(first_ray(), n - 1u))].job].scene);
+    tlas_cache_fill(job_view<kOne>(jt, one, ps[entry(min(first_ray(), n - 1u))].job).scene);
     // per lane: queue index, slot, kind of ray and shade-bin bits, job; the ray
     __shared__ uint4 cold[256];
     __shared__ float4 cold_o[256], cold_d[256], cold_best[256];
@@ -841,7 +856,7 @@ __global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_trace(JobTable j
                 const Hit h = trace_best(ray);
                 const uint32_t key = c.z >> 3;
                 if (c.z & kColdShadow) {
-                    walk = shadow_finish(jt.jobs[job], ps, c.y, h);
+                    walk = shadow_finish(job_view<kOne>(jt, one, job), ps, c.y, h);
                     walk_slot = c.y;
                     state = kLaneFree;
                 } else if ((c.z & kColdFused) && key == 0 && h.inst != kNoHit && h.t < kExtTmin) {
@@ -851,13 +866,13 @@ __global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_trace(JobTable j
                     // extension ray from its tmin
                     cold[threadIdx.x].z = kColdFused | (4u << 3);
                     const float3 o = f3(ray.o_slack), d = f3(ray.d_tmin);
-                    trace_begin(st, ray, jt.jobs[job].scene, o, d, kExtTmin, kExtTmax, no_hit());
+                    trace_begin(st, ray, job_view<kOne>(jt, one, job).scene, o, d, kExtTmin, kExtTmax, no_hit());
                     state = kLaneTracing;
                 } else {
                     ps[c.y].hit = make_float4(h.t, h.u, h.v, __uint_as_float(h.prim));
                     ps[c.y].hit_inst = h.inst;
                     if (!(c.z & kColdEmitter))
-                        q.ext_key[c.x] = extend_key(jt.jobs[job].scene, h, (c.z & kColdFused) != 0, key);
+                        q.ext_key[c.x] = extend_key(job_view<kOne>(jt, one, job).scene, h, (c.z & kColdFused) != 0, key);
                     state = kLaneFree;
                 }
             }
@@ -883,12 +898,12 @@ __global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_trace(JobTable j
                     const bool fused = ext && (flags & F_NEE_FUSED) != 0;
                     cold[threadIdx.x] =
                         make_uint4(i, slot, shadow ? kColdShadow : (!ext ? kColdEmitter : (fused ? kColdFused : 0u)), 0u);
-                    const float tmax = ext ? kExtTmax : (shadow ? d.w - kConnTmin : jt.jobs[job].params.zfar);
+                    const float tmax = ext ? kExtTmax : (shadow ? d.w - kConnTmin : job_view<kOne>(jt, one, job).params.zfar);
                     // the emitter ray of a path that goes on (zfar beyond the
                     // extension rays' range) takes the walk as a whole: the
                     // path's hit record belongs to its extension ray
                     if (ext || shadow || (flags & F_DONE)) {
-                        trace_begin(st, ray, jt.jobs[job].scene, f3(o), f3(d),
+                        trace_begin(st, ray, job_view<kOne>(jt, one, job).scene, f3(o), f3(d),
                                     ext && !fused ? kExtTmin : kConnTmin, tmax, no_hit());
                         state = kLaneTracing;
                     }
@@ -901,7 +916,7 @@ __global__ void __launch_bounds__(256, VVPT_TRACE_MIN_BLOCKS) k_trace(JobTable j
                 continue;
             }
         }
-        if (trace_turn(st, ray, stack, jt.jobs[job].scene, state == kLaneTracing, __popc(tr), err))
+        if (trace_turn(st, ray, stack, job_view<kOne>(jt, one, job).scene, state == kLaneTracing, __popc(tr), err))
             state = kLaneDone;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1041,9 +1056,9 @@ __device__ __noinline__ float3 fused_nee(const SceneView &s, const RenderParams 
 #ifndef VVPT_SHADE_SHARED_BSDF
 #define VVPT_SHADE_SHARED_BSDF 1
 #endif
-template <int KIND>
+template <int KIND, bool kOne>
 __global__ void __launch_bounds__(256, KIND == 0 || KIND == 2 ? VVPT_SHADE_LM_MIN_BLOCKS : VVPT_SHADE_MIN_BLOCKS)
-    k_shade(JobTable jt, PathState ps, Queues q, int pp)
+    k_shade(JobTable jt, PathState ps, Queues q, int pp, const __grid_constant__ JobView one)
 {
     // KIND 3: all three queues in one launch (VVPT_SHADE_SPLIT = 0)
     const uint32_t nl = q.counters[C_SHADE_L], np = q.counters[C_SHADE_P];
@@ -1059,7 +1074,7 @@ __global__ void __launch_bounds__(256, KIND == 0 || KIND == 2 ? VVPT_SHADE_LM_MI
     {
         const uint32_t f = blockIdx.x * blockDim.x;
         if (f < n)
-            tlas_cache_fill(jt.jobs[ps[entry(f)].job].scene);
+            tlas_cache_fill(job_view<kOne>(jt, one, ps[entry(f)].job).scene);
         else
             tlas_cache_none();
     }
@@ -1074,7 +1089,7 @@ __global__ void __launch_bounds__(256, KIND == 0 || KIND == 2 ? VVPT_SHADE_LM_MI
         load_pair(ps[slot].hit, hv, mv);
         load_pair(ps[slot].beta, bv, rv);
         load_pair(ps[slot].o, ov, dv);
-        const JobView &J = jt.jobs[__float_as_uint(mv.z)];
+        const JobView &J = job_view<kOne>(jt, one, __float_as_uint(mv.z));
         const SceneView &s = J.scene;
         const RenderParams &p = J.params;
 
@@ -1930,8 +1945,22 @@ void launch_iteration(const JobTable &jt, const PathState &ps, const Queues &q, 
         launch_kernel((KernelId)k, jt, ps, q, pp, shape, stream);
 }
 
+template <bool kOne>
+static void launch_one(KernelId k, const JobTable &jt, const PathState &ps, const Queues &q, int pp,
+                       const LaunchShape &shape, const JobView &one, cudaStream_t stream);
+
 void launch_kernel(KernelId k, const JobTable &jt, const PathState &ps, const Queues &q, int pp,
                    const LaunchShape &shape, cudaStream_t stream)
+{
+    if (jt.only)
+        launch_one<true>(k, jt, ps, q, pp, shape, *jt.only, stream);
+    else
+        launch_one<false>(k, jt, ps, q, pp, shape, JobView{}, stream);
+}
+
+template <bool kOne>
+static void launch_one(KernelId k, const JobTable &jt, const PathState &ps, const Queues &q, int pp,
+                       const LaunchShape &shape, const JobView &one, cudaStream_t stream)
 {
     // At most `grid` blocks. Those past what the slots can occupy (`per_block`
     // each), or past what fits at once, only cost their launch: the loops
@@ -1948,13 +1977,13 @@ void launch_kernel(KernelId k, const JobTable &jt, const PathState &ps, const Qu
     const uint32_t block = (uint32_t)shape.block;
     switch (k) {
     case K_REGEN:
-        k_regen<<<blocks(shape.grid, 2, block), shape.block, 0, stream>>>(jt, ps, q, pp);
+        k_regen<kOne><<<blocks(shape.grid, 2, block), shape.block, 0, stream>>>(jt, ps, q, pp, one);
         break;
     case K_TRACE:
         // five blocks of k_trace fit an SM where the other kernels' shape counts
         // four; two per SM stay even for few slots, whose rays are spread thin
-        k_trace<<<blocks(shape.grid + shape.grid / 4, 8, std::min(block, shape.slots / (2u * shape.num_sms) + 1u)),
-                  shape.block, kTlasCacheBytes, stream>>>(jt, ps, q, pp);
+        k_trace<kOne><<<blocks(shape.grid + shape.grid / 4, 8, std::min(block, shape.slots / (2u * shape.num_sms) + 1u)),
+                  shape.block, kTlasCacheBytes, stream>>>(jt, ps, q, pp, one);
         break;
     case K_PARTITION:
         k_partition<<<blocks(shape.grid, 8, 4 * block), shape.block, 0, stream>>>(ps, q, pp);
@@ -1964,11 +1993,11 @@ void launch_kernel(KernelId k, const JobTable &jt, const PathState &ps, const Qu
         break;
     case K_SHADE:
 #if VVPT_SHADE_SPLIT
-        k_shade<0><<<shape.grid, shape.block, kTlasCacheBytes, stream>>>(jt, ps, q, pp);
-        k_shade<1><<<shape.grid, shape.block, kTlasCacheBytes, stream>>>(jt, ps, q, pp);
-        k_shade<2><<<shape.grid, shape.block, kTlasCacheBytes, stream>>>(jt, ps, q, pp);
+        k_shade<0, kOne><<<shape.grid, shape.block, kTlasCacheBytes, stream>>>(jt, ps, q, pp, one);
+        k_shade<1, kOne><<<shape.grid, shape.block, kTlasCacheBytes, stream>>>(jt, ps, q, pp, one);
+        k_shade<2, kOne><<<shape.grid, shape.block, kTlasCacheBytes, stream>>>(jt, ps, q, pp, one);
 #else
-        k_shade<3><<<blocks(shape.grid, VVPT_SHADE_MIN_BLOCKS, block), shape.block, kTlasCacheBytes, stream>>>(jt, ps, q, pp);
+        k_shade<3, kOne><<<blocks(shape.grid, VVPT_SHADE_MIN_BLOCKS, block), shape.block, kTlasCacheBytes, stream>>>(jt, ps, q, pp, one);
 #endif
         break;
     default:

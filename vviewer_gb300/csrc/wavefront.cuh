@@ -137,6 +137,7 @@ struct JobView {
 // all live jobs; a path finds its job through ps.job.
 struct JobTable {
     const JobView *jobs;                   // per job slot
+    const JobView *only = nullptr;         // host copy of the table's one job (a render), or null
     const unsigned long long *range_begin; // per hand-out range, ascending
     const uint32_t *range_job;
     uint32_t *item_done;                   // per job slot: work items finished
