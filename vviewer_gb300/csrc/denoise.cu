@@ -108,6 +108,8 @@ struct vvpt_denoiser {
     // gskip[l]: gradient of e_l through the decoder's concat (gradient pool only)
     Tensor x[kLevels], a[kLevels], e[kLevels], u[kLevels - 1], b[kLevels - 1], d[kLevels - 1], gskip[kLevels - 1];
     bool weights_dirty = true;
+    // floats between the gradients' copies (even: pairs are added at once)
+    size_t grad_stride() const { return (nparams + 1) & ~size_t(1); }
 };
 
 namespace {
@@ -249,7 +251,8 @@ void conv_wgrad(vvpt_denoiser *dn, int li, const bf16 *dout, const bf16 *in, int
     const Layer &L = dn->layers[li];
     vvdn::conv3x3_wgrad(dout, L.cout, in, L.cin, dn->n, dn->h >> level, dn->w >> level,
                         dn->grads.as<float>() + L.w_off, dn->grads.as<float>() + L.b_off, s,
-                        dn->conv_kind == vvdn::kConvWgradTc ? dn->err.as<uint32_t>() : nullptr);
+                        dn->conv_kind == vvdn::kConvWgradTc ? dn->err.as<uint32_t>() : nullptr,
+                        (long)dn->grad_stride());
 }
 
 // inference (fuse_concat): the decoder's first convolution of a level reads
@@ -339,7 +342,7 @@ vvpt_status check_shape(vvpt_ctx *ctx, uint32_t n, uint32_t w, uint32_t h)
     return VVPT_OK;
 }
 
-// forward + loss + backward into dn->grads; loss returned on the host
+// forward + loss + backward into the copies of dn->grads; loss returned on the host
 vvpt_status loss_and_grads(vvpt_denoiser *dn, const vvpt_denoise_batch *bt, float *loss_out)
 {
     vvpt_ctx *ctx = dn->ctx;
@@ -355,7 +358,7 @@ vvpt_status loss_and_grads(vvpt_denoiser *dn, const vvpt_denoise_batch *bt, floa
     forward(dn, bt->radiance, bt->albedo, bt->normal, s);
     VV_CUDA(cudaMemsetAsync(dn->loss.ptr, 0, sizeof(float), s), "clear loss");
     vvdn::l1_loss(dn->out_f32.as<float>(), kOutCh, bt->target, dn->dout.as<bf16>(), dn->loss.as<float>(), p0, s);
-    VV_CUDA(cudaMemsetAsync(dn->grads.ptr, 0, dn->nparams * sizeof(float), s), "clear gradients");
+    VV_CUDA(cudaMemsetAsync(dn->grads.ptr, 0, dn->grads.bytes, s), "clear gradients");
     backward(dn, s);
     VV_CUDA(cudaGetLastError(), "denoiser kernels");
     float l = 0.0f;
@@ -395,7 +398,7 @@ VVPT_API vvpt_status vvpt_denoiser_create(vvpt_ctx *ctx, uint64_t seed, vvpt_den
                 p[L.w_off + (size_t)co * 9 * L.cin + k] = (float)(std_ * rng.normal());
     }
     VV_CUDA(dn->params.alloc(dn->nparams * sizeof(float)), "cudaMalloc denoiser parameters");
-    VV_CUDA(dn->grads.alloc(dn->nparams * sizeof(float)), "cudaMalloc denoiser gradients");
+    VV_CUDA(dn->grads.alloc(vvdn::kGradCopies * dn->grad_stride() * sizeof(float)), "cudaMalloc denoiser gradients");
     VV_CUDA(dn->adam_m.alloc(dn->nparams * sizeof(float)), "cudaMalloc denoiser optimiser");
     VV_CUDA(dn->adam_v.alloc(dn->nparams * sizeof(float)), "cudaMalloc denoiser optimiser");
     VV_CUDA(dn->w16.alloc(dn->nw16 * sizeof(bf16)), "cudaMalloc denoiser weights");
@@ -462,7 +465,11 @@ VVPT_API vvpt_status vvpt_denoiser_gradients(vvpt_denoiser *dn, const vvpt_denoi
     vvpt_status st = loss_and_grads(dn, batch, loss);
     if (st != VVPT_OK)
         return st;
-    VV_CUDA(cudaMemcpy(grads_host, dn->grads.ptr, n * sizeof(float), cudaMemcpyDeviceToHost), "read gradients");
+    cudaStream_t s = vv_stream(ctx);
+    vvdn::sum_grads(dn->grads.as<float>(), dn->grad_stride(), s);
+    VV_CUDA(cudaGetLastError(), "sum gradients");
+    VV_CUDA(cudaMemcpyAsync(grads_host, dn->grads.ptr, n * sizeof(float), cudaMemcpyDeviceToHost, s), "read gradients");
+    VV_CUDA(cudaStreamSynchronize(s), "read gradients");
     return VVPT_OK;
 }
 
@@ -479,8 +486,8 @@ VVPT_API vvpt_status vvpt_denoiser_train_step(vvpt_denoiser *dn, const vvpt_deno
         return st;
     cudaStream_t s = vv_stream(ctx);
     dn->step++;
-    vvdn::adam(dn->params.as<float>(), dn->grads.as<float>(), dn->adam_m.as<float>(), dn->adam_v.as<float>(),
-               dn->nparams, lr, 0.9f, 0.999f, 1e-8f, dn->step, s);
+    vvdn::adam(dn->params.as<float>(), dn->grads.as<float>(), dn->grad_stride(), dn->adam_m.as<float>(),
+               dn->adam_v.as<float>(), dn->nparams, lr, 0.9f, 0.999f, 1e-8f, dn->step, s);
     dn->weights_dirty = true;
     VV_CUDA(cudaGetLastError(), "adam");
     return VVPT_OK;

@@ -206,6 +206,17 @@ __global__ void __launch_bounds__(256) k_conv3x3(ConvArgs a)
         }
 }
 
+__device__ __forceinline__ void unpack8(const uint4 &v, float (&f)[8])
+{
+    const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&v);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float2 t = __bfloat1622float2(h[k]);
+        f[2 * k] = t.x;
+        f[2 * k + 1] = t.y;
+    }
+}
+
 // Weight (and bias) gradient, all nine taps in one pass over the pixels:
 // dW_tap[co][ci] = sum_p dout[p][co] * in[p shifted by the tap][ci] on the
 // warp-level mma.sync m16n8k16. A block owns 32 output x BN input channels and
@@ -214,13 +225,22 @@ __global__ void __launch_bounds__(256) k_conv3x3(ConvArgs a)
 // units. Rows arrive by cp.async, two ahead: output row y reads input rows
 // y - 1, y, y + 1 from a ring of five and its dout row, so a row of either is
 // staged once for the nine taps. A tap's operand is the staged row shifted by
-// a pixel or two, which ldmatrix takes as it is. The warp of the middle tap
-// also multiplies dout by ones: the bias gradient. Partial sums are added to
-// dw and dbias with atomics.
+// a pixel or two, which ldmatrix takes as it is. The bias gradient is added up
+// in FP32 by the threads that staged the values (the tensor cores cut the sums
+// they accumulate off where an addition rounds: -1.3 units in the last place on
+// average over rows of 64 pixels). Partial sums are added to dw and dbias with
+// atomics, block b to copy b % copies of the gradients: hundreds of blocks
+// adding to one value round as often, and with copies that are summed at the
+// end the errors of n additions shrink from sqrt(n) to sqrt(n) / copies.
 // Bound by shared-memory reads and MMA issue of the nine warps. Against one
 // launch per layer that staged both tensors again for every tap (and a launch
 // for the bias): 32 x 32 channels over 8 x 256 x 256 pixels 45 us, 157 + 10
-// before; 80 x 32 channels 136 us, 314 + 10 before.
+// before; 80 x 32 channels 136 us, 314 + 10 before. With the bias in FP32 and
+// the copies a training step over 8 x 256 x 256 pixels went from 1715 to 1651 us
+// and the weights' error against 64-bit sums of the same inputs, all layers,
+// from 1.94e-6 to 1.93e-6 there, from 2.1e-7 to 0.8e-7 at 8 x 64 x 64 (before the
+// taps were taken together: 4.6e-6 and 1.9e-7); the bias's from 2 to 4 times the
+// separate pass's at 8 x 64 x 64 to 0.6 times.
 constexpr int kWgPx = 64, kWgM = 32, kWgThreads = 288, kWgRing = 5, kWgDRing = 3, kWgDRow = kWgM + 8;
 template <int BN>
 constexpr int wg_smem()
@@ -231,7 +251,8 @@ constexpr int wg_smem()
 template <int BN>
 __global__ void __launch_bounds__(kWgThreads, BN == 32 ? 3 : 2) k_conv3x3_wgrad(const bf16 *__restrict__ dout, int cout,
                                                               const bf16 *__restrict__ in, int cin, int n, int h,
-                                                              int w, float *dw, float *dbias, int segs, int seg_rows)
+                                                              int w, float *dw, float *dbias, int segs, int seg_rows,
+                                                              int copies, long copy_stride)
 {
     constexpr int G = BN / 8, XRow = BN + 8, XSlot = (kWgPx + 2) * XRow, DSlot = kWgPx * kWgDRow, NT = BN / 8;
     extern __shared__ __align__(16) uint8_t wg_raw[];
@@ -242,7 +263,8 @@ __global__ void __launch_bounds__(kWgThreads, BN == 32 ? 3 : 2) k_conv3x3_wgrad(
     const int co0 = ((int)blockIdx.y / tiles_ci) * kWgM, ci0 = ((int)blockIdx.y % tiles_ci) * BN;
     const int cols = (w + kWgPx - 1) / kWgPx, units = n * cols * segs;
     const int dy = tap / 3, dx = tap % 3;
-    const bool bias = dbias && tap == 4 && ci0 == 0;
+    const bool bias = dbias && ci0 == 0 && tid < kWgPx * (kWgM / 8);
+    const long copy = (long)((int)blockIdx.x % copies) * copy_stride;
 
     // A unit's copies: what a thread copies of a row is fixed within a unit
     // (element offsets within the row, -1: zeros), so a row costs it no
@@ -299,7 +321,7 @@ __global__ void __launch_bounds__(kWgThreads, BN == 32 ? 3 : 2) k_conv3x3_wgrad(
         }
     };
 
-    float acc[2][NT][4] = {}, sum[2][2] = {}; // sum: output channels g and g + 8 of both halves
+    float acc[2][NT][4] = {}, sum[8] = {}; // sum: of the 8 output channels and the pixel this thread stages
     Unit cu = unit((int)blockIdx.x), lu = cu;
     int cr = 0, lr = 0;
     for (int k = 0; k < 2; k++) {
@@ -321,7 +343,6 @@ __global__ void __launch_bounds__(kWgThreads, BN == 32 ? 3 : 2) k_conv3x3_wgrad(
             const bf16 *D = Ds + (at % kWgDRing) * DSlot;
             const bf16 *X = Xs + ((at - 2 + dy) % kWgRing) * XSlot + dx * XRow;
             const int steps = (min(kWgPx, w - cu.x0) + 15) >> 4;
-            float row_sum[2][4] = {};
             for (int ks = 0; ks < 16 * steps; ks += 16) {
                 // A[m = cout][k = pixel] from D[k][m], B[k = pixel][n = cin]
                 // from X[k][n] (transposed loads)
@@ -343,19 +364,14 @@ __global__ void __launch_bounds__(kWgThreads, BN == 32 ? 3 : 2) k_conv3x3_wgrad(
                         mma_bf16(acc[m][2 * j + 1], a[m][0], a[m][1], a[m][2], a[m][3], b2, b3);
                     }
                 }
-                if (bias) {
-                    constexpr uint32_t kOnes = 0x3F803F80u; // two bf16 ones
-#pragma unroll
-                    for (int m = 0; m < 2; m++)
-                        mma_bf16(row_sum[m], a[m][0], a[m][1], a[m][2], a[m][3], kOnes, kOnes);
-                }
             }
-            if (bias) // row by row, so that the sums over all rows round to nearest
+            if (bias) {
+                float v[8];
+                unpack8(*reinterpret_cast<const uint4 *>(D + dpx * kWgDRow + 8 * dg), v);
 #pragma unroll
-                for (int m = 0; m < 2; m++) {
-                    sum[m][0] += row_sum[m][0];
-                    sum[m][1] += row_sum[m][2];
-                }
+                for (int k = 0; k < 8; k++)
+                    sum[k] += v[k];
+            }
         }
         advance(cu, cr);
     }
@@ -372,29 +388,39 @@ __global__ void __launch_bounds__(kWgThreads, BN == 32 ? 3 : 2) k_conv3x3_wgrad(
             for (int j = 0; j < NT; j++) {
                 const int ci = ci0 + 8 * j + 2 * t;
                 if (ci < cin)
-                    atomicAdd(reinterpret_cast<float2 *>(dw + ((long)co * 9 + tap) * cin + ci),
+                    atomicAdd(reinterpret_cast<float2 *>(dw + copy + ((long)co * 9 + tap) * cin + ci),
                               make_float2(acc[m][j][2 * half], acc[m][j][2 * half + 1]));
             }
-            if (bias && t == 0)
-                atomicAdd(dbias + co, sum[m][half]);
         }
+    if (!dbias || ci0 != 0)
+        return;
+    // bias: over a warp's 8 pixels by halves, then the 8 warps' sums
+    __syncthreads(); // the staged rows are read
+    float(*red)[kWgM] = reinterpret_cast<float(*)[kWgM]>(wg_raw);
+    if (tid < kWgPx * (kWgM / 8)) {
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1)
+                sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
+            if (lane < 4)
+                red[tid >> 5][8 * lane + k] = sum[k];
+        }
+    }
+    __syncthreads();
+    if (tid < kWgM && co0 + tid < cout) {
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            v[k] = red[k][tid];
+        atomicAdd(dbias + copy + co0 + tid, ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])));
+    }
 }
 
 // The layout kernels below move 8 channels (16 bytes) per thread: channel
 // counts are multiples of 8, so every access is one aligned 128-bit load or
 // store and a warp covers 512 consecutive bytes. Index arithmetic is 32-bit
 // (element counts stay below 2^31; the host checks).
-__device__ __forceinline__ void unpack8(const uint4 &v, float (&f)[8])
-{
-    const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&v);
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const float2 t = __bfloat1622float2(h[k]);
-        f[2 * k] = t.x;
-        f[2 * k + 1] = t.y;
-    }
-}
-
 __device__ __forceinline__ uint4 pack8(const float (&f)[8])
 {
     uint4 v;
@@ -635,11 +661,23 @@ __global__ void __launch_bounds__(256) k_l1_loss(const float *out, int cout, con
     }
 }
 
-__global__ void k_adam(float *p, const float *g, float *m, float *v, size_t n, float lr, float b1, float b2, float eps,
-                       float c1, float c2)
+// The sum of a gradient's copies (see k_conv3x3_wgrad).
+__device__ __forceinline__ float sum_copies(const float *g, size_t stride)
+{
+    static_assert(kGradCopies == 4, "summed by halves");
+    return (g[0] + g[stride]) + (g[2 * stride] + g[3 * stride]);
+}
+__global__ void k_sum_grads(float *g, size_t stride)
+{
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < stride; i += (size_t)gridDim.x * blockDim.x)
+        g[i] = sum_copies(g + i, stride);
+}
+
+__global__ void k_adam(float *p, const float *g, size_t stride, float *m, float *v, size_t n, float lr, float b1,
+                       float b2, float eps, float c1, float c2)
 {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const float gi = g[i];
+        const float gi = sum_copies(g + i, stride);
         const float mi = b1 * m[i] + (1.0f - b1) * gi;
         const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
         m[i] = mi;
@@ -2079,7 +2117,7 @@ bool conv3x3(const ConvArgs &a_in, cudaStream_t s, uint32_t *err, ConvKernels ki
 }
 
 void conv3x3_wgrad(const bf16 *dout, int cout, const bf16 *in, int cin, int n, int h, int w, float *dw, float *dbias,
-                   cudaStream_t s, uint32_t *err)
+                   cudaStream_t s, uint32_t *err, long copy_stride)
 {
     const long P = (long)n * h * w;
     if (err) {
@@ -2103,7 +2141,7 @@ void conv3x3_wgrad(const bf16 *dout, int cout, const bf16 *in, int cin, int n, i
         dim3 grid((unsigned)slices, (unsigned)(9 * tiles));
         k_conv3x3_wgrad_tc<<<grid, 128, smem, s>>>(dout, cout, in, cin, n, h, w, dw, slice, ntile, ncols, err);
     } else {
-        wgrad_mma_sync(dout, cout, in, cin, n, h, w, dw, dbias, s);
+        wgrad_mma_sync(dout, cout, in, cin, n, h, w, dw, dbias, s, copy_stride);
     }
     if (err && dbias) {
         // channel counts are multiples of 8 up to 256: 1-32 groups per pixel lane
@@ -2115,7 +2153,7 @@ void conv3x3_wgrad(const bf16 *dout, int cout, const bf16 *in, int cin, int n, i
 
 template <int BN>
 static void launch_wgrad(const bf16 *dout, int cout, const bf16 *in, int cin, int n, int h, int w, float *dw,
-                         float *dbias, cudaStream_t s)
+                         float *dbias, cudaStream_t s, long copy_stride)
 {
     static bool attr_set = false;
     if (!attr_set) {
@@ -2130,18 +2168,19 @@ static void launch_wgrad(const bf16 *dout, int cout, const bf16 *in, int cin, in
     const int seg_rows = (h + segs - 1) / segs;
     segs = (h + seg_rows - 1) / seg_rows;
     dim3 grid((unsigned)std::min<long>(cols * segs, blocks), (unsigned)tiles);
-    k_conv3x3_wgrad<BN><<<grid, kWgThreads, wg_smem<BN>(), s>>>(dout, cout, in, cin, n, h, w, dw, dbias, segs, seg_rows);
+    k_conv3x3_wgrad<BN><<<grid, kWgThreads, wg_smem<BN>(), s>>>(dout, cout, in, cin, n, h, w, dw, dbias, segs, seg_rows,
+                                                          copy_stride ? kGradCopies : 1, copy_stride);
 }
 
 void wgrad_mma_sync(const bf16 *dout, int cout, const bf16 *in, int cin, int n, int h, int w, float *dw, float *dbias,
-                    cudaStream_t s)
+                    cudaStream_t s, long copy_stride)
 {
     // 64 input channels per block where that leaves no more of them empty
     // than 32 would (64, 112, 128 channels)
     if ((cin + 63) / 64 * 64 == (cin + 31) / 32 * 32)
-        launch_wgrad<64>(dout, cout, in, cin, n, h, w, dw, dbias, s);
+        launch_wgrad<64>(dout, cout, in, cin, n, h, w, dw, dbias, s, copy_stride);
     else
-        launch_wgrad<32>(dout, cout, in, cin, n, h, w, dw, dbias, s);
+        launch_wgrad<32>(dout, cout, in, cin, n, h, w, dw, dbias, s, copy_stride);
 }
 
 void prepare_weights(const float *params, const WeightTable &t, bf16 *w16, bf16 *wt16, cudaStream_t s)
@@ -2192,11 +2231,16 @@ void l1_loss(const float *out, int cout, const float *target, bf16 *dout, float 
                                                                 dout, loss_sum, npix);
 }
 
-void adam(float *p, const float *g, float *m, float *v, size_t n, float lr, float b1, float b2, float eps, int t,
+void sum_grads(float *g, size_t stride, cudaStream_t s)
+{
+    k_sum_grads<<<grid_for((long)stride), 256, 0, s>>>(g, stride);
+}
+
+void adam(float *p, const float *g, size_t stride, float *m, float *v, size_t n, float lr, float b1, float b2, float eps, int t,
           cudaStream_t s)
 {
     const float c1 = 1.0f - powf(b1, (float)t), c2 = 1.0f - powf(b2, (float)t);
-    k_adam<<<grid_for((long)n), 256, 0, s>>>(p, g, m, v, n, lr, b1, b2, eps, c1, c2);
+    k_adam<<<grid_for((long)n), 256, 0, s>>>(p, g, stride, m, v, n, lr, b1, b2, eps, c1, c2);
 }
 
 void unpack_output(const float *y, int cout, float *out_rgba, int npix, cudaStream_t s)

@@ -69,11 +69,17 @@ void inject_wait_timeout();
 // bit if a wait timed out), with err null on the warp-level mma.sync kernel
 // (the faster of the two for this network: gradients of 8 x 256 x 256
 // pixels 2.25 vs 4.1 ms).
+// copy_stride: with 0 everything is added to dw and dbias; else the mma.sync
+// kernel's blocks share out kGradCopies copies of both, copy_stride floats
+// apart, which sum_grads and adam add up.
+constexpr int kGradCopies = 4;
 void conv3x3_wgrad(const bf16 *dout, int cout, const bf16 *in, int cin, int n, int h, int w, float *dw,
-                   float *dbias, cudaStream_t s, uint32_t *err = nullptr);
+                   float *dbias, cudaStream_t s, uint32_t *err = nullptr, long copy_stride = 0);
 // the mma.sync weight and bias gradient
 void wgrad_mma_sync(const bf16 *dout, int cout, const bf16 *in, int cin, int n, int h, int w, float *dw, float *dbias,
-                    cudaStream_t s);
+                    cudaStream_t s, long copy_stride = 0);
+// the first of kGradCopies arrays of `stride` floats becomes their sum
+void sum_grads(float *g, size_t stride, cudaStream_t s);
 
 // The layers' weights: first element in the bf16 copies (start[layers]: their
 // end) and in the f32 parameters.
@@ -106,8 +112,9 @@ void pool_backward_combine(const bf16 *dskip, const bf16 *dpooled, const bf16 *e
 // log(1 + max(target, 0)) of the RGBA32F target; dout (bf16, stride cout, zero
 // beyond channel 3) = sign(out - t) / (3 * npix); loss_sum += |diff|
 void l1_loss(const float *out, int cout, const float *target, bf16 *dout, float *loss_sum, int npix, cudaStream_t s);
-// Adam (Kingma and Ba 2015) with bias correction; t = step number from 1
-void adam(float *p, const float *g, float *m, float *v, size_t n, float lr, float b1, float b2, float eps, int t,
+// Adam (Kingma and Ba 2015) with bias correction on the sum of the gradients'
+// copies, `stride` floats apart; t = step number from 1
+void adam(float *p, const float *g, size_t stride, float *m, float *v, size_t n, float lr, float b1, float b2, float eps, int t,
           cudaStream_t s);
 // out RGBA32F = exp(max(y, 0)) - 1 for the first 3 channels, A = 1
 void unpack_output(const float *y, int cout, float *out_rgba, int npix, cudaStream_t s);
