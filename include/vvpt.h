@@ -353,7 +353,8 @@ VVPT_API vvpt_status vvpt_render_noalloc(vvpt_ctx *ctx,
 VVPT_API vvpt_status vvpt_progress(vvpt_ctx *ctx, float *out_progress);
 
 /* Closest hit for a batch of rays against the scene (no shading). rays/hits
- * are host pointers unless on_device != 0. */
+ * are host pointers unless on_device != 0. The arrays may overlap: the hits
+ * are then stored after all rays have been read. */
 VVPT_API vvpt_status vvpt_trace_closest(vvpt_ctx *ctx,
                                         vvpt_scene *scene,
                                         const vvpt_ray *rays,

@@ -827,6 +827,21 @@ VVPT_API vvpt_status vvpt_autotune(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_
     return VVPT_OK;
 }
 
+// Whether kernels can write `out` while they read `in`: apart from it, aligned
+// for 4-byte stores, memory of the context's device.
+static bool own_device_array(const vvpt_ctx *ctx, const void *in, size_t in_bytes, const void *out, size_t out_bytes)
+{
+    const uintptr_t a = (uintptr_t)in, b = (uintptr_t)out;
+    if (b % 4 || (a < b + out_bytes && b < a + in_bytes))
+        return false;
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, out) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeManaged || (at.type == cudaMemoryTypeDevice && at.device == ctx->device);
+}
+
 VVPT_API vvpt_status vvpt_trace_closest(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_ray *rays, uint32_t n,
                                         vvpt_hit *hits, int32_t on_device)
 {
@@ -845,9 +860,15 @@ VVPT_API vvpt_status vvpt_trace_closest(vvpt_ctx *ctx, vvpt_scene *scene, const 
         VV_CUDA(cudaMemcpyAsync(ctx->rays.ptr, rays, (size_t)n * 32, cudaMemcpyHostToDevice, vv_stream(ctx)), "upload rays");
         d_rays = ctx->rays.as<float4>();
     }
-    // hits of a caller on the host come back in one copy, straight into its array
+    // The kernels write a device caller's array directly, while other rays are
+    // still being read. Hits of a caller on the host come back in one copy,
+    // straight into its array; any other array (one that overlaps the rays, is
+    // not aligned to its members, or is not this device's memory) is stored once
+    // all rays are traced.
+    const bool direct = on_device && own_device_array(ctx, rays, (size_t)n * sizeof(vvpt_ray), hits,
+                                                      (size_t)n * sizeof(vvpt_hit));
     vvpt_hit *d_hits = hits;
-    if (!on_device) {
+    if (!direct) {
         VV_CUDA(ctx->hits.reserve((size_t)n * sizeof(vvpt_hit)), "cudaMalloc hits");
         d_hits = ctx->hits.as<vvpt_hit>();
     }
@@ -857,11 +878,15 @@ VVPT_API vvpt_status vvpt_trace_closest(vvpt_ctx *ctx, vvpt_scene *scene, const 
                          vv_stream(ctx));
     VV_CUDA(cudaGetLastError(), "launch trace");
     uint32_t err = 0;
-    if (!on_device)
-        VV_CUDA(cudaMemcpyAsync(hits, d_hits, (size_t)n * sizeof(vvpt_hit), cudaMemcpyDeviceToHost, vv_stream(ctx)),
+    std::vector<vvpt_hit> stored(on_device && !direct ? n : 0);
+    if (!direct)
+        VV_CUDA(cudaMemcpyAsync(on_device ? stored.data() : hits, d_hits, (size_t)n * sizeof(vvpt_hit),
+                                cudaMemcpyDeviceToHost, vv_stream(ctx)),
                 "d2h");
     VV_CUDA(cudaMemcpyAsync(&err, ctx->err_word.ptr, 4, cudaMemcpyDeviceToHost, vv_stream(ctx)), "d2h");
     VV_CUDA(cudaStreamSynchronize(vv_stream(ctx)), "trace");
+    if (!stored.empty())
+        VV_CUDA(cudaMemcpy(hits, stored.data(), (size_t)n * sizeof(vvpt_hit), cudaMemcpyHostToDevice), "store hits");
     if (err)
         return fail(ctx, VVPT_ERR_DEVICE, "traversal status word set: " + std::to_string(err));
     return VVPT_OK;
