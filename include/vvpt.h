@@ -326,7 +326,7 @@ VVPT_API vvpt_status vvpt_render(vvpt_ctx *ctx,
  * the same way, VVPT_RENDER_ENV_IS honoured); the PMJ sampler, whose tables
  * would need an allocation, is refused with VVPT_ERR_UNSUPPORTED. All scratch
  * (parameters, counters, ray queues,
- * path state for up to 63,488 paths in flight, per-batch sums) comes from one
+ * path state for up to 64,512 paths in flight, per-batch sums) comes from one
  * 64 MiB array the library defines at file scope, which every GPU that loads
  * the library holds until the process exits. Limit: the request must fit it:
  * width * height * (samples / batch_size) <= 993,936 work items (48 bytes

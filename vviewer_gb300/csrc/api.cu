@@ -97,13 +97,6 @@ vvpt_status make_render_params(vvpt_ctx *ctx, const vvpt_scene *scene, const vvp
 // their scenes, 180 ms against 219 with 2^22 for twelve previews.)
 constexpr uint32_t kDefaultSlots = 1u << 24, kSmallPoolSlots = 1u << 20;
 
-size_t path_state_bytes(size_t slots) { return slots * sizeof(PathRecord); }
-
-size_t queue_bytes(size_t slots)
-{
-    return 11 * aligned256(slots * sizeof(uint32_t)) + aligned256(C_COUNT * sizeof(uint32_t));
-}
-
 Queues carve_queues(char *base, size_t n)
 {
     const size_t u4 = aligned256(n * sizeof(uint32_t));
@@ -964,14 +957,11 @@ VVPT_API vvpt_status vvpt_render_noalloc(vvpt_ctx *ctx, vvpt_scene *scene, const
     const uint64_t items64 = hp.total_items;
     const uint64_t slots64 = std::max<uint64_t>(32, std::min<uint64_t>(items64, kNoAllocMaxSlots));
     auto aligned = [](uint64_t b) { return (b + 255) & ~uint64_t(255); };
-    const uint64_t f4 = slots64 * sizeof(float4), u4 = slots64 * sizeof(uint32_t);
-    // (path state counted as 14 f4 and 7 u4 arrays, 252 bytes a slot, which sets
-    // the renders that are refused; a record takes 256, so one slot in 32 stays
-    // unused)
-    const uint64_t need = aligned(sizeof(SingleJobBlock)) + aligned(C_COUNT * sizeof(uint32_t)) + 14 * aligned(f4) +
-                          7 * aligned(u4) + aligned(u4) /* idle slots */ + 11 * aligned(u4) +
+    const uint64_t u4 = slots64 * sizeof(uint32_t);
+    const uint64_t need = aligned(sizeof(SingleJobBlock)) + aligned(C_COUNT * sizeof(uint32_t)) +
+                          path_member_bytes(slots64) + aligned(u4) /* idle slots */ + 11 * aligned(u4) +
                           3 * aligned(items64 * sizeof(float4));
-    const uint32_t slots = (uint32_t)std::max<uint64_t>(32, slots64 - slots64 / 32);
+    const uint32_t slots = slots_within_members((uint32_t)slots64);
     if (need > kNoAllocScratchBytes)
         return fail(ctx, VVPT_ERR_INVALID_ARG,
                     "render needs " + std::to_string(need) + " bytes of scratch; vvpt_render_noalloc has " +

@@ -167,7 +167,7 @@ bool Engine::init_device(std::string &err)
 
     const vvpt_tuning &t = ctx->tuning;
     slots = t.slots ? t.slots : (1u << 20);
-    slots = std::max<uint32_t>(slots, 32u);
+    slots = slots_within_members(std::max<uint32_t>(slots, 32u));
     graph_iters = t.iterations_per_graph ? (int)t.iterations_per_graph : 8;
     graph_iters = (graph_iters + 1) & ~1;
     if (!ck(state_buf.alloc(path_state_bytes(slots)), "cudaMalloc path state") ||
@@ -177,7 +177,7 @@ bool Engine::init_device(std::string &err)
     q = carve_queues(queue_buf.as<char>(), slots);
     const size_t tb = aligned256(kMaxJobSlots * sizeof(JobView)) + aligned256(kMaxRanges * 8) +
                       aligned256(kMaxRanges * 4) + aligned256(kMaxJobSlots * 4) + aligned256(sizeof(TableCounters)) +
-                      aligned256((size_t)slots * 4);
+                      idle_bytes(slots);
     if (!ck(table_buf.alloc(tb), "cudaMalloc job table"))
         return false;
     char *base = table_buf.as<char>();

@@ -14,6 +14,7 @@
 #include "../../include/vvpt.h"
 #include "bvh_build.h"
 #include "scene_gpu.h"
+#include "slot_pool.h"
 #include "wavefront.cuh"
 
 namespace vvpt {
@@ -139,17 +140,13 @@ inline vvpt_status cuda_fail(vvpt_ctx *ctx, cudaError_t e, const char *what)
             return cuda_fail(ctx, _e, what); \
     } while (0)
 
-constexpr size_t aligned256(size_t b) { return (b + 255) & ~size_t(255); }
-
 // RenderParams of one render request (SceneData and RenderInfo of the
 // reference: VulkanRendererPathTracing.cpp:143-199, raygen.rgen.glsl:24-40).
 // Checks the request; on error sets ctx's message and returns its status.
 vvpt_status make_render_params(vvpt_ctx *ctx, const vvpt_scene *scene, const vvpt_scene_data *sd,
                                const vvpt_render_info *info, RenderParams &hp);
 
-// Path state and queues for `slots` paths carved from one allocation each.
-size_t path_state_bytes(size_t slots);
-size_t queue_bytes(size_t slots);
+// The queues of `slots` paths (queue_bytes) in one allocation.
 Queues carve_queues(char *base, size_t slots);
 
 // Engine teardown (vvpt_destroy): stops the worker, fails unfinished jobs.
