@@ -399,7 +399,15 @@ VVPT_API vvpt_status vvpt_last_kernel_profile(vvpt_ctx *ctx, vvpt_kernel_profile
 VVPT_API vvpt_status vvpt_set_stream(vvpt_ctx *ctx, void *cuda_stream);
 
 /* Tuning knobs (path-slot pool size and blocks per SM for the wavefront
- * kernels); 0 = automatic. */
+ * kernels); 0 = automatic.
+ *
+ * slots: a slot takes 304 bytes of device memory. Automatic: for vvpt_render
+ * one per work item (width * height * samples / batch_size) up to 2^24
+ * (5.1 GB), fewer where that is more than an eighth of the device's free
+ * memory or than vvpt_set_budget allows, but 2^20 (0.3 GB) at least; for the
+ * job engine 2^20. vvpt_render keeps its slots' memory for the next render
+ * until the context is destroyed, a smaller number is set here, or another
+ * allocation of a context on the device in this process needs the room. */
 typedef struct vvpt_tuning {
     uint32_t slots;
     uint32_t blocks_per_sm;
@@ -486,7 +494,8 @@ VVPT_API vvpt_status vvpt_wait(vvpt_ctx *ctx, vvpt_job job, double timeout_ms);
 VVPT_API vvpt_status vvpt_job_release(vvpt_ctx *ctx, vvpt_job job);
 /* Device-memory budget of the engine in bytes (path state, queues, per-job
  * batch sums and output staging); 0 = no limit but the device's memory.
- * Applies to admissions after the call. */
+ * Applies to admissions after the call. vvpt_render's automatic path slots
+ * stay within it too, down to 2^20 of them (0.3 GB). */
 VVPT_API vvpt_status vvpt_set_budget(vvpt_ctx *ctx, uint64_t bytes);
 /* Engine occupancy: its fixed pool (path slots, queues, job table), the
  * memory admitted jobs hold, and job counts by state (records not yet

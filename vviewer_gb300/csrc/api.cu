@@ -87,15 +87,19 @@ vvpt_status make_render_params(vvpt_ctx *ctx, const vvpt_scene *scene, const vvp
     return VVPT_OK;
 }
 
-// Path slots of a render whose tuning leaves them open. More slots mean fewer,
-// larger launches, and paths that start together: their rays stay neighbours
-// on the image for longer, and less of the time goes by waiting for a launch's
-// last rays. 2^20 slots (0.3 GB with their queues), 2^22 and 2^24 (4.8 GB):
-// 225, 196 and 184 ms on the 1080p x 32 medium scene, 62, 52 and 51 ms on the
-// 1919 x 1079 x 16 sky scene. A render has at most one slot per work item. (The
-// job engine keeps 2^20: with several jobs in flight a larger pool only mixes
-// their scenes, 180 ms against 219 with 2^22 for twelve previews.)
-constexpr uint32_t kDefaultSlots = 1u << 24, kSmallPoolSlots = 1u << 20;
+namespace {
+Pools<DeviceMem> &pools()
+{
+    static Pools<DeviceMem> p;
+    return p;
+}
+}  // namespace
+
+bool reclaim_pools()
+{
+    int device = 0;
+    return cudaGetDevice(&device) == cudaSuccess && pools().reclaim(device);
+}
 
 Queues carve_queues(char *base, size_t n)
 {
@@ -214,6 +218,7 @@ VVPT_API vvpt_status vvpt_create(int device, vvpt_ctx **out_ctx)
         delete ctx;
         return VVPT_ERR_OOM;
     }
+    pools().add(&ctx->pool, device);
     *out_ctx = ctx;
     return VVPT_OK;
 }
@@ -223,6 +228,7 @@ VVPT_API vvpt_status vvpt_destroy(vvpt_ctx *ctx)
     if (!ctx)
         return VVPT_ERR_INVALID_ARG;
     engine_shutdown(ctx);
+    pools().remove(&ctx->pool);
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(vv_stream(ctx));
     if (ctx->counters_pinned)
@@ -249,6 +255,10 @@ VVPT_API vvpt_status vvpt_set_tuning(vvpt_ctx *ctx, const vvpt_tuning *t)
         return fail(ctx, VVPT_ERR_INVALID_ARG, "blocks_per_sm at most 64, iterations_per_graph at most 256");
     std::lock_guard<std::mutex> lk(ctx->mu);
     ctx->tuning = *t;
+    if (t->slots) {
+        cudaSetDevice(ctx->device);
+        ctx->pool.give_back(pool_bytes(t->slots));
+    }
     return VVPT_OK;
 }
 
@@ -481,21 +491,17 @@ VVPT_API vvpt_status vvpt_render(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_sc
                 VV_CUDA(cudaMemsetAsync(d_out[k], 0, img_bytes, vv_stream(ctx)), "clear outputs");
     } else {
         // ---- path state and queues
-        uint32_t slots = ctx->tuning.slots ? ctx->tuning.slots : kDefaultSlots;
-        slots = std::max<uint32_t>(32u, std::min<uint32_t>(slots, hp.total_items));
         const size_t rb = (size_t)hp.total_items * sizeof(float4);
         VV_CUDA(ctx->results.reserve(3 * aligned256(rb)), "cudaMalloc batch results");
-        if (!ctx->tuning.slots && slots > kSmallPoolSlots &&
-            (ctx->state.reserve(path_state_bytes(slots)) != cudaSuccess ||
-             ctx->queues.reserve(queue_bytes(slots)) != cudaSuccess)) {
-            // no room for the default pool
-            cudaGetLastError();
-            ctx->state.release();
-            ctx->queues.release();
-            slots = kSmallPoolSlots;
-        }
+        VV_CUDA(ctx->params.reserve(aligned256(sizeof(SingleJobBlock))), "cudaMalloc job table");
+        const uint32_t slots = ctx->pool.acquire(hp.total_items, ctx->tuning.slots, ctx->budget_bytes.load());
+        if (!slots)
+            return cuda_fail(ctx, cudaErrorMemoryAllocation, "cudaMalloc path state");
+        struct PoolGuard {
+            SlotPool<DeviceMem> &pool;
+            ~PoolGuard() { pool.done(); }
+        } pool_guard{ctx->pool};
         const size_t n = slots;
-        const size_t u4 = n * sizeof(uint32_t);
         auto aligned = [](size_t b) { return aligned256(b); };
         char *base = nullptr;
         auto take = [&](size_t b) {
@@ -503,10 +509,10 @@ VVPT_API vvpt_status vvpt_render(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_sc
             base += aligned(b);
             return p;
         };
-        VV_CUDA(ctx->state.reserve(path_state_bytes(n)), "cudaMalloc path state");
-        const PathState ps{ctx->state.as<PathRecord>()};
-        VV_CUDA(ctx->queues.reserve(queue_bytes(n)), "cudaMalloc queues");
-        const Queues q = carve_queues(ctx->queues.as<char>(), n);
+        base = static_cast<char *>(ctx->pool.ptr());
+        const PathState ps{(PathRecord *)take(path_state_bytes(n))};
+        const Queues q = carve_queues(take(queue_bytes(n)), n);
+        uint32_t *const d_idle = (uint32_t *)take(idle_bytes(n));
 
         base = ctx->results.as<char>();
         BatchResults br;
@@ -514,11 +520,9 @@ VVPT_API vvpt_status vvpt_render(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_sc
         br.alb = (float4 *)take(rb);
         br.nrm = (float4 *)take(rb);
 
-        VV_CUDA(ctx->params.reserve(aligned(sizeof(SingleJobBlock)) + u4), "cudaMalloc job table");
-        base = ctx->params.as<char>();
-        SingleJobBlock *djob = (SingleJobBlock *)take(sizeof(SingleJobBlock));
+        SingleJobBlock *djob = ctx->params.as<SingleJobBlock>();
         const SingleJobBlock hjob = single_job_host(scene->view, hp, br);
-        const JobTable jt = single_job_table(djob, &hjob, (uint32_t *)take(u4));
+        const JobTable jt = single_job_table(djob, &hjob, d_idle);
         VV_CUDA(cudaMemcpyAsync(djob, &hjob, sizeof(hjob), cudaMemcpyHostToDevice, vv_stream(ctx)), "upload job");
         uint32_t *d_item_done = &djob->item_done;
 

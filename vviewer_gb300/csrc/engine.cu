@@ -332,10 +332,16 @@ void Engine::run()
                 if (ctx->budget_bytes && fixed_bytes + used_bytes + need > ctx->budget_bytes)
                     break;
                 void *res = nullptr, *stg = nullptr;
-                cudaError_t e1 = cudaMallocFromPoolAsync(&res, j->bytes_results, pool, stream);
-                cudaError_t e2 = e1 == cudaSuccess && j->bytes_staging
-                                     ? cudaMallocFromPoolAsync(&stg, j->bytes_staging, pool, stream)
-                                     : cudaSuccess;
+                auto take = [&](void **p, size_t n) {
+                    cudaError_t e = cudaMallocFromPoolAsync(p, n, pool, stream);
+                    if (e == cudaErrorMemoryAllocation && reclaim_pools()) {
+                        cudaGetLastError();
+                        e = cudaMallocFromPoolAsync(p, n, pool, stream);
+                    }
+                    return e;
+                };
+                cudaError_t e1 = take(&res, j->bytes_results);
+                cudaError_t e2 = e1 == cudaSuccess && j->bytes_staging ? take(&stg, j->bytes_staging) : cudaSuccess;
                 if (e1 != cudaSuccess || e2 != cudaSuccess) {
                     cudaGetLastError();
                     if (res)
@@ -616,7 +622,7 @@ VVPT_API vvpt_status vvpt_submit(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_sc
         return fail(ctx, VVPT_ERR_BUDGET_EXCEEDED,
                     "job needs " + std::to_string(j->bytes_results + j->bytes_staging) +
                         " bytes beside the engine's " + std::to_string(e->fixed_bytes) + "; budget " +
-                        std::to_string(ctx->budget_bytes));
+                        std::to_string(ctx->budget_bytes.load()));
     j->id = e->next_id++;
     j->submit_ms = e->now_ms();
     scene->jobs_in_flight.fetch_add(1);
@@ -704,6 +710,10 @@ VVPT_API vvpt_status vvpt_set_budget(vvpt_ctx *ctx, uint64_t bytes)
 {
     if (!ctx)
         return VVPT_ERR_INVALID_ARG;
+    if (bytes) {
+        cudaSetDevice(ctx->device);
+        ctx->pool.give_back(std::max<uint64_t>(bytes, pool_bytes(kSmallPoolSlots)));
+    }
     std::lock_guard<std::mutex> lk(ctx->engine_mu);
     if (ctx->engine) {
         std::lock_guard<std::mutex> lk2(ctx->engine->m);

@@ -19,6 +19,10 @@
 
 namespace vvpt {
 
+// Gives back the path pools of the current device's contexts that no render
+// uses; whether that freed memory.
+bool reclaim_pools();
+
 struct DevBuf {
     void *ptr = nullptr;
     size_t bytes = 0;
@@ -39,6 +43,10 @@ struct DevBuf {
         if (n == 0)
             n = 16;
         cudaError_t e = cudaMalloc(&ptr, n);
+        if (e == cudaErrorMemoryAllocation && reclaim_pools()) {
+            cudaGetLastError();
+            e = cudaMalloc(&ptr, n);
+        }
         if (e == cudaSuccess)
             bytes = n;
         else
@@ -56,6 +64,32 @@ struct DevBuf {
     T *as() const
     {
         return reinterpret_cast<T *>(ptr);
+    }
+};
+
+struct DeviceMem {
+    static void *alloc(size_t n)
+    {
+        void *p = nullptr;
+        if (cudaMalloc(&p, n) == cudaSuccess)
+            return p;
+        cudaGetLastError();
+        return nullptr;
+    }
+    static void *alloc_or_reclaim(size_t n)
+    {
+        void *p = alloc(n);
+        return p || !reclaim_pools() ? p : alloc(n);
+    }
+    static void free(void *p) { cudaFree(p); }
+    static size_t free_bytes()
+    {
+        size_t free = 0, total = 0;
+        if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        return free;
     }
 };
 
@@ -99,7 +133,8 @@ struct vvpt_ctx {
     vvpt_render_stats stats{};
     vvpt_tuning tuning{};
     // render buffers (grow-only, reused across renders)
-    vvpt::DevBuf state, queues, results, params, outputs;
+    vvpt::SlotPool<vvpt::DeviceMem> pool;
+    vvpt::DevBuf results, params, outputs;
     uint32_t *counters_pinned = nullptr;
     vvpt::DevBuf rays, hits, err_word;
     cudaStream_t user_stream = nullptr;
@@ -107,7 +142,7 @@ struct vvpt_ctx {
     // job engine (vvpt_submit ...), created on first use
     std::mutex engine_mu;
     vvpt::Engine *engine = nullptr;
-    uint64_t budget_bytes = 0; // 0: no limit beyond the device's memory
+    std::atomic<uint64_t> budget_bytes{0}; // 0: no limit beyond the device's memory
     int bvh_builder = 0;       // VVPT_BVH_BUILDER_*
     // low-discrepancy sampler tables (VVPT_RENDER_SAMPLER_PMJ), uploaded on first use
     std::mutex sampler_mu;
