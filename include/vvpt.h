@@ -407,7 +407,11 @@ VVPT_API vvpt_status vvpt_set_stream(vvpt_ctx *ctx, void *cuda_stream);
  * memory or than vvpt_set_budget allows, but 2^20 (0.3 GB) at least; for the
  * job engine 2^20. vvpt_render keeps its slots' memory for the next render
  * until the context is destroyed, a smaller number is set here, or another
- * allocation of a context on the device in this process needs the room. */
+ * allocation of a context on the device in this process needs the room.
+ *
+ * blocks_per_sm: blocks of threads_per_block threads (256) of every wavefront
+ * kernel per SM (a quarter more of the tracing kernel's). Automatic: four, and
+ * no more of a kernel than run on an SM at once. */
 typedef struct vvpt_tuning {
     uint32_t slots;
     uint32_t blocks_per_sm;

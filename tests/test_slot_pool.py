@@ -170,3 +170,19 @@ def test_pool_is_kept_given_back_and_never_lost_to_a_larger_one(tmp_path):
         }""")
     assert out == [str(x) for x in (1 << 20, 1 << 20, 1, 1 << 24, 0, 1, 0, 1000, 1 << 20, 1 << 24, 1, 1, 1 << 20, 77, 2,
                                     0)]
+
+
+def test_blocks_per_sm_reach_every_kernel(tmp_path):
+    """A caller's blocks_per_sm is every kernel's grid, up to one thread per
+    slot; the default keeps to the blocks that run at once."""
+    out = run_host(tmp_path, """
+        int main()
+        {
+            for (int automatic = 0; automatic < 2; automatic++)
+                for (int per_sm : {2, 8}) {
+                    const LaunchShape s{152 * 6, 256, 152, 1u << 24, automatic != 0}, few{152 * 6, 128, 152, 1000,
+                                                                                                  automatic != 0};
+                    std::printf("%d %d\\n", launch_blocks(s, s.grid, per_sm, 256), launch_blocks(few, few.grid, per_sm, 128));
+                }
+        }""")
+    assert out == ["912", "8", "912", "8", "304", "8", "912", "8"]

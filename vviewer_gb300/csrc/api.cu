@@ -532,6 +532,7 @@ VVPT_API vvpt_status vvpt_render(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_sc
         shape.grid = std::max(1, ctx->num_sms * bps);
         shape.num_sms = ctx->num_sms;
         shape.slots = slots;
+        shape.automatic = !ctx->tuning.blocks_per_sm;
         // Iterations between checks of the counters. Up to this many and as
         // many again in flight run empty once the last path has ended: 8 took
         // 48 iterations, 4 takes 40, where a 256 x 256 preview needs 34
@@ -1022,6 +1023,7 @@ VVPT_API vvpt_status vvpt_render_noalloc(vvpt_ctx *ctx, vvpt_scene *scene, const
     shape.grid = std::max(1, ctx->num_sms * 4);
     shape.num_sms = ctx->num_sms;
     shape.slots = slots;
+    shape.automatic = true;
     launch_init_slots(q, ps, jt, slots, stream);
     VV_CUDA(cudaGetLastError(), "launch init");
     const uint64_t max_iters =

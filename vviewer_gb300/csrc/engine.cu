@@ -218,6 +218,7 @@ bool Engine::init_device(std::string &err)
     shape.grid = std::max(1, ctx->num_sms * (t.blocks_per_sm ? (int)t.blocks_per_sm : 4));
     shape.num_sms = ctx->num_sms;
     shape.slots = slots;
+    shape.automatic = !t.blocks_per_sm;
     cudaGraph_t graph;
     if (!ck(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture"))
         return false;

@@ -1962,18 +1962,12 @@ template <bool kOne>
 static void launch_one(KernelId k, const JobTable &jt, const PathState &ps, const Queues &q, int pp,
                        const LaunchShape &shape, const JobView &one, cudaStream_t stream)
 {
-    // At most `grid` blocks. Those past what the slots can occupy (`per_block`
-    // each), or past what fits at once, only cost their launch: the loops
-    // stride over the grid. k_shade's 128 registers let two blocks of 256 share
-    // an SM, and two also serve k_regen best, whose accesses get in each other's
-    // way beyond that (1080p x 32 medium scene, four and two per SM: shading 47.7
-    // and 46.9 ms, regeneration 14.3 and 13.6 ms). With all limits 256 x 256
-    // previews, 131,072 slots, went from 2.63 to 2.37 ms on the device.
-    auto blocks = [&](int grid, int per_sm, uint32_t per_block) {
-        const uint64_t fit = (uint64_t)shape.num_sms * per_sm * 256 / shape.block;
-        const uint64_t full = ((uint64_t)shape.slots + per_block - 1) / per_block;
-        return (int)std::max<uint64_t>(1, std::min(std::min((uint64_t)grid, fit), full));
-    };
+    // By default: k_shade's 128 registers let two blocks of 256 share an SM, and
+    // two also serve k_regen best, whose accesses get in each other's way beyond
+    // that (1080p x 32 medium scene, four and two per SM: shading 47.7 and 46.9
+    // ms, regeneration 14.3 and 13.6 ms). With all limits 256 x 256 previews,
+    // 131,072 slots, went from 2.63 to 2.37 ms on the device.
+    auto blocks = [&](int grid, int per_sm, uint32_t per_block) { return launch_blocks(shape, grid, per_sm, per_block); };
     const uint32_t block = (uint32_t)shape.block;
     switch (k) {
     case K_REGEN:

@@ -1,5 +1,7 @@
 // Wavefront path-tracer state and launch interface.
 #pragma once
+#include <algorithm>
+
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -153,7 +155,21 @@ struct LaunchShape {
     int block;
     int num_sms;
     uint32_t slots; // path slots: the most entries a queue can hold
+    bool automatic; // `grid` is the default, not a caller's blocks_per_sm
 };
+
+// Grid of a kernel: at most `grid` blocks, and none past what the slots can
+// occupy (`per_block` each): they would only cost their launch, since the loops
+// stride over the grid. The default shape also stays within what fits at once,
+// `per_sm` blocks of 256 threads; a caller's number reaches every kernel.
+inline int launch_blocks(const LaunchShape &shape, int grid, int per_sm, uint32_t per_block)
+{
+    const uint64_t full = ((uint64_t)shape.slots + per_block - 1) / per_block;
+    uint64_t n = std::min<uint64_t>((uint64_t)grid, full);
+    if (shape.automatic)
+        n = std::min(n, (uint64_t)shape.num_sms * per_sm * 256 / shape.block);
+    return (int)std::max<uint64_t>(1, n);
+}
 
 // Kernel launchers (wavefront.cu). Each reads its work count from `counters`,
 // so a sequence of them can be captured in a CUDA graph.
