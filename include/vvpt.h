@@ -426,8 +426,10 @@ VVPT_API vvpt_status vvpt_get_tuning(vvpt_ctx *ctx, vvpt_tuning *out_tuning);
  * budget_ms / 12 each) and picks blocks per SM, path slots and iterations
  * per CUDA graph by coordinate descent on measured paths/s. The result is
  * stored as the context's tuning (used by vvpt_render and by a job engine
- * started afterwards) and returned in out_tuning (may be NULL). Images do
- * not depend on the tuning. */
+ * started afterwards) and returned in out_tuning (may be NULL). A value of 0
+ * stands for vvpt_render's automatic choice, which no candidate beat; a job
+ * engine's automatic slots and iterations are its own (2^20 and 8), not the
+ * ones measured here. Images do not depend on the tuning. */
 VVPT_API vvpt_status vvpt_autotune(vvpt_ctx *ctx,
                                    vvpt_scene *scene,
                                    const vvpt_scene_data *scene_data,

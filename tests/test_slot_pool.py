@@ -186,3 +186,17 @@ def test_blocks_per_sm_reach_every_kernel(tmp_path):
                 }
         }""")
     assert out == ["912", "8", "912", "8", "304", "8", "912", "8"]
+
+
+def test_autotuner_tries_slots_up_to_the_default(tmp_path):
+    out = run_host(tmp_path, """
+        int main()
+        {
+            for (uint32_t items : {1u, 1u << 19, (1u << 20) + 1, 33000000u}) {
+                for (uint32_t s : autotune_slots(items))
+                    std::printf("%u,", s);
+                std::printf("end\\n");
+            }
+        }""")
+    small = f"{1 << 19},{1 << 20},"
+    assert out == ["end", "end", small + "end", small + f"{3 << 19},{1 << 21},{1 << 22},{1 << 24},end"]

@@ -790,7 +790,7 @@ VVPT_API vvpt_status vvpt_autotune(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_
     if ((st = trial(best, best_ppm)) != VVPT_OK)
         return st;
     // coordinate descent: blocks per SM, slots, iterations per graph
-    auto sweep = [&](auto apply, std::initializer_list<uint32_t> values) -> vvpt_status {
+    auto sweep = [&](auto apply, const std::vector<uint32_t> &values) -> vvpt_status {
         vvpt_tuning base = best;
         for (uint32_t v : values) {
             vvpt_tuning t = base;
@@ -810,14 +810,16 @@ VVPT_API vvpt_status vvpt_autotune(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_
     };
     if ((st = sweep([](vvpt_tuning &t, uint32_t v) { t.blocks_per_sm = v; }, {2u, 3u, 4u, 6u, 8u})) != VVPT_OK)
         return st;
-    if ((st = sweep([](vvpt_tuning &t, uint32_t v) { t.slots = v; }, {1u << 19, 1u << 20, 3u << 19, 1u << 21})) !=
-        VVPT_OK)
+    if ((st = sweep([](vvpt_tuning &t, uint32_t v) { t.slots = v; },
+                    autotune_slots(hp.width * hp.height * batches))) != VVPT_OK)
         return st;
     if ((st = sweep([](vvpt_tuning &t, uint32_t v) { t.iterations_per_graph = v; }, {4u, 8u, 16u})) != VVPT_OK)
         return st;
     {
         std::lock_guard<std::mutex> lk(ctx->mu);
         ctx->tuning = best;
+        if (best.slots)
+            ctx->pool.give_back(pool_bytes(best.slots));
         outb.release();
     }
     if (out)

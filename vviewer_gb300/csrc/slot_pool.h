@@ -63,6 +63,17 @@ inline uint32_t default_slots(uint32_t items, size_t room, size_t budget)
     return s;
 }
 
+// Numbers of slots that vvpt_autotune tries for a render of `items` work items:
+// below the default's where it has more, and the default's steps above 2^21 for
+// a tuning that starts from a smaller number. As many slots as items or more
+// are all the same render.
+inline std::vector<uint32_t> autotune_slots(uint32_t items)
+{
+    std::vector<uint32_t> v{1u << 19, 1u << 20, 3u << 19, 1u << 21, 1u << 22, kDefaultSlots};
+    v.erase(std::remove_if(v.begin(), v.end(), [items](uint32_t s) { return s >= items; }), v.end());
+    return v;
+}
+
 // The memory of one context's renders, kept between them. Other allocations that
 // find no room take it back while no render runs (Pools::reclaim).
 // Mem: static void *alloc(size_t) (null: no room), void free(void *), size_t
