@@ -439,7 +439,8 @@ VVPT_API vvpt_status vvpt_autotune(vvpt_ctx *ctx,
 
 /* BVH builder of vvpt_scene_upload: AUTO builds meshes of at least 512
  * triangles on the GPU (binned SAH, all meshes in the same launches) and the
- * rest, the baked small instances and the TLAS on the host; HOST builds
+ * rest, the baked small instances and the TLAS on the host (all of them where
+ * the device has no room for the builder's working memory); HOST builds
  * every tree on the host (binned SAH with FP64 costs); GPU builds every BLAS,
  * the baked small instances' BLAS and the TLAS on the GPU (trees of at most
  * one leaf stay on the host). All give the same closest hits. */

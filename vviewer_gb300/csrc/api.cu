@@ -129,12 +129,16 @@ Queues carve_queues(char *base, size_t n)
 
 namespace {
 
-// `front`: bytes left free before the uploaded array (what the device built)
+// `front`: bytes before the uploaded array (what the device built); a buffer
+// that is there already is large enough for both
 template <class T>
 vvpt_status upload(vvpt_ctx *ctx, DevBuf &buf, const std::vector<T> &v, uint64_t &bytes, size_t front = 0)
 {
     size_t n = v.size() * sizeof(T);
-    VV_CUDA(buf.alloc(front + n), "cudaMalloc scene buffer");
+    if (!buf.ptr)
+        VV_CUDA(buf.alloc(front + n), "cudaMalloc scene buffer");
+    if (buf.bytes < front + n)
+        return fail(ctx, VVPT_ERR_DEVICE, "scene buffer smaller than planned");
     if (n)
         VV_CUDA(cudaMemcpyAsync(buf.as<char>() + front, v.data(), n, cudaMemcpyHostToDevice, vv_stream(ctx)),
                 "upload scene buffer");
@@ -296,8 +300,30 @@ VVPT_API vvpt_status vvpt_scene_upload(vvpt_ctx *ctx, const vvpt_scene_desc *des
     outside.tree = [bs](const std::vector<Box3> &boxes, const BVHBuildOptions &opt, BVHBuildResult &res,
                         std::string &e) { return build_bvh2_gpu(boxes, opt, bs, res, e); };
     outside.build = [&](const std::vector<uint32_t> &meshes, std::vector<MeshPlace> &places, std::string &e) {
-        if (!build_meshes_gpu(desc, meshes, BVHBuildOptions(), bs, dm, e))
+        // what the host adds to the scene's arrays: the other meshes, and at most
+        // the small meshes' triangles once more per instance (scene_pack.cpp)
+        std::vector<uint8_t> here(desc->num_meshes, 1);
+        for (uint32_t m : meshes)
+            here[m] = 0;
+        for (uint32_t m = 0; m < desc->num_meshes; m++)
+            if (here[m]) {
+                dm.host_index_tris += desc->meshes[m].num_triangles;
+                dm.host_verts += desc->meshes[m].num_vertices;
+            }
+        dm.host_tris = dm.host_index_tris;
+        for (uint32_t i = 0; i < desc->num_instances; i++) {
+            const vvpt_instance &in = desc->instances[i];
+            if ((in.flags & VVPT_INSTANCE_IN_TLAS) && desc->meshes[in.mesh_index].num_triangles <= kFlattenMaxTriangles)
+                dm.host_tris += desc->meshes[in.mesh_index].num_triangles;
+        }
+        if (!build_meshes_gpu(desc, meshes, BVHBuildOptions(), bs, dm, e)) {
+            // no room for the arrays or the working memory: the host builder, whose
+            // scene needs neither
+            dm.release();
+            if (dm.no_room && ctx->bvh_builder == VVPT_BVH_BUILDER_AUTO)
+                e.clear();
             return false;
+        }
         for (const DeviceMeshes::Placed &p : dm.placed) {
             MeshPlace mp{p.node_offset, p.tri_offset, p.vertex_offset, 3u * p.tri_offset, {}, {}};
             std::copy(p.root.lo, p.root.lo + 3, mp.lo);
@@ -322,6 +348,9 @@ VVPT_API vvpt_status vvpt_scene_upload(vvpt_ctx *ctx, const vvpt_scene_desc *des
 
     // ---- upload
     uint64_t bytes = 0;
+    scene->tris.swap(dm.tris);
+    scene->verts.swap(dm.verts);
+    scene->indices.swap(dm.indices);
     if ((st = upload(ctx, scene->nodes, pk.nodes, bytes, dm.num_nodes * sizeof(BVHNode))) != VVPT_OK)
         return st;
     if ((st = upload(ctx, scene->wnodes, pk.wnodes, bytes)) != VVPT_OK)
@@ -357,9 +386,6 @@ VVPT_API vvpt_status vvpt_scene_upload(vvpt_ctx *ctx, const vvpt_scene_desc *des
             VV_CUDA(copy(to, *nb, nb->bytes), "place nodes");
             to += nb->bytes;
         }
-        VV_CUDA(copy(scene->tris.ptr, dm.tris, dm.num_tris * sizeof(TriVerts)), "place triangles");
-        VV_CUDA(copy(scene->verts.ptr, dm.verts, dm.num_verts * sizeof(ShadeVertex)), "place vertices");
-        VV_CUDA(copy(scene->indices.ptr, dm.indices, dm.num_tris * 12ull), "place indices");
     }
     VV_CUDA(cudaStreamSynchronize(vv_stream(ctx)), "scene upload");
 

@@ -736,7 +736,7 @@ struct Forest {
         return off;
     }
 
-    bool begin(const std::vector<int> &counts, cudaStream_t s, std::string &err)
+    cudaError_t alloc(const std::vector<int> &counts)
     {
         n = 0;
         meshes = (int)counts.size();
@@ -746,9 +746,14 @@ struct Forest {
             n += c;
         }
         cap = n / (kSmall + 1) + 1; // a task has more than kSmall primitives
-        if (!ck(err, mem.alloc(carve(nullptr)), "alloc"))
-            return false;
-        carve(mem.as<char>());
+        const cudaError_t e = mem.alloc(carve(nullptr));
+        if (e == cudaSuccess)
+            carve(mem.as<char>());
+        return e;
+    }
+
+    bool begin(cudaStream_t s, std::string &err)
+    {
         const int start[kCounters] = {meshes, 0, 0, 0};
         if (!ck(err, cudaMemcpyAsync(ranges, ranges_h.data(), sizeof(int2) * meshes, cudaMemcpyHostToDevice, s),
                 "upload") ||
@@ -827,7 +832,7 @@ bool build_bvh2_gpu(const std::vector<Box3> &boxes, const BVHBuildOptions &opt, 
     static_assert(sizeof(GBox) == sizeof(Box3), "box layout");
     Forest f;
     DevBuf given;
-    if (!f.begin({n}, s, err) || !ck(err, given.alloc(sizeof(GBox) * n), "alloc") ||
+    if (!ck(err, f.alloc({n}), "alloc") || !f.begin(s, err) || !ck(err, given.alloc(sizeof(GBox) * n), "alloc") ||
         !ck(err, cudaMemcpyAsync(given.ptr, boxes.data(), sizeof(GBox) * n, cudaMemcpyHostToDevice, s), "upload"))
         return false;
     f.add(0, nullptr, nullptr, given.as<GBox>(), s);
@@ -843,13 +848,17 @@ bool build_bvh2_gpu(const std::vector<Box3> &boxes, const BVHBuildOptions &opt, 
            ck(err, cudaStreamSynchronize(s), "sync");
 }
 
-// The device part of a scene. Meshes are taken in groups of at most
-// kGroupTriangles triangles (or one mesh), which bounds the working memory to
-// a few gigabytes however large the scene is.
+// The device part of a scene, in the scene's own arrays. Meshes are taken in
+// groups of at most VVPT_GROUP_TRIANGLES triangles (or one mesh): the working
+// memory, about 320 bytes a triangle beside the group's vertices as they were
+// given, is a group's and not the scene's. Only the nodes, whose number a build
+// finds out, are there twice at the end.
+#ifndef VVPT_GROUP_TRIANGLES
+#define VVPT_GROUP_TRIANGLES (16u << 20)
+#endif
 bool build_meshes_gpu(const vvpt_scene_desc *desc, const std::vector<uint32_t> &meshes, const BVHBuildOptions &opt,
                       cudaStream_t s, DeviceMeshes &out, std::string &err)
 {
-    constexpr uint64_t kGroupTriangles = 16u << 20;
     out.placed.assign(meshes.size(), DeviceMeshes::Placed{});
     uint64_t nt = 0, nv = 0;
     for (size_t k = 0; k < meshes.size(); k++) {
@@ -861,9 +870,13 @@ bool build_meshes_gpu(const vvpt_scene_desc *desc, const std::vector<uint32_t> &
     }
     out.num_tris = (uint32_t)nt;
     out.num_verts = (uint32_t)nv;
-    if (!ck(err, out.tris.alloc(sizeof(TriVerts) * nt), "alloc") ||
-        !ck(err, out.verts.alloc(sizeof(ShadeVertex) * nv), "alloc") ||
-        !ck(err, out.indices.alloc(12ull * nt), "alloc"))
+    auto room = [&](cudaError_t e) {
+        out.no_room |= e == cudaErrorMemoryAllocation;
+        return ck(err, e, "alloc");
+    };
+    if (!room(out.tris.alloc(sizeof(TriVerts) * (nt + out.host_tris))) ||
+        !room(out.verts.alloc(sizeof(ShadeVertex) * (nv + out.host_verts))) ||
+        !room(out.indices.alloc(12ull * (nt + out.host_index_tris))))
         return false;
     for (size_t first = 0; first < meshes.size();) {
         size_t end = first;
@@ -871,7 +884,7 @@ bool build_meshes_gpu(const vvpt_scene_desc *desc, const std::vector<uint32_t> &
         uint64_t tris = 0, verts = 0;
         while (end < meshes.size()) {
             const vvpt_mesh_desc &md = desc->meshes[meshes[end]];
-            if (end > first && tris + md.num_triangles > kGroupTriangles)
+            if (end > first && tris + md.num_triangles > VVPT_GROUP_TRIANGLES)
                 break;
             tris += md.num_triangles;
             verts += md.num_vertices;
@@ -880,7 +893,7 @@ bool build_meshes_gpu(const vvpt_scene_desc *desc, const std::vector<uint32_t> &
         }
         Forest f;
         DevBuf raw;
-        if (!f.begin(counts, s, err) || !ck(err, raw.alloc(sizeof(vvpt_vertex) * verts), "alloc"))
+        if (!room(f.alloc(counts)) || !room(raw.alloc(sizeof(vvpt_vertex) * verts)) || !f.begin(s, err))
             return false;
         vvpt_vertex *rv = raw.as<vvpt_vertex>();
         const uint32_t t0 = out.placed[first].tri_offset, v0 = out.placed[first].vertex_offset;
@@ -907,7 +920,7 @@ bool build_meshes_gpu(const vvpt_scene_desc *desc, const std::vector<uint32_t> &
         out.nodes.emplace_back(new DevBuf());
         DevBuf &nb = *out.nodes.back();
         std::vector<int> bounds((size_t)kBoundInts * f.meshes);
-        if (!ck(err, nb.alloc(sizeof(BVHNode) * (size_t)nnodes), "alloc") ||
+        if (!room(nb.alloc(sizeof(BVHNode) * (size_t)nnodes)) ||
             !ck(err, cudaMemcpyAsync(nb.ptr, f.nodes, sizeof(BVHNode) * (size_t)nnodes, cudaMemcpyDeviceToDevice, s),
                 "copy") ||
             !ck(err, cudaMemcpyAsync(bounds.data(), f.bounds, 4 * bounds.size(), cudaMemcpyDeviceToHost, s), "download") ||

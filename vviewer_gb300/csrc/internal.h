@@ -53,6 +53,11 @@ struct DevBuf {
             ptr = nullptr;
         return e;
     }
+    void swap(DevBuf &o)
+    {
+        std::swap(ptr, o.ptr);
+        std::swap(bytes, o.bytes);
+    }
     // grow-only reuse
     cudaError_t reserve(size_t n)
     {
@@ -105,9 +110,21 @@ struct DeviceMeshes {
     };
     std::vector<Placed> placed;                 // per mesh, in the order given
     std::vector<std::unique_ptr<DevBuf>> nodes; // in order, num_nodes in all
+    // the scene's arrays themselves: behind the device's part there is room for
+    // `host_tris`, `host_verts` and `host_index_tris` more elements
     DevBuf tris, verts, indices;
+    uint64_t host_tris = 0, host_verts = 0, host_index_tris = 0;
     uint32_t num_nodes = 0, num_tris = 0, num_verts = 0;
     int depth = 0;
+    bool no_room = false; // an allocation failed for lack of memory
+
+    void release()
+    {
+        nodes.clear();
+        for (DevBuf *b : {&tris, &verts, &indices})
+            b->release();
+        num_nodes = num_tris = num_verts = 0;
+    }
 };
 bool build_meshes_gpu(const vvpt_scene_desc *desc, const std::vector<uint32_t> &meshes, const BVHBuildOptions &opt,
                       cudaStream_t stream, DeviceMeshes &out, std::string &err);

@@ -243,7 +243,6 @@ vvpt_status pack_scene(const vvpt_scene_desc *desc, PackedScene &out, std::strin
         order[i] = i;
     std::sort(order.begin(), order.end(),
               [&](uint32_t a, uint32_t b) { return desc->meshes[a].num_triangles > desc->meshes[b].num_triangles; });
-    std::atomic<uint32_t> next{0};
     const BVHBuildOptions blas_opt;
     std::vector<uint32_t> away; // meshes built outside
     std::vector<MeshPlace> places;
@@ -271,14 +270,12 @@ vvpt_status pack_scene(const vvpt_scene_desc *desc, PackedScene &out, std::strin
         return built;
     };
 #endif
-    auto worker = [&]() {
+    auto build_here = [&](const std::vector<uint32_t> &todo, std::atomic<uint32_t> &next) {
         for (;;) {
             uint32_t k = next.fetch_add(1);
-            if (k >= nm)
+            if (k >= todo.size())
                 break;
-            uint32_t m = order[k];
-            if (is_away[m])
-                continue;
+            uint32_t m = todo[k];
             const vvpt_mesh_desc &md = desc->meshes[m];
             std::vector<Box3> boxes(md.num_triangles);
             for (uint32_t t = 0; t < md.num_triangles; t++) {
@@ -319,18 +316,34 @@ vvpt_status pack_scene(const vvpt_scene_desc *desc, PackedScene &out, std::strin
         }
     };
     {
-        std::vector<std::thread> th;
-        unsigned nth = std::min<unsigned>(hw, std::max<uint32_t>(nm - (uint32_t)away.size(), 1));
-        for (unsigned i = 0; i < nth; i++)
-            th.emplace_back(worker);
+        // the meshes of one list on the host threads, beside what `meanwhile` does
+        auto on_threads = [&](const std::vector<uint32_t> &todo, auto meanwhile) {
+            std::atomic<uint32_t> next{0};
+            std::vector<std::thread> th;
+            const unsigned nth = std::min<unsigned>(hw, std::max<uint32_t>((uint32_t)todo.size(), 1));
+            for (unsigned i = 0; i < nth; i++)
+                th.emplace_back([&] { build_here(todo, next); });
+            meanwhile();
+            for (auto &t : th)
+                t.join();
+        };
+        std::vector<uint32_t> here, left;
+        for (uint32_t m : order)
+            (is_away[m] ? left : here).push_back(m);
         bool ok = true;
         std::string e;
-        if (!away.empty())
-            ok = outside->build(away, places, e);
-        for (auto &t : th)
-            t.join();
-        if (!ok)
+        on_threads(here, [&] {
+            if (!away.empty())
+                ok = outside->build(away, places, e);
+        });
+        if (!ok && !e.empty())
             return fail(err, VVPT_ERR_DEVICE, e);
+        if (!ok) {
+            on_threads(left, [] {});
+            away.clear();
+            places.clear();
+            std::fill(is_away.begin(), is_away.end(), 0);
+        }
     }
 #if VVPT_BLAS_WIDE
     if (!outside_err.empty())

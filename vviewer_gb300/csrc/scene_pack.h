@@ -66,7 +66,8 @@ struct OutsideMeshes {
     uint32_t min_triangles = 512;
     bool other_trees = false;       // the baked small instances' BLAS and the TLAS go to `tree` too
     BlasBuilder tree;
-    // builds the given meshes; false with err set on failure
+    // Builds the given meshes. False with err set on failure, or without when it
+    // leaves them all to the host (no room on the device).
     std::function<bool(const std::vector<uint32_t> &meshes, std::vector<MeshPlace> &places, std::string &err)> build;
     uint32_t nodes = 0, tris = 0, verts = 0; // set by build: elements in front of the packed arrays
     int depth = 0;
