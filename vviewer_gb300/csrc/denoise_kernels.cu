@@ -10,6 +10,7 @@
 #include <cudaTypedefs.h>
 
 #include "denoise_kernels.cuh"
+#include "per_device.h"
 
 namespace vvdn {
 
@@ -1847,6 +1848,44 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
     return fn;
 }
 
+// The current device and what plans and launches need to know of it.
+struct DeviceProps {
+    int sms = 0, sm_smem = 0, optin = 0, reserved = 0;
+};
+int current_device()
+{
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return dev;
+}
+const DeviceProps &device_props()
+{
+    static vvpt::PerDevice<DeviceProps> props;
+    const int dev = current_device();
+    return props.get(dev, [dev] {
+        DeviceProps p;
+        cudaDeviceGetAttribute(&p.sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaDeviceGetAttribute(&p.sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+        cudaDeviceGetAttribute(&p.optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        cudaDeviceGetAttribute(&p.reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
+        return p;
+    });
+}
+
+// Lets a kernel have up to `most` bytes of dynamic shared memory on the current
+// device, once and for every launch of it there.
+template <auto kernel>
+void allow_smem(int most, bool carveout = false)
+{
+    static vvpt::PerDevice<bool> done;
+    done.get(current_device(), [&] {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (carveout)
+            cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        return true;
+    });
+}
+
 // Launch that may start while the previous one runs (see pdl_wait).
 template <class... P, class... A>
 void launch_pdl(void (*kernel)(P...), dim3 grid, int threads, int smem, cudaStream_t s, A... args)
@@ -1870,10 +1909,12 @@ void launch_pdl(void (*kernel)(P...), dim3 grid, int threads, int smem, cudaStre
 int split_channels(int N, long ctas)
 {
     for (int nt = 16; nt < N; nt += 16)
-        if (N % nt == 0 && ctas * (N / nt) <= 152)
+        if (N % nt == 0 && ctas * (N / nt) <= device_props().sms)
             return nt;
     return N;
 }
+
+constexpr int kStStatic = 2048; // the strip kernel's mbarriers, TMEM address, flags (1 KB aligned)
 
 struct StripPlan {
     int ntile = 0; // output channels per CTA
@@ -1891,15 +1932,8 @@ bool plan_strip(const ConvArgs &a, StripPlan &pl)
         return false;
     if (a.cc && (a.cc % 16 || a.cc >= a.cin || a.h % 2 || a.wd % 2 || (reinterpret_cast<uintptr_t>(a.coarse) & 15)))
         return false;
-    static int nsm = 0, sm_smem = 0, optin = 0, reserved = 0;
-    if (!nsm) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-        cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
-    }
+    const DeviceProps &dp = device_props();
+    const int nsm = dp.sms;
     if (!tensor_map_encoder())
         return false;
     const int N = (a.cout + 15) & ~15;
@@ -1908,9 +1942,8 @@ bool plan_strip(const ConvArgs &a, StripPlan &pl)
     int ncols = 32;
     while (ncols < 2 * N)
         ncols <<= 1;
-    constexpr int kStatic = 2048; // mbarriers, TMEM address, flags (1 KB aligned)
     auto ring_of = [&](int c) {
-        const int dyn = std::min(optin - kStatic, sm_smem / c - reserved - kStatic);
+        const int dyn = std::min(dp.optin - kStStatic, dp.sm_smem / c - dp.reserved - kStStatic);
         return std::min(kStMaxRing, (dyn - 1024 - 9 * share * a.cin * 2) / slot);
     };
     // accumulators per row (independent MMA chains, whose sums the drain adds):
@@ -2011,13 +2044,7 @@ template <int nacc, bool pool>
 void launch_strip_as(const ConvArgs &a, const CUtensorMap &tmap, const StripPlan &pl, int withhold, cudaStream_t s,
                        uint32_t *err)
 {
-    static int attr_smem = 0;
-    if (pl.smem > attr_smem) {
-        cudaFuncSetAttribute(k_conv3x3_strip<nacc, pool>, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem);
-        cudaFuncSetAttribute(k_conv3x3_strip<nacc, pool>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared);
-        attr_smem = pl.smem;
-    }
+    allow_smem<k_conv3x3_strip<nacc, pool>>(device_props().optin - kStStatic, true);
     launch_pdl(k_conv3x3_strip<nacc, pool>, dim3((unsigned)pl.grid, (unsigned)(((a.cout + 15) & ~15) / pl.ntile)),
                kStThreads + 128 * (pl.dsets - 1) + (a.cc ? 32 * kStUpWarps : 0), pl.smem, s, a, tmap, pl.ncols, pl.ring,
                pl.segs, pl.seg_rows, pl.ntile, pl.dsets, err, withhold);
@@ -2065,14 +2092,10 @@ bool conv3x3(const ConvArgs &a_in, cudaStream_t s, uint32_t *err, ConvKernels ki
         return a.pool != nullptr;
     a.pool = nullptr;
     if (err && a.cout <= 256) {
-        static bool attr_set = false;
-        if (!attr_set) {
-            cudaFuncSetAttribute(k_conv3x3_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_smem_bytes(256));
-            cudaFuncSetAttribute(k_conv3x3_tc_chunk, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 std::max(tc_chunk_smem_bytes(128, 2, tc_chunk_rows(128)),
-                                          tc_chunk_smem_bytes(64, 2, tc_chunk_rows(64))));
-            attr_set = true;
-        }
+        allow_smem<k_conv3x3_tc>(tc_smem_bytes(256));
+        allow_smem<k_conv3x3_tc_chunk>(std::max(tc_chunk_smem_bytes(128, 2, tc_chunk_rows(128)),
+                                                tc_chunk_smem_bytes(64, 2, tc_chunk_rows(64))));
+        const int sms = device_props().sms;
         const int N = (a.cout + 15) & ~15;
         int ncols = 32;
         while (ncols < N)
@@ -2086,7 +2109,7 @@ bool conv3x3(const ConvArgs &a_in, cudaStream_t s, uint32_t *err, ConvKernels ki
             // a small image leaves SMs idle: fewer rows per CTA while the
             // CTAs still run at once, one per SM (224 to 96 channels at 32 x 32:
             // 28 us on 32 CTAs, 19 us on 96)
-            while (rows > 1 && 2 * columns * ((a.h + rows - 1) / rows) <= 152)
+            while (rows > 1 && 2 * columns * ((a.h + rows - 1) / rows) <= sms)
                 rows /= 2;
             const long blocks = columns * ((a.h + rows - 1) / rows);
             // ... and then fewer output channels per CTA, which share the
@@ -2127,17 +2150,12 @@ void conv3x3_wgrad(const bf16 *dout, int cout, const bf16 *in, int cin, int n, i
         while (ncols < ntile)
             ncols <<= 1;
         const int tiles = ((cout + kWtM - 1) / kWtM) * ((cin + ntile - 1) / ntile);
-        long slices = std::max<long>(1, (152L * 4) / (9L * tiles));
+        long slices = std::max<long>(1, (device_props().sms * 4L) / (9L * tiles));
         long slice = (P + slices - 1) / slices;
         slice = std::max<long>(kWtK, (slice + kWtK - 1) / kWtK * kWtK);
         slices = (P + slice - 1) / slice;
         const int smem = kWtStages * wt_stage_bytes(ntile);
-        static bool attr_set = false;
-        if (!attr_set) {
-            cudaFuncSetAttribute(k_conv3x3_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kWtStages * wt_stage_bytes(128));
-            attr_set = true;
-        }
+        allow_smem<k_conv3x3_wgrad_tc>(kWtStages * wt_stage_bytes(128));
         dim3 grid((unsigned)slices, (unsigned)(9 * tiles));
         k_conv3x3_wgrad_tc<<<grid, 128, smem, s>>>(dout, cout, in, cin, n, h, w, dw, slice, ntile, ncols, err);
     } else {
@@ -2155,15 +2173,11 @@ template <int BN>
 static void launch_wgrad(const bf16 *dout, int cout, const bf16 *in, int cin, int n, int h, int w, float *dw,
                          float *dbias, cudaStream_t s, long copy_stride)
 {
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaFuncSetAttribute(k_conv3x3_wgrad<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, wg_smem<BN>());
-        attr_set = true;
-    }
+    allow_smem<k_conv3x3_wgrad<BN>>(wg_smem<BN>());
     // three (BN = 32) or two blocks fit an SM: about one unit per block over
     // all channel tiles
     const int tiles = ((cout + kWgM - 1) / kWgM) * ((cin + BN - 1) / BN);
-    const long cols = (long)n * ((w + kWgPx - 1) / kWgPx), blocks = std::max<long>(1, 152L * (BN == 32 ? 3 : 2) / tiles);
+    const long cols = (long)n * ((w + kWgPx - 1) / kWgPx), blocks = std::max<long>(1, (long)device_props().sms * (BN == 32 ? 3 : 2) / tiles);
     int segs = (int)std::max<long>(1, std::min<long>(h, blocks / cols));
     const int seg_rows = (h + segs - 1) / segs;
     segs = (h + seg_rows - 1) / seg_rows;
