@@ -10,7 +10,7 @@ extern "C" __attribute__((visibility("default"))) int device_wgrad(const void *d
 {
     const vvdn::bf16 *d = static_cast<const vvdn::bf16 *>(dout), *x = static_cast<const vvdn::bf16 *>(in);
     vvdn::wgrad_mma_sync(d, cout, x, cin, n, h, w, g, g + 9 * cin * cout, nullptr, stride);
-    vvdn::sum_grads(g, stride, nullptr);
+    vvdn::sum_grads(g, stride, g, 9 * cin * cout + cout, nullptr);
     const cudaError_t launch = cudaGetLastError(), sync = cudaDeviceSynchronize();
     return (int)(launch != cudaSuccess ? launch : sync);
 }

@@ -96,7 +96,8 @@ struct vvpt_denoiser {
     vvpt_ctx *ctx = nullptr;
     std::vector<Layer> layers;
     size_t nparams = 0, nw16 = 0;
-    DevBuf params, grads, adam_m, adam_v, w16, wt16;
+    DevBuf params, adam_m, adam_v, w16, wt16;
+    DevBuf grads; // the copies' sum, on its way to the host
     int step = 0;
     // shape-dependent buffers
     int n = 0, h = 0, w = 0;
@@ -108,8 +109,12 @@ struct vvpt_denoiser {
     // gskip[l]: gradient of e_l through the decoder's concat (gradient pool only)
     Tensor x[kLevels], a[kLevels], e[kLevels], u[kLevels - 1], b[kLevels - 1], d[kLevels - 1], gskip[kLevels - 1];
     bool weights_dirty = true;
-    // floats between the gradients' copies (even: pairs are added at once)
+    // the parameters' gradients, vvdn::kGradCopies copies behind the activations'
+    // in gacts, grad_stride() floats apart (even: pairs are added at once)
+    size_t copies_off = 0;
     size_t grad_stride() const { return (nparams + 1) & ~size_t(1); }
+    size_t copies_bytes() const { return vvdn::kGradCopies * grad_stride() * sizeof(float); }
+    float *grad_copies() const { return reinterpret_cast<float *>(gacts.as<char>() + copies_off); }
 };
 
 namespace {
@@ -149,7 +154,8 @@ vvpt_status ensure_shape(vvpt_denoiser *dn, int n, int h, int w, bool with_grads
     VV_CUDA(dn->acts.reserve(off * sizeof(bf16)), "cudaMalloc denoiser activations");
     VV_CUDA(dn->out_f32.reserve(p0 * kOutCh * sizeof(float)), "cudaMalloc denoiser output");
     if (dn->with_grads) {
-        VV_CUDA(dn->gacts.reserve(off * sizeof(bf16)), "cudaMalloc denoiser gradients");
+        dn->copies_off = aligned256(off * sizeof(bf16));
+        VV_CUDA(dn->gacts.reserve(dn->copies_off + dn->copies_bytes()), "cudaMalloc denoiser gradients");
         VV_CUDA(dn->dout.reserve(p0 * kOutCh * sizeof(bf16)), "cudaMalloc denoiser output gradient");
         VV_CUDA(dn->loss.reserve(sizeof(float)), "cudaMalloc loss");
     }
@@ -250,7 +256,7 @@ void conv_wgrad(vvpt_denoiser *dn, int li, const bf16 *dout, const bf16 *in, int
 {
     const Layer &L = dn->layers[li];
     vvdn::conv3x3_wgrad(dout, L.cout, in, L.cin, dn->n, dn->h >> level, dn->w >> level,
-                        dn->grads.as<float>() + L.w_off, dn->grads.as<float>() + L.b_off, s,
+                        dn->grad_copies() + L.w_off, dn->grad_copies() + L.b_off, s,
                         dn->conv_kind == vvdn::kConvWgradTc ? dn->err.as<uint32_t>() : nullptr,
                         (long)dn->grad_stride());
 }
@@ -342,7 +348,7 @@ vvpt_status check_shape(vvpt_ctx *ctx, uint32_t n, uint32_t w, uint32_t h)
     return VVPT_OK;
 }
 
-// forward + loss + backward into the copies of dn->grads; loss returned on the host
+// forward + loss + backward into the gradients' copies; loss returned on the host
 vvpt_status loss_and_grads(vvpt_denoiser *dn, const vvpt_denoise_batch *bt, float *loss_out)
 {
     vvpt_ctx *ctx = dn->ctx;
@@ -358,7 +364,7 @@ vvpt_status loss_and_grads(vvpt_denoiser *dn, const vvpt_denoise_batch *bt, floa
     forward(dn, bt->radiance, bt->albedo, bt->normal, s);
     VV_CUDA(cudaMemsetAsync(dn->loss.ptr, 0, sizeof(float), s), "clear loss");
     vvdn::l1_loss(dn->out_f32.as<float>(), kOutCh, bt->target, dn->dout.as<bf16>(), dn->loss.as<float>(), p0, s);
-    VV_CUDA(cudaMemsetAsync(dn->grads.ptr, 0, dn->grads.bytes, s), "clear gradients");
+    VV_CUDA(cudaMemsetAsync(dn->grad_copies(), 0, dn->copies_bytes(), s), "clear gradients");
     backward(dn, s);
     VV_CUDA(cudaGetLastError(), "denoiser kernels");
     float l = 0.0f;
@@ -398,7 +404,7 @@ VVPT_API vvpt_status vvpt_denoiser_create(vvpt_ctx *ctx, uint64_t seed, vvpt_den
                 p[L.w_off + (size_t)co * 9 * L.cin + k] = (float)(std_ * rng.normal());
     }
     VV_CUDA(dn->params.alloc(dn->nparams * sizeof(float)), "cudaMalloc denoiser parameters");
-    VV_CUDA(dn->grads.alloc(vvdn::kGradCopies * dn->grad_stride() * sizeof(float)), "cudaMalloc denoiser gradients");
+    VV_CUDA(dn->grads.alloc(dn->nparams * sizeof(float)), "cudaMalloc denoiser gradients");
     VV_CUDA(dn->adam_m.alloc(dn->nparams * sizeof(float)), "cudaMalloc denoiser optimiser");
     VV_CUDA(dn->adam_v.alloc(dn->nparams * sizeof(float)), "cudaMalloc denoiser optimiser");
     VV_CUDA(dn->w16.alloc(dn->nw16 * sizeof(bf16)), "cudaMalloc denoiser weights");
@@ -466,7 +472,7 @@ VVPT_API vvpt_status vvpt_denoiser_gradients(vvpt_denoiser *dn, const vvpt_denoi
     if (st != VVPT_OK)
         return st;
     cudaStream_t s = vv_stream(ctx);
-    vvdn::sum_grads(dn->grads.as<float>(), dn->grad_stride(), s);
+    vvdn::sum_grads(dn->grad_copies(), dn->grad_stride(), dn->grads.as<float>(), dn->nparams, s);
     VV_CUDA(cudaGetLastError(), "sum gradients");
     VV_CUDA(cudaMemcpyAsync(grads_host, dn->grads.ptr, n * sizeof(float), cudaMemcpyDeviceToHost, s), "read gradients");
     VV_CUDA(cudaStreamSynchronize(s), "read gradients");
@@ -486,7 +492,7 @@ VVPT_API vvpt_status vvpt_denoiser_train_step(vvpt_denoiser *dn, const vvpt_deno
         return st;
     cudaStream_t s = vv_stream(ctx);
     dn->step++;
-    vvdn::adam(dn->params.as<float>(), dn->grads.as<float>(), dn->grad_stride(), dn->adam_m.as<float>(),
+    vvdn::adam(dn->params.as<float>(), dn->grad_copies(), dn->grad_stride(), dn->adam_m.as<float>(),
                dn->adam_v.as<float>(), dn->nparams, lr, 0.9f, 0.999f, 1e-8f, dn->step, s);
     dn->weights_dirty = true;
     VV_CUDA(cudaGetLastError(), "adam");

@@ -668,10 +668,10 @@ __device__ __forceinline__ float sum_copies(const float *g, size_t stride)
     static_assert(kGradCopies == 4, "summed by halves");
     return (g[0] + g[stride]) + (g[2 * stride] + g[3 * stride]);
 }
-__global__ void k_sum_grads(float *g, size_t stride)
+__global__ void k_sum_grads(const float *g, size_t stride, float *sum, size_t n)
 {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < stride; i += (size_t)gridDim.x * blockDim.x)
-        g[i] = sum_copies(g + i, stride);
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+        sum[i] = sum_copies(g + i, stride);
 }
 
 __global__ void k_adam(float *p, const float *g, size_t stride, float *m, float *v, size_t n, float lr, float b1,
@@ -2245,9 +2245,9 @@ void l1_loss(const float *out, int cout, const float *target, bf16 *dout, float 
                                                                 dout, loss_sum, npix);
 }
 
-void sum_grads(float *g, size_t stride, cudaStream_t s)
+void sum_grads(const float *g, size_t stride, float *sum, size_t n, cudaStream_t s)
 {
-    k_sum_grads<<<grid_for((long)stride), 256, 0, s>>>(g, stride);
+    k_sum_grads<<<grid_for((long)n), 256, 0, s>>>(g, stride, sum, n);
 }
 
 void adam(float *p, const float *g, size_t stride, float *m, float *v, size_t n, float lr, float b1, float b2, float eps, int t,

@@ -78,8 +78,8 @@ void conv3x3_wgrad(const bf16 *dout, int cout, const bf16 *in, int cin, int n, i
 // the mma.sync weight and bias gradient
 void wgrad_mma_sync(const bf16 *dout, int cout, const bf16 *in, int cin, int n, int h, int w, float *dw, float *dbias,
                     cudaStream_t s, long copy_stride = 0);
-// the first of kGradCopies arrays of `stride` floats becomes their sum
-void sum_grads(float *g, size_t stride, cudaStream_t s);
+// sum = the sum of kGradCopies arrays of n floats, `stride` floats apart
+void sum_grads(const float *g, size_t stride, float *sum, size_t n, cudaStream_t s);
 
 // The layers' weights: first element in the bf16 copies (start[layers]: their
 // end) and in the f32 parameters.
