@@ -126,6 +126,14 @@ vvpt_status ensure_shape(vvpt_denoiser *dn, int n, int h, int w, bool with_grads
     vvpt_ctx *ctx = dn->ctx;
     if (dn->n == n && dn->h == h && dn->w == w && (dn->with_grads || !with_grads))
         return VVPT_OK;
+    // until every buffer is there the denoiser has no shape, and is not held to
+    // gradients that it never had room for
+    const bool had_grads = dn->with_grads;
+    auto incomplete = [&](const char *what, cudaError_t e) {
+        dn->n = dn->h = dn->w = 0;
+        dn->with_grads = had_grads;
+        return cuda_fail(ctx, e, what);
+    };
     dn->n = n;
     dn->h = h;
     dn->w = w;
@@ -151,13 +159,19 @@ vvpt_status ensure_shape(vvpt_denoiser *dn, int n, int h, int w, bool with_grads
         place(dn->gskip[l], l, kCh[l]);
     }
     const size_t p0 = level_pixels(dn, 0);
-    VV_CUDA(dn->acts.reserve(off * sizeof(bf16)), "cudaMalloc denoiser activations");
-    VV_CUDA(dn->out_f32.reserve(p0 * kOutCh * sizeof(float)), "cudaMalloc denoiser output");
+    cudaError_t e;
+    if ((e = dn->acts.reserve(off * sizeof(bf16))) != cudaSuccess)
+        return incomplete("cudaMalloc denoiser activations", e);
+    if ((e = dn->out_f32.reserve(p0 * kOutCh * sizeof(float))) != cudaSuccess)
+        return incomplete("cudaMalloc denoiser output", e);
     if (dn->with_grads) {
         dn->copies_off = aligned256(off * sizeof(bf16));
-        VV_CUDA(dn->gacts.reserve(dn->copies_off + dn->copies_bytes()), "cudaMalloc denoiser gradients");
-        VV_CUDA(dn->dout.reserve(p0 * kOutCh * sizeof(bf16)), "cudaMalloc denoiser output gradient");
-        VV_CUDA(dn->loss.reserve(sizeof(float)), "cudaMalloc loss");
+        if ((e = dn->gacts.reserve(dn->copies_off + dn->copies_bytes())) != cudaSuccess)
+            return incomplete("cudaMalloc denoiser gradients", e);
+        if ((e = dn->dout.reserve(p0 * kOutCh * sizeof(bf16))) != cudaSuccess)
+            return incomplete("cudaMalloc denoiser output gradient", e);
+        if ((e = dn->loss.reserve(sizeof(float))) != cudaSuccess)
+            return incomplete("cudaMalloc loss", e);
     }
     return VVPT_OK;
 }
