@@ -17,6 +17,16 @@ static bool same(const std::vector<T> &a, const std::vector<T> &b)
     return a.size() == b.size() && (a.empty() || std::memcmp(a.data(), b.data(), a.size() * sizeof(T)) == 0);
 }
 
+extern "C" int host_pack_status(const vvpt_scene_desc *desc, char *msg, int msg_len)
+{
+    PackedScene packed;
+    std::string err;
+    const vvpt_status st = pack_scene(desc, packed, err, 2);
+    std::strncpy(msg, err.c_str(), msg_len - 1);
+    msg[msg_len - 1] = 0;
+    return (int)st;
+}
+
 // 0: the packed scenes are the same; else the status with `msg`, or -1 where
 // they differ. `failure`: what the outside builder reports ("" declines).
 extern "C" int host_pack_outside(const vvpt_scene_desc *desc, const char *failure, int *asked, char *msg, int msg_len)

@@ -9,6 +9,7 @@ from pathlib import Path
 import pytest
 
 from raygen import HIT_SCENES
+from vviewer_gb300 import _native as N
 
 ROOT = Path(__file__).resolve().parent.parent
 CSRC = ROOT / "vviewer_gb300" / "csrc"
@@ -28,6 +29,7 @@ def host_lib():
                     f"{cuda}/include", "-I", str(ROOT / "include"), "-I", str(CSRC), *map(str, srcs), "-o", str(OUT)],
                    check=True, capture_output=True)
     lib = C.CDLL(str(OUT))
+    lib.host_pack_status.argtypes = [C.c_void_p, C.c_char_p, C.c_int]
     lib.host_pack_outside.argtypes = [C.c_void_p, C.c_char_p, C.POINTER(C.c_int), C.c_char_p, C.c_int]
     return lib
 
@@ -45,3 +47,18 @@ def test_declined_meshes_are_built_on_the_host(host_lib, name):
     if large:
         assert pack(host_lib, flat, b"broken") == (5, large, b"broken")  # VVPT_ERR_DEVICE
     assert name != "displaced_spheres" or large > 0
+
+
+def test_scenes_beyond_the_reference_bits_are_refused(host_lib):
+    """Counts that an index of 30 bits (or 32-bit offsets) cannot name: refused
+    before anything is read (the arrays here hold one element)."""
+    for meshes, tris, verts in ((1, 1 << 30, 3), (2, (1 << 30) - 1, 3), (3, 1, 1 << 31)):
+        vertex, corner = N.Vertex(), (C.c_uint32 * 3)()
+        md = (N.MeshDesc * meshes)()
+        for m in md:
+            m.vertices, m.num_vertices = C.addressof(vertex), verts
+            m.indices, m.num_triangles = C.addressof(corner), tris
+        desc = N.SceneDesc()
+        desc.meshes, desc.num_meshes = md, meshes
+        msg = C.create_string_buffer(256)
+        assert host_lib.host_pack_status(C.addressof(desc), msg, 256) == 8, msg.value  # VVPT_ERR_UNSUPPORTED

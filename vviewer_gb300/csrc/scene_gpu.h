@@ -12,6 +12,10 @@ namespace vvpt {
 // scene builder rejects BVHs whose worst-case depth would not fit.
 constexpr int kTraversalStack = 128;
 
+// A traversal reference (traverse.cuh) holds an index in 30 bits: nodes and
+// triangles of one BLAS, instances.
+constexpr uint32_t kMaxRefIndex = (1u << 30) - 1u;
+
 // Binary BVH node, 64 bytes: both children's boxes plus child links, so one
 // node visit is four 128-bit loads. lxy = (l.lo.x, l.lo.y, l.hi.x, l.hi.y),
 // rxy likewise, lrz = (l.lo.z, l.hi.z, r.lo.z, r.hi.z): each half of a word is

@@ -173,6 +173,18 @@ vvpt_status pack_scene(const vvpt_scene_desc *desc, PackedScene &out, std::strin
         (desc->num_materials && !desc->materials) || (desc->num_lights && !desc->lights) ||
         (desc->num_light_data && !desc->light_data) || (desc->num_textures && !desc->textures))
         return fail(err, VVPT_ERR_INVALID_ARG, "array pointer is null while its count is not zero");
+    // larger ones would run into the bits of a reference that name its kind
+    uint64_t triangles = 0, vertices = 0;
+    for (uint32_t m = 0; m < desc->num_meshes; m++) {
+        if (desc->meshes[m].num_triangles > kMaxRefIndex)
+            return fail(err, VVPT_ERR_UNSUPPORTED, "mesh " + std::to_string(m) + ": 2^30 triangles or more");
+        triangles += desc->meshes[m].num_triangles;
+        vertices += desc->meshes[m].num_vertices;
+    }
+    if (desc->num_instances > kMaxRefIndex)
+        return fail(err, VVPT_ERR_UNSUPPORTED, "2^30 instances or more");
+    if (3 * triangles > 0xFFFFFFFFull || vertices > 0xFFFFFFFFull)
+        return fail(err, VVPT_ERR_UNSUPPORTED, "2^32 vertices or triangle corners or more");
     for (uint32_t m = 0; m < desc->num_meshes; m++) {
         const vvpt_mesh_desc &md = desc->meshes[m];
         if ((md.num_vertices && !md.vertices) || (md.num_triangles && !md.indices))
@@ -614,6 +626,8 @@ vvpt_status pack_scene(const vvpt_scene_desc *desc, PackedScene &out, std::strin
                 fb.push_back(b);
             }
         }
+        if (ft.size() > kMaxRefIndex)
+            return fail(err, VVPT_ERR_UNSUPPORTED, "2^30 triangles or more in small instances");
         BVHBuildResult fbvh;
         if (!build_other(fb, BVHBuildOptions(), fbvh))
             return VVPT_ERR_DEVICE;

@@ -441,7 +441,7 @@ __device__ __forceinline__ BVHNode load_node_cached(int idx)
 // marks the last), an instance run of a TLAS leaf (index into tlas_order, whose
 // top bit marks the last), the return from an instance; kRefDone ends the ray.
 constexpr uint32_t kRefLeaf = 1u << 30, kRefInst = 2u << 30, kRefReturn = 3u << 30, kRefDone = 0xFFFFFFFFu;
-constexpr uint32_t kRefIndex = (1u << 30) - 1u;
+constexpr uint32_t kRefIndex = kMaxRefIndex;
 #if VVPT_BLAS_WIDE
 constexpr uint32_t kRefWide = 1u << 30; // wide children still to visit (its BLAS has no leaf references)
 #endif
