@@ -203,7 +203,7 @@ public:
         auto box_or_empty = [](const Link &k, float *lo, float *hi) {
             for (int a = 0; a < 3; a++) {
                 lo[a] = k.box.valid() ? k.box.lo[a] : 1.0f;
-                hi[a] = k.box.valid() ? k.box.hi[a] : -1.0f; // empty box never hit
+                hi[a] = k.box.valid() ? k.box.hi[a] : -1.0f; // visited like any box: nothing in it can be hit
             }
         };
         float llo[3], lhi[3], rlo[3], rhi[3];

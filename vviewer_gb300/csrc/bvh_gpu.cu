@@ -25,8 +25,8 @@
 // Bound by atomics and latency at the top levels (few tasks, all primitives in
 // one) and by launches below. Building eight meshes of 124,820 triangles one
 // after the other, a thread per split, took 60 ms; together, with the boxes
-// and the packing on the device, the whole scene uploads in 7.5 ms instead
-// of 97 (k_bin 1.7 ms in all, k_small 1.1).
+// and the packing on the device, the whole scene uploads in 7.4 ms instead
+// of 107 (k_bin 1.7 ms in all, k_small 1.1).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -850,7 +850,7 @@ bool build_bvh2_gpu(const std::vector<Box3> &boxes, const BVHBuildOptions &opt, 
 
 // The device part of a scene, in the scene's own arrays. Meshes are taken in
 // groups of at most VVPT_GROUP_TRIANGLES triangles (or one mesh): the working
-// memory, about 320 bytes a triangle beside the group's vertices as they were
+// memory, about 310 bytes a triangle beside the group's vertices as they were
 // given, is a group's and not the scene's. Only the nodes, whose number a build
 // finds out, are there twice at the end.
 #ifndef VVPT_GROUP_TRIANGLES

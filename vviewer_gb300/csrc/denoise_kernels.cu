@@ -235,13 +235,12 @@ __device__ __forceinline__ void unpack8(const uint4 &v, float (&f)[8])
 // end the errors of n additions shrink from sqrt(n) to sqrt(n) / copies.
 // Bound by shared-memory reads and MMA issue of the nine warps. Against one
 // launch per layer that staged both tensors again for every tap (and a launch
-// for the bias): 32 x 32 channels over 8 x 256 x 256 pixels 45 us, 157 + 10
-// before; 80 x 32 channels 136 us, 314 + 10 before. With the bias in FP32 and
-// the copies a training step over 8 x 256 x 256 pixels went from 1715 to 1651 us
-// and the weights' error against 64-bit sums of the same inputs, all layers,
-// from 1.94e-6 to 1.93e-6 there, from 2.1e-7 to 0.8e-7 at 8 x 64 x 64 (before the
-// taps were taken together: 4.6e-6 and 1.9e-7); the bias's from 2 to 4 times the
-// separate pass's at 8 x 64 x 64 to 0.6 times.
+// for the bias): 32 x 32 channels over 8 x 256 x 256 pixels 42 us, 157 + 10
+// before; 80 x 32 channels 113 us, 314 + 10 before. (47 and 137 us with the bias
+// as an MMA by ones and one copy of the gradients.) The weights' error against 64-bit sums of the same inputs, all layers,
+// is 1.93e-6 there and 0.8e-7 at 8 x 64 x 64 (before the taps were taken together
+// 4.6e-6 and 1.9e-7; with one copy 1.94e-6 and 2.1e-7), the bias's 0.2 to 0.6
+// times that of the separate pass.
 constexpr int kWgPx = 64, kWgM = 32, kWgThreads = 288, kWgRing = 5, kWgDRing = 3, kWgDRow = kWgM + 8;
 template <int BN>
 constexpr int wg_smem()
@@ -1919,7 +1918,7 @@ constexpr int kStStatic = 2048; // the strip kernel's mbarriers, TMEM address, f
 struct StripPlan {
     int ntile = 0; // output channels per CTA
     int dsets = 1; // drain sets of four warps
-    int ring = 0, smem = 0, grid = 0, segs = 0, seg_rows = 0, ncols = 0, nacc = 1, per_sm = 1;
+    int ring = 0, smem = 0, grid = 0, segs = 0, seg_rows = 0, ncols = 0, nacc = 1;
 };
 
 // Occupancy first (up to 4 CTAs per SM, bounded by shared memory and by the
@@ -2011,7 +2010,6 @@ bool plan_strip(const ConvArgs &a, StripPlan &pl)
     pl.seg_rows = seg_rows;
     pl.ncols = tcols;
     pl.nacc = nacc;
-    pl.per_sm = c;
     // A second set of drain warps where the registers of the CTAs of an SM
     // leave room for it and there are channels to share (64 channels at
     // 960 x 540: 72 to 52 us; 48 at 1920 x 1080: 114 to 95). A fused

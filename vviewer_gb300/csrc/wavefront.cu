@@ -778,8 +778,6 @@ __device__ __forceinline__ bool trace_turn(TraceState &st, const TraceCold &ray,
     return tracing && st.cur == kRefDone;
 }
 
-__device__ __forceinline__ float3 medium_transmittance(const SceneView &s, uint32_t vol, float vtstart, float vtend);
-
 // A shadow ray whose nearest candidate is known: opaque, the light is hidden;
 // none, the light is seen through the medium at the event (the miss shader of
 // raySecondary.rmiss.glsl:17-44); transparent, the candidates have to be
