@@ -90,8 +90,8 @@ vvpt_status make_render_params(vvpt_ctx *ctx, const vvpt_scene *scene, const vvp
 namespace {
 Pools<DeviceMem> &pools()
 {
-    static Pools<DeviceMem> p;
-    return p;
+    static Pools<DeviceMem> *p = new Pools<DeviceMem>(); // contexts may go after the process's statics
+    return *p;
 }
 }  // namespace
 
@@ -523,10 +523,16 @@ VVPT_API vvpt_status vvpt_render(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_sc
         const uint32_t slots = ctx->pool.acquire(hp.total_items, ctx->tuning.slots, ctx->budget_bytes.load());
         if (!slots)
             return cuda_fail(ctx, cudaErrorMemoryAllocation, "cudaMalloc path state");
-        struct PoolGuard {
-            SlotPool<DeviceMem> &pool;
-            ~PoolGuard() { pool.done(); }
-        } pool_guard{ctx->pool};
+        struct PoolGuard { // a render that returns early leaves kernels behind that use the pool
+            vvpt_ctx *ctx;
+            bool finished;
+            ~PoolGuard()
+            {
+                if (!finished)
+                    cudaStreamSynchronize(vv_stream(ctx));
+                ctx->pool.done();
+            }
+        } pool_guard{ctx, false};
         const size_t n = slots;
         auto aligned = [](size_t b) { return aligned256(b); };
         char *base = nullptr;
@@ -747,6 +753,7 @@ VVPT_API vvpt_status vvpt_render(vvpt_ctx *ctx, vvpt_scene *scene, const vvpt_sc
         float ms = 0.0f;
         cudaEventElapsedTime(&ms, tev[0], tev[1]);
         stats.device_ms = ms;
+        pool_guard.finished = true;
     }
 
     if (!out->on_device) {
